@@ -72,9 +72,14 @@ typedef struct ss2d_scan_params {
     void *checkpoints;                  /* optional, fp32 (batch, dim, ceil(seqlen / 128), dstate) contiguous: the state
                                            in front of every 128th element, for ss2d_selective_scan_bwd (the reference
                                            hands its backward the chunk states `x` the same way, selective_scan_oflex.cpp:208) */
+    int64_t checkpoint_every;           /* spacing of the checkpoints; 0 = 128.  A multiple of ss2d_selective_scan_checkpoint_every() */
+    void *workspace;                    /* optional, 16-byte aligned: with ss2d_selective_scan_fwd_workspace_bytes() bytes, rows too */
+    int64_t workspace_bytes;            /* few to fill the GPU are cut into segments that are walked side by side */
 } ss2d_scan_params;
 
 int ss2d_selective_scan_fwd(const ss2d_scan_params *p, void *cuda_stream);
+int64_t ss2d_selective_scan_fwd_workspace_bytes(const ss2d_scan_params *p);       /* < 0: invalid arguments; 0: none is used */
+int64_t ss2d_selective_scan_checkpoint_every(int64_t dstate, int64_t delta_ratio);   /* the spacing that the backward call reads */
 
 /* ------------------------------------------------------------------------------------
  * Selective-scan backward.  Replaces selective_scan_cuda_oflex.bwd

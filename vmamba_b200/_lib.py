@@ -27,7 +27,7 @@ class ScanParams(ctypes.Structure):
                                     "out_batch_stride", "out_dim_stride",
                                     "B_batch_stride", "B_group_stride", "B_state_stride",
                                     "C_batch_stride", "C_group_stride", "C_state_stride")] + \
-               [("checkpoints", _vp)]
+               [("checkpoints", _vp), ("checkpoint_every", _i64), ("workspace", _vp), ("workspace_bytes", _i64)]
 
 
 class ScanBwdParams(ctypes.Structure):
@@ -112,6 +112,8 @@ class LinearParams(ctypes.Structure):
 EXPORTS = {
     # name: (restype, argtypes)
     "ss2d_selective_scan_fwd": (ctypes.c_int, [ctypes.POINTER(ScanParams), _vp]),
+    "ss2d_selective_scan_fwd_workspace_bytes": (_i64, [ctypes.POINTER(ScanParams)]),
+    "ss2d_selective_scan_checkpoint_every": (_i64, [_i64, _i64]),
     "ss2d_selective_scan_bwd": (ctypes.c_int, [ctypes.POINTER(ScanBwdParams), _vp]),
     "ss2d_selective_scan_bwd_workspace_bytes": (_i64, [ctypes.POINTER(ScanBwdParams)]),
     "ss2d_cross_scan": (ctypes.c_int, [ctypes.POINTER(CrossParams), _vp]),

@@ -9,6 +9,8 @@
 
 namespace ss2d {
 int selective_scan_fwd(const ss2d_scan_params* p, cudaStream_t st);
+long long selective_scan_fwd_workspace_bytes(const ss2d_scan_params* p);
+long long selective_scan_checkpoint_every(int64_t dstate, int64_t delta_ratio);
 int selective_scan_bwd(const ss2d_scan_bwd_params* p, cudaStream_t st);
 long long selective_scan_bwd_workspace_bytes(const ss2d_scan_bwd_params* p);
 int cross_scan(const ss2d_cross_params* p, cudaStream_t st);
@@ -72,8 +74,12 @@ int ss2d_set_debug_checks(int on) { return ss2d::g_debug_checks.exchange(on ? 1 
 
 int ss2d_selective_scan_fwd(const ss2d_scan_params* p, void* stream) {
     ss2d::Range nvtx_("ss2d_selective_scan_fwd");
-    if (p) SS2D_CHECK_PTRS(p->u, p->delta, p->A, p->B, p->C, p->D, p->delta_bias, p->out, p->checkpoints);
+    if (p) SS2D_CHECK_PTRS(p->u, p->delta, p->A, p->B, p->C, p->D, p->delta_bias, p->out, p->checkpoints, p->workspace);
     return ss2d::selective_scan_fwd(p, (cudaStream_t)stream);
+}
+int64_t ss2d_selective_scan_fwd_workspace_bytes(const ss2d_scan_params* p) { return ss2d::selective_scan_fwd_workspace_bytes(p); }
+int64_t ss2d_selective_scan_checkpoint_every(int64_t dstate, int64_t delta_ratio) {
+    return ss2d::selective_scan_checkpoint_every(dstate, delta_ratio);
 }
 int ss2d_selective_scan_bwd(const ss2d_scan_bwd_params* p, void* stream) {
     ss2d::Range nvtx_("ss2d_selective_scan_bwd");

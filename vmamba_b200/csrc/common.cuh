@@ -198,6 +198,46 @@ __device__ __forceinline__ AB warp_scan_inclusive_rev(AB v, int lane) {
     return v;
 }
 
+// One step of an inclusive (a, b) scan across the lanes: the shuffle's own "source lane in range" predicate guards the
+// combine, so a step is two shuffles and two predicated arithmetic instructions (no lane test, no select).
+// WIDTH: lanes per segment (aligned groups of lanes that are scanned on their own).
+template <int OFF, int WIDTH = 32> __device__ __forceinline__ void scan_step_up(float& a, float& b) {
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .f32 pa, pb;\n"
+        " shfl.sync.up.b32 pa|p, %0, %2, %3, 0xffffffff;\n"
+        " shfl.sync.up.b32 pb, %1, %2, %3, 0xffffffff;\n"
+        " @p fma.rn.f32 %1, %0, pb, %1;\n"
+        " @p mul.f32 %0, %0, pa;\n}"
+        : "+f"(a), "+f"(b) : "n"(OFF), "n"((32 - WIDTH) << 8));
+}
+template <int OFF> __device__ __forceinline__ void scan_step_down(float& a, float& b) {
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .f32 pa, pb;\n"
+        " shfl.sync.down.b32 pa|p, %0, %2, 31, 0xffffffff;\n"
+        " shfl.sync.down.b32 pb, %1, %2, 31, 0xffffffff;\n"
+        " @p fma.rn.f32 %1, %0, pb, %1;\n"
+        " @p mul.f32 %0, %0, pa;\n}"
+        : "+f"(a), "+f"(b) : "n"(OFF));
+}
+// Inclusive state of the neighbouring lane (the lane before, or after when walking backwards); on the first lane of
+// the walk, which has no neighbour, the state carried over from the previous chunk.
+template <bool kBack, int WIDTH = 32> __device__ __forceinline__ float entering_state(float inc_b, float carry) {
+    float r;
+    if constexpr (kBack)
+        asm volatile(
+            "{\n .reg .pred p;\n"
+            " shfl.sync.down.b32 %0|p, %1, 1, 31, 0xffffffff;\n"
+            " @!p mov.f32 %0, %2;\n}"
+            : "=&f"(r) : "f"(inc_b), "f"(carry));
+    else
+        asm volatile(
+            "{\n .reg .pred p;\n"
+            " shfl.sync.up.b32 %0|p, %1, 1, %3, 0xffffffff;\n"
+            " @!p mov.f32 %0, %2;\n}"
+            : "=&f"(r) : "f"(inc_b), "f"(carry), "n"((32 - WIDTH) << 8));
+    return r;
+}
+
 // ---- warp-level tensor-core step: D (16 x 8, fp32) += A (16 x 16, row-major) . B (16 x 8, column-major) -------
 template <typename T> struct MmaK16;
 template <> struct MmaK16<__nv_bfloat16> {

@@ -48,45 +48,6 @@ __device__ __forceinline__ void pair_barrier(bool col) {
     else asm volatile("bar.sync 1, 64;" ::: "memory");
 }
 
-// One step of an inclusive (a, b) scan across the lanes: the shuffle's own "source lane in range" predicate guards the
-// combine, so a step is two shuffles and two predicated arithmetic instructions (no lane test, no select).
-template <int OFF> __device__ __forceinline__ void scan_step_up(float& a, float& b) {
-    asm volatile(
-        "{\n .reg .pred p;\n .reg .f32 pa, pb;\n"
-        " shfl.sync.up.b32 pa|p, %0, %2, 0, 0xffffffff;\n"
-        " shfl.sync.up.b32 pb, %1, %2, 0, 0xffffffff;\n"
-        " @p fma.rn.f32 %1, %0, pb, %1;\n"
-        " @p mul.f32 %0, %0, pa;\n}"
-        : "+f"(a), "+f"(b) : "n"(OFF));
-}
-template <int OFF> __device__ __forceinline__ void scan_step_down(float& a, float& b) {
-    asm volatile(
-        "{\n .reg .pred p;\n .reg .f32 pa, pb;\n"
-        " shfl.sync.down.b32 pa|p, %0, %2, 31, 0xffffffff;\n"
-        " shfl.sync.down.b32 pb, %1, %2, 31, 0xffffffff;\n"
-        " @p fma.rn.f32 %1, %0, pb, %1;\n"
-        " @p mul.f32 %0, %0, pa;\n}"
-        : "+f"(a), "+f"(b) : "n"(OFF));
-}
-// Inclusive state of the neighbouring lane (the lane before, or after when walking backwards); on the first lane of
-// the walk, which has no neighbour, the state carried over from the previous chunk.
-template <bool kBack> __device__ __forceinline__ float entering_state(float inc_b, float carry) {
-    float r;
-    if constexpr (kBack)
-        asm volatile(
-            "{\n .reg .pred p;\n"
-            " shfl.sync.down.b32 %0|p, %1, 1, 31, 0xffffffff;\n"
-            " @!p mov.f32 %0, %2;\n}"
-            : "=&f"(r) : "f"(inc_b), "f"(carry));
-    else
-        asm volatile(
-            "{\n .reg .pred p;\n"
-            " shfl.sync.up.b32 %0|p, %1, 1, 0, 0xffffffff;\n"
-            " @!p mov.f32 %0, %2;\n}"
-            : "=&f"(r) : "f"(inc_b), "f"(carry));
-    return r;
-}
-
 // One route of one plane (k: route; kBack: routes 2, 3).  `xsrc` is the plane's x in the orientation order of the route
 // (global memory for the row-major routes, the shared column-major copy for the others: a generic address); `acc`
 // the fp32 plane of the orientation, in orientation order.  kRoll chooses where the loads of the next chunk are issued:

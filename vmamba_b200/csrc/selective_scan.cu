@@ -7,7 +7,8 @@
 // a register (d_state 1) or in shared memory (d_state > 1).  The next step's vectors are
 // fetched before the current step's arithmetic.  Traffic per row: u and delta read once, out
 // written once; B/C rows are shared by all channels of a group and come from L2.
-#include "common.cuh"
+#include "scan_row.cuh"
+#include "scan_states_fwd.cuh"
 
 namespace ss2d {
 
@@ -22,77 +23,157 @@ struct ScanArgs {
     int64_t dratio;   // channels per delta row
     float* ckpt;      // (rows, nck, dstate) or null
     int64_t nck;
+    int every;        // elements between the states kept in ckpt
+    bool states_only; // no result, the states alone
 };
 
 constexpr int kWarpsPerCta = 4;
 
-template <typename Tin, typename Tout, int VEC>
-__global__ void __launch_bounds__(kWarpsPerCta * 32) selscan_fwd_n1_kernel(const ScanArgs a) {
-    const int lane = threadIdx.x & 31;
-    const int64_t row = (int64_t)blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
-    if (row >= a.rows) return;
-    const int64_t b = row / a.dim, r = row % a.dim, k = r / a.group_size;
+// d_state 1: W warps per row (1: four rows per CTA; 2 .. 8: the CTA is one row).  Per step a warp takes 256 elements, eight
+// per lane, and scans its lanes' (a, b) pairs by shuffle; with several warps per row their totals meet in shared memory
+// (one barrier per step) and every warp folds the ones in front of it.  One warp per row is the faster form where the rows
+// fill the chip; fewer rows get the more warps (try: rows * W up to 20 warps per SM).
+// AL is the vector width of every access (8 or 4 elements), or 0 for rows of any alignment: a row is then walked from
+// the 16-byte boundary in front of its result, so that the results leave as vectors, and the inputs are cut out of the
+// aligned pieces around them.
+// `every` (a multiple of 8): spacing of the states kept for the backward pass.
+// Rows of at most 128 (64) elements share a warp, two (four) at a time, LPR = 16 (8) lanes each.
+template <typename Tin, typename Tout, int AL, int W, int LPR>
+__global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32) selscan_fwd_n1_kernel(const ScanArgs a) {
+    static_assert(W == 1 || LPR == 32, "rows of several warps take whole warps");
+    constexpr int VEC = 8, WSTEP = LPR * VEC, STEP = W * WSTEP, NL = AL ? VEC / AL : 1;
+    constexpr int AW = AL ? AL : 1;
+    __shared__ AB agg[2][W];
+    const int lane = threadIdx.x & (LPR - 1), wi = W == 1 ? 0 : threadIdx.x >> 5;
+    int64_t row = W == 1 ? ((int64_t)blockIdx.x * (kWarpsPerCta * 32) + threadIdx.x) / LPR : (int64_t)blockIdx.x;
+    if (row - (threadIdx.x & 31) / LPR >= a.rows) return;      // whole warps (whole CTAs where W > 1)
+    const bool real = LPR == 32 || row < a.rows;               // the last warp's spare lanes repeat its last row, unseen
+    if (!real) row = a.rows - 1;
+    const int64_t b = row / a.dim, r = row - b * a.dim, k = r / a.group_size;
+    const int64_t rd_ = a.dratio == 1 ? r : r / a.dratio;
     const Tin* __restrict__ u = (const Tin*)a.u + b * a.u_bs + r * a.u_ds;
-    const Tin* __restrict__ dt = (const Tin*)a.delta + b * a.d_bs + (r / a.dratio) * a.d_ds;
+    const Tin* __restrict__ dt = (const Tin*)a.delta + b * a.d_bs + rd_ * a.d_ds;
     const Tin* __restrict__ Bm = (const Tin*)a.B + b * a.B_bs + k * a.B_gs;
     const Tin* __restrict__ Cm = (const Tin*)a.C + b * a.C_bs + k * a.C_gs;
     Tout* __restrict__ out = (Tout*)a.out + b * a.o_bs + r * a.o_ds;
     const float A2 = __ldg(a.A + r) * kLog2e;
-    const bool has_D = a.D != nullptr;
-    const float Dv = has_D ? __ldg(a.D + r) : 0.f;
-    const float bias = a.bias ? __ldg(a.bias + r / a.dratio) : 0.f;
+    const float Dv = a.D ? __ldg(a.D + r) : 0.f;
+    const float bias = a.bias ? __ldg(a.bias + rd_) : 0.f;
     const bool sp = a.softplus != 0;
     const int L = (int)a.seqlen;
-    constexpr int STEP = 32 * VEC;
-    using VI = Vec<Tin, VEC>;
-    using VO = Vec<Tout, VEC>;
+    constexpr int OV = 16 / (int)sizeof(Tout);       // elements per 16-byte store
+    const int ph = AL ? 0 : (int)((reinterpret_cast<uintptr_t>(out) / sizeof(Tout)) & (OV - 1));
+    constexpr int ph_max = AL ? 0 : OV - 1;
+    using VI = Vec<Tin, AW>;
+    using Raw = typename VI::Raw;
 
-    typename VI::Raw ru = {}, rd = {}, rb = {}, rc = {};
-    int pos = lane * VEC;
-    if (pos < L) {   // L % VEC == 0: a lane's vector lies wholly inside or outside the row
-        ru = VI::load_raw(u + pos); rd = VI::load_raw(dt + pos);
-        rb = VI::load_raw(Bm + pos); rc = VI::load_raw(Cm + pos);
-    }
-    float hc = 0.f;   // state entering this step
-    for (int base = 0; base < L; base += STEP) {
-        typename VI::Raw nu = {}, nd = {}, nb = {}, nc = {};
-        const int npos = pos + STEP;
-        if (npos < L) {
-            nu = VI::load_raw(u + npos); nd = VI::load_raw(dt + npos);
-            nb = VI::load_raw(Bm + npos); nc = VI::load_raw(Cm + npos);
+    Raw ru[NL], rd[NL], rb[NL], rc[NL];
+    auto fetch = [&](int at) {
+        if constexpr (AL != 0) {
+#pragma unroll
+            for (int j = 0; j < NL; ++j) {
+                const int p = min(at + j * AL, L - AL);          // vectors beyond the row re-read its end and are ignored
+                ru[j] = VI::load_raw(u + p); rd[j] = VI::load_raw(dt + p);
+                rb[j] = VI::load_raw(Bm + p); rc[j] = VI::load_raw(Cm + p);
+            }
         }
+    };
+    int pos = wi * WSTEP + lane * VEC - ph;
+    fetch(pos);
+    float hc = 0.f;                                  // state entering this step
+    // rows that share a warp may start at different phases: they take the same number of steps
+    for (int base = LPR < 32 ? -ph_max : -ph, it = 0; base < L; base += STEP, ++it) {
         float uv[VEC], dv[VEC], bv[VEC], cv[VEC], P[VEC], hl[VEC];
-        VI::unpack(ru, uv); VI::unpack(rd, dv); VI::unpack(rb, bv); VI::unpack(rc, cv);
+        if constexpr (AL != 0) {
+#pragma unroll
+            for (int j = 0; j < NL; ++j) {
+                float x[AW];
+                VI::unpack(ru[j], x);
+#pragma unroll
+                for (int e = 0; e < AW; ++e) uv[j * AW + e] = x[e];
+                VI::unpack(rd[j], x);
+#pragma unroll
+                for (int e = 0; e < AW; ++e) dv[j * AW + e] = x[e];
+                VI::unpack(rb[j], x);
+#pragma unroll
+                for (int e = 0; e < AW; ++e) bv[j * AW + e] = x[e];
+                VI::unpack(rc[j], x);
+#pragma unroll
+                for (int e = 0; e < AW; ++e) cv[j * AW + e] = x[e];
+            }
+            fetch(pos + STEP);
+        } else {
+            load8_any<Tin>(u, pos, L, uv); load8_any<Tin>(dt, pos, L, dv);
+            load8_any<Tin>(Bm, pos, L, bv); load8_any<Tin>(Cm, pos, L, cv);
+        }
         float p = 1.f, h = 0.f;
 #pragma unroll
         for (int i = 0; i < VEC; ++i) {
             float dl = dv[i] + bias;
             if (sp) dl = softplus_fast(dl);
+            // outside the row: a step of zero leaves the state as it is (whole vectors are tested once below)
+            if constexpr (AL != 8) dl = (AL == 4 ? pos + (i & 4) : pos + i) < L && (AL || pos + i >= 0) ? dl : 0.f;
             const float aa = decay_fast(dl, A2);
             h = fmaf(aa, h, dl * bv[i] * uv[i]);
             p *= aa;
             P[i] = p; hl[i] = h;
         }
-        const AB inc = warp_scan_inclusive(AB{p, h}, lane);
-        float ea = __shfl_up_sync(0xffffffffu, inc.a, 1);
-        float eb = __shfl_up_sync(0xffffffffu, inc.b, 1);
-        if (lane == 0) { ea = 1.f; eb = 0.f; }
-        const float hin = fmaf(ea, hc, eb);
-        if (a.ckpt && (pos & 127) == 0 && pos < L) a.ckpt[row * a.nck + (pos >> 7)] = hin;     // state in front of element pos
-        const float ta = __shfl_sync(0xffffffffu, inc.a, 31);
-        const float tb = __shfl_sync(0xffffffffu, inc.b, 31);
-        hc = fmaf(ta, hc, tb);
-        if (pos < L) {
+        float ia = p, ib = h;
+        if constexpr (AL == 8) { const bool in = pos < L; ia = in ? p : 1.f; ib = in ? h : 0.f; }
+        float hin;
+        if constexpr (W == 1) {
+            if (lane == 0) ib = fmaf(ia, hc, ib);
+            scan_step_up<1, LPR>(ia, ib); scan_step_up<2, LPR>(ia, ib); scan_step_up<4, LPR>(ia, ib);
+            if constexpr (LPR > 8) scan_step_up<8, LPR>(ia, ib);
+            if constexpr (LPR > 16) scan_step_up<16, LPR>(ia, ib);
+            hin = entering_state<false, LPR>(ib, hc);
+            hc = __shfl_sync(0xffffffffu, ib, LPR - 1, LPR);
+        } else {
+            scan_step_up<1>(ia, ib); scan_step_up<2>(ia, ib); scan_step_up<4>(ia, ib); scan_step_up<8>(ia, ib); scan_step_up<16>(ia, ib);
+            if (lane == 31) agg[it & 1][wi] = AB{ia, ib};
+            float ea = __shfl_up_sync(0xffffffffu, ia, 1), eb = __shfl_up_sync(0xffffffffu, ib, 1);
+            if (lane == 0) { ea = 1.f; eb = 0.f; }
+            __syncthreads();        // the buffer of this step was last read two steps ago, in front of the barrier in between
+            float hw = hc;
+#pragma unroll
+            for (int j = 0; j < W; ++j) {
+                if (j == wi) hw = hc;
+                const AB g = agg[it & 1][j];
+                hc = fmaf(g.a, hc, g.b);
+            }
+            hin = fmaf(ea, hw, eb);
+        }
+        if (a.ckpt && real) {
+            if constexpr (AL != 0) {
+                if (pos < L && pos % a.every == 0) a.ckpt[row * a.nck + pos / a.every] = hin;
+            } else {
+#pragma unroll
+                for (int i = 0; i < VEC; ++i)
+                    if (pos + i >= 0 && pos + i < L && (pos + i) % a.every == 0)
+                        a.ckpt[row * a.nck + (pos + i) / a.every] = i == 0 ? hin : fmaf(P[i > 0 ? i - 1 : 0], hin, hl[i > 0 ? i - 1 : 0]);
+            }
+        }
+        if (!a.states_only && real) {
             float ov[VEC];
 #pragma unroll
-            for (int i = 0; i < VEC; ++i) {
-                const float y = cv[i] * fmaf(P[i], hin, hl[i]);
-                ov[i] = has_D ? fmaf(Dv, uv[i], y) : y;
+            for (int i = 0; i < VEC; ++i) ov[i] = fmaf(Dv, uv[i], cv[i] * fmaf(P[i], hin, hl[i]));
+            constexpr int SV = AL == 4 && OV > 4 ? 4 : OV;       // elements per store
+#pragma unroll
+            for (int j = 0; j < VEC; j += SV) {
+                const int q = pos + j;
+                if (AL != 0 ? q < L : (q >= 0 && q + SV <= L)) {
+                    float o[SV];
+#pragma unroll
+                    for (int e = 0; e < SV; ++e) o[e] = ov[j + e];
+                    Vec<Tout, SV>::store(out + q, o);
+                } else if (AL == 0) {
+#pragma unroll
+                    for (int e = 0; e < SV; ++e)
+                        if (q + e >= 0 && q + e < L) out[q + e] = from_f<Tout>(ov[j + e]);
+                }
             }
-            VO::store(out + pos, ov);
         }
-        ru = nu; rd = nd; rb = nb; rc = nc;
-        pos = npos;
+        pos += STEP;
     }
 }
 
@@ -163,7 +244,7 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) selscan_fwd_nx_kernel(const
             if (lane == 0) { ea = 1.f; eb = 0.f; }
             const float hc = carry_s[warp][n];
             const float hin = fmaf(ea, hc, eb);
-            if (a.ckpt && (pos & 127) == 0 && in) a.ckpt[(row * a.nck + (pos >> 7)) * N + n] = hin;
+            if (a.ckpt && pos % a.every == 0 && in) a.ckpt[(row * a.nck + pos / a.every) * N + n] = hin;
             __syncwarp();
             if (lane == 31) carry_s[warp][n] = fmaf(inc.a, hc, inc.b);
 #pragma unroll
@@ -174,227 +255,50 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) selscan_fwd_nx_kernel(const
     }
 }
 
-// d_state 4 / 8 / 16 with many rows: LANES ARE ROWS.  A warp owns 32 consecutive rows of one (image, group) and every
-// lane walks its own row element by element with all NS states in registers: the recurrence is a plain fused
-// multiply-add per (element, state) - no running products, no fix-up, no shuffle scan (the warp-per-row kernel above
-// spends 13.7 instructions per (element, state), 2.2 of them in the scans; this form needs 5: scale, ex2, B u, h, y) -
-// and the NS states of a lane are NS independent dependency chains.  The B / C values of an element are the same for
-// the 32 rows of the warp: they are staged once per tile as fp32 and read as broadcast 16-byte loads.  Tiles of 16
-// elements: u and delta (32 rows x 16 elements) and B / C (NS rows x 16 elements) are loaded as 16-byte pieces, unpacked
-// and stored transposed ([element][row], pitch 33: conflict-free both ways); the outputs leave through the same buffer
-// as 16-byte vectors.  Warps of a CTA never wait for each other.  The kernel is bound by the MUFU pipe (NS + 2
-// transcendentals per element and lane).
-constexpr int kRowsTile = 16;          // elements per tile: 6.8 KB of shared memory per warp at 16 states, six CTAs per SM
-constexpr int kRowsWarps = 4;
-template <int NS> struct RowsSmem {
-    static constexpr int kPitch = 33;
-    static constexpr int kBCPitch = NS >= 4 ? NS + 4 : NS;       // 16-byte aligned rows for the 16-byte reads of four states
-    static constexpr int kFloatsPerWarp = 2 * kRowsTile * kPitch + 2 * kRowsTile * kBCPitch;
-};
-
-template <typename Tin, typename Tout, int NS, int EPP>
-__global__ void __launch_bounds__(kRowsWarps * 32, 6) selscan_fwd_rows_kernel(const ScanArgs a) {
-    using S = RowsSmem<NS>;
-    // EPP: elements per piece moved by one load (16 bytes; 8 bytes for 16-bit rows whose length is a multiple of 4 only)
-    constexpr int PPR = kRowsTile / EPP;                         // pieces per row of a tile
-    constexpr int OPP = EPP < 16 / (int)sizeof(Tout) ? EPP : 16 / (int)sizeof(Tout), OPR = kRowsTile / OPP;
-    extern __shared__ __align__(16) float rows_sm[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float* su = rows_sm + (size_t)warp * S::kFloatsPerWarp;       // [t][row]; overwritten by the outputs
-    float* sd = su + kRowsTile * S::kPitch;
-    float* sB = sd + kRowsTile * S::kPitch;                      // [t][n]
-    float* sC = sB + kRowsTile * S::kBCPitch;
-    const int64_t row0 = ((int64_t)blockIdx.x * kRowsWarps + warp) * 32;
-    if (row0 >= a.rows) return;
-    const int64_t b = row0 / a.dim, r0 = row0 % a.dim, k = r0 / a.group_size;     // 32 rows: one image, one group
-    const int64_t r = r0 + lane;
-    const Tin* __restrict__ u = (const Tin*)a.u + b * a.u_bs + r0 * a.u_ds;
-    const Tin* __restrict__ dt = (const Tin*)a.delta + b * a.d_bs + r0 * a.d_ds;
-    const Tin* __restrict__ Bm = (const Tin*)a.B + b * a.B_bs + k * a.B_gs;
-    const Tin* __restrict__ Cm = (const Tin*)a.C + b * a.C_bs + k * a.C_gs;
-    Tout* __restrict__ out = (Tout*)a.out + b * a.o_bs + r0 * a.o_ds;
-    float A2[NS], h[NS];
-#pragma unroll
-    for (int n = 0; n < NS; ++n) { A2[n] = __ldg(a.A + r * NS + n) * kLog2e; h[n] = 0.f; }
-    const bool has_D = a.D != nullptr;
-    const float Dv = has_D ? __ldg(a.D + r) : 0.f;
-    const float bias = a.bias ? __ldg(a.bias + r) : 0.f;
-    const bool sp = a.softplus != 0;
-    const int L = (int)a.seqlen;
-    using VI = Vec<Tin, EPP>;
-    using VO = Vec<Tout, OPP>;
-
-    for (int t0 = 0; t0 < L; t0 += kRowsTile) {
-        // ---- stage the tile: 16-byte pieces in, fp32 transposed out (L is a multiple of the piece: a piece is inside or outside)
-#pragma unroll
-        for (int j = 0; j < PPR; ++j) {
-            const int idx = j * 32 + lane, rr = idx / PPR, piece = idx - rr * PPR;
-            const int pos = t0 + piece * EPP;
-            float uv[EPP], dv[EPP];
-            if (pos < L) {
-                VI::load(u + rr * a.u_ds + pos, uv);
-                VI::load(dt + rr * a.d_ds + pos, dv);
-            } else {
-#pragma unroll
-                for (int e = 0; e < EPP; ++e) { uv[e] = 0.f; dv[e] = 0.f; }
-            }
-#pragma unroll
-            for (int e = 0; e < EPP; ++e) {
-                su[(piece * EPP + e) * S::kPitch + rr] = uv[e];
-                sd[(piece * EPP + e) * S::kPitch + rr] = dv[e];
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < (NS * PPR + 31) / 32; ++j) {
-            const int idx = j * 32 + lane, n = idx / PPR, piece = idx - n * PPR;
-            const int pos = t0 + piece * EPP;
-            if (n < NS) {
-                float bv[EPP], cv[EPP];
-                if (pos < L) {
-                    VI::load(Bm + n * a.B_ss + pos, bv);
-                    VI::load(Cm + n * a.C_ss + pos, cv);
-                } else {
-#pragma unroll
-                    for (int e = 0; e < EPP; ++e) { bv[e] = 0.f; cv[e] = 0.f; }
-                }
-#pragma unroll
-                for (int e = 0; e < EPP; ++e) {
-                    sB[(piece * EPP + e) * S::kBCPitch + n] = bv[e];
-                    sC[(piece * EPP + e) * S::kBCPitch + n] = cv[e];
-                }
-            }
-        }
-        __syncwarp();
-        // ---- the recurrence: this lane's row, element by element
-        const int tn = min(kRowsTile, L - t0);
-#pragma unroll 2
-        for (int t = 0; t < tn; ++t) {
-            const float uv = su[t * S::kPitch + lane];
-            float d = sd[t * S::kPitch + lane] + bias;
-            if (sp) d = softplus_fast(d);
-            const float du = d * uv;
-            float y = has_D ? Dv * uv : 0.f, y1 = 0.f;           // two partial sums: half the dependent chain
-            if (a.ckpt && ((t0 + t) & 127) == 0) {               // the states in front of element t0 + t
-                float* ck = a.ckpt + ((row0 + lane) * a.nck + ((t0 + t) >> 7)) * NS;
-                if constexpr (NS >= 4) {
-#pragma unroll
-                    for (int n = 0; n < NS; n += 4) *reinterpret_cast<float4*>(ck + n) = make_float4(h[n], h[n + 1], h[n + 2], h[n + 3]);
-                } else {
-#pragma unroll
-                    for (int n = 0; n < NS; ++n) ck[n] = h[n];
-                }
-            }
-            if constexpr (NS >= 4) {
-#pragma unroll
-                for (int n4 = 0; n4 < NS; n4 += 4) {
-                    const float4 b4 = *reinterpret_cast<const float4*>(sB + t * S::kBCPitch + n4);
-                    const float4 c4 = *reinterpret_cast<const float4*>(sC + t * S::kBCPitch + n4);
-                    const float bb[4] = {b4.x, b4.y, b4.z, b4.w}, cc[4] = {c4.x, c4.y, c4.z, c4.w};
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int n = n4 + i;
-                        h[n] = fmaf(decay_fast(d, A2[n]), h[n], du * bb[i]);
-                        if (i & 1) y1 = fmaf(cc[i], h[n], y1);
-                        else y = fmaf(cc[i], h[n], y);
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int n = 0; n < NS; ++n) {
-                    h[n] = fmaf(decay_fast(d, A2[n]), h[n], du * sB[t * S::kBCPitch + n]);
-                    y = fmaf(sC[t * S::kBCPitch + n], h[n], y);
-                }
-            }
-            su[t * S::kPitch + lane] = y + y1;
-        }
-        __syncwarp();
-        // ---- outputs: 16-byte pieces along each row
-#pragma unroll
-        for (int j = 0; j < OPR; ++j) {
-            const int idx = j * 32 + lane, rr = idx / OPR, piece = idx - rr * OPR;
-            const int pos = t0 + piece * OPP;
-            if (pos < L) {
-                float ov[OPP];
-#pragma unroll
-                for (int e = 0; e < OPP; ++e) ov[e] = su[(piece * OPP + e) * S::kPitch + rr];
-                VO::store(out + rr * a.o_ds + pos, ov);
-            }
-        }
-        __syncwarp();
-    }
+// d_state 1: warps per row.  Rows that fill the chip (20 warps on each of 148 SMs) get one; fewer rows more, as long as a
+// step of all of them is not longer than the row.
+static int n1_warps(int64_t rows, int64_t L) {
+    int w = 1;
+    while (w < 8 && rows * w < 148 * 20 && (int64_t)w * 256 < L) w *= 2;
+    return w;
 }
 
-template <typename Tin, typename Tout, int NS, int EPP>
-static int launch_rows(const ScanArgs& a, cudaStream_t st) {
-    using S = RowsSmem<NS>;
-    const size_t smem = (size_t)kRowsWarps * S::kFloatsPerWarp * sizeof(float);
-    auto kern = selscan_fwd_rows_kernel<Tin, Tout, NS, EPP>;
-    static bool attr_ok[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!attr_ok[dev & 63]) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
-        attr_ok[dev & 63] = true;
-    }
-    const int64_t warps = a.rows / 32;
-    const int64_t ctas = (warps + kRowsWarps - 1) / kRowsWarps;
+template <typename Tin, typename Tout, int AL>
+static int launch_n1(const ScanArgs& a, cudaStream_t st) {
+    const int w = n1_warps(a.rows, a.seqlen), lpr = w > 1 ? 32 : a.seqlen <= 64 ? 8 : a.seqlen <= 128 ? 16 : 32;
+    const int64_t per_cta = kWarpsPerCta * (32 / lpr), ctas = w == 1 ? (a.rows + per_cta - 1) / per_cta : a.rows;
     if (ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
-    kern<<<(unsigned)ctas, kRowsWarps * 32, smem, st>>>(a);
+    const unsigned g = (unsigned)ctas;
+    if (w == 8) selscan_fwd_n1_kernel<Tin, Tout, AL, 8, 32><<<g, 256, 0, st>>>(a);
+    else if (w == 4) selscan_fwd_n1_kernel<Tin, Tout, AL, 4, 32><<<g, 128, 0, st>>>(a);
+    else if (w == 2) selscan_fwd_n1_kernel<Tin, Tout, AL, 2, 32><<<g, 64, 0, st>>>(a);
+    else if (lpr == 8) selscan_fwd_n1_kernel<Tin, Tout, AL, 1, 8><<<g, kWarpsPerCta * 32, 0, st>>>(a);
+    else if (lpr == 16) selscan_fwd_n1_kernel<Tin, Tout, AL, 1, 16><<<g, kWarpsPerCta * 32, 0, st>>>(a);
+    else selscan_fwd_n1_kernel<Tin, Tout, AL, 1, 32><<<g, kWarpsPerCta * 32, 0, st>>>(a);
     count_launch();
     return check_launch();
-}
-
-// The lanes-are-rows kernel takes a problem when its rows come in whole groups of 32 per (image, group), every tensor
-// allows pieces of at least 8 bytes, each row has its own delta row, and there are enough rows (below).
-template <typename Tin, typename Tout, int EPP>
-static int rows_by_state(const ScanArgs& a, cudaStream_t st) {
-    if (a.dstate == 16) return launch_rows<Tin, Tout, 16, EPP>(a, st);
-    if (a.dstate == 8) return launch_rows<Tin, Tout, 8, EPP>(a, st);
-    if (a.dstate == 4) return launch_rows<Tin, Tout, 4, EPP>(a, st);
-    return launch_rows<Tin, Tout, 1, EPP>(a, st);
-}
-template <typename Tin, typename Tout>
-static int try_rows(const ScanArgs& a, int vec, cudaStream_t st, bool& taken) {
-    taken = false;
-    // d_state 1: short rows only (bf16, fraction of the copy bandwidth, this kernel against the warp-per-row one: 0.42 / 0.35
-    // at L = 196, 0.42 / 0.54 at L = 784; the warp-per-row kernel reaches 0.8 from L = 3136 up)
-    if (a.dstate == 1 ? a.seqlen > 256 : (a.dstate != 4 && a.dstate != 8 && a.dstate != 16)) return SS2D_OK;
-    // enough rows to fill the GPU with warps of 32 rows.  Measured crossover against the warp-per-row kernels (d_state 16,
-    // bf16): 12 288 rows tie, 26 112 rows 0.105 against 0.067 of the copy bandwidth, 6 144 rows 0.027 against 0.058
-    const long long min_rows = 32LL * 148 * (a.dstate == 1 ? 8 : 3);
-    if (vec < 4 || a.dratio != 1 || a.group_size % 32 != 0 || a.rows < min_rows || !rows_kernels_enabled()) return SS2D_OK;
-    taken = true;
-    if constexpr (sizeof(Tin) == 2) {
-        if (vec >= 8) return rows_by_state<Tin, Tout, 8>(a, st);
-    }
-    return rows_by_state<Tin, Tout, 4>(a, st);
 }
 
 template <typename Tin, typename Tout, int VEC>
-static int launch_scan(const ScanArgs& a, cudaStream_t st) {
+static int launch_nx(const ScanArgs& a, cudaStream_t st) {
     const int64_t ctas = (a.rows + kWarpsPerCta - 1) / kWarpsPerCta;
     if (ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
-    if (a.dstate == 1)
-        selscan_fwd_n1_kernel<Tin, Tout, VEC><<<(unsigned)ctas, kWarpsPerCta * 32, 0, st>>>(a);
-    else
-        selscan_fwd_nx_kernel<Tin, Tout, VEC><<<(unsigned)ctas, kWarpsPerCta * 32, 0, st>>>(a);
+    selscan_fwd_nx_kernel<Tin, Tout, VEC><<<(unsigned)ctas, kWarpsPerCta * 32, 0, st>>>(a);
     count_launch();
     return check_launch();
 }
 
+// `vec`: widest vector, in elements and at most 8, that every row start of every tensor allows
 template <typename Tin, typename Tout>
 static int dispatch_vec(const ScanArgs& a, int vec, cudaStream_t st) {
-    {
-        bool taken;
-        const int rc = try_rows<Tin, Tout>(a, vec, st, taken);
-        if (taken) return rc;
-    }
+    if (a.dstate == 1)
+        return vec >= 8 ? launch_n1<Tin, Tout, 8>(a, st) : vec >= 4 ? launch_n1<Tin, Tout, 4>(a, st) : launch_n1<Tin, Tout, 0>(a, st);
     if constexpr (sizeof(Tin) == 2) {
-        if (vec >= 8) return launch_scan<Tin, Tout, 8>(a, st);
+        if (vec >= 8) return launch_nx<Tin, Tout, 8>(a, st);
     }
-    if (vec >= 4) return launch_scan<Tin, Tout, 4>(a, st);
-    if (vec >= 2) return launch_scan<Tin, Tout, 2>(a, st);
-    return launch_scan<Tin, Tout, 1>(a, st);
+    if (vec >= 4) return launch_nx<Tin, Tout, 4>(a, st);
+    if (vec >= 2) return launch_nx<Tin, Tout, 2>(a, st);
+    return launch_nx<Tin, Tout, 1>(a, st);
 }
 
 // largest power of two v <= cap such that every listed quantity is a multiple of v
@@ -407,7 +311,10 @@ static int common_pow2(std::initializer_list<int64_t> xs, int cap) {
     return v;
 }
 
-int selective_scan_fwd(const ss2d_scan_params* p, cudaStream_t st) {
+// What the kernels of scan_states.cuh take: 2 .. 16 states, a row of step sizes per row.
+static bool st_states(const ss2d_scan_params* p) { return p->dstate >= 2 && p->dstate <= 16 && p->delta_ratio <= 1; }
+
+static int validate_fwd(const ss2d_scan_params* p) {
     if (!p) return SS2D_EINVAL_NULL;
     if (!p->u || !p->delta || !p->A || !p->B || !p->C || !p->out) return SS2D_EINVAL_NULL;
     if (!dtype_ok(p->in_dtype) || !dtype_ok(p->out_dtype)) return SS2D_EINVAL_DTYPE;
@@ -429,6 +336,86 @@ int selective_scan_fwd(const ss2d_scan_params* p, cudaStream_t st) {
         !aligned_to(p->out, so) || !aligned_to(p->checkpoints, 4) || !aligned_to(p->A, 4) || !aligned_to(p->D, 4) || !aligned_to(p->delta_bias, 4))
         return SS2D_EINVAL_ALIGN;
 
+    if (p->checkpoints && p->checkpoint_every < 0) return SS2D_EINVAL_SHAPE;
+    if (p->checkpoint_every % (p->dstate == 1 ? 8 : st_states(p) ? 32 : 128) != 0) return SS2D_EINVAL_SHAPE;
+    return SS2D_OK;
+}
+
+// Widest vector (in elements, at most 8) that keeps every row start aligned for every tensor.
+static int fwd_vec(const ss2d_scan_params* p) {
+    const size_t si = dtype_size(p->in_dtype), so = dtype_size(p->out_dtype);
+    auto ptr_el = [](const void* q, size_t s) { return (int64_t)(reinterpret_cast<uintptr_t>(q) / s); };
+    return common_pow2({p->seqlen, p->u_batch_stride, p->u_dim_stride, p->delta_batch_stride, p->delta_dim_stride, p->out_batch_stride,
+                        p->out_dim_stride, p->B_batch_stride, p->B_group_stride, p->B_state_stride, p->C_batch_stride, p->C_group_stride,
+                        p->C_state_stride, ptr_el(p->u, si), ptr_el(p->delta, si), ptr_el(p->B, si), ptr_el(p->C, si), ptr_el(p->out, so)}, 8);
+}
+
+// How the rows of a 2 .. 16 state problem are cut: segments, and the floats of their end states and sums.
+static StSegments fwd_segments(const ss2d_scan_params* p, int64_t& floats) {
+    const int NS = st_pad_states(p->dstate), parts = st_parts(p->dim / p->n_groups);
+    const StSegments s = st_segments(p->batch * p->n_groups * parts * (NS / 4), p->seqlen);
+    floats = s.count > 1 ? p->batch * p->dim * s.count * (NS + 1) : 0;
+    return s;
+}
+
+long long selective_scan_checkpoint_every(int64_t dstate, int64_t delta_ratio) {
+    return dstate == 1 ? 8 : dstate >= 2 && dstate <= 16 && delta_ratio <= 1 ? 32 : 128;
+}
+
+long long selective_scan_fwd_workspace_bytes(const ss2d_scan_params* p) {
+    if (validate_fwd(p) != SS2D_OK) return -1;
+    if (!st_states(p)) return 0;
+    int64_t floats;
+    fwd_segments(p, floats);
+    return (long long)floats * 4;
+}
+
+template <typename Tin, typename Tout>
+static int states_fwd(StFwdArgs& a, const ss2d_scan_params* p, int vw, cudaStream_t st) {
+    if (a.S > 1) {
+        a.fold = 0;
+        float* ck = a.ckpt;
+        a.ckpt = nullptr;
+        const int rc = st_dispatch_fwd<Tin, Tin, false>(a, p->batch, vw, st);
+        if (rc != SS2D_OK) return rc;
+        a.ckpt = ck;
+        a.fold = 1;
+    }
+    return st_dispatch_fwd<Tin, Tout, true>(a, p->batch, vw, st);
+}
+
+static int selective_scan_states(const ss2d_scan_params* p, cudaStream_t st) {
+    StFwdArgs a = {};
+    a.u = p->u; a.delta = p->delta; a.B = p->B; a.C = p->C; a.out = p->out;
+    a.A = (const float*)p->A; a.D = (const float*)p->D; a.bias = (const float*)p->delta_bias;
+    a.dim = p->dim; a.group_size = p->dim / p->n_groups;
+    a.u_bs = p->u_batch_stride; a.u_ds = p->u_dim_stride; a.d_bs = p->delta_batch_stride; a.d_ds = p->delta_dim_stride;
+    a.o_bs = p->out_batch_stride; a.o_ds = p->out_dim_stride;
+    a.B_bs = p->B_batch_stride; a.B_gs = p->B_group_stride; a.B_ss = p->B_state_stride;
+    a.C_bs = p->C_batch_stride; a.C_gs = p->C_group_stride; a.C_ss = p->C_state_stride;
+    a.L = (int)p->seqlen; a.N = (int)p->dstate; a.n_groups = (int)p->n_groups; a.softplus = p->delta_softplus;
+    a.parts = st_parts(a.group_size);
+    a.every = p->checkpoint_every ? (int)p->checkpoint_every : 128;
+    a.ckpt = (float*)p->checkpoints; a.nck = (p->seqlen + a.every - 1) / a.every;
+    int64_t floats;
+    StSegments s = fwd_segments(p, floats);
+    if (floats && (!p->workspace || p->workspace_bytes < floats * 4)) { s = {1, (a.L + 127) / 128 * 128}; floats = 0; }   // uncut: slower, same result
+    if (floats && !aligned_to(p->workspace, 16)) return SS2D_EINVAL_ALIGN;
+    a.S = s.count; a.seg_len = s.len;
+    a.ends = floats ? (float*)p->workspace : nullptr;
+    a.sums = floats ? a.ends + p->batch * p->dim * s.count * st_pad_states(p->dstate) : nullptr;
+    const int v = fwd_vec(p), vw = v >= 8 ? 8 : v >= 4 ? 4 : 1;
+    const bool of32 = p->out_dtype == SS2D_F32;
+    if (p->in_dtype == SS2D_F32) return states_fwd<float, float>(a, p, vw, st);
+    if (p->in_dtype == SS2D_BF16) return of32 ? states_fwd<__nv_bfloat16, float>(a, p, vw, st) : states_fwd<__nv_bfloat16, __nv_bfloat16>(a, p, vw, st);
+    return of32 ? states_fwd<__half, float>(a, p, vw, st) : states_fwd<__half, __half>(a, p, vw, st);
+}
+
+int selective_scan_fwd(const ss2d_scan_params* p, cudaStream_t st) {
+    const int rc = validate_fwd(p);
+    if (rc != SS2D_OK) return rc;
+    if (st_states(p)) return selective_scan_states(p, st);
+    const int64_t L = p->seqlen;
     ScanArgs a;
     a.u = p->u; a.delta = p->delta; a.B = p->B; a.C = p->C;
     a.A = (const float*)p->A; a.D = (const float*)p->D; a.bias = (const float*)p->delta_bias;
@@ -442,14 +429,12 @@ int selective_scan_fwd(const ss2d_scan_params* p, cudaStream_t st) {
     a.C_bs = p->C_batch_stride; a.C_gs = p->C_group_stride; a.C_ss = p->C_state_stride;
     a.softplus = p->delta_softplus;
     a.dratio = p->delta_ratio > 1 ? p->delta_ratio : 1;
-    a.ckpt = (float*)p->checkpoints; a.nck = (L + 127) / 128;
+    a.ckpt = (float*)p->checkpoints;
 
-    // widest vector (in elements) that keeps every row start aligned for every tensor
-    const int cap = (si == 2) ? 8 : 4;
-    auto ptr_el = [](const void* q, size_t s) { return (int64_t)(reinterpret_cast<uintptr_t>(q) / s); };
-    int vec = common_pow2({L, a.u_bs, a.u_ds, a.d_bs, a.d_ds, a.o_bs, a.o_ds, a.B_bs, a.B_gs, a.B_ss, a.C_bs, a.C_gs,
-                           a.C_ss, ptr_el(p->u, si), ptr_el(p->delta, si), ptr_el(p->B, si), ptr_el(p->C, si),
-                           ptr_el(p->out, so)}, cap);
+    a.every = p->checkpoint_every ? (int)p->checkpoint_every : 128;
+    a.nck = (L + a.every - 1) / a.every;
+    a.states_only = false;
+    const int vec = fwd_vec(p);
 
     const int in = p->in_dtype;
     const bool of32 = p->out_dtype == SS2D_F32;

@@ -104,6 +104,10 @@ def selective_scan_fwd(u, delta, A, B, C, D=None, delta_bias=None, delta_softplu
     if return_checkpoints:
         ckpt = torch.empty((batch, dim, (L + 127) // 128, N), device=u.device, dtype=torch.float32)
         p.checkpoints = ckpt.data_ptr()
+    need = int(lib().ss2d_selective_scan_fwd_workspace_bytes(p)) if N > 1 else 0
+    if need > 0:        # rows too few to fill the GPU are walked in segments
+        ws = torch.empty(need, device=u.device, dtype=torch.uint8)
+        p.workspace, p.workspace_bytes = ws.data_ptr(), need
     with torch.cuda.device(u.device):
         check(lib().ss2d_selective_scan_fwd(p, _stream(u)), "ss2d_selective_scan_fwd")
     return (out, ckpt) if return_checkpoints else out
