@@ -75,6 +75,7 @@ typedef struct ss2d_scan_params {
     int64_t checkpoint_every;           /* spacing of the checkpoints; 0 = 128.  A multiple of ss2d_selective_scan_checkpoint_every() */
     void *workspace;                    /* optional, 16-byte aligned: with ss2d_selective_scan_fwd_workspace_bytes() bytes, rows too */
     int64_t workspace_bytes;            /* few to fill the GPU are cut into segments that are walked side by side */
+    int64_t states_only;                /* non-zero: write the checkpoints, not `out` (dstate <= 16, delta_ratio <= 1 or dstate 1) */
 } ss2d_scan_params;
 
 int ss2d_selective_scan_fwd(const ss2d_scan_params *p, void *cuda_stream);
@@ -115,6 +116,9 @@ typedef struct ss2d_scan_bwd_params {
     int64_t B_batch_stride, B_group_stride, B_state_stride;
     int64_t C_batch_stride, C_group_stride, C_state_stride;
     const void *checkpoints;            /* optional: what the forward call wrote; saves the pass that recomputes the states */
+    int64_t checkpoint_every;           /* their spacing.  0 = 128, and the kernels and the workspace size that go with it.  Callers
+                                           with checkpoints at ss2d_selective_scan_checkpoint_every(), or none, give that
+                                           value here and get the faster kernels for dstate <= 16 */
 } ss2d_scan_bwd_params;
 
 int64_t ss2d_selective_scan_bwd_workspace_bytes(const ss2d_scan_bwd_params *p);   /* < 0: invalid or unsupported arguments */

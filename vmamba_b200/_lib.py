@@ -27,7 +27,8 @@ class ScanParams(ctypes.Structure):
                                     "out_batch_stride", "out_dim_stride",
                                     "B_batch_stride", "B_group_stride", "B_state_stride",
                                     "C_batch_stride", "C_group_stride", "C_state_stride")] + \
-               [("checkpoints", _vp), ("checkpoint_every", _i64), ("workspace", _vp), ("workspace_bytes", _i64)]
+               [("checkpoints", _vp), ("checkpoint_every", _i64), ("workspace", _vp), ("workspace_bytes", _i64),
+                ("states_only", _i64)]
 
 
 class ScanBwdParams(ctypes.Structure):
@@ -40,7 +41,7 @@ class ScanBwdParams(ctypes.Structure):
                                     "dout_batch_stride", "dout_dim_stride",
                                     "B_batch_stride", "B_group_stride", "B_state_stride",
                                     "C_batch_stride", "C_group_stride", "C_state_stride")] + \
-               [("checkpoints", _vp)]
+               [("checkpoints", _vp), ("checkpoint_every", _i64)]
 
 
 class CrossParams(ctypes.Structure):

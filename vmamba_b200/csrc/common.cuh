@@ -210,14 +210,14 @@ template <int OFF, int WIDTH = 32> __device__ __forceinline__ void scan_step_up(
         " @p mul.f32 %0, %0, pa;\n}"
         : "+f"(a), "+f"(b) : "n"(OFF), "n"((32 - WIDTH) << 8));
 }
-template <int OFF> __device__ __forceinline__ void scan_step_down(float& a, float& b) {
+template <int OFF, int WIDTH = 32> __device__ __forceinline__ void scan_step_down(float& a, float& b) {
     asm volatile(
         "{\n .reg .pred p;\n .reg .f32 pa, pb;\n"
-        " shfl.sync.down.b32 pa|p, %0, %2, 31, 0xffffffff;\n"
-        " shfl.sync.down.b32 pb, %1, %2, 31, 0xffffffff;\n"
+        " shfl.sync.down.b32 pa|p, %0, %2, %3, 0xffffffff;\n"
+        " shfl.sync.down.b32 pb, %1, %2, %3, 0xffffffff;\n"
         " @p fma.rn.f32 %1, %0, pb, %1;\n"
         " @p mul.f32 %0, %0, pa;\n}"
-        : "+f"(a), "+f"(b) : "n"(OFF));
+        : "+f"(a), "+f"(b) : "n"(OFF), "n"(((32 - WIDTH) << 8) | 31));
 }
 // Inclusive state of the neighbouring lane (the lane before, or after when walking backwards); on the first lane of
 // the walk, which has no neighbour, the state carried over from the previous chunk.
@@ -226,9 +226,9 @@ template <bool kBack, int WIDTH = 32> __device__ __forceinline__ float entering_
     if constexpr (kBack)
         asm volatile(
             "{\n .reg .pred p;\n"
-            " shfl.sync.down.b32 %0|p, %1, 1, 31, 0xffffffff;\n"
+            " shfl.sync.down.b32 %0|p, %1, 1, %3, 0xffffffff;\n"
             " @!p mov.f32 %0, %2;\n}"
-            : "=&f"(r) : "f"(inc_b), "f"(carry));
+            : "=&f"(r) : "f"(inc_b), "f"(carry), "n"(((32 - WIDTH) << 8) | 31));
     else
         asm volatile(
             "{\n .reg .pred p;\n"

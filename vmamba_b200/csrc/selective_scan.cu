@@ -336,6 +336,7 @@ static int validate_fwd(const ss2d_scan_params* p) {
         !aligned_to(p->out, so) || !aligned_to(p->checkpoints, 4) || !aligned_to(p->A, 4) || !aligned_to(p->D, 4) || !aligned_to(p->delta_bias, 4))
         return SS2D_EINVAL_ALIGN;
 
+    if (p->states_only && (!p->checkpoints || (p->dstate != 1 && !st_states(p)))) return SS2D_ENOTSUP;
     if (p->checkpoints && p->checkpoint_every < 0) return SS2D_EINVAL_SHAPE;
     if (p->checkpoint_every % (p->dstate == 1 ? 8 : st_states(p) ? 32 : 128) != 0) return SS2D_EINVAL_SHAPE;
     return SS2D_OK;
@@ -381,7 +382,7 @@ static int states_fwd(StFwdArgs& a, const ss2d_scan_params* p, int vw, cudaStrea
         a.ckpt = ck;
         a.fold = 1;
     }
-    return st_dispatch_fwd<Tin, Tout, true>(a, p->batch, vw, st);
+    return p->states_only ? st_dispatch_fwd<Tin, Tin, false>(a, p->batch, vw, st) : st_dispatch_fwd<Tin, Tout, true>(a, p->batch, vw, st);
 }
 
 static int selective_scan_states(const ss2d_scan_params* p, cudaStream_t st) {
@@ -433,7 +434,7 @@ int selective_scan_fwd(const ss2d_scan_params* p, cudaStream_t st) {
 
     a.every = p->checkpoint_every ? (int)p->checkpoint_every : 128;
     a.nck = (L + a.every - 1) / a.every;
-    a.states_only = false;
+    a.states_only = p->states_only != 0;
     const int vec = fwd_vec(p);
 
     const int in = p->in_dtype;

@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "selective_scan_grad.cuh"
 
 namespace ss2d {
 
@@ -840,7 +841,7 @@ __global__ void __launch_bounds__(kBwdRowsWarps * 32, 2) selscan_bwd_rows_nx_ker
 // them to the storage type).  One thread per output element, fixed summation order.
 template <typename Tin>
 __global__ void selscan_bwd_fold_kernel(const float* rowred, const float* bcpart, float* dA, float* dD, float* dbias,
-                                        Tin* dB, Tin* dC, int64_t batch, int64_t dim, int N, int64_t L,
+                                        Tin* dB, Tin* dC, int64_t batch, int64_t images, int64_t dim, int N, int64_t L, int64_t Lp,
                                         int n_groups, int parts) {
     const int64_t n_small = dim * (N + 2);
     const int64_t n_bc = batch * n_groups * N * L;       // per tensor
@@ -850,7 +851,7 @@ __global__ void selscan_bwd_fold_kernel(const float* rowred, const float* bcpart
             const int64_t r = i / (N + 2);
             const int j = (int)(i - r * (N + 2));
             float acc = 0.f;
-            for (int64_t b = 0; b < batch; ++b) acc += rowred[(b * dim + r) * (N + 2) + j];
+            for (int64_t b = 0; b < images; ++b) acc += rowred[(b * dim + r) * (N + 2) + j];
             if (j < N) dA[r * N + j] = acc;
             else if (j == N) { if (dD) dD[r] = acc; }
             else if (dbias) dbias[r] = acc;
@@ -860,9 +861,9 @@ __global__ void selscan_bwd_fold_kernel(const float* rowred, const float* bcpart
             if (which) q -= n_bc;
             const int64_t l = q % L; int64_t t = q / L;
             const int n = (int)(t % N); t /= N;                 // t = b * n_groups + k
-            const float* src = bcpart + ((size_t)t * parts * 2 + which) * (size_t)N * L + (size_t)n * L + l;
+            const float* src = bcpart + ((size_t)t * parts * 2 + which) * (size_t)N * Lp + (size_t)n * Lp + l;
             float acc = 0.f;
-            for (int pq = 0; pq < parts; ++pq) acc += src[(size_t)pq * 2 * N * L];
+            for (int pq = 0; pq < parts; ++pq) acc += src[(size_t)pq * 2 * N * Lp];
             (which ? dC : dB)[q] = from_f<Tin>(acc);
         }
     }
@@ -965,6 +966,7 @@ static int plan_bwd(const ss2d_scan_bwd_params* p, BwdPlan& c) {
 
 long long selective_scan_bwd_workspace_bytes(const ss2d_scan_bwd_params* p) {
     if (validate_bwd(p) != SS2D_OK) return -1;
+    if (selective_scan_grad_takes(p)) return selective_scan_grad_workspace_bytes(p);
     BwdPlan c;
     if (plan_bwd(p, c) != SS2D_OK) return -1;
     return (long long)c.ws_floats * 4;
@@ -1009,20 +1011,31 @@ static int dispatch_bwd(const BwdArgs& a, const BwdPlan& c, int64_t ctas, cudaSt
 }
 
 template <typename Tin>
-static int launch_fold(const ss2d_scan_bwd_params* p, const BwdArgs& a, const BwdPlan& c, cudaStream_t st) {
+static int launch_fold(const ss2d_scan_bwd_params* p, const BwdFold& f, cudaStream_t st) {
     const int64_t total = p->dim * (p->dstate + 2) + 2 * p->batch * p->n_groups * p->dstate * p->seqlen;
     int64_t blocks = (total + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    selscan_bwd_fold_kernel<Tin><<<(unsigned)blocks, 256, 0, st>>>(a.rowred, a.bcpart, (float*)p->dA, (float*)p->dD,
-                                                                  (float*)p->ddelta_bias, (Tin*)p->dB, (Tin*)p->dC, p->batch,
-                                                                  p->dim, (int)p->dstate, p->seqlen, (int)p->n_groups, c.parts);
+    selscan_bwd_fold_kernel<Tin><<<(unsigned)blocks, 256, 0, st>>>(f.rowred, f.bcpart, (float*)p->dA, (float*)p->dD, (float*)p->ddelta_bias,
+                                                                   (Tin*)p->dB, (Tin*)p->dC, p->batch, f.images, p->dim, (int)p->dstate,
+                                                                   p->seqlen, f.Lp, (int)p->n_groups, f.parts);
     count_launch();
     return check_launch();
+}
+
+static int fold_bwd(const ss2d_scan_bwd_params* p, const BwdFold& f, cudaStream_t st) {
+    if (p->in_dtype == SS2D_F32) return launch_fold<float>(p, f, st);
+    if (p->in_dtype == SS2D_BF16) return launch_fold<__nv_bfloat16>(p, f, st);
+    return launch_fold<__half>(p, f, st);
 }
 
 int selective_scan_bwd(const ss2d_scan_bwd_params* p, cudaStream_t st) {
     const int rc = validate_bwd(p);
     if (rc != SS2D_OK) return rc;
+    BwdFold fold;
+    if (selective_scan_grad_takes(p)) {
+        const int r = selective_scan_grad(p, fold, st);
+        return r != SS2D_OK ? r : fold_bwd(p, fold, st);
+    }
     BwdPlan c;
     const int pr = plan_bwd(p, c);
     if (pr != SS2D_OK) return pr;
@@ -1052,9 +1065,8 @@ int selective_scan_bwd(const ss2d_scan_bwd_params* p, cudaStream_t st) {
     else
         r = gf32 ? dispatch_bwd<__half, float>(a, c, ctas, st) : dispatch_bwd<__half, __half>(a, c, ctas, st);
     if (r != SS2D_OK) return r;
-    if (p->in_dtype == SS2D_F32) return launch_fold<float>(p, a, c, st);
-    if (p->in_dtype == SS2D_BF16) return launch_fold<__nv_bfloat16>(p, a, c, st);
-    return launch_fold<__half>(p, a, c, st);
+    fold = {a.rowred, a.bcpart, p->batch, p->seqlen, c.parts};
+    return fold_bwd(p, fold, st);
 }
 
 }  // namespace ss2d

@@ -52,7 +52,8 @@ def selective_scan_fwd(u, delta, A, B, C, D=None, delta_bias=None, delta_softplu
     u, delta: (batch, K*C, L); A: (K*C, N); B, C: (batch, K, N, L); D, delta_bias: (K*C,) fp32.
     Output fp32 if `out_float` (the reference's "oflex") else u.dtype.  With `return_checkpoints` also the fp32
     states in front of every 128th element, (batch, K*C, ceil(L/128), N), which `selective_scan_bwd` accepts
-    instead of recomputing them.  `out`: optional result tensor of that shape and type (any batch / row strides,
+    instead of recomputing them; `return_checkpoints="grad"` gives them at the spacing the gradient kernels read
+    (`ss2d_selective_scan_checkpoint_every`).  `out`: optional result tensor of that shape and type (any batch / row strides,
     elements of a row contiguous), e.g. a permuted view, so that the result lands in the caller's layout.
     """
     _require_cuda(u, delta, A, B, C, D, delta_bias)
@@ -102,8 +103,9 @@ def selective_scan_fwd(u, delta, A, B, C, D=None, delta_bias=None, delta_softplu
     p.C_batch_stride, p.C_group_stride, p.C_state_stride = C.stride(0), C.stride(1), C.stride(2)
     ckpt = None
     if return_checkpoints:
-        ckpt = torch.empty((batch, dim, (L + 127) // 128, N), device=u.device, dtype=torch.float32)
-        p.checkpoints = ckpt.data_ptr()
+        every = 128 if return_checkpoints is True else lib().ss2d_selective_scan_checkpoint_every(N, ratio)
+        ckpt = torch.empty((batch, dim, (L + every - 1) // every, N), device=u.device, dtype=torch.float32)
+        p.checkpoints, p.checkpoint_every = ckpt.data_ptr(), every
     need = int(lib().ss2d_selective_scan_fwd_workspace_bytes(p)) if N > 1 else 0
     if need > 0:        # rows too few to fill the GPU are walked in segments
         ws = torch.empty(need, device=u.device, dtype=torch.uint8)
@@ -150,11 +152,17 @@ def selective_scan_bwd(u, delta, A, B, C, D, delta_bias, dout, delta_softplus=Fa
     p.dout_batch_stride, p.dout_dim_stride = dout.stride(0), dout.stride(1)
     p.B_batch_stride, p.B_group_stride, p.B_state_stride = B.stride(0), B.stride(1), B.stride(2)
     p.C_batch_stride, p.C_group_stride, p.C_state_stride = C.stride(0), C.stride(1), C.stride(2)
+    every = lib().ss2d_selective_scan_checkpoint_every(N, ratio)
+    p.checkpoint_every = every
     if checkpoints is not None:
-        if checkpoints.dtype != torch.float32 or tuple(checkpoints.shape) != (batch, dim, (L + 127) // 128, N) \
+        n_ck = [(L + e - 1) // e for e in (128, every)]
+        if checkpoints.dtype != torch.float32 or checkpoints.dim() != 4 or checkpoints.shape[2] not in n_ck \
+                or tuple(checkpoints.shape) != (batch, dim, checkpoints.shape[2], N) \
                 or not checkpoints.is_contiguous() or checkpoints.device != u.device:
             raise RuntimeError("checkpoints must be the fp32 (batch, dim, ceil(L/128), dstate) tensor of the forward call")
-        p.checkpoints = checkpoints.data_ptr()
+        # the gradient kernels form their own states where the ones at hand are too far apart
+        if checkpoints.shape[2] == n_ck[1]:
+            p.checkpoints = checkpoints.data_ptr()
     need = int(lib().ss2d_selective_scan_bwd_workspace_bytes(p))
     if need < 0:
         raise RuntimeError("ss2d_selective_scan_bwd_workspace_bytes: invalid or unsupported arguments")
@@ -185,7 +193,7 @@ class SelectiveScanCuda(torch.autograd.Function):
         ctx.backend = backend
         ctx.has_D, ctx.has_bias = D is not None, delta_bias is not None
         # the step states go to the backward call, as the reference's `x` does (csms6s.py:81-86)
-        out, ckpt = selective_scan_fwd(u, delta, A, B, C, D, delta_bias, delta_softplus, bool(oflex), return_checkpoints=True)
+        out, ckpt = selective_scan_fwd(u, delta, A, B, C, D, delta_bias, delta_softplus, bool(oflex), return_checkpoints="grad")
         saved = [u, delta, A, B, C, ckpt] + ([D] if ctx.has_D else []) + ([delta_bias] if ctx.has_bias else [])
         ctx.save_for_backward(*saved)
         return out
