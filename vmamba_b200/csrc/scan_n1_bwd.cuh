@@ -31,36 +31,13 @@ struct N1BwdArgs {
     int L, Lp, n_groups, parts, R, S, seg_len, softplus;
 };
 
-// Eight elements of a row from `pos`: AL 8 or 4 as vectors (row starts aligned, L a multiple of AL), 0 any alignment.
-template <typename T, int AL> struct Row8 {
-    static constexpr int kV = AL ? AL : 1, kN = AL ? 8 / AL : 1;
-    typename Vec<T, kV>::Raw w[kN];
-    __device__ __forceinline__ void load(const T* row, int pos, int L) {
-        if constexpr (AL != 0) {
+template <typename T, int AL>
+__device__ __forceinline__ void row8_pairs(const Row8<T, AL>& w, const T* row, int pos, int L, float2 (&v)[4]) {
+    float x[8];
+    w.get(row, pos, L, x);
 #pragma unroll
-            for (int j = 0; j < kN; ++j) {
-                w[j] = {};
-                if (pos + j * AL < L) w[j] = Vec<T, kV>::load_raw(row + pos + j * AL);
-            }
-        }
-    }
-    __device__ __forceinline__ void get(const T* row, int pos, int L, float2 (&v)[4]) const {
-        float x[8];
-        if constexpr (AL != 0) {
-#pragma unroll
-            for (int j = 0; j < kN; ++j) {
-                float y[kV];
-                Vec<T, kV>::unpack(w[j], y);
-#pragma unroll
-                for (int e = 0; e < kV; ++e) x[j * kV + e] = y[e];
-            }
-        } else {
-            load8_any<T>(row, pos, L, x);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = make_float2(x[2 * i], x[2 * i + 1]);
-    }
-};
+    for (int i = 0; i < 4; ++i) v[i] = make_float2(x[2 * i], x[2 * i + 1]);
+}
 template <typename T, int AL, int LPR>
 __device__ __forceinline__ void row8_store(T* row, int pos, int L, const float2 (&v)[4], float* stage, int lane) {
     const float x[8] = {v[0].x, v[0].y, v[1].x, v[1].y, v[2].x, v[2].y, v[3].x, v[3].y};
@@ -168,7 +145,7 @@ __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArg
         {
             Row8<Tin, AL> rb, rc;
             rb.load(Bm, pos, L); rc.load(Cm, pos, L);
-            rb.get(Bm, pos, L, bv); rc.get(Cm, pos, L, cv);
+            row8_pairs(rb, Bm, pos, L, bv); row8_pairs(rc, Cm, pos, L, cv);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) accB[i] = accC[i] = pk(0.f);
@@ -176,7 +153,7 @@ __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArg
         for (int i = 0; i < mine; ++i) {
             const int64_t r = row_of(i);
             float2 uv[4], d[4], g[4];
-            nu.get(u + r * a.u_ds, pos, L, uv); nd.get(delta_row(r), pos, L, d); ng.get(gp + r * a.g_ds, pos, L, g);
+            row8_pairs(nu, u + r * a.u_ds, pos, L, uv); row8_pairs(nd, delta_row(r), pos, L, d); row8_pairs(ng, gp + r * a.g_ds, pos, L, g);
             float h = nh;
             if (i + 1 < mine) fetch(i + 1, pos);
             const float4 pr = par[i * kStep + wr];
@@ -319,7 +296,7 @@ __global__ void __launch_bounds__(kN1Warps * 32) n1_bwd_segments_kernel(const N1
             Row8<Tin, AL> xd, xc;
             Row8<Tg, AL> xg;
             xd.load(dt, pos, L); xg.load(gp, pos, L); xc.load(Cm, pos, L);
-            xd.get(dt, pos, L, d); xg.get(gp, pos, L, g); xc.get(Cm, pos, L, cv);
+            row8_pairs(xd, dt, pos, L, d); row8_pairs(xg, gp, pos, L, g); row8_pairs(xc, Cm, pos, L, cv);
         }
         float le = 0.f, ls = 0.f;
 #pragma unroll

@@ -8,7 +8,7 @@
 // is staged in shared memory, and the chunk is then read back as four elements per load.  The B / C values of a chunk are
 // staged once per CTA (all rows of a CTA belong to one image and one group).
 //
-// Segments.  Where the rows of a problem do not fill the chip, every row is cut into S segments of a multiple of 128
+// Segments.  Where the rows of a problem do not fill the chip, every row is cut into S segments of a multiple of 64
 // elements that are walked side by side.  A first kernel leaves what a segment does to a state that enters it (its
 // end state from zero and the sum of its step sizes; the decay over the segment is exp(A * sum)), and the main kernel
 // folds the segments in front of its own.  The extra pass costs at most as many exponentials as the main one.
@@ -174,11 +174,11 @@ template <typename T, int NS, int VW, int WARPS> struct StRawBC {
 struct StSegments { int count, len; };
 inline StSegments st_segments(int64_t warps, int64_t L) {
     const int64_t want = 148 * 16;
-    if (warps * 4 > want || L < 512) return {1, (int)((L + 127) / 128 * 128)};
+    if (warps * 4 > want || L < 192) return {1, (int)((L + 63) / 64 * 64)};
     int64_t s = (want + warps - 1) / warps;
-    const int64_t most = (L + 127) / 128;
+    const int64_t most = (L + 63) / 64;
     if (s > most) s = most;
-    const int64_t len = (((L + s - 1) / s) + 127) / 128 * 128;
+    const int64_t len = (((L + s - 1) / s) + 63) / 64 * 64;
     s = (L + len - 1) / len;
     return {(int)s, (int)len};
 }

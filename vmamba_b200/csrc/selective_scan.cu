@@ -32,7 +32,7 @@ constexpr int kWarpsPerCta = 4;
 // d_state 1: W warps per row (1: four rows per CTA; 2 .. 8: the CTA is one row).  Per step a warp takes 256 elements, eight
 // per lane, and scans its lanes' (a, b) pairs by shuffle; with several warps per row their totals meet in shared memory
 // (one barrier per step) and every warp folds the ones in front of it.  One warp per row is the faster form where the rows
-// fill the chip; fewer rows get the more warps (try: rows * W up to 20 warps per SM).
+// fill the chip; fewer rows get the more warps (up to 32 per SM).
 // AL is the vector width of every access (8 or 4 elements), or 0 for rows of any alignment: a row is then walked from
 // the 16-byte boundary in front of its result, so that the results leave as vectors, and the inputs are cut out of the
 // aligned pieces around them.
@@ -41,8 +41,7 @@ constexpr int kWarpsPerCta = 4;
 template <typename Tin, typename Tout, int AL, int W, int LPR>
 __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32) selscan_fwd_n1_kernel(const ScanArgs a) {
     static_assert(W == 1 || LPR == 32, "rows of several warps take whole warps");
-    constexpr int VEC = 8, WSTEP = LPR * VEC, STEP = W * WSTEP, NL = AL ? VEC / AL : 1;
-    constexpr int AW = AL ? AL : 1;
+    constexpr int VEC = 8, WSTEP = LPR * VEC, STEP = W * WSTEP;
     __shared__ AB agg[2][W];
     const int lane = threadIdx.x & (LPR - 1), wi = W == 1 ? 0 : threadIdx.x >> 5;
     int64_t row = W == 1 ? ((int64_t)blockIdx.x * (kWarpsPerCta * 32) + threadIdx.x) / LPR : (int64_t)blockIdx.x;
@@ -64,55 +63,23 @@ __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32) selscan_f
     constexpr int OV = 16 / (int)sizeof(Tout);       // elements per 16-byte store
     const int ph = AL ? 0 : (int)((reinterpret_cast<uintptr_t>(out) / sizeof(Tout)) & (OV - 1));
     constexpr int ph_max = AL ? 0 : OV - 1;
-    using VI = Vec<Tin, AW>;
-    using Raw = typename VI::Raw;
-
-    Raw ru[NL], rd[NL], rb[NL], rc[NL];
-    auto fetch = [&](int at) {
-        if constexpr (AL != 0) {
-#pragma unroll
-            for (int j = 0; j < NL; ++j) {
-                const int p = min(at + j * AL, L - AL);          // vectors beyond the row re-read its end and are ignored
-                ru[j] = VI::load_raw(u + p); rd[j] = VI::load_raw(dt + p);
-                rb[j] = VI::load_raw(Bm + p); rc[j] = VI::load_raw(Cm + p);
-            }
-        }
-    };
+    Row8<Tin, AL> ru, rd, rb, rc;
+    auto fetch = [&](int at) { ru.load(u, at, L); rd.load(dt, at, L); rb.load(Bm, at, L); rc.load(Cm, at, L); };
     int pos = wi * WSTEP + lane * VEC - ph;
     fetch(pos);
     float hc = 0.f;                                  // state entering this step
     // rows that share a warp may start at different phases: they take the same number of steps
     for (int base = LPR < 32 ? -ph_max : -ph, it = 0; base < L; base += STEP, ++it) {
         float uv[VEC], dv[VEC], bv[VEC], cv[VEC], P[VEC], hl[VEC];
-        if constexpr (AL != 0) {
-#pragma unroll
-            for (int j = 0; j < NL; ++j) {
-                float x[AW];
-                VI::unpack(ru[j], x);
-#pragma unroll
-                for (int e = 0; e < AW; ++e) uv[j * AW + e] = x[e];
-                VI::unpack(rd[j], x);
-#pragma unroll
-                for (int e = 0; e < AW; ++e) dv[j * AW + e] = x[e];
-                VI::unpack(rb[j], x);
-#pragma unroll
-                for (int e = 0; e < AW; ++e) bv[j * AW + e] = x[e];
-                VI::unpack(rc[j], x);
-#pragma unroll
-                for (int e = 0; e < AW; ++e) cv[j * AW + e] = x[e];
-            }
-            fetch(pos + STEP);
-        } else {
-            load8_any<Tin>(u, pos, L, uv); load8_any<Tin>(dt, pos, L, dv);
-            load8_any<Tin>(Bm, pos, L, bv); load8_any<Tin>(Cm, pos, L, cv);
-        }
+        ru.get(u, pos, L, uv); rd.get(dt, pos, L, dv); rb.get(Bm, pos, L, bv); rc.get(Cm, pos, L, cv);
+        fetch(pos + STEP);
         float p = 1.f, h = 0.f;
 #pragma unroll
         for (int i = 0; i < VEC; ++i) {
             float dl = dv[i] + bias;
             if (sp) dl = softplus_fast(dl);
             // outside the row: a step of zero leaves the state as it is (whole vectors are tested once below)
-            if constexpr (AL != 8) dl = (AL == 4 ? pos + (i & 4) : pos + i) < L && (AL || pos + i >= 0) ? dl : 0.f;
+            if constexpr (AL != 8) dl = pos + (AL ? i / (AL ? AL : 1) * AL : i) < L && (AL || pos + i >= 0) ? dl : 0.f;
             const float aa = decay_fast(dl, A2);
             h = fmaf(aa, h, dl * bv[i] * uv[i]);
             p *= aa;
@@ -157,7 +124,7 @@ __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32) selscan_f
             float ov[VEC];
 #pragma unroll
             for (int i = 0; i < VEC; ++i) ov[i] = fmaf(Dv, uv[i], cv[i] * fmaf(P[i], hin, hl[i]));
-            constexpr int SV = AL == 4 && OV > 4 ? 4 : OV;       // elements per store
+            constexpr int SV = AL && AL < OV ? AL : OV;          // elements per store
 #pragma unroll
             for (int j = 0; j < VEC; j += SV) {
                 const int q = pos + j;
@@ -255,11 +222,11 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) selscan_fwd_nx_kernel(const
     }
 }
 
-// d_state 1: warps per row.  Rows that fill the chip (20 warps on each of 148 SMs) get one; fewer rows more, as long as a
+// d_state 1: warps per row.  Rows that fill the chip (32 warps on each of 148 SMs) get one; fewer rows more, as long as a
 // step of all of them is not longer than the row.
 static int n1_warps(int64_t rows, int64_t L) {
     int w = 1;
-    while (w < 8 && rows * w < 148 * 20 && (int64_t)w * 256 < L) w *= 2;
+    while (w < 8 && rows * w < 148 * 32 && (int64_t)w * 256 < L) w *= 2;
     return w;
 }
 
@@ -292,7 +259,10 @@ static int launch_nx(const ScanArgs& a, cudaStream_t st) {
 template <typename Tin, typename Tout>
 static int dispatch_vec(const ScanArgs& a, int vec, cudaStream_t st) {
     if (a.dstate == 1)
-        return vec >= 8 ? launch_n1<Tin, Tout, 8>(a, st) : vec >= 4 ? launch_n1<Tin, Tout, 4>(a, st) : launch_n1<Tin, Tout, 0>(a, st);
+        return vec >= 8   ? launch_n1<Tin, Tout, 8>(a, st)
+               : vec >= 4 ? launch_n1<Tin, Tout, 4>(a, st)
+               : vec >= 2 && sizeof(Tin) == 4 ? launch_n1<Tin, Tout, sizeof(Tin) == 4 ? 2 : 0>(a, st)
+                          : launch_n1<Tin, Tout, 0>(a, st);
     if constexpr (sizeof(Tin) == 2) {
         if (vec >= 8) return launch_nx<Tin, Tout, 8>(a, st);
     }
@@ -400,7 +370,7 @@ static int selective_scan_states(const ss2d_scan_params* p, cudaStream_t st) {
     a.ckpt = (float*)p->checkpoints; a.nck = (p->seqlen + a.every - 1) / a.every;
     int64_t floats;
     StSegments s = fwd_segments(p, floats);
-    if (floats && (!p->workspace || p->workspace_bytes < floats * 4)) { s = {1, (a.L + 127) / 128 * 128}; floats = 0; }   // uncut: slower, same result
+    if (floats && (!p->workspace || p->workspace_bytes < floats * 4)) { s = {1, (a.L + 63) / 64 * 64}; floats = 0; }   // uncut: slower, same result
     if (floats && !aligned_to(p->workspace, 16)) return SS2D_EINVAL_ALIGN;
     a.S = s.count; a.seg_len = s.len;
     a.ends = floats ? (float*)p->workspace : nullptr;

@@ -81,8 +81,8 @@ static int plan_grad(const ss2d_scan_bwd_params* p, GradPlan& c) {
         c.S = 0;
         for (int sets = 1; sets <= kStMaxSets && sets <= parts1; sets *= 2) {
             const int64_t parts = (parts1 + sets - 1) / sets, ctas = groups * parts;
-            for (int64_t s = 1; s <= 16 && (s == 1 || L >= s * 128); ++s) {
-                const int64_t len = ((L + s - 1) / s + 127) / 128 * 128, S = (L + len - 1) / len, waves = (ctas * S + slots - 1) / slots;
+            for (int64_t s = 1; s <= 64 && (s == 1 || L >= s * 64); ++s) {
+                const int64_t len = ((L + s - 1) / s + 63) / 64 * 64, S = (L + len - 1) / len, waves = (ctas * S + slots - 1) / slots;
                 const double cost = (double)waves * (100 * sets + 29) * (double)len / (double)L + (S > 1 ? 25.0 * (double)(groups * parts1) / (double)slots : 0.0);
                 if (c.S == 0 || cost < 0.97 * best) { best = cost; c.sets = sets; c.parts = (int)parts; c.S = (int)S; c.seg_len = (int)len; }
             }
