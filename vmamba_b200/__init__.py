@@ -1,8 +1,11 @@
 """vmamba_b200: the SS2D core of VMamba as hand-written sm_100a CUDA behind the reference's
 operator surface.  Importing the package loads libss2d_b200.so and fails loudly if it is absent."""
+import torch  # noqa: F401  the host extension links against its libraries
+
 from . import _lib
 
 _lib.lib()   # no CUDA library, no package: there is no CPU or eager fallback
+from . import _host  # noqa: E402,F401  the host extension of the same build
 
 from .ops import (CrossMerge, CrossMergeF, CrossMergeTritonF, CrossScan, CrossScanF, CrossScanTritonF,  # noqa: E402
                   SelectiveScanCuda, SelectiveScanOflex, cross_merge_fn, cross_merge_fwd, cross_scan_fn,

@@ -1,0 +1,57 @@
+// Shared parts of the host extension (_host.so): the torch side of libss2d_b200.so.
+// Every function here only prepares arguments and launches; the kernels are behind the C interface of ss2d_b200.h.
+#pragma once
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/extension.h>
+
+#include "ss2d_b200.h"
+
+namespace host {
+
+using at::Tensor;
+using OptT = std::optional<Tensor>;
+
+// A status of the library, raised in Python as vmamba_b200._lib.Ss2dError(status, where).
+struct LibError {
+    int status;
+    const char* where;
+};
+inline void check(int status, const char* where) {
+    if (status != SS2D_OK) throw LibError{status, where};
+}
+
+inline int dtype_code(at::ScalarType t) {
+    switch (t) {
+        case at::kFloat: return SS2D_F32;
+        case at::kHalf: return SS2D_F16;
+        case at::kBFloat16: return SS2D_BF16;
+        default: TORCH_CHECK_TYPE(false, "unsupported dtype ", t, ": expected float32, float16 or bfloat16");
+    }
+}
+inline int dtype_code(const Tensor& t) { return dtype_code(t.scalar_type()); }
+
+inline void require_cuda(std::initializer_list<const Tensor*> ts) {
+    for (const Tensor* t : ts)
+        TORCH_CHECK(!t->defined() || t->is_cuda(),
+                    "vmamba_b200 operators run on CUDA tensors only (no CPU fallback); use the oracle under oracle/ for CPU reference values");
+}
+inline void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
+inline Tensor opt(const OptT& t) { return t.has_value() ? *t : Tensor(); }
+inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+inline Tensor f32(const Tensor& t) {
+    if (!t.defined() || (t.scalar_type() == at::kFloat && t.is_contiguous())) return t;
+    return t.contiguous().to(at::kFloat);
+}
+inline Tensor rows(const Tensor& t) { return t.stride(-1) == 1 ? t : t.contiguous(); }
+inline Tensor bytes(int64_t n, const Tensor& like) { return at::empty({n}, like.options().dtype(at::kByte)); }
+
+// host_ops.cpp
+std::pair<Tensor, Tensor> scan_fwd(Tensor u, Tensor delta, Tensor A, Tensor B, Tensor C, Tensor D, Tensor bias, bool softplus, bool out_float,
+                                   int64_t every, Tensor out);
+std::vector<Tensor> scan_bwd(Tensor u, Tensor delta, Tensor A, Tensor B, Tensor C, Tensor D, Tensor bias, Tensor dout, bool softplus, Tensor ckpt);
+Tensor cross_scan(const Tensor& x, int64_t scans);       // (B, C, H, W) -> (B, 4, C, L)
+Tensor cross_merge(const Tensor& ys, int64_t scans);     // (B, 4, C, H, W) -> (B, C, L)
+int64_t scan_ratio(const Tensor& u, const Tensor& delta);
+
+}  // namespace host

@@ -1,4 +1,5 @@
-"""Operator surface of the reference, backed by the sm_100a kernels of libss2d_b200.so.
+"""Operator surface of the reference, backed by the sm_100a kernels of libss2d_b200.so (the hot calls through the host
+extension _host.so, the others through ctypes).
 
 Mirrors, name for name, what MzeroMiko/VMamba's modules resolve at call time:
   selective_scan_fn, SelectiveScanCuda (+ alias SelectiveScanOflex)   classification/models/csms6s.py:71-126,
@@ -13,8 +14,8 @@ from __future__ import annotations
 
 import torch
 
-from . import _lib
-from ._lib import (CrossExParams, CrossParams, NormParams, PointwiseParams, RelayoutParams, ScanBwdParams, ScanParams, StemParams,
+from . import _host, _lib
+from ._lib import (CrossExParams, NormParams, PointwiseParams, RelayoutParams, StemParams,
                    check, lib)
 
 _DTYPES = {torch.float32: _lib.SS2D_F32, torch.float16: _lib.SS2D_F16, torch.bfloat16: _lib.SS2D_BF16}
@@ -56,62 +57,11 @@ def selective_scan_fwd(u, delta, A, B, C, D=None, delta_bias=None, delta_softplu
     (`ss2d_selective_scan_checkpoint_every`).  `out`: optional result tensor of that shape and type (any batch / row strides,
     elements of a row contiguous), e.g. a permuted view, so that the result lands in the caller's layout.
     """
-    _require_cuda(u, delta, A, B, C, D, delta_bias)
-    if u.dim() != 3 or delta.dim() != 3 or delta.shape[0] != u.shape[0] or delta.shape[2] != u.shape[2] \
-            or delta.shape[1] == 0 or u.shape[1] % delta.shape[1] != 0:
-        raise RuntimeError(f"u must be (batch, dim, L) and delta (batch, dim / r, L), got {tuple(u.shape)} {tuple(delta.shape)}")
-    if B.dim() != 4 or C.shape != B.shape:
-        raise RuntimeError("B and C must be (batch, n_groups, dstate, L) with equal shapes")
-    batch, dim, L = u.shape
-    _, K, N, Lb = B.shape
-    if B.shape[0] != batch or Lb != L or dim % K != 0:
-        raise RuntimeError("B/C shape does not match u")
-    if tuple(A.shape) != (dim, N):
-        raise RuntimeError(f"A must be (dim, dstate) = ({dim}, {N}), got {tuple(A.shape)}")
-    if delta.dtype != u.dtype or B.dtype != u.dtype or C.dtype != u.dtype:
-        raise RuntimeError("u, delta, B, C must share one dtype")
-    if u.stride(-1) != 1:
-        u = u.contiguous()
-    if delta.stride(-1) != 1:
-        delta = delta.contiguous()
-    if B.stride(-1) != 1:
-        B = B.contiguous()
-    if C.stride(-1) != 1:
-        C = C.contiguous()
-    A = A.contiguous().float()
-    D = None if D is None else D.contiguous().float()
-    delta_bias = None if delta_bias is None else delta_bias.contiguous().float()
-    if D is not None and D.numel() != dim:
-        raise RuntimeError("D must have dim elements")
-    ratio = dim // delta.shape[1]        # channels sharing one delta row (selective_scan_oflex.cpp:59)
-    if delta_bias is not None and delta_bias.numel() != delta.shape[1]:
-        raise RuntimeError("delta_bias must have one element per delta row")
-    out_dtype = torch.float32 if out_float else u.dtype
-    if out is None:
-        out = torch.empty((batch, dim, L), device=u.device, dtype=out_dtype)
-    elif tuple(out.shape) != (batch, dim, L) or out.dtype != out_dtype or out.stride(-1) != 1 or out.device != u.device:
-        raise RuntimeError("out must be (batch, dim, L) of the result type on u's device with contiguous rows")
-    p = ScanParams()
-    p.u, p.delta, p.A, p.B, p.C, p.D, p.delta_bias, p.out = (_ptr(t) for t in (u, delta, A, B, C, D, delta_bias, out))
-    p.in_dtype, p.out_dtype = dtype_code(u), dtype_code(out)
-    p.delta_softplus, p.delta_ratio = int(bool(delta_softplus)), ratio
-    p.batch, p.dim, p.dstate, p.seqlen, p.n_groups = batch, dim, N, L, K
-    p.u_batch_stride, p.u_dim_stride = u.stride(0), u.stride(1)
-    p.delta_batch_stride, p.delta_dim_stride = delta.stride(0), delta.stride(1)
-    p.out_batch_stride, p.out_dim_stride = out.stride(0), out.stride(1)
-    p.B_batch_stride, p.B_group_stride, p.B_state_stride = B.stride(0), B.stride(1), B.stride(2)
-    p.C_batch_stride, p.C_group_stride, p.C_state_stride = C.stride(0), C.stride(1), C.stride(2)
-    ckpt = None
+    every = 0
     if return_checkpoints:
-        every = 128 if return_checkpoints is True else lib().ss2d_selective_scan_checkpoint_every(N, ratio)
-        ckpt = torch.empty((batch, dim, (L + every - 1) // every, N), device=u.device, dtype=torch.float32)
-        p.checkpoints, p.checkpoint_every = ckpt.data_ptr(), every
-    need = int(lib().ss2d_selective_scan_fwd_workspace_bytes(p)) if N > 1 else 0
-    if need > 0:        # rows too few to fill the GPU are walked in segments
-        ws = torch.empty(need, device=u.device, dtype=torch.uint8)
-        p.workspace, p.workspace_bytes = ws.data_ptr(), need
-    with torch.cuda.device(u.device):
-        check(lib().ss2d_selective_scan_fwd(p, _stream(u)), "ss2d_selective_scan_fwd")
+        every = 128 if return_checkpoints is True else \
+            lib().ss2d_selective_scan_checkpoint_every(A.shape[1], u.shape[1] // delta.shape[1])
+    out, ckpt = _host.selective_scan_fwd(u, delta, A, B, C, D, delta_bias, bool(delta_softplus), bool(out_float), every, out)
     return (out, ckpt) if return_checkpoints else out
 
 
@@ -121,60 +71,7 @@ def selective_scan_bwd(u, delta, A, B, C, D, delta_bias, dout, delta_softplus=Fa
     `checkpoints`: what `selective_scan_fwd(..., return_checkpoints=True)` returned (optional).
     Shapes and types of the results as selective_scan_cuda_oflex.bwd returns them
     (selective_scan_oflex.cpp:308-353)."""
-    _require_cuda(u, delta, A, B, C, D, delta_bias, dout)
-    batch, dim, L = u.shape
-    _, K, N, _ = B.shape
-    if dout.shape != u.shape:
-        raise RuntimeError(f"dout must have the shape of u, got {tuple(dout.shape)}")
-    if dout.dtype not in (torch.float32, u.dtype):
-        raise RuntimeError("dout must be fp32 or of u's dtype")
-    cont = lambda t: t if t.stride(-1) == 1 else t.contiguous()
-    u, delta, B, C, dout = cont(u), cont(delta), cont(B), cont(C), cont(dout)
-    A = A.contiguous().float()
-    D = None if D is None else D.contiguous().float()
-    delta_bias = None if delta_bias is None else delta_bias.contiguous().float()
-    du = torch.empty((batch, dim, L), device=u.device, dtype=u.dtype)
-    ddelta = torch.empty_like(du)
-    dA = torch.empty((dim, N), device=u.device, dtype=torch.float32)
-    dB = torch.empty((batch, K, N, L), device=u.device, dtype=u.dtype)
-    dC = torch.empty_like(dB)
-    dD = None if D is None else torch.empty(dim, device=u.device, dtype=torch.float32)
-    dbias = None if delta_bias is None else torch.empty(dim, device=u.device, dtype=torch.float32)
-    p = ScanBwdParams()
-    p.u, p.delta, p.A, p.B, p.C, p.D, p.delta_bias, p.dout = (_ptr(t) for t in (u, delta, A, B, C, D, delta_bias, dout))
-    p.du, p.ddelta, p.dA, p.dB, p.dC, p.dD, p.ddelta_bias = (_ptr(t) for t in (du, ddelta, dA, dB, dC, dD, dbias))
-    p.in_dtype, p.dout_dtype = dtype_code(u), dtype_code(dout)
-    ratio = dim // delta.shape[1]
-    p.delta_softplus, p.delta_ratio = int(bool(delta_softplus)), ratio
-    p.batch, p.dim, p.dstate, p.seqlen, p.n_groups = batch, dim, N, L, K
-    p.u_batch_stride, p.u_dim_stride = u.stride(0), u.stride(1)
-    p.delta_batch_stride, p.delta_dim_stride = delta.stride(0), delta.stride(1)
-    p.dout_batch_stride, p.dout_dim_stride = dout.stride(0), dout.stride(1)
-    p.B_batch_stride, p.B_group_stride, p.B_state_stride = B.stride(0), B.stride(1), B.stride(2)
-    p.C_batch_stride, p.C_group_stride, p.C_state_stride = C.stride(0), C.stride(1), C.stride(2)
-    every = lib().ss2d_selective_scan_checkpoint_every(N, ratio)
-    p.checkpoint_every = every
-    if checkpoints is not None:
-        n_ck = [(L + e - 1) // e for e in (128, every)]
-        if checkpoints.dtype != torch.float32 or checkpoints.dim() != 4 or checkpoints.shape[2] not in n_ck \
-                or tuple(checkpoints.shape) != (batch, dim, checkpoints.shape[2], N) \
-                or not checkpoints.is_contiguous() or checkpoints.device != u.device:
-            raise RuntimeError("checkpoints must be the fp32 (batch, dim, ceil(L/128), dstate) tensor of the forward call")
-        # the gradient kernels form their own states where the ones at hand are too far apart
-        if checkpoints.shape[2] == n_ck[1]:
-            p.checkpoints = checkpoints.data_ptr()
-    need = int(lib().ss2d_selective_scan_bwd_workspace_bytes(p))
-    if need < 0:
-        raise RuntimeError("ss2d_selective_scan_bwd_workspace_bytes: invalid or unsupported arguments")
-    ws = torch.empty(max(need, 16), device=u.device, dtype=torch.uint8)
-    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
-    with torch.cuda.device(u.device):
-        check(lib().ss2d_selective_scan_bwd(p, _stream(u)), "ss2d_selective_scan_bwd")
-    if ratio > 1:       # rows that shared a delta row: their gradients add up (selective_scan_oflex.cpp:348-352)
-        ddelta = ddelta.view(batch, dim // ratio, ratio, L).float().sum(2).to(u.dtype)
-        if dbias is not None:
-            dbias = dbias.view(dim // ratio, ratio).sum(1)
-    return du, ddelta, dA, dB, dC, dD, dbias
+    return tuple(_host.selective_scan_bwd(u, delta, A, B, C, D, delta_bias, dout, bool(delta_softplus), checkpoints))
 
 
 class SelectiveScanCuda(torch.autograd.Function):
@@ -225,10 +122,11 @@ def selective_scan_fn(u, delta, A, B, C, D=None, delta_bias=None, delta_softplus
     if backend == "torch":
         raise NotImplementedError("backend='torch' is not provided: vmamba_b200 has no eager/CPU path "
                                   "(reference values come from the oracle under oracle/)")
-    if torch.is_grad_enabled() and any(isinstance(t, torch.Tensor) and t.requires_grad for t in (u, delta, A, B, C, D, delta_bias)):
+    if torch._C._get_tracing_state() is not None:        # a traced graph names the operator (selective_scan_flop_jit)
         return SelectiveScanCuda.apply(u, delta, A, B, C, D, delta_bias, delta_softplus, oflex, backend)
-    with torch.autocast("cuda", enabled=False):
-        return selective_scan_fwd(u, delta, A, B, C, D, delta_bias, delta_softplus, bool(oflex))
+    if torch.is_autocast_enabled("cuda") and torch.is_grad_enabled():     # the Function's casts under autocast
+        return SelectiveScanCuda.apply(u, delta, A, B, C, D, delta_bias, delta_softplus, oflex, backend)
+    return _host.selective_scan_fn(u, delta, A, B, C, D, delta_bias, bool(delta_softplus), bool(oflex))
 
 
 def flops_selective_scan_fn(B=1, L=256, D=768, N=16, with_D=True, with_Z=False, with_complex=False):
@@ -297,18 +195,11 @@ def cross_scan_fwd(x: torch.Tensor, scans: int = 0, in_channel_first=True, out_c
     """cross_scan_fwd / cross_scan1b1_fwd of the reference (vmamba.py:41-84, 130-183).  Default flags:
     (B, C, H, W) -> (B, 4, C, H*W) through the tuned kernels; channel-last sides and one_by_one through the
     index-only kernels (`ss2d_cross_scan_ex`)."""
-    _require_cuda(x)
     _check_flags(in_channel_first, out_channel_first, one_by_one, scans)
-    x = x.contiguous()
     if _plain(in_channel_first, out_channel_first, one_by_one):
-        if x.dim() != 4:
-            raise RuntimeError("cross_scan expects a (B, C, H, W) tensor")
-        B, C, H, W = x.shape
-        y = torch.empty((B, 4, C, H * W), device=x.device, dtype=x.dtype)
-        p = CrossParams(x.data_ptr(), y.data_ptr(), dtype_code(x), scans, B, C, H, W)
-        with torch.cuda.device(x.device):
-            check(lib().ss2d_cross_scan(p, _stream(x)), "ss2d_cross_scan")
-        return y
+        return _host.cross_scan(x, scans)
+    _require_cuda(x)
+    x = x.contiguous()
     if one_by_one:
         if in_channel_first:
             B, K, C, H, W = x.shape
@@ -342,20 +233,13 @@ def cross_merge_fwd(ys: torch.Tensor, scans: int = 0, in_channel_first=True, out
     """cross_merge_fwd / cross_merge1b1_fwd of the reference (vmamba.py:87-130, 186-245).  `out_channel_first` names
     the layout of ys ((B, 4, C, H, W) or (B, H, W, 4, C)), `in_channel_first` the layout of the result ((B, C, L)
     or (B, L, C)), as there."""
-    _require_cuda(ys)
     _check_flags(in_channel_first, out_channel_first, one_by_one, scans)
+    if _plain(in_channel_first, out_channel_first, one_by_one):
+        return _host.cross_merge(ys, scans)
+    _require_cuda(ys)
     ys = ys.contiguous()
     if ys.dim() != 5:
         raise RuntimeError("cross_merge expects a 5-d tensor of four routes")
-    if _plain(in_channel_first, out_channel_first, one_by_one):
-        B, K, C, H, W = ys.shape
-        if K != 4:
-            raise RuntimeError("cross_merge expects (B, 4, C, H, W)")
-        y = torch.empty((B, C, H * W), device=ys.device, dtype=ys.dtype)
-        p = CrossParams(ys.data_ptr(), y.data_ptr(), dtype_code(ys), scans, B, C, H, W)
-        with torch.cuda.device(ys.device):
-            check(lib().ss2d_cross_merge(p, _stream(ys)), "ss2d_cross_merge")
-        return y
     if out_channel_first:
         B, K, C, H, W = ys.shape
     else:
@@ -446,6 +330,8 @@ def cross_scan_fn(x, in_channel_first=True, out_channel_first=True, one_by_one=F
     """Drop-in for cross_scan_fn (vmamba.py:577-588).  `force_torch` is accepted and ignored:
     there is one implementation."""
     _check_flags(in_channel_first, out_channel_first, one_by_one, scans)
+    if _plain(in_channel_first, out_channel_first, one_by_one):
+        return _host.cross_scan_fn(x, scans)
     if torch.is_grad_enabled() and x.requires_grad:
         return CrossScanF.apply(x, in_channel_first, out_channel_first, one_by_one, scans)
     return cross_scan_fwd(x, scans, in_channel_first, out_channel_first, one_by_one)
@@ -454,6 +340,8 @@ def cross_scan_fn(x, in_channel_first=True, out_channel_first=True, one_by_one=F
 def cross_merge_fn(y, in_channel_first=True, out_channel_first=True, one_by_one=False, scans=0, force_torch=False):
     """Drop-in for cross_merge_fn (vmamba.py:591-601)."""
     _check_flags(in_channel_first, out_channel_first, one_by_one, scans)
+    if _plain(in_channel_first, out_channel_first, one_by_one):
+        return _host.cross_merge_fn(y, scans)
     if torch.is_grad_enabled() and y.requires_grad:
         return CrossMergeF.apply(y, in_channel_first, out_channel_first, one_by_one, scans)
     return cross_merge_fwd(y, scans, in_channel_first, out_channel_first, one_by_one)
