@@ -32,7 +32,7 @@ constexpr int kWarpsPerCta = 4;
 // d_state 1: W warps per row (1: four rows per CTA; 2 .. 8: the CTA is one row).  Per step a warp takes 256 elements, eight
 // per lane, and scans its lanes' (a, b) pairs by shuffle; with several warps per row their totals meet in shared memory
 // (one barrier per step) and every warp folds the ones in front of it.  One warp per row is the faster form where the rows
-// fill the chip; fewer rows get the more warps (up to 32 per SM).
+// fill the chip; fewer rows get the more warps (up to 24 per SM).
 // AL is the vector width of every access (8 or 4 elements), or 0 for rows of any alignment: a row is then walked from
 // the 16-byte boundary in front of its result, so that the results leave as vectors, and the inputs are cut out of the
 // aligned pieces around them.
@@ -222,11 +222,11 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) selscan_fwd_nx_kernel(const
     }
 }
 
-// d_state 1: warps per row.  Rows that fill the chip (32 warps on each of 148 SMs) get one; fewer rows more, as long as a
+// d_state 1: warps per row.  Rows that fill the chip (24 warps on each of 148 SMs) get one; fewer rows more, as long as a
 // step of all of them is not longer than the row.
 static int n1_warps(int64_t rows, int64_t L) {
     int w = 1;
-    while (w < 8 && rows * w < 148 * 32 && (int64_t)w * 256 < L) w *= 2;
+    while (w < 8 && rows * w < 148 * 24 && (int64_t)w * 256 < L) w *= 2;
     return w;
 }
 
