@@ -8,6 +8,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "cross_flat.cuh"
 
 namespace ss2d {
 
@@ -418,6 +419,41 @@ static int merge_plane_v(const PlaneArgs& a, int scans, int pv, size_t smem, cud
     return launch_merge_plane<T, 1>(a, scans, smem, st);
 }
 
+// Whether the flat kernels take the planes, and how.  `copies`: shared planes per plane (1 scan, 2 merge).
+static bool plan_flat(const ss2d_cross_params* p, size_t esize, int copies, FlatArgs& a, int& threads, size_t& smem) {
+    const long long L = p->H * p->W, Lp = copies == 1 ? p->H * (p->W | 1) : p->W * (p->H | 1);
+    if (Lp * (long long)esize * copies > 200 * 1024 || L > 65536) return false;      // 65 536: the divisions by multiplication are exact
+    long long PP = std::min<long long>(std::max<long long>(1, 4096 / L), p->C);
+    while (PP > 1 && PP * Lp * (long long)esize * copies > 48 * 1024) --PP;
+    a.in = p->in; a.out = p->out; a.C = (int)p->C; a.H = (int)p->H; a.W = (int)p->W; a.L = (int)L; a.PP = (int)PP;
+    a.blocks = (int)((p->C + PP - 1) / PP);
+    for (int k = 0; k < 4; ++k) {
+        const RouteMap m = route_map(p->scans, k, p->H, p->W);
+        a.route[k] = {m.col_like, m.sh > 0, m.sw > 0};
+    }
+    auto magic = [](long long d) { return d > 1 ? (unsigned)(((1ULL << 32) + (unsigned long long)d - 1) / (unsigned long long)d) : 0u; };
+    a.magic_H = magic(p->H); a.magic_W = magic(p->W); a.magic_L = magic(L);
+    smem = (size_t)PP * Lp * esize * copies;
+    threads = smem > 40 * 1024 ? 512 : 256;
+    return p->B * a.blocks <= 0x7fffffffLL;
+}
+template <typename T>
+static int launch_scan_flat(const FlatArgs& a, int64_t B, int threads, size_t smem, cudaStream_t st) {
+    auto k = cross_scan_flat_kernel<T>;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
+    k<<<(unsigned)(B * a.blocks), threads, smem, st>>>(a);
+    count_launch();
+    return check_launch();
+}
+template <typename T>
+static int launch_merge_flat(const FlatArgs& a, int64_t B, int scans, int threads, size_t smem, cudaStream_t st) {
+    auto k = cross_merge_flat_kernel<T>;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
+    k<<<(unsigned)(B * a.blocks), threads, smem, st>>>(a, scans);
+    count_launch();
+    return check_launch();
+}
+
 static int fill_args(const ss2d_cross_params* p, CrossArgs& a) {
     if (!p) return SS2D_EINVAL_NULL;
     if (!p->in || !p->out) return SS2D_EINVAL_NULL;
@@ -446,8 +482,13 @@ int cross_scan(const ss2d_cross_params* p, cudaStream_t st) {
     const bool pairs = p->dtype != SS2D_F32 && p->H % 2 == 0 && p->W % 2 == 0 && aligned_to(p->in, 4) && aligned_to(p->out, 4);
     if (!(pairs && p->H >= 48 && p->W >= 48)) {
         PlaneArgs pa; int pv; size_t smem;
-        if (p->dtype == SS2D_F32) { if (plan_plane<float>(p, 1, pa, pv, smem)) return scan_plane_v<float>(pa, pv, smem, st); }
-        else if (plan_plane<uint16_t>(p, 1, pa, pv, smem)) return scan_plane_v<uint16_t>(pa, pv, smem, st);
+        const bool f32 = p->dtype == SS2D_F32, plane = f32 ? plan_plane<float>(p, 1, pa, pv, smem) : plan_plane<uint16_t>(p, 1, pa, pv, smem);
+        if (!plane || pv < 2) {      // with pairs the plane kernel is the faster one (57 x 58 maps: 15 against 18 us)
+            FlatArgs fa; int threads; size_t fs;
+            if (plan_flat(p, f32 ? 4 : 2, 1, fa, threads, fs) && (plane || !f32))
+                return f32 ? launch_scan_flat<float>(fa, p->B, threads, fs, st) : launch_scan_flat<uint16_t>(fa, p->B, threads, fs, st);
+        }
+        if (plane) return f32 ? scan_plane_v<float>(pa, pv, smem, st) : scan_plane_v<uint16_t>(pa, pv, smem, st);
     }
     if (pairs) {
         CrossArgs q = a;
@@ -471,9 +512,19 @@ int cross_merge(const ss2d_cross_params* p, cudaStream_t st) {
     if (rc != SS2D_OK) return rc;
     {
         PlaneArgs pa; int pv; size_t smem;
-        if (p->dtype == SS2D_F32) { if (plan_plane<float>(p, 2, pa, pv, smem)) return merge_plane_v<float>(pa, p->scans, pv, smem, st); }
-        else if (p->dtype == SS2D_BF16) { if (plan_plane<__nv_bfloat16>(p, 2, pa, pv, smem)) return merge_plane_v<__nv_bfloat16>(pa, p->scans, pv, smem, st); }
-        else if (plan_plane<__half>(p, 2, pa, pv, smem)) return merge_plane_v<__half>(pa, p->scans, pv, smem, st);
+        const bool f32 = p->dtype == SS2D_F32, bf = p->dtype == SS2D_BF16;
+        const bool plane = f32 ? plan_plane<float>(p, 2, pa, pv, smem) : plan_plane<__half>(p, 2, pa, pv, smem);
+        if (!plane || pv < 4) {
+            FlatArgs fa; int threads; size_t fs;
+            if (plan_flat(p, f32 ? 4 : 2, 2, fa, threads, fs) && (plane || !f32))
+                return f32 ? launch_merge_flat<float>(fa, p->B, p->scans, threads, fs, st)
+                     : bf  ? launch_merge_flat<__nv_bfloat16>(fa, p->B, p->scans, threads, fs, st)
+                           : launch_merge_flat<__half>(fa, p->B, p->scans, threads, fs, st);
+        }
+        if (plane)
+            return f32 ? merge_plane_v<float>(pa, p->scans, pv, smem, st)
+                 : bf  ? merge_plane_v<__nv_bfloat16>(pa, p->scans, pv, smem, st)
+                       : merge_plane_v<__half>(pa, p->scans, pv, smem, st);
     }
     const dim3 blk(kTile, kMergeRows);
     if (p->dtype == SS2D_F32) cross_merge_kernel<float><<<(unsigned)a.n_tiles, blk, 0, st>>>(a, p->scans);
