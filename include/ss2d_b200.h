@@ -119,7 +119,23 @@ typedef struct ss2d_scan_bwd_params {
     int64_t checkpoint_every;           /* their spacing.  0 = 128, and the kernels and the workspace size that go with it.  Callers
                                            with checkpoints at ss2d_selective_scan_checkpoint_every(), or none, give that
                                            value here and get the faster kernels for dstate <= 16 */
+    int64_t bc_out_group_stride;        /* elements between the (batch, group) blocks of dB and dC; 0 = dense (dstate * seqlen) */
 } ss2d_scan_bwd_params;
+
+/* Backward of the channel LayerNorm of ss2d_layer_norm_cf (no add): from y fp32 (B, D, L) and the gradient g (B, D, L) of the
+ * result, dy fp32 (B, D, L) and dweight, dbias (D) fp32; all dense.  workspace: ss2d_layer_norm_cf_bwd_workspace_bytes().
+ * No atomics: repeated calls give bit-identical results. */
+typedef struct ss2d_norm_bwd_params {
+    const void *y, *g, *weight;
+    void *dy, *dweight, *dbias;
+    int64_t B, D, L;
+    int32_t g_dtype;
+    float eps;
+    void *workspace;
+    int64_t workspace_bytes;
+} ss2d_norm_bwd_params;
+int64_t ss2d_layer_norm_cf_bwd_workspace_bytes(const ss2d_norm_bwd_params *p);
+int ss2d_layer_norm_cf_bwd(const ss2d_norm_bwd_params *p, void *cuda_stream);
 
 int64_t ss2d_selective_scan_bwd_workspace_bytes(const ss2d_scan_bwd_params *p);   /* < 0: invalid or unsupported arguments */
 int ss2d_selective_scan_bwd(const ss2d_scan_bwd_params *p, void *cuda_stream);
@@ -140,10 +156,16 @@ typedef struct ss2d_cross_params {
     int32_t dtype;
     int32_t scans;
     int64_t B, C, H, W;
+    int64_t route_stride;      /* elements between the rows of the routes tensor; 0 or H * W = dense.  A larger multiple of 8 pads
+                                  them (scan writes the padding as zero, merge skips it), so that rows of any length start
+                                  aligned: ss2d_cross_padding_supported() says whether every such call takes the map */
 } ss2d_cross_params;
 
 int ss2d_cross_scan(const ss2d_cross_params *p, void *cuda_stream);
 int ss2d_cross_merge(const ss2d_cross_params *p, void *cuda_stream);
+/* rows (B, 4, C, H * W), route_stride apart: row (k, c) from pixel order into the order of route k, or back.  in != out. */
+int ss2d_cross_rows(const ss2d_cross_params *p, int back, void *cuda_stream);
+int ss2d_cross_padding_supported(const ss2d_cross_params *p);    /* 1 / 0; of scan, merge and rows, any dtype */
 
 /* ------------------------------------------------------------------------------------
  * CrossScan / CrossMerge with the reference's layout flags (cross_scan_fwd / cross_merge_fwd / their one-by-one

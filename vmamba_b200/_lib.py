@@ -41,12 +41,12 @@ class ScanBwdParams(ctypes.Structure):
                                     "dout_batch_stride", "dout_dim_stride",
                                     "B_batch_stride", "B_group_stride", "B_state_stride",
                                     "C_batch_stride", "C_group_stride", "C_state_stride")] + \
-               [("checkpoints", _vp), ("checkpoint_every", _i64)]
+               [("checkpoints", _vp), ("checkpoint_every", _i64), ("bc_out_group_stride", _i64)]
 
 
 class CrossParams(ctypes.Structure):
     _fields_ = [("in_", _vp), ("out", _vp), ("dtype", _i32), ("scans", _i32),
-                ("B", _i64), ("C", _i64), ("H", _i64), ("W", _i64)]
+                ("B", _i64), ("C", _i64), ("H", _i64), ("W", _i64), ("route_stride", _i64)]
 
 
 class CrossExParams(ctypes.Structure):

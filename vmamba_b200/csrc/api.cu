@@ -15,6 +15,10 @@ int selective_scan_bwd(const ss2d_scan_bwd_params* p, cudaStream_t st);
 long long selective_scan_bwd_workspace_bytes(const ss2d_scan_bwd_params* p);
 int cross_scan(const ss2d_cross_params* p, cudaStream_t st);
 int cross_merge(const ss2d_cross_params* p, cudaStream_t st);
+int cross_rows(const ss2d_cross_params* p, int back, cudaStream_t st);
+int cross_padding_supported(const ss2d_cross_params* p);
+long long layer_norm_cf_bwd_workspace_bytes(const ss2d_norm_bwd_params* p);
+int layer_norm_cf_bwd(const ss2d_norm_bwd_params* p, cudaStream_t st);
 int cross_scan_ex(const ss2d_cross_ex_params* p, cudaStream_t st);
 int cross_merge_ex(const ss2d_cross_ex_params* p, cudaStream_t st);
 int layer_norm_cf(const ss2d_norm_params* p, cudaStream_t st);
@@ -97,6 +101,18 @@ int ss2d_cross_merge(const ss2d_cross_params* p, void* stream) {
     ss2d::Range nvtx_("ss2d_cross_merge");
     if (p) SS2D_CHECK_PTRS(p->in, p->out);
     return ss2d::cross_merge(p, (cudaStream_t)stream);
+}
+int ss2d_cross_rows(const ss2d_cross_params* p, int back, void* stream) {
+    ss2d::Range nvtx_("ss2d_cross_rows");
+    if (p) SS2D_CHECK_PTRS(p->in, p->out);
+    return ss2d::cross_rows(p, back, (cudaStream_t)stream);
+}
+int ss2d_cross_padding_supported(const ss2d_cross_params* p) { return ss2d::cross_padding_supported(p); }
+int64_t ss2d_layer_norm_cf_bwd_workspace_bytes(const ss2d_norm_bwd_params* p) { return ss2d::layer_norm_cf_bwd_workspace_bytes(p); }
+int ss2d_layer_norm_cf_bwd(const ss2d_norm_bwd_params* p, void* stream) {
+    ss2d::Range nvtx_("ss2d_layer_norm_cf_bwd");
+    if (p) SS2D_CHECK_PTRS(p->y, p->g, p->weight, p->dy, p->dweight, p->dbias, p->workspace);
+    return ss2d::layer_norm_cf_bwd(p, (cudaStream_t)stream);
 }
 int ss2d_cross_scan_ex(const ss2d_cross_ex_params* p, void* stream) {
     ss2d::Range nvtx_("ss2d_cross_scan_ex");

@@ -7,6 +7,9 @@
 // Bound by that index arithmetic (flat runs with the two divisions for every element, and lines of a group of lanes, were
 // slower).  37 x 53 maps, 8 x 192 planes, bf16: scan 32 -> 21 us, merge 48 -> 22 us; fp32 32 -> 22, 49 -> 26 us against the
 // single-element form of the plane kernels.
+// The rows of the routes may be padded to a multiple of eight elements (`stride` > L), which gives the kernels behind them
+// aligned rows whatever L is: the run is then taken over the padded rows, whose words never cross planes, and the
+// padding is written as zero.
 #pragma once
 #include "common.cuh"
 
@@ -14,7 +17,7 @@ namespace ss2d {
 
 constexpr int kWordBytes = 8;
 struct Walk {            // constants of a walk over the lines of shared planes
-    int len, lines, plane;         // elements per line, lines per plane, elements per plane
+    int len, lines, plane;         // elements per line, lines per plane, elements of the run per plane (with padding)
     unsigned magic_len, magic_plane;
     int o0, line, step, next;      // place of element j of line i of plane p: o0 + i * line + j * step + p * next
 };
@@ -29,7 +32,7 @@ __device__ __forceinline__ void advance(const Walk& w, Place& q) {
     if (++q.j == w.len) {
         q.j = 0;
         q.at += w.line - w.len * w.step;
-        if (++q.i == w.lines) { q.i = 0; q.at += w.next - w.lines * w.line; }
+        if (++q.i == w.lines && w.len * w.lines == w.plane) { q.i = 0; q.at += w.next - w.lines * w.line; }
     }
 }
 template <typename T> union Word { T e[kWordBytes / sizeof(T)]; uint2 w; };
@@ -68,7 +71,7 @@ template <typename T> __device__ __forceinline__ void run_in(const Walk& w, cons
 #pragma unroll
             for (int e = 0; e < E; ++e)
                 if (f + e >= 0) {
-                    if (f + e < n) sm[q.at] = v[i].e[e];
+                    if (f + e < n && q.i < w.lines) sm[q.at] = v[i].e[e];
                     advance(w, q);
                 }
         }
@@ -82,7 +85,7 @@ template <typename T> __device__ __forceinline__ void run_out(const Walk& w, con
 #pragma unroll
         for (int e = 0; e < E; ++e)
             if (f + e >= 0) {
-                if (f + e < n) v.e[e] = sm[q.at];
+                if (f + e < n) v.e[e] = q.i < w.lines ? sm[q.at] : static_cast<T>(0.f);
                 advance(w, q);
             }
         store_word(v, run, f, n);
@@ -94,9 +97,20 @@ struct FlatArgs {
     const void* in;
     void* out;
     int C, H, W, L, PP, blocks;                      // blocks: CTAs per image
+    int stride;                                      // elements between the rows of a route
     FlatRoute route[4];
-    unsigned magic_H, magic_W, magic_L;
+    unsigned magic_H, magic_W, magic_L, magic_S;         // S: stride
 };
+
+// Route k over row-major shared planes of pitch W | 1.
+__device__ __forceinline__ Walk route_walk(const FlatArgs& a, int k) {
+    const FlatRoute m = a.route[k];
+    const int H = a.H, W = a.W, Wp = W | 1, Lp = H * Wp;
+    if (m.col_like)
+        return {H, W, a.stride, a.magic_H, a.magic_S, (m.w_up ? 0 : W - 1) + (m.h_up ? 0 : (H - 1) * Wp), m.w_up ? 1 : -1, m.h_up ? Wp : -Wp, Lp};
+    if (!m.w_up) return {W, H, a.stride, a.magic_W, a.magic_S, (H - 1) * Wp + W - 1, -Wp, -1, Lp};
+    return {W, H, a.stride, a.magic_W, a.magic_S, 0, Wp, 1, Lp};
+}
 
 template <typename T>
 __global__ void __launch_bounds__(512) cross_scan_flat_kernel(const FlatArgs a) {
@@ -104,19 +118,26 @@ __global__ void __launch_bounds__(512) cross_scan_flat_kernel(const FlatArgs a) 
     T* sm = reinterpret_cast<T*>(smraw);             // [PP][H][W | 1]
     const int b = blockIdx.x / a.blocks, c0 = (blockIdx.x - b * a.blocks) * a.PP, np = min(a.PP, a.C - c0);
     const int L = a.L, H = a.H, W = a.W, Wp = W | 1, Lp = H * Wp, n = np * L;
-    const Walk by_row = {W, H, L, a.magic_W, a.magic_L, 0, Wp, 1, Lp};
-    run_in<T>(by_row, (const T*)a.in + ((long long)b * a.C + c0) * L, n, sm);
+    run_in<T>({W, H, L, a.magic_W, a.magic_L, 0, Wp, 1, Lp}, (const T*)a.in + ((long long)b * a.C + c0) * L, n, sm);
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const FlatRoute m = a.route[k];
-        Walk w = by_row;
-        if (m.col_like)
-            w = {H, W, L, a.magic_H, a.magic_L, (m.w_up ? 0 : W - 1) + (m.h_up ? 0 : (H - 1) * Wp), m.w_up ? 1 : -1, m.h_up ? Wp : -Wp, Lp};
-        else if (!m.w_up)
-            w = {W, H, L, a.magic_W, a.magic_L, (H - 1) * Wp + W - 1, -Wp, -1, Lp};
-        run_out<T>(w, sm, (T*)a.out + ((long long)(b * 4 + k) * a.C + c0) * L, n);
-    }
+    for (int k = 0; k < 4; ++k)
+        run_out<T>(route_walk(a, k), sm, (T*)a.out + ((long long)(b * 4 + k) * a.C + c0) * a.stride, np * a.stride);
+}
+
+// Rows (B, 4, C, H x W), `stride` elements apart: row (k, c) is brought from pixel order into the order of route k (or back,
+// with `back`).  The CrossScan of rows that each belong to one route.
+template <typename T>
+__global__ void __launch_bounds__(512) cross_rows_kernel(const FlatArgs a, const int back) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    T* sm = reinterpret_cast<T*>(smraw);             // [PP][H][W | 1]
+    const int bk = blockIdx.x / a.blocks, k = bk & 3, c0 = (blockIdx.x - bk * a.blocks) * a.PP, np = min(a.PP, a.C - c0);
+    const int H = a.H, W = a.W, Wp = W | 1, n = np * a.stride;
+    const long long at = ((long long)bk * a.C + c0) * a.stride;
+    const Walk by_row = {W, H, a.stride, a.magic_W, a.magic_S, 0, Wp, 1, H * Wp}, by_route = route_walk(a, k);
+    run_in<T>(back ? by_route : by_row, (const T*)a.in + at, n, sm);
+    __syncthreads();
+    run_out<T>(back ? by_row : by_route, sm, (T*)a.out + at, n);
 }
 
 // Sum of four routes in the association order of the reference's additions, rounded to the storage type after each.
@@ -134,7 +155,7 @@ __global__ void __launch_bounds__(512) cross_merge_flat_kernel(const FlatArgs a,
     T* sm = reinterpret_cast<T*>(smraw);             // [column-like route][PP][W][H | 1]
     constexpr int E = kWordBytes / (int)sizeof(T);
     const int b = blockIdx.x / a.blocks, c0 = (blockIdx.x - b * a.blocks) * a.PP, np = min(a.PP, a.C - c0);
-    const int L = a.L, H = a.H, W = a.W, Hp = H | 1, Lp = W * Hp, n = np * L;
+    const int L = a.L, S = a.stride, H = a.H, W = a.W, Hp = H | 1, Lp = W * Hp, n = np * L;
     const T* in[4];
     bool col[4], fwd[4], same[4];
     Walk w[4];                                       // of the column-like routes, in the order of the result
@@ -143,13 +164,13 @@ __global__ void __launch_bounds__(512) cross_merge_flat_kernel(const FlatArgs a,
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const FlatRoute m = a.route[k];
-        in[k] = (const T*)a.in + ((long long)(b * 4 + k) * a.C + c0) * L;
+        in[k] = (const T*)a.in + ((long long)(b * 4 + k) * a.C + c0) * S;
         col[k] = m.col_like != 0;
         fwd[k] = m.w_up != 0;
-        same[k] = phase_of(in[k]) == phase_of(out);
+        same[k] = S == L && phase_of(in[k]) == phase_of(out);
         w[k] = {W, H, L, a.magic_W, a.magic_L, 0, 0, 0, 0};
         if (!col[k]) continue;
-        run_in<T>({H, W, L, a.magic_H, a.magic_L, 0, Hp, 1, Lp}, in[k], n, sm + slots * a.PP * Lp);
+        run_in<T>({H, W, S, a.magic_H, a.magic_S, 0, Hp, 1, Lp}, in[k], np * S, sm + slots * a.PP * Lp);
         w[k] = {W, H, L, a.magic_W, a.magic_L, slots * a.PP * Lp + (m.w_up ? 0 : (W - 1) * Hp) + (m.h_up ? 0 : H - 1), m.h_up ? 1 : -1,
                 m.w_up ? Hp : -Hp, Lp};
         ++slots;
@@ -171,18 +192,23 @@ __global__ void __launch_bounds__(512) cross_merge_flat_kernel(const FlatArgs a,
             } else if (fwd[k]) {
                 if (same[k]) load_word(v[k], in[k], f, n);
                 else {
+                    int at = p * S + l, gone = l;
 #pragma unroll
                     for (int e = 0; e < E; ++e)
-                        if (f + e >= 0 && f + e < n) v[k].e[e] = __ldg(in[k] + f + e);
+                        if (f + e >= 0) {
+                            if (f + e < n) v[k].e[e] = __ldg(in[k] + at);
+                            ++at;
+                            if (++gone == L) { gone = 0; at += S - L; }
+                        }
                 }
             } else {
-                int at = p * L + L - 1 - l, gone = l;
+                int at = p * S + L - 1 - l, gone = l;
 #pragma unroll
                 for (int e = 0; e < E; ++e)
                     if (f + e >= 0) {
                         if (f + e < n) v[k].e[e] = __ldg(in[k] + at);
                         --at;
-                        if (++gone == L) { gone = 0; at += 2 * L; }
+                        if (++gone == L) { gone = 0; at += S + L; }
                     }
             }
         }

@@ -421,18 +421,18 @@ static int merge_plane_v(const PlaneArgs& a, int scans, int pv, size_t smem, cud
 
 // Whether the flat kernels take the planes, and how.  `copies`: shared planes per plane (1 scan, 2 merge).
 static bool plan_flat(const ss2d_cross_params* p, size_t esize, int copies, FlatArgs& a, int& threads, size_t& smem) {
-    const long long L = p->H * p->W, Lp = copies == 1 ? p->H * (p->W | 1) : p->W * (p->H | 1);
-    if (Lp * (long long)esize * copies > 200 * 1024 || L > 65536) return false;      // 65 536: the divisions by multiplication are exact
+    const long long L = p->H * p->W, Lp = copies == 1 ? p->H * (p->W | 1) : p->W * (p->H | 1), S = p->route_stride ? p->route_stride : L;
+    if (Lp * (long long)esize * copies > 200 * 1024 || S > 65536) return false;      // 65 536: the divisions by multiplication are exact
     long long PP = std::min<long long>(std::max<long long>(1, 4096 / L), p->C);
     while (PP > 1 && PP * Lp * (long long)esize * copies > 48 * 1024) --PP;
-    a.in = p->in; a.out = p->out; a.C = (int)p->C; a.H = (int)p->H; a.W = (int)p->W; a.L = (int)L; a.PP = (int)PP;
+    a.in = p->in; a.out = p->out; a.C = (int)p->C; a.H = (int)p->H; a.W = (int)p->W; a.L = (int)L; a.PP = (int)PP; a.stride = (int)S;
     a.blocks = (int)((p->C + PP - 1) / PP);
     for (int k = 0; k < 4; ++k) {
         const RouteMap m = route_map(p->scans, k, p->H, p->W);
         a.route[k] = {m.col_like, m.sh > 0, m.sw > 0};
     }
     auto magic = [](long long d) { return d > 1 ? (unsigned)(((1ULL << 32) + (unsigned long long)d - 1) / (unsigned long long)d) : 0u; };
-    a.magic_H = magic(p->H); a.magic_W = magic(p->W); a.magic_L = magic(L);
+    a.magic_H = magic(p->H); a.magic_W = magic(p->W); a.magic_L = magic(L); a.magic_S = magic(S);
     smem = (size_t)PP * Lp * esize * copies;
     threads = smem > 40 * 1024 ? 512 : 256;
     return p->B * a.blocks <= 0x7fffffffLL;
@@ -454,6 +454,20 @@ static int launch_merge_flat(const FlatArgs& a, int64_t B, int scans, int thread
     return check_launch();
 }
 
+static int launch_rows(const ss2d_cross_params* p, bool back, cudaStream_t st) {
+    FlatArgs a; int threads; size_t smem;
+    const bool f32 = p->dtype == SS2D_F32;
+    if (!plan_flat(p, f32 ? 4 : 2, 1, a, threads, smem) || p->B * 4 * a.blocks > 0x7fffffffLL) return SS2D_ENOTSUP;
+    if (!aligned_to(p->in, 8) || !aligned_to(p->out, 8) || (a.stride != a.L && a.stride % 8 != 0)) return SS2D_EINVAL_ALIGN;
+    const void* k = f32 ? (const void*)cross_rows_kernel<float> : (const void*)cross_rows_kernel<uint16_t>;
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
+    const unsigned grid = (unsigned)(p->B * 4 * a.blocks);
+    if (f32) cross_rows_kernel<float><<<grid, threads, smem, st>>>(a, back);
+    else cross_rows_kernel<uint16_t><<<grid, threads, smem, st>>>(a, back);
+    count_launch();
+    return check_launch();
+}
+
 static int fill_args(const ss2d_cross_params* p, CrossArgs& a) {
     if (!p) return SS2D_EINVAL_NULL;
     if (!p->in || !p->out) return SS2D_EINVAL_NULL;
@@ -463,6 +477,7 @@ static int fill_args(const ss2d_cross_params* p, CrossArgs& a) {
     if (p->H * p->W > 0x3fffffffLL || p->C > 0x7fffffffLL || p->B * p->C > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;   // 32-bit indices inside a plane
     const size_t s = dtype_size(p->dtype);
     if (!aligned_to(p->in, s) || !aligned_to(p->out, s)) return SS2D_EINVAL_ALIGN;
+    if (p->route_stride && p->route_stride < p->H * p->W) return SS2D_EINVAL_STRIDE;
     a.in = p->in; a.out = p->out;
     a.C = p->C; a.H = p->H; a.W = p->W;
     a.tiles_h = (p->H + kTile - 1) / kTile;
@@ -473,10 +488,19 @@ static int fill_args(const ss2d_cross_params* p, CrossArgs& a) {
     return SS2D_OK;
 }
 
+// Routes with padded rows: the flat kernels alone take them.
+static bool padded(const ss2d_cross_params* p) { return p->route_stride && p->route_stride != p->H * p->W; }
+
 int cross_scan(const ss2d_cross_params* p, cudaStream_t st) {
     CrossArgs a;
     const int rc = fill_args(p, a);
     if (rc != SS2D_OK) return rc;
+    if (padded(p)) {
+        FlatArgs fa; int threads; size_t fs;
+        if (p->route_stride % 8 != 0 || !aligned_to(p->out, 8)) return SS2D_EINVAL_ALIGN;
+        if (!plan_flat(p, dtype_size(p->dtype), 1, fa, threads, fs)) return SS2D_ENOTSUP;
+        return p->dtype == SS2D_F32 ? launch_scan_flat<float>(fa, p->B, threads, fs, st) : launch_scan_flat<uint16_t>(fa, p->B, threads, fs, st);
+    }
     // 16-bit maps with even sides: the pair kernel for every map that fills most of a 64 x 64 tile (0.87 of the copy
     // bandwidth on 256 x 256 planes against 0.60 for the whole-plane kernel on 128 x 128 ones)
     const bool pairs = p->dtype != SS2D_F32 && p->H % 2 == 0 && p->W % 2 == 0 && aligned_to(p->in, 4) && aligned_to(p->out, 4);
@@ -506,10 +530,29 @@ int cross_scan(const ss2d_cross_params* p, cudaStream_t st) {
     return check_launch();
 }
 
+int cross_rows(const ss2d_cross_params* p, int back, cudaStream_t st) {
+    CrossArgs a;
+    const int rc = fill_args(p, a);
+    return rc != SS2D_OK ? rc : launch_rows(p, back != 0, st);
+}
+
+int cross_padding_supported(const ss2d_cross_params* p) {
+    FlatArgs a; int threads; size_t smem;
+    return p && dtype_ok(p->dtype) && p->H > 0 && p->W > 0 && p->C > 0 && plan_flat(p, 4, 2, a, threads, smem) ? 1 : 0;
+}
+
 int cross_merge(const ss2d_cross_params* p, cudaStream_t st) {
     CrossArgs a;
     const int rc = fill_args(p, a);
     if (rc != SS2D_OK) return rc;
+    if (padded(p)) {
+        FlatArgs fa; int threads; size_t fs;
+        if (p->route_stride % 8 != 0 || !aligned_to(p->in, 8)) return SS2D_EINVAL_ALIGN;
+        if (!plan_flat(p, dtype_size(p->dtype), 2, fa, threads, fs)) return SS2D_ENOTSUP;
+        return p->dtype == SS2D_F32    ? launch_merge_flat<float>(fa, p->B, p->scans, threads, fs, st)
+               : p->dtype == SS2D_BF16 ? launch_merge_flat<__nv_bfloat16>(fa, p->B, p->scans, threads, fs, st)
+                                       : launch_merge_flat<__half>(fa, p->B, p->scans, threads, fs, st);
+    }
     {
         PlaneArgs pa; int pv; size_t smem;
         const bool f32 = p->dtype == SS2D_F32, bf = p->dtype == SS2D_BF16;

@@ -50,6 +50,9 @@ inline Tensor bytes(int64_t n, const Tensor& like) { return at::empty({n}, like.
 std::pair<Tensor, Tensor> scan_fwd(Tensor u, Tensor delta, Tensor A, Tensor B, Tensor C, Tensor D, Tensor bias, bool softplus, bool out_float,
                                    int64_t every, Tensor out);
 std::vector<Tensor> scan_bwd(Tensor u, Tensor delta, Tensor A, Tensor B, Tensor C, Tensor D, Tensor bias, Tensor dout, bool softplus, Tensor ckpt);
+// the same with dB and dC (B, K, N, L) written into views of a larger tensor whose (image, group) blocks are evenly spaced
+std::vector<Tensor> scan_bwd_into(Tensor u, Tensor delta, Tensor A, Tensor B, Tensor C, Tensor D, Tensor bias, Tensor dout, bool softplus, Tensor ckpt,
+                                  Tensor dB, Tensor dC);
 Tensor cross_scan(const Tensor& x, int64_t scans);       // (B, C, H, W) -> (B, 4, C, L)
 Tensor cross_merge(const Tensor& ys, int64_t scans);     // (B, 4, C, H, W) -> (B, C, L)
 int64_t scan_ratio(const Tensor& u, const Tensor& delta);

@@ -1,0 +1,157 @@
+// The differentiable SS2D core (fused.ss2d_core_autograd) as one autograd node.
+//
+// Forward: CrossScan of x; x_proj ONCE on the un-scanned map (a 1 x 1 projection commutes with the permutation: a quarter of
+// the reads), its rows permuted into route order; dt_projs; selective scan; CrossMerge; LayerNorm.  Backward: LayerNorm,
+// the scan of its gradient, the selective-scan gradients (dB, dC written in place into the rows of x_dbl's gradient), the
+// four small contractions, CrossMerge.  Rows are padded to a multiple of eight elements where the map's pixel count is
+// none, so that the scan and the library's GEMMs see aligned rows whatever H and W are.
+#include "host_common.h"
+
+namespace host {
+
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+static Tensor cross(const Tensor& in, Tensor out, int64_t B, int64_t C, int64_t H, int64_t W, int64_t stride, int op) {
+    ss2d_cross_params p = {in.data_ptr(), out.data_ptr(), dtype_code(in), 0, B, C, H, W, stride};
+    void* st = stream_of(in);
+    if (op == 0) check(ss2d_cross_scan(&p, st), "ss2d_cross_scan");
+    else if (op == 1) check(ss2d_cross_merge(&p, st), "ss2d_cross_merge");
+    else check(ss2d_cross_rows(&p, op == 3, st), "ss2d_cross_rows");
+    return out;
+}
+
+// Row stride of the core's route tensors: H * W, or that rounded up to a multiple of eight where the kernels take padded rows.
+static int64_t padded_row(int64_t B, int64_t C, int64_t H, int64_t W) {
+    const int64_t L = H * W, Lp = (L + 7) / 8 * 8;
+    if (Lp == L) return L;
+    ss2d_cross_params p = {nullptr, nullptr, SS2D_F32, 0, B, C, H, W, Lp};
+    return ss2d_cross_padding_supported(&p) ? Lp : L;
+}
+// cross_rows keeps whole planes in shared memory: 200 KB
+static bool rows_fit(int64_t H, int64_t W, int64_t esize) { return H * (W | 1) * esize <= 200 * 1024 && H * W <= 65536; }
+
+// (b, k) weights of a batched product: the four routes' matrices, repeated over the images
+static Tensor per_image(const Tensor& w, int64_t B) {
+    return w.unsqueeze(0).expand({B, 4, w.size(1), w.size(2)}).reshape({B * 4, w.size(1), w.size(2)});
+}
+
+// sum over the images of a . b^T (rows of equal length): per-image products accumulated and summed in fp32
+static Tensor row_products(const Tensor& a, const Tensor& b, int64_t groups) {
+    const Tensor bt = b.transpose(1, 2);
+    const Tensor p = a.scalar_type() == at::kFloat ? at::bmm(a, bt) : at::bmm(a, bt, at::kFloat);
+    return p.view({-1, groups, p.size(1), p.size(2)}).sum(0);
+}
+
+struct CoreNode : public torch::autograd::Function<CoreNode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x_, const Tensor& x_proj, const Tensor& dt_projs, const Tensor& dt_bias,
+                          const Tensor& A_logs, const Tensor& Ds, const Tensor& ln_w, const Tensor& ln_b, int64_t N, int64_t R, double eps) {
+        const Tensor x = x_.contiguous();
+        const c10::cuda::OptionalCUDAGuard guard(x.device());
+        const int64_t B = x.size(0), D = x.size(1), H = x.size(2), W = x.size(3), L = H * W, C = R + 2 * N, S = padded_row(B, D, H, W);
+        const auto of = x.options();
+        const Tensor wx = x_proj.reshape({4 * C, D}).to(x.scalar_type()), wdt = dt_projs.reshape({4, D, R}).to(x.scalar_type()).contiguous();
+        const Tensor A = A_logs.to(at::kFloat).exp().neg().contiguous(), bias = f32(dt_bias.reshape(-1)), Dp = f32(Ds.reshape(-1));
+        const Tensor xs = cross(x, at::empty({B, 4, D, S}, of), B, D, H, W, S, 0);
+        Tensor xd = at::empty({B, 4, C, S}, of);
+        if (rows_fit(H, W, x.element_size())) {
+            const Tensor nat = at::bmm(wx.unsqueeze(0).expand({B, 4 * C, D}), S == L ? x.view({B, D, L}) : xs.select(1, 0));
+            cross(nat, xd, B, C, H, W, S, 2);
+        } else {
+            Tensor out = xd.view({B * 4, C, S});
+            at::bmm_out(out, per_image(wx.view({4, C, D}), B), xs.view({B * 4, D, S}));
+        }
+        Tensor dts = at::empty({B, 4, D, S}, of);
+        const Tensor bc = expand(xd, wdt, dts, B, D, R, N, S);
+        auto [ys, states] = scan_fwd(xs.view({B, 4 * D, S}), dts.view({B, 4 * D, S}), A, bc.narrow(2, 0, N), bc.narrow(2, N, N), Dp, bias, true, true,
+                                     ss2d_selective_scan_checkpoint_every(N, 1), Tensor());
+        const Tensor y = cross(ys, at::empty({B, D, L}, of.dtype(at::kFloat)), B, D, H, W, S, 1);
+        Tensor out = at::empty({B, D, H, W}, of);
+        const Tensor lw = f32(ln_w), lb = f32(ln_b);
+        ss2d_norm_params n = {};
+        n.in = y.data_ptr(); n.weight = lw.data_ptr(); n.bias = lb.data_ptr(); n.out = out.data_ptr();
+        n.B = B; n.D = D; n.L = L; n.io_dtype = dtype_code(x); n.eps = (float)eps;
+        check(ss2d_layer_norm_cf(&n, stream_of(x)), "ss2d_layer_norm_cf");
+        ctx->save_for_backward({x_, x_proj, dt_projs, dt_bias, A_logs, Ds, ln_w, ln_b});
+        ctx->saved_data["t"] = std::vector<Tensor>{xs, xd, dts, bc, states, y, wx, wdt, A};
+        ctx->saved_data["n"] = std::vector<int64_t>{B, D, H, W, N, R, S};
+        ctx->saved_data["eps"] = eps;
+        return out;
+    }
+
+    // step sizes (B, 4, D, S) of the low-rank rows, and the B / C rows as a tensor of their own
+    static Tensor expand(const Tensor& xd, const Tensor& wdt, Tensor dts, int64_t B, int64_t D, int64_t R, int64_t N, int64_t S) {
+        const int64_t C = R + 2 * N;
+        Tensor bc = at::empty({B, 4, 2 * N, S}, xd.options());
+        ss2d_expand_params p = {};
+        p.x_dbl = xd.data_ptr(); p.dt_weight = wdt.data_ptr();
+        p.x_dbl_batch_stride = 4 * C * S; p.x_dbl_route_stride = C * S; p.x_dbl_row_stride = S;
+        const int64_t e = xd.element_size();
+        for (int64_t k = 0; k < 4; ++k) {
+            p.delta[k] = (char*)dts.data_ptr() + k * D * S * e; p.delta_batch_stride[k] = 4 * D * S; p.delta_channel_stride[k] = S;
+            p.bc[k] = (char*)bc.data_ptr() + k * 2 * N * S * e; p.bc_batch_stride[k] = 8 * N * S; p.bc_row_stride[k] = S;
+        }
+        p.B = B; p.D = D; p.R = R; p.N = N; p.H = 1; p.W = S;      // the rows are in route order already: one long row each
+        p.act_dtype = dtype_code(xd);
+        check(ss2d_route_expand(&p, stream_of(xd)), "ss2d_route_expand");
+        return bc;
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const auto in = ctx->get_saved_variables();
+        const auto t = ctx->saved_data["t"].toTensorVector();
+        const auto sz = ctx->saved_data["n"].toIntVector();
+        const Tensor &xs = t[0], &xd = t[1], &dts = t[2], &bc = t[3], &states = t[4], &y = t[5], &wx = t[6], &wdt = t[7], &A = t[8];
+        const int64_t B = sz[0], D = sz[1], H = sz[2], W = sz[3], N = sz[4], R = sz[5], S = sz[6], L = H * W, C = R + 2 * N;
+        const c10::cuda::OptionalCUDAGuard guard(xs.device());
+        const auto of = xs.options(), of32 = of.dtype(at::kFloat);
+        const Tensor g = grads[0].contiguous(), lw = f32(in[6]);
+        Tensor dy = at::empty({B, D, L}, of32), dlw = at::empty({D}, of32), dlb = at::empty({D}, of32);
+        {
+            ss2d_norm_bwd_params p = {};
+            p.y = y.data_ptr(); p.g = g.data_ptr(); p.weight = lw.data_ptr(); p.dy = dy.data_ptr(); p.dweight = dlw.data_ptr(); p.dbias = dlb.data_ptr();
+            p.B = B; p.D = D; p.L = L; p.g_dtype = dtype_code(g); p.eps = (float)ctx->saved_data["eps"].toDouble();
+            const Tensor ws = bytes(ss2d_layer_norm_cf_bwd_workspace_bytes(&p), xs);
+            p.workspace = ws.data_ptr(); p.workspace_bytes = ws.numel();
+            check(ss2d_layer_norm_cf_bwd(&p, stream_of(xs)), "ss2d_layer_norm_cf_bwd");
+        }
+        Tensor dys = cross(dy, at::empty({B, 4, D, S}, of32), B, D, H, W, S, 0);
+        dy = Tensor();
+        // gradient of x_dbl in route order: rows 0 .. R from the step sizes, the others are dB and dC
+        Tensor dxd = at::empty({B, 4, C, S}, of);
+        const Tensor bias = f32(in[3].reshape(-1)), Dp = f32(in[5].reshape(-1));
+        auto r = scan_bwd_into(xs.view({B, 4 * D, S}), dts.view({B, 4 * D, S}), A, bc.narrow(2, 0, N), bc.narrow(2, N, N), Dp, bias,
+                               dys.view({B, 4 * D, S}), true, states, dxd.narrow(2, R, N), dxd.narrow(2, R + N, N));
+        dys = Tensor();
+        Tensor du = r[0].view({B * 4, D, S});
+        const Tensor dd = r[1].view({B * 4, D, S});
+        Tensor low = dxd.view({B * 4, C, S}).narrow(1, 0, R);
+        at::bmm_out(low, per_image(wdt.transpose(1, 2), B), dd);
+        const Tensor dwdt = row_products(dd, xd.view({B * 4, C, S}).narrow(1, 0, R), 4);        // (4, D, R)
+        Tensor dwx;
+        if (rows_fit(H, W, xs.element_size())) {
+            const Tensor nat = cross(dxd, at::empty({B, 4 * C, S}, of), B, C, H, W, S, 3), x0 = xs.select(1, 0);
+            dwx = row_products(nat, x0, 1).view({4 * C, D});
+            Tensor du0 = du.view({B, 4, D, S}).select(1, 0);                                    // route 0 is the pixel order
+            at::baddbmm_out(du0, du0, wx.t().unsqueeze(0).expand({B, D, 4 * C}), nat);
+        } else {
+            dwx = row_products(dxd.view({B * 4, C, S}), xs.view({B * 4, D, S}), 4).view({4 * C, D});
+            at::baddbmm_out(du, du, per_image(wx.view({4, C, D}).transpose(1, 2), B), dxd.view({B * 4, C, S}));
+        }
+        const Tensor dx = cross(du, at::empty({B, D, H, W}, of), B, D, H, W, S, 1);
+        auto as = [](const Tensor& v, const Tensor& like) { return v.reshape(like.sizes()).to(like.scalar_type()); };
+        return {dx, as(dwx, in[1]), as(dwdt, in[2]), as(r[6], in[3]), as(r[2].mul(A), in[4]), as(r[5], in[5]), as(dlw, in[6]), as(dlb, in[7]),
+                Tensor(), Tensor(), Tensor()};
+    }
+};
+
+void bind_core(pybind11::module_& m) {
+    namespace py = pybind11;
+    m.def("ss2d_core_autograd",
+          [](const Tensor& x, const Tensor& x_proj, const Tensor& dt_projs, const Tensor& dt_bias, const Tensor& A_logs, const Tensor& Ds,
+             const Tensor& ln_w, const Tensor& ln_b, int64_t N, int64_t R, double eps) {
+              return CoreNode::apply(x, x_proj, dt_projs, dt_bias, A_logs, Ds, ln_w, ln_b, N, R, eps);
+          }, py::call_guard<py::gil_scoped_release>());
+}
+
+}  // namespace host

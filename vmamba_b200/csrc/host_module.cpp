@@ -3,6 +3,7 @@
 
 namespace host {
 void bind_ops(pybind11::module_& m);
+void bind_core(pybind11::module_& m);
 }  // namespace host
 
 PYBIND11_MODULE(_host, m) {
@@ -17,4 +18,5 @@ PYBIND11_MODULE(_host, m) {
         }
     });
     host::bind_ops(m);
+    host::bind_core(m);
 }

@@ -55,6 +55,11 @@ std::pair<Tensor, Tensor> scan_fwd(Tensor u, Tensor delta, Tensor A, Tensor B, T
 }
 
 std::vector<Tensor> scan_bwd(Tensor u, Tensor delta, Tensor A, Tensor B, Tensor C, Tensor D, Tensor bias, Tensor dout, bool softplus, Tensor ckpt) {
+    return scan_bwd_into(u, delta, A, B, C, D, bias, dout, softplus, ckpt, Tensor(), Tensor());
+}
+
+std::vector<Tensor> scan_bwd_into(Tensor u, Tensor delta, Tensor A, Tensor B, Tensor C, Tensor D, Tensor bias, Tensor dout, bool softplus, Tensor ckpt,
+                                  Tensor dB, Tensor dC) {
     require_cuda({&u, &delta, &A, &B, &C, &D, &bias, &dout});
     TORCH_CHECK(dout.sizes() == u.sizes(), "dout must have the shape of u, got ", dout.sizes());
     TORCH_CHECK(dout.scalar_type() == at::kFloat || dout.scalar_type() == u.scalar_type(), "dout must be fp32 or of u's dtype");
@@ -63,7 +68,7 @@ std::vector<Tensor> scan_bwd(Tensor u, Tensor delta, Tensor A, Tensor B, Tensor 
     A = f32(A); D = f32(D); bias = f32(bias);
     const auto of = u.options(), of32 = of.dtype(at::kFloat);
     Tensor du = at::empty({batch, dim, L}, of), ddelta = at::empty({batch, dim, L}, of), dA = at::empty({dim, N}, of32);
-    Tensor dB = at::empty({batch, K, N, L}, of), dC = at::empty({batch, K, N, L}, of);
+    if (!dB.defined()) { dB = at::empty({batch, K, N, L}, of); dC = at::empty({batch, K, N, L}, of); }
     Tensor dD = D.defined() ? at::empty({dim}, of32) : Tensor(), dbias = bias.defined() ? at::empty({dim}, of32) : Tensor();
     ss2d_scan_bwd_params p = {};
     p.u = u.data_ptr(); p.delta = delta.data_ptr(); p.A = A.data_ptr(); p.B = B.data_ptr(); p.C = C.data_ptr(); p.D = ptr(D);
@@ -79,6 +84,7 @@ std::vector<Tensor> scan_bwd(Tensor u, Tensor delta, Tensor A, Tensor B, Tensor 
     p.dout_batch_stride = dout.stride(0); p.dout_dim_stride = dout.stride(1);
     p.B_batch_stride = B.stride(0); p.B_group_stride = B.stride(1); p.B_state_stride = B.stride(2);
     p.C_batch_stride = C.stride(0); p.C_group_stride = C.stride(1); p.C_state_stride = C.stride(2);
+    p.bc_out_group_stride = dB.stride(1);
     const int64_t every = ss2d_selective_scan_checkpoint_every(N, ratio);
     p.checkpoint_every = every;
     if (ckpt.defined()) {

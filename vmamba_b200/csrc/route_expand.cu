@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kExpThreads) route_expand_kernel(const ExpandA
     float* s_rows = sm;                                  // [C][NI * VEC]
     float* s_w = sm + (size_t)a.C * NI * VEC;            // [R][kDChunk] (transposed: 4 channels = one float4)
     const int k = blockIdx.y;
-    const bool col = (k & 1) != 0;
+    const bool col = (k & 1) != 0 && a.H > 1 && a.W > 1;      // a single row or column: both orders are one
     const int tid = threadIdx.x;
     const int item0 = blockIdx.x * NI;
     const T* __restrict__ xd = (const T*)a.xd + (long long)k * a.xd_ks;
@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(256) route_expand_mma_kernel(const ExpandArgs 
     __shared__ __align__(16) T Xt[PIX * KPAD];     // [pixel][k]
     __shared__ __align__(16) T Os[kDChunk * OPAD];     // [channel][pixel]
     const int k = blockIdx.y;
-    const bool col = (k & 1) != 0;
+    const bool col = (k & 1) != 0 && a.H > 1 && a.W > 1;      // a single row or column: both orders are one
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tiles_per_run = (a.L + PIX - 1) / PIX;
     const int groups_per_run = (tiles_per_run + a.mma_tiles - 1) / a.mma_tiles;
@@ -401,7 +401,7 @@ static bool transpose_fits(const ss2d_expand_params* p) {
 
 long long route_expand_workspace_bytes(const ss2d_expand_params* p) {
     if (!p || !dtype_ok(p->act_dtype) || p->B <= 0 || p->R <= 0 || p->N <= 0 || p->H <= 0 || p->W <= 0) return -1;
-    if (!transpose_fits(p)) return 0;
+    if (!transpose_fits(p) || p->H == 1 || p->W == 1) return 0;
     return 2 * (p->R + 2 * p->N) * p->B * p->H * p->W * (long long)dtype_size(p->act_dtype);
 }
 
@@ -480,7 +480,7 @@ int route_expand(const ss2d_expand_params* p, cudaStream_t st) {
     a.B = (int)p->B; a.D = (int)p->D; a.R = (int)p->R; a.N2 = (int)(2 * p->N); a.C = (int)C;
     a.H = (int)p->H; a.W = (int)p->W; a.L = (int)run; a.Limg = (int)L;
     a.xt = nullptr; a.xt_rs = p->B * L;
-    if (p->workspace && transpose_fits(p)) {
+    if (p->workspace && transpose_fits(p) && p->H > 1 && p->W > 1) {
         if (p->workspace_bytes < route_expand_workspace_bytes(p)) return SS2D_EWORKSPACE;
         if (!aligned_to(p->workspace, 16)) return SS2D_EINVAL_ALIGN;
         int tr;

@@ -842,7 +842,7 @@ __global__ void __launch_bounds__(kBwdRowsWarps * 32, 2) selscan_bwd_rows_nx_ker
 template <typename Tin>
 __global__ void selscan_bwd_fold_kernel(const float* rowred, const float* bcpart, float* dA, float* dD, float* dbias,
                                         Tin* dB, Tin* dC, int64_t batch, int64_t images, int64_t dim, int N, int64_t L, int64_t Lp,
-                                        int n_groups, int parts) {
+                                        int n_groups, int parts, int64_t out_gs) {
     const int64_t n_small = dim * (N + 2);
     const int64_t n_bc = batch * n_groups * N * L;       // per tensor
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_small + 2 * n_bc;
@@ -864,7 +864,7 @@ __global__ void selscan_bwd_fold_kernel(const float* rowred, const float* bcpart
             const float* src = bcpart + ((size_t)t * parts * 2 + which) * (size_t)N * Lp + (size_t)n * Lp + l;
             float acc = 0.f;
             for (int pq = 0; pq < parts; ++pq) acc += src[(size_t)pq * 2 * N * Lp];
-            (which ? dC : dB)[q] = from_f<Tin>(acc);
+            (which ? dC : dB)[t * out_gs + n * L + l] = from_f<Tin>(acc);
         }
     }
 }
@@ -892,6 +892,7 @@ static int validate_bwd(const ss2d_scan_bwd_params* p) {
     if (p->dim % p->n_groups != 0) return SS2D_EINVAL_SHAPE;
     if (p->delta_ratio < 0 || (p->delta_ratio > 1 && p->dim % p->delta_ratio != 0)) return SS2D_EINVAL_SHAPE;
     if (p->seqlen > 0x3fffffffLL) return SS2D_ENOTSUP;
+    if (p->bc_out_group_stride && p->bc_out_group_stride < p->dstate * p->seqlen) return SS2D_EINVAL_STRIDE;
     const int64_t L = p->seqlen;
     if (p->u_dim_stride < L || p->delta_dim_stride < L || p->dout_dim_stride < L) return SS2D_EINVAL_STRIDE;
     if (p->B_state_stride < L || p->C_state_stride < L) return SS2D_EINVAL_STRIDE;
@@ -1017,7 +1018,8 @@ static int launch_fold(const ss2d_scan_bwd_params* p, const BwdFold& f, cudaStre
     if (blocks > 148 * 16) blocks = 148 * 16;
     selscan_bwd_fold_kernel<Tin><<<(unsigned)blocks, 256, 0, st>>>(f.rowred, f.bcpart, (float*)p->dA, (float*)p->dD, (float*)p->ddelta_bias,
                                                                    (Tin*)p->dB, (Tin*)p->dC, p->batch, f.images, p->dim, (int)p->dstate,
-                                                                   p->seqlen, f.Lp, (int)p->n_groups, f.parts);
+                                                                   p->seqlen, f.Lp, (int)p->n_groups, f.parts,
+                                                                   p->bc_out_group_stride ? p->bc_out_group_stride : p->dstate * p->seqlen);
     count_launch();
     return check_launch();
 }

@@ -20,7 +20,7 @@ from typing import Optional
 
 import torch
 
-from . import _lib, ops
+from . import _host, _lib, ops
 from ._lib import CoreParams, check, lib
 
 K = 4
@@ -280,6 +280,10 @@ def ss2d_core_autograd(x, x_proj_weight, dt_projs_weight, dt_projs_bias, A_logs,
     CrossMerge, and torch for the projections and the LayerNorm.  Gradients flow to x and to every
     parameter; this is what a reference module computes after `vmamba_b200.install()`.
     x: (B, D, H, W); x_proj_weight: (K*(R+2N), D) or (K, R+2N, D); dt_projs_weight: (K*D, R) or (K, D, R)."""
+    params = (x_proj_weight, dt_projs_weight, dt_projs_bias, A_logs, Ds, ln_weight, ln_bias)
+    if oflex and x.is_cuda and x.dtype in ops._DTYPES and not torch.is_autocast_enabled("cuda") \
+            and all(t is not None and t.is_cuda for t in params) and int(d_state) <= 16 and int(dt_rank) <= 1024:
+        return _host.ss2d_core_autograd(x, *params, int(d_state), int(dt_rank), float(eps))     # the same statements as one node
     B, D, H, W = x.shape
     L, N, R = H * W, int(d_state), int(dt_rank)
     xs = ops.cross_scan_fn(x, True, True, False, 0)                                     # (B, K, D, L)
