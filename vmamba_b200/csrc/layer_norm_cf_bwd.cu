@@ -2,11 +2,12 @@
 //
 //   xhat = (y - mean) rstd,  dy = rstd (g w - mean_D(g w) - xhat mean_D(g w xhat)),  dw = sum g xhat,  db = sum g
 //
-// A CTA of eight warps takes tiles of 32 pixels of one image: a lane is a pixel, a warp every eighth group of four channels.
+// A CTA of eight warps takes tiles of 32 pixels (or pixel pairs) of one image: a lane is a pixel, a warp every eighth group of four channels.
 // Three passes over the tile (mean; squares and the two sums of g w; results), of which the first reads memory and the
 // others the caches.  dw / db: the eight values of a warp's four channels are summed over its pixels by halving exchanges
 // (nine shuffles) and kept per CTA in shared memory over all its tiles; a second kernel folds the CTAs in a fixed order.
-// Bound: HBM, 6 + 4 bytes per value in 16 bits.
+// Bound: HBM, 6 + 4 bytes per value in 16 bits (32 x 96 x 3 136: 21 us, 0.7 of the copy bandwidth; a pixel per lane, the tile
+// read three times and 64-bit addresses for each value took 91 us).
 #include "common.cuh"
 
 namespace ss2d {
@@ -22,64 +23,128 @@ struct NormBwdArgs {
     float eps;
 };
 
-template <typename Tg>
-__global__ void __launch_bounds__(kLnbWarps * 32) layer_norm_cf_bwd_kernel(const NormBwdArgs a) {
+// PV: pixels per lane (neighbours, one access).  IT > 0: a warp's IT groups of channels stay in registers (D <= 32 * IT).
+template <typename Tg, int PV, int IT>
+__global__ void __launch_bounds__(kLnbWarps * 32, 3) layer_norm_cf_bwd_kernel(const NormBwdArgs a) {
     extern __shared__ float lnb_sm[];                // [2][D] sums of dw, db
-    __shared__ float red[3][kLnbWarps][32];
+    __shared__ float red[3][kLnbWarps][32 * PV];
+    using VY = Vec<float, PV>;
+    using VG = Vec<Tg, PV>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, D = a.D, L = a.L;
     for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) lnb_sm[i] = 0.f;
-    __syncthreads();
     const float inv_d = 1.f / (float)D;
-    auto total = [&](int which) {
-        float t = 0.f;
+    auto put = [&](int which, const float (&v)[PV]) {
 #pragma unroll
-        for (int w = 0; w < kLnbWarps; ++w) t += red[which][w][lane];
-        return t;
+        for (int p = 0; p < PV; ++p) red[which][warp][p * 32 + lane] = v[p];
     };
+    auto total = [&](int which, float (&t)[PV]) {
+#pragma unroll
+        for (int p = 0; p < PV; ++p) {
+            t[p] = 0.f;
+#pragma unroll
+            for (int w = 0; w < kLnbWarps; ++w) t[p] += red[which][w][p * 32 + lane];
+        }
+    };
+    constexpr int C = IT > 0 ? IT : 1;
     for (long long tile = blockIdx.x; tile < a.tiles; tile += gridDim.x) {
         const long long b = tile / a.tiles_per_image;
-        const int l = (int)(tile - b * a.tiles_per_image) * 32 + lane;
-        const bool in = l < L;
-        const long long at = b * D * (long long)L + (in ? l : L - 1);
+        const int l = ((int)(tile - b * a.tiles_per_image) * 32 + lane) * PV;
+        const bool in = l < L;                       // L is a multiple of PV
+        const long long at = b * D * (long long)L + (in ? l : L - PV);
         const float* __restrict__ y = a.y + at;
         const Tg* __restrict__ g = (const Tg*)a.g + at;
-        float s = 0.f;
-#pragma unroll 2
-        for (int d0 = warp * 4; d0 < D; d0 += kLnbWarps * 4)
+        typename VY::Raw ry[C][4];
+        typename VG::Raw rg[C][4];
+        auto channel = [&](int j, int i) { return (j * kLnbWarps + warp) * 4 + i; };
+        // body(j, d of the group's first channel, y values, g values) for every group of four channels of the warp
+        auto groups = [&](bool with_g, auto body) {
+            if constexpr (IT > 0) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (d0 + i < D) s += __ldg(y + (long long)(d0 + i) * L);
-        red[0][warp][lane] = s;
-        __syncthreads();
-        const float mean = total(0) * inv_d;
-        __syncthreads();
-        float q = 0.f, s1 = 0.f, s2 = 0.f;
+                for (int j = 0; j < IT; ++j) body(ry[j], rg[j], channel(j, 0));
+            } else {
 #pragma unroll 2
-        for (int d0 = warp * 4; d0 < D; d0 += kLnbWarps * 4)
+                for (int d0 = warp * 4; d0 < D; d0 += kLnbWarps * 4) {
+                    typename VY::Raw qy[4];
+                    typename VG::Raw qg[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (d0 + i < D) {
-                    const float v = __ldg(y + (long long)(d0 + i) * L) - mean;
-                    const float gw = to_f<Tg>(__ldg(g + (long long)(d0 + i) * L)) * (a.w ? __ldg(a.w + d0 + i) : 1.f);
-                    q = fmaf(v, v, q); s1 += gw; s2 = fmaf(gw, v, s2);
+                    for (int i = 0; i < 4; ++i) {
+                        const long long o = (long long)min(d0 + i, D - 1) * L;
+                        qy[i] = VY::load_raw(y + o);
+                        if (with_g) qg[i] = VG::load_raw(g + o);
+                    }
+                    body(qy, qg, d0);
                 }
-        red[0][warp][lane] = q; red[1][warp][lane] = s1; red[2][warp][lane] = s2;
+            }
+        };
+        if constexpr (IT > 0) {
+#pragma unroll
+            for (int j = 0; j < IT; ++j)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const long long o = (long long)min(channel(j, i), D - 1) * L;
+                    ry[j][i] = VY::load_raw(y + o); rg[j][i] = VG::load_raw(g + o);
+                }
+        }
+        float s[PV], mean[PV];
+#pragma unroll
+        for (int p = 0; p < PV; ++p) s[p] = 0.f;
+        groups(false, [&](const typename VY::Raw (&qy)[4], const typename VG::Raw (&)[4], int d0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float v[PV];
+                VY::unpack(qy[i], v);
+#pragma unroll
+                for (int p = 0; p < PV; ++p) s[p] += d0 + i < D ? v[p] : 0.f;
+            }
+        });
+        put(0, s);
         __syncthreads();
-        const float rstd = rsqrtf(fmaf(total(0), inv_d, a.eps));
-        const float c1 = total(1) * inv_d, c2 = total(2) * inv_d * rstd * rstd;
+        total(0, mean);
+        float q[PV], s1[PV], s2[PV];
+#pragma unroll
+        for (int p = 0; p < PV; ++p) { mean[p] *= inv_d; q[p] = s1[p] = s2[p] = 0.f; }
+        groups(true, [&](const typename VY::Raw (&qy)[4], const typename VG::Raw (&qg)[4], int d0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float v[PV], gv[PV];
+                VY::unpack(qy[i], v); VG::unpack(qg[i], gv);
+                const float w = d0 + i < D ? (a.w ? __ldg(a.w + d0 + i) : 1.f) : 0.f;
+#pragma unroll
+                for (int p = 0; p < PV; ++p) {
+                    const float c = d0 + i < D ? v[p] - mean[p] : 0.f, gw = gv[p] * w;
+                    q[p] = fmaf(c, c, q[p]); s1[p] += gw; s2[p] = fmaf(gw, c, s2[p]);
+                }
+            }
+        });
+        __syncthreads();
+        put(0, q); put(1, s1); put(2, s2);
+        __syncthreads();
+        float rstd[PV], c1[PV], c2[PV];
+        total(0, rstd); total(1, c1); total(2, c2);
+#pragma unroll
+        for (int p = 0; p < PV; ++p) {
+            rstd[p] = rsqrtf(fmaf(rstd[p], inv_d, a.eps));
+            c1[p] *= inv_d; c2[p] *= inv_d * rstd[p] * rstd[p];
+        }
         __syncthreads();
         float* __restrict__ dy = a.dy + at;
-        for (int d0 = warp * 4; d0 < D; d0 += kLnbWarps * 4) {
+        groups(true, [&](const typename VY::Raw (&qy)[4], const typename VG::Raw (&qg)[4], int d0) {
             float v[8];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
+                float c[PV], gv[PV], o[PV];
+                VY::unpack(qy[i], c); VG::unpack(qg[i], gv);
+                const bool real = d0 + i < D && in;
+                const float w = d0 + i < D ? (a.w ? __ldg(a.w + d0 + i) : 1.f) : 0.f;
                 v[2 * i] = v[2 * i + 1] = 0.f;
-                if (d0 + i < D && in) {
-                    const float c = __ldg(y + (long long)(d0 + i) * L) - mean, gv = to_f<Tg>(__ldg(g + (long long)(d0 + i) * L));
-                    const float gw = gv * (a.w ? __ldg(a.w + d0 + i) : 1.f);
-                    dy[(long long)(d0 + i) * L] = rstd * (gw - c1 - c * c2);
-                    v[2 * i] = gv * c * rstd; v[2 * i + 1] = gv;
+#pragma unroll
+                for (int p = 0; p < PV; ++p) {
+                    c[p] -= mean[p];
+                    o[p] = rstd[p] * (gv[p] * w - c1[p] - c[p] * c2[p]);
+                    v[2 * i] = fmaf(gv[p], c[p] * rstd[p], v[2 * i]); v[2 * i + 1] += gv[p];
                 }
+                if (real) VY::store(dy + (long long)(d0 + i) * L, o);
+                else v[2 * i] = v[2 * i + 1] = 0.f;
             }
             int at_v = 0;
 #pragma unroll
@@ -93,10 +158,23 @@ __global__ void __launch_bounds__(kLnbWarps * 32) layer_norm_cf_bwd_kernel(const
             v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
             const int d = d0 + (at_v >> 1);
             if ((lane & 3) == 0 && d < D) lnb_sm[(at_v & 1) * D + d] += v[0];
-        }
+        });
     }
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) a.part[(long long)blockIdx.x * 2 * D + i] = lnb_sm[i];
+}
+
+template <typename Tg>
+static void launch_lnb(const NormBwdArgs& a, int pv, unsigned ctas, cudaStream_t st) {
+    const size_t smem = (size_t)2 * a.D * sizeof(float);
+    const int threads = kLnbWarps * 32;
+    if (pv == 2) {
+        if (a.D <= 96) layer_norm_cf_bwd_kernel<Tg, 2, 3><<<ctas, threads, smem, st>>>(a);
+        else layer_norm_cf_bwd_kernel<Tg, 2, 0><<<ctas, threads, smem, st>>>(a);
+    } else {
+        if (a.D <= 96) layer_norm_cf_bwd_kernel<Tg, 1, 3><<<ctas, threads, smem, st>>>(a);
+        else layer_norm_cf_bwd_kernel<Tg, 1, 0><<<ctas, threads, smem, st>>>(a);
+    }
 }
 
 __global__ void __launch_bounds__(256) layer_norm_cf_bwd_fold_kernel(const float* part, int ctas, int D, float* dw, float* db) {
@@ -116,9 +194,14 @@ __global__ void __launch_bounds__(256) layer_norm_cf_bwd_fold_kernel(const float
     }
 }
 
+// Pixel pairs where they are aligned and leave a tile for every CTA.
+static int lnb_pv(const ss2d_norm_bwd_params* p) {
+    const bool even = p->L % 2 == 0 && aligned_to(p->y, 8) && aligned_to(p->dy, 8) && aligned_to(p->g, 2 * dtype_size(p->g_dtype));
+    return even && p->B * ((p->L + 63) / 64) >= 148 * 3 ? 2 : 1;
+}
 static long long lnb_ctas(const ss2d_norm_bwd_params* p) {
-    const long long tiles = p->B * ((p->L + 31) / 32);
-    return tiles < 148 * 6 ? tiles : 148 * 6;
+    const long long px = 32 * lnb_pv(p), tiles = p->B * ((p->L + px - 1) / px);
+    return tiles < 148 * 3 ? tiles : 148 * 3;        // resident at once
 }
 
 static int validate_lnb(const ss2d_norm_bwd_params* p) {
@@ -142,12 +225,12 @@ int layer_norm_cf_bwd(const ss2d_norm_bwd_params* p, cudaStream_t st) {
     if (!p->workspace || p->workspace_bytes < layer_norm_cf_bwd_workspace_bytes(p)) return SS2D_EWORKSPACE;
     NormBwdArgs a;
     a.y = (const float*)p->y; a.g = p->g; a.w = (const float*)p->weight; a.dy = (float*)p->dy; a.part = (float*)p->workspace;
-    a.D = (int)p->D; a.L = (int)p->L; a.tiles_per_image = (int)((p->L + 31) / 32); a.tiles = p->B * a.tiles_per_image; a.eps = p->eps;
+    const int pv = lnb_pv(p);
+    a.D = (int)p->D; a.L = (int)p->L; a.tiles_per_image = (int)((p->L + 32 * pv - 1) / (32 * pv)); a.tiles = p->B * a.tiles_per_image; a.eps = p->eps;
     const unsigned ctas = (unsigned)lnb_ctas(p);
-    const size_t smem = (size_t)2 * p->D * sizeof(float);
-    if (p->g_dtype == SS2D_F32) layer_norm_cf_bwd_kernel<float><<<ctas, kLnbWarps * 32, smem, st>>>(a);
-    else if (p->g_dtype == SS2D_BF16) layer_norm_cf_bwd_kernel<__nv_bfloat16><<<ctas, kLnbWarps * 32, smem, st>>>(a);
-    else layer_norm_cf_bwd_kernel<__half><<<ctas, kLnbWarps * 32, smem, st>>>(a);
+    if (p->g_dtype == SS2D_F32) launch_lnb<float>(a, pv, ctas, st);
+    else if (p->g_dtype == SS2D_BF16) launch_lnb<__nv_bfloat16>(a, pv, ctas, st);
+    else launch_lnb<__half>(a, pv, ctas, st);
     layer_norm_cf_bwd_fold_kernel<<<(unsigned)((2 * p->D + 31) / 32), 256, 0, st>>>(a.part, (int)ctas, a.D, (float*)p->dweight, (float*)p->dbias);
     count_launch(2);
     return check_launch();
