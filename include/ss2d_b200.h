@@ -262,6 +262,7 @@ typedef struct ss2d_pointwise_params {
     int32_t dtype, act;
     int32_t channel_major;   /* 0: maps are (B, D, H, W); 1: (D, B, H, W) */
     int32_t reserved0;
+    int64_t channel_stride;  /* dwconv, channel_major: elements between channels; 0 = B*H*W */
 } ss2d_pointwise_params;
 
 int ss2d_bias_act(const ss2d_pointwise_params *p, void *cuda_stream);
@@ -294,7 +295,8 @@ typedef struct ss2d_expand_params {
     int64_t bc_row_stride[SS2D_ROUTES];          /* 0 = L; (2N, B, L) outputs: batch stride L, row stride B*L */
     int64_t B, D, R, N, H, W;
     int32_t act_dtype;
-    int32_t reserved0;
+    int32_t padded_rows;                /* non-zero, images adjacent in every row (batch strides L): rows have room for B*L rounded
+                                           up to a multiple of 8 and may be read and written up to there */
     void *workspace;                    /* optional: ss2d_route_expand_workspace_bytes() bytes, 16-byte aligned */
     int64_t workspace_bytes;
 } ss2d_expand_params;

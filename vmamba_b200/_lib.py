@@ -72,13 +72,13 @@ class ExpandParams(ctypes.Structure):
                 ("delta_batch_stride", _i64 * ROUTES), ("bc_batch_stride", _i64 * ROUTES),
                 ("delta_channel_stride", _i64 * ROUTES), ("bc_row_stride", _i64 * ROUTES),
                 ("B", _i64), ("D", _i64), ("R", _i64), ("N", _i64), ("H", _i64), ("W", _i64),
-                ("act_dtype", _i32), ("reserved0", _i32), ("workspace", _vp), ("workspace_bytes", _i64)]
+                ("act_dtype", _i32), ("padded_rows", _i32), ("workspace", _vp), ("workspace_bytes", _i64)]
 
 
 class PointwiseParams(ctypes.Structure):
     _fields_ = [("x", _vp), ("weight", _vp), ("bias", _vp), ("y", _vp),
                 ("B", _i64), ("D", _i64), ("H", _i64), ("W", _i64), ("dtype", _i32), ("act", _i32),
-                ("channel_major", _i32), ("reserved0", _i32)]
+                ("channel_major", _i32), ("reserved0", _i32), ("channel_stride", _i64)]
 
 
 class NormParams(ctypes.Structure):
@@ -86,6 +86,11 @@ class NormParams(ctypes.Structure):
                 ("out", _vp), ("B", _i64), ("D", _i64), ("L", _i64), ("batch_stride", _i64), ("channel_stride", _i64),
                 ("out_batch_stride", _i64), ("out_channel_stride", _i64), ("io_dtype", _i32), ("eps", _f32),
                 ("skip_norm", _i32), ("descending", _i32)]
+
+
+class NormBwdParams(ctypes.Structure):
+    _fields_ = [(n, _vp) for n in ("y", "g", "weight", "dy", "dweight", "dbias")] + \
+               [("B", _i64), ("D", _i64), ("L", _i64), ("g_dtype", _i32), ("eps", _f32), ("workspace", _vp), ("workspace_bytes", _i64)]
 
 
 class StemParams(ctypes.Structure):
@@ -119,6 +124,10 @@ EXPORTS = {
     "ss2d_selective_scan_bwd_workspace_bytes": (_i64, [ctypes.POINTER(ScanBwdParams)]),
     "ss2d_cross_scan": (ctypes.c_int, [ctypes.POINTER(CrossParams), _vp]),
     "ss2d_cross_merge": (ctypes.c_int, [ctypes.POINTER(CrossParams), _vp]),
+    "ss2d_cross_rows": (ctypes.c_int, [ctypes.POINTER(CrossParams), ctypes.c_int, _vp]),
+    "ss2d_cross_padding_supported": (ctypes.c_int, [ctypes.POINTER(CrossParams)]),
+    "ss2d_layer_norm_cf_bwd": (ctypes.c_int, [ctypes.POINTER(NormBwdParams), _vp]),
+    "ss2d_layer_norm_cf_bwd_workspace_bytes": (_i64, [ctypes.POINTER(NormBwdParams)]),
     "ss2d_cross_scan_ex": (ctypes.c_int, [ctypes.POINTER(CrossExParams), _vp]),
     "ss2d_cross_merge_ex": (ctypes.c_int, [ctypes.POINTER(CrossExParams), _vp]),
     "ss2d_core_workspace_bytes": (_i64, [ctypes.POINTER(CoreParams)]),

@@ -14,15 +14,13 @@ the scan.
 """
 from __future__ import annotations
 
-import math
 import re
 from typing import Dict, List, Optional, Sequence
 
 import torch
-import torch.nn.functional as F
 
-from . import ops
-from .fused import CoreWeights, ss2d_core
+from . import _host
+from .fused import CoreWeights
 
 # vmamba.py:2286-2300 (tiny), 2250-2264 (small), 2268-2282 (base)
 CONFIGS = dict(
@@ -80,6 +78,7 @@ class VSSMInfer:
         self.outnorm: Dict[int, tuple] = {}
         self.dtype = torch.bfloat16
         self.device = torch.device("cuda")
+        self._native = None
 
     # ------------------------------------------------------------------ construction
     @staticmethod
@@ -144,118 +143,38 @@ class VSSMInfer:
                           w=T("classifier.head.weight", dtype), b=T("classifier.head.bias", dtype))
         return m
 
-    # ------------------------------------------------------------------ layers
-    # Between the stem and the head every map is kept CHANNEL-MAJOR, (C, B, H, W): each 1x1 projection
-    # is then ONE GEMM  (C_out x C_in) . (C_in x B*H*W)  whose long dimension is a multiple of 8 for any
-    # map size (14x14 and 7x7 maps would otherwise give 128 small GEMMs with unaligned leading dimensions),
-    # while every (channel, image) plane stays a contiguous run of H*W pixels for the scan kernels.
-    def _ln(self, x, w, b, out_dtype=None, cm=True, out_cm=None):
-        """channel-first LayerNorm (vmamba.py:1078-1093), fp32 statistics."""
-        return ops.layer_norm_cf(x, w, b, 1e-5, out_dtype or self.dtype, channel_major=cm, out_channel_major=out_cm)
-
-    @staticmethod
-    def _pw(w, x):
-        """1x1 convolution of a channel-major map as one GEMM (vmamba.py:1060-1064)."""
-        C, B, H, W = x.shape
-        return torch.matmul(w, x.view(C, B * H * W)).view(w.shape[0], B, H, W)
-
-    def _block(self, x: torch.Tensor, h: torch.Tensor, b: _Block, nxt):
-        """VSSBlock._forward, eval mode (vmamba.py:1766-1778).  x: fp32 residual stream (updated in
-        place), h = norm(x) of this block.  Returns (x, norm_next(x)) where norm_next is the first
-        norm of the following block (`nxt` = its weight/bias) or None at the end of a stage: both
-        residual additions are fused into the LayerNorm that consumes their result."""
-        h = self._pw(b.w_in, h)                                                   # in_proj          :1574
-        h = ops.dwconv3x3_act(h, b.w_dw, None, "silu", channel_major=True)        # dwconv 3x3, SiLU :1582-1583
-        h = ss2d_core(h, b.core, channel_major=True)                              # forward_core     :1584
-        o = self._pw(b.w_out, h)                                                  # out_proj         :1588
-        h = ops.layer_norm_cf(x, b.n2w, b.n2b, 1e-5, self.dtype, add=o, update=True, channel_major=True)   # :1772, 1777
-        if ops.mlp_supported(h.shape[0], b.w1.shape[0], h.numel() // h.shape[0], h.dtype):
-            m = ops.mlp_fused(h, b.w1, b.b1f, b.w2)                               # Mlp: fc1 + GELU + fc2, one kernel :1151-1167
-        else:
-            h = ops.bias_act_(self._pw(b.w1, h), b.b1f, "gelu", channel_major=True)   # Mlp fc1 + GELU   :1160-1163
-            m = self._pw(b.w2, h)                                                 # fc2 (its bias joins the residual update)
-        if nxt is None:          # end of a stage: the caller decides what consumes x + m + bias
-            return x, (m, b.b2f)
-        return x, ops.layer_norm_cf(x, nxt[0], nxt[1], 1e-5, self.dtype, add=m, add_bias=b.b2f, update=True,
-                                    channel_major=True)
-
-    @staticmethod
-    def _conv_s2(rows, w_cl):
-        """3x3 stride-2 convolution (library) of a pixel-major (B, H, W, C) map; returns pixel-major.
-        The tensor is handed over as a channels-last view, so the library runs its pixel-major kernel
-        without converting."""
-        y = F.conv2d(rows.permute(0, 3, 1, 2), w_cl, None, stride=2, padding=1)
-        y = y.permute(0, 2, 3, 1)
-        return y if y.is_contiguous() else y.contiguous()
-
-    def _stem(self, img):
-        """patch embed v2 (vmamba.py:1928-1942): conv+LayerNorm+GELU in one kernel, the second convolution in
-        the library on the pixel-major map, its bias + LayerNorm + the change to channel planes in one kernel."""
-        s = self.stem
-        img = img.to(self.dtype)
-        if ops.stem_supported(img.shape[1], s["w0"].shape[0]):
-            x = ops.stem_conv_norm_act(img, s["w0"], s["b0"], s["n0w"], s["n0b"])            # (B, H/2, W/2, C0)
-        else:
-            x = F.conv2d(img, s["w0"], None, stride=2, padding=1)
-            x = F.gelu(ops.layer_norm_cf(None, s["n0w"], s["n0b"], 1e-5, self.dtype, add=x, add_bias=s["b0"]))
-            x = x.permute(0, 2, 3, 1).contiguous()
-        x = self._conv_s2(x, s["w1"])
-        return ops.pixels_norm_to_planes(x, s["b1"], s["n1w"], s["n1b"])                     # -> (C, B, H, W) fp32
-
-    def _stages(self, img, want_features=False, head_norm=None):
-        """Runs the stages.  Returns (per-stage residual maps if wanted, last value):
-        the last value is the classifier-normalised (B, C, H, W) map when `head_norm` is given."""
-        x = self._stem(img)
-        outs = []
-        last = None
-        for i, stage in enumerate(self.blocks):
-            h = self._ln(x, stage[0].n1w, stage[0].n1b)
-            pend = None
-            for j, b in enumerate(stage):
-                nxt = (stage[j + 1].n1w, stage[j + 1].n1b) if j + 1 < len(stage) else None
-                x, h = self._block(x, h, b, nxt)
-                if nxt is None:
-                    pend = h            # (m, bias): the last residual update of the stage, not applied yet
-            m, mb = pend
-            d = self.down[i]
-            if d is not None:
-                # downsample v3 (vmamba.py:1964-1971): x + m + bias as the pixel-major 16-bit input of the strided
-                # convolution in one pass (the sum goes back into x only when the stage's map is asked for: the
-                # convolution's output replaces the residual stream); its bias + LayerNorm + the way back to planes in another
-                xin = ops.planes_to_pixels(x, add=m, add_bias=mb, update=want_features, out_dtype=self.dtype)
-                if want_features:
-                    outs.append(x.clone())
-                x = ops.pixels_norm_to_planes(self._conv_s2(xin, d["w"]), d["bf"], d["nw"], d["nb"])
-            else:
-                if head_norm is not None:     # classifier norm fused with the last residual update
-                    last = ops.layer_norm_cf(x, head_norm[0], head_norm[1], 1e-5, torch.float32, add=m, add_bias=mb,
-                                             update=True, channel_major=True, out_channel_major=False)
-                else:
-                    ops.layer_norm_cf(x, None, None, 1e-5, self.dtype, add=m, add_bias=mb, update=True,
-                                      channel_major=True, normalize=False)
-                if want_features:
-                    outs.append(x)
-        return outs, (last if last is not None else x)
-
     # ------------------------------------------------------------------ public
-    @torch.no_grad()
+    # The forward itself (patch embedding, blocks, downsampling, norms) runs in the host extension: a forward is 120 to 300
+    # launches, which Python issues more slowly than the GPU runs them (csrc/host_backbone.cpp).
+    @property
+    def native(self):
+        if self._native is None:
+            n = _host.Backbone()
+            n.dtype = self.dtype
+            s = self.stem
+            n.stem = [s["w0"], s["b0"], s["n0w"], s["n0b"], s["w1"], s["b1"], s["n1w"], s["n1b"]]
+            for stage, down in zip(self.blocks, self.down):
+                for j, b in enumerate(stage):
+                    c = b.core
+                    n.add_block(j == 0, [b.n1w, b.n1b, b.n2w, b.n2b, b.w_in, b.w_dw, b.w_out, b.w1, b.b1f, b.w2, b.b2f,
+                                         c.wx, c.wdt, c.A, c.Ds, c.dt_bias], [c.ln_weight, c.ln_bias], c.d_state, c.dt_rank, c.eps)
+                n.add_down([] if down is None else [down["w"], down["bf"], down["nw"], down["nb"]])
+            if self.head is not None:
+                n.head = [self.head["nw"], self.head["nb"], self.head["w"], self.head["b"]]
+            for i, (w, b) in self.outnorm.items():
+                n.add_outnorm(i, w, b)
+            self._native = n
+        return self._native
+
     def __call__(self, img: torch.Tensor) -> torch.Tensor:
         """VSSM.forward (vmamba.py:2027-2035): (B, 3, H, W) -> (B, num_classes) logits."""
         if self.head is None:
             raise RuntimeError("this model was built without a classifier")
-        hd = self.head
-        _, x = self._stages(img, head_norm=(hd["nw"], hd["nb"]))
-        return F.linear(x.mean(dim=(2, 3)).to(self.dtype), hd["w"], hd["b"])
+        return self.native.forward(img)
 
-    @torch.no_grad()
     def features(self, img: torch.Tensor, out_indices: Sequence[int] = (0, 1, 2, 3)):
         """Backbone_VSSM.forward (vmamba.py:2133-2153): LayerNorm'ed per-stage maps."""
-        outs, _ = self._stages(img, want_features=True)
-        res = []
-        for i in out_indices:
-            w, b = self.outnorm[i]
-            res.append(self._ln(outs[i], w, b, torch.float32, out_cm=False))
-        return res
+        return self.native.features(img, list(out_indices))
 
 
 class AcceleratedVSSM(torch.nn.Module):

@@ -57,4 +57,11 @@ Tensor cross_scan(const Tensor& x, int64_t scans);       // (B, C, H, W) -> (B, 
 Tensor cross_merge(const Tensor& ys, int64_t scans);     // (B, 4, C, H, W) -> (B, C, L)
 int64_t scan_ratio(const Tensor& u, const Tensor& delta);
 
+// host_core.cpp: CrossScan (op 0), CrossMerge (1), rows into (2) and out of (3) route order, rows of a route `stride` apart
+Tensor cross(const Tensor& in, Tensor out, int64_t B, int64_t C, int64_t H, int64_t W, int64_t stride, int op);
+int64_t padded_row(int64_t B, int64_t C, int64_t H, int64_t W);
+bool rows_fit(int64_t H, int64_t W, int64_t esize);
+// step sizes (B, 4, D, S) of rows in route order (B, 4, R + 2N, S); returns the B / C rows (B, 4, 2N, S)
+Tensor expand_rows(const Tensor& xd, const Tensor& wdt, Tensor dts, int64_t B, int64_t D, int64_t R, int64_t N, int64_t S);
+
 }  // namespace host

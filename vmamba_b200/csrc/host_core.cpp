@@ -12,7 +12,7 @@ namespace host {
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
-static Tensor cross(const Tensor& in, Tensor out, int64_t B, int64_t C, int64_t H, int64_t W, int64_t stride, int op) {
+Tensor cross(const Tensor& in, Tensor out, int64_t B, int64_t C, int64_t H, int64_t W, int64_t stride, int op) {
     ss2d_cross_params p = {in.data_ptr(), out.data_ptr(), dtype_code(in), 0, B, C, H, W, stride};
     void* st = stream_of(in);
     if (op == 0) check(ss2d_cross_scan(&p, st), "ss2d_cross_scan");
@@ -22,14 +22,14 @@ static Tensor cross(const Tensor& in, Tensor out, int64_t B, int64_t C, int64_t 
 }
 
 // Row stride of the core's route tensors: H * W, or that rounded up to a multiple of eight where the kernels take padded rows.
-static int64_t padded_row(int64_t B, int64_t C, int64_t H, int64_t W) {
+int64_t padded_row(int64_t B, int64_t C, int64_t H, int64_t W) {
     const int64_t L = H * W, Lp = (L + 7) / 8 * 8;
     if (Lp == L) return L;
     ss2d_cross_params p = {nullptr, nullptr, SS2D_F32, 0, B, C, H, W, Lp};
     return ss2d_cross_padding_supported(&p) ? Lp : L;
 }
 // cross_rows keeps whole planes in shared memory: 200 KB
-static bool rows_fit(int64_t H, int64_t W, int64_t esize) { return H * (W | 1) * esize <= 200 * 1024 && H * W <= 65536; }
+bool rows_fit(int64_t H, int64_t W, int64_t esize) { return H * (W | 1) * esize <= 200 * 1024 && H * W <= 65536; }
 
 // (b, k) weights of a batched product: the four routes' matrices, repeated over the images
 static Tensor per_image(const Tensor& w, int64_t B) {
@@ -41,6 +41,23 @@ static Tensor row_products(const Tensor& a, const Tensor& b, int64_t groups) {
     const Tensor bt = b.transpose(1, 2);
     const Tensor p = a.scalar_type() == at::kFloat ? at::bmm(a, bt) : at::bmm(a, bt, at::kFloat);
     return p.view({-1, groups, p.size(1), p.size(2)}).sum(0);
+}
+
+Tensor expand_rows(const Tensor& xd, const Tensor& wdt, Tensor dts, int64_t B, int64_t D, int64_t R, int64_t N, int64_t S) {
+    const int64_t C = R + 2 * N;
+    Tensor bc = at::empty({B, 4, 2 * N, S}, xd.options());
+    ss2d_expand_params p = {};
+    p.x_dbl = xd.data_ptr(); p.dt_weight = wdt.data_ptr();
+    p.x_dbl_batch_stride = 4 * C * S; p.x_dbl_route_stride = C * S; p.x_dbl_row_stride = S;
+    const int64_t e = xd.element_size();
+    for (int64_t k = 0; k < 4; ++k) {
+        p.delta[k] = (char*)dts.data_ptr() + k * D * S * e; p.delta_batch_stride[k] = 4 * D * S; p.delta_channel_stride[k] = S;
+        p.bc[k] = (char*)bc.data_ptr() + k * 2 * N * S * e; p.bc_batch_stride[k] = 8 * N * S; p.bc_row_stride[k] = S;
+    }
+    p.B = B; p.D = D; p.R = R; p.N = N; p.H = 1; p.W = S;      // the rows are in route order already: one long row each
+    p.act_dtype = dtype_code(xd);
+    check(ss2d_route_expand(&p, stream_of(xd)), "ss2d_route_expand");
+    return bc;
 }
 
 struct CoreNode : public torch::autograd::Function<CoreNode> {
@@ -62,7 +79,7 @@ struct CoreNode : public torch::autograd::Function<CoreNode> {
             at::bmm_out(out, per_image(wx.view({4, C, D}), B), xs.view({B * 4, D, S}));
         }
         Tensor dts = at::empty({B, 4, D, S}, of);
-        const Tensor bc = expand(xd, wdt, dts, B, D, R, N, S);
+        const Tensor bc = expand_rows(xd, wdt, dts, B, D, R, N, S);
         auto [ys, states] = scan_fwd(xs.view({B, 4 * D, S}), dts.view({B, 4 * D, S}), A, bc.narrow(2, 0, N), bc.narrow(2, N, N), Dp, bias, true, true,
                                      ss2d_selective_scan_checkpoint_every(N, 1), Tensor());
         const Tensor y = cross(ys, at::empty({B, D, L}, of.dtype(at::kFloat)), B, D, H, W, S, 1);
@@ -77,24 +94,6 @@ struct CoreNode : public torch::autograd::Function<CoreNode> {
         ctx->saved_data["n"] = std::vector<int64_t>{B, D, H, W, N, R, S};
         ctx->saved_data["eps"] = eps;
         return out;
-    }
-
-    // step sizes (B, 4, D, S) of the low-rank rows, and the B / C rows as a tensor of their own
-    static Tensor expand(const Tensor& xd, const Tensor& wdt, Tensor dts, int64_t B, int64_t D, int64_t R, int64_t N, int64_t S) {
-        const int64_t C = R + 2 * N;
-        Tensor bc = at::empty({B, 4, 2 * N, S}, xd.options());
-        ss2d_expand_params p = {};
-        p.x_dbl = xd.data_ptr(); p.dt_weight = wdt.data_ptr();
-        p.x_dbl_batch_stride = 4 * C * S; p.x_dbl_route_stride = C * S; p.x_dbl_row_stride = S;
-        const int64_t e = xd.element_size();
-        for (int64_t k = 0; k < 4; ++k) {
-            p.delta[k] = (char*)dts.data_ptr() + k * D * S * e; p.delta_batch_stride[k] = 4 * D * S; p.delta_channel_stride[k] = S;
-            p.bc[k] = (char*)bc.data_ptr() + k * 2 * N * S * e; p.bc_batch_stride[k] = 8 * N * S; p.bc_row_stride[k] = S;
-        }
-        p.B = B; p.D = D; p.R = R; p.N = N; p.H = 1; p.W = S;      // the rows are in route order already: one long row each
-        p.act_dtype = dtype_code(xd);
-        check(ss2d_route_expand(&p, stream_of(xd)), "ss2d_route_expand");
-        return bc;
     }
 
     static variable_list backward(AutogradContext* ctx, variable_list grads) {

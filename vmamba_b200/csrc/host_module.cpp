@@ -4,6 +4,7 @@
 namespace host {
 void bind_ops(pybind11::module_& m);
 void bind_core(pybind11::module_& m);
+void bind_backbone(pybind11::module_& m);
 }  // namespace host
 
 PYBIND11_MODULE(_host, m) {
@@ -19,4 +20,5 @@ PYBIND11_MODULE(_host, m) {
     });
     host::bind_ops(m);
     host::bind_core(m);
+    host::bind_backbone(m);
 }

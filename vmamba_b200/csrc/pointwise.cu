@@ -127,6 +127,8 @@ struct DwStripArgs {
     void* y;
     int D, H, W, nseg, nrb, total;  // nseg = W / PV strips per row, nrb = row blocks per plane, total threads with work
     unsigned magic_nseg, magic_nrb, magic_ppc;
+    int ppc;                        // planes per channel
+    long long cstride;              // elements between channels
 };
 
 template <typename T, int PV, int KR, int ACT>
@@ -138,7 +140,7 @@ __global__ void __launch_bounds__(256, PV == 8 ? 2 : 3) dwconv3x3_strip_kernel(c
     const int i = valid ? (int)gi : a.total - 1;      // spare threads shadow the last strip (they join the shuffles, store nothing)
     const int t = mdiv(i, a.magic_nseg), seg = i - t * a.nseg;
     const int plane = mdiv(t, a.magic_nrb), rb = t - plane * a.nrb;
-    const int d = mdiv(plane, a.magic_ppc) % a.D;
+    const int chan = mdiv(plane, a.magic_ppc), d = chan % a.D;      // batch-major maps: one plane per (image, channel)
     float k[9];
     {
         const T* __restrict__ wk = (const T*)a.w + d * 9;
@@ -146,7 +148,7 @@ __global__ void __launch_bounds__(256, PV == 8 ? 2 : 3) dwconv3x3_strip_kernel(c
         for (int j = 0; j < 9; ++j) k[j] = to_f<T>(wk[j]);
     }
     const float b = a.bias ? __ldg(a.bias + d) : 0.f;
-    const long long origin = (long long)plane * H * W + seg * PV;
+    const long long origin = chan * a.cstride + (long long)(plane - chan * a.ppc) * H * W + seg * PV;
     const T* __restrict__ px = (const T*)a.x + origin;
     T* __restrict__ py = (T*)a.y + origin;
     const bool at_left = seg == 0, at_right = seg == a.nseg - 1;
@@ -290,7 +292,9 @@ int dwconv3x3_act(const ss2d_pointwise_params* p, cudaStream_t st) {
     const long long L = p->H * p->W;
     int pv = (s == 2) ? 8 : 4;
     auto fit = [&](long long x) { while (pv > 1 && (x % pv) != 0) pv >>= 1; };
-    fit(p->W); fit(L);
+    const long long cstride = p->channel_major ? (p->channel_stride ? p->channel_stride : p->B * L) : L;
+    if (cstride < (p->channel_major ? p->B * L : L)) return SS2D_EINVAL_STRIDE;
+    fit(p->W); fit(L); fit(cstride);
     fit((long long)(reinterpret_cast<uintptr_t>(p->x) / s));
     fit((long long)(reinterpret_cast<uintptr_t>(p->y) / s));
     const int kr = (p->H % 8 == 0 || p->H % 7 != 0) ? 8 : 7;      // rows per thread: whichever divides the map better
@@ -304,6 +308,7 @@ int dwconv3x3_act(const ss2d_pointwise_params* p, cudaStream_t st) {
     a.x = p->x; a.w = p->weight; a.bias = (const float*)p->bias; a.y = p->y;
     a.D = (int)p->D; a.H = (int)p->H; a.W = (int)p->W; a.nseg = (int)nseg; a.nrb = (int)nrb; a.total = (int)total;
     a.magic_nseg = magic(nseg); a.magic_nrb = magic(nrb); a.magic_ppc = magic(p->channel_major ? p->B : 1);
+    a.ppc = p->channel_major ? (int)p->B : 1; a.cstride = cstride;
     const unsigned grid = (unsigned)((total + 255) / 256);
     if (p->dtype == SS2D_F32) return launch_dw_strip<float>(a, pv, kr, p->act, grid, st);
     if (p->dtype == SS2D_BF16) return launch_dw_strip<__nv_bfloat16>(a, pv, kr, p->act, grid, st);

@@ -349,6 +349,7 @@ struct TransArgs {
     const void* xd;
     void* xt;
     long long xd_bs, xd_ks, xd_rs;
+    long long xt_rs;
     int C, B, H, W, L, planes, vec_ok;  // planes = 2 * C * B; vec_ok: every plane start is 16-byte aligned
 };
 
@@ -363,7 +364,7 @@ __global__ void __launch_bounds__(256) plane_transpose_kernel(const TransArgs a)
     for (int pid = blockIdx.x * nwarps + warp; pid < a.planes; pid += gridDim.x * nwarps) {
         const int b = pid % a.B, c = (pid / a.B) % a.C, kk = pid / (a.B * a.C);
         const T* src = (const T*)a.xd + (long long)(2 * kk + 1) * a.xd_ks + (long long)b * a.xd_bs + (long long)c * a.xd_rs;
-        T* dst = (T*)a.xt + (long long)pid * a.L;
+        T* dst = (T*)a.xt + (long long)(pid / a.B) * a.xt_rs + (long long)b * a.L;
         if (vec) {
             for (int e = lane * PV; e < a.L; e += 32 * PV) {
                 T v[PV];
@@ -399,10 +400,16 @@ static bool transpose_fits(const ss2d_expand_params* p) {
     return (size_t)p->H * (p->W + 1) * dtype_size(p->act_dtype) <= 16 * 1024;
 }
 
+// Elements of a row over all images (rows of a workspace, adjacent images).
+static long long expand_run(const ss2d_expand_params* p) {
+    const long long n = p->B * p->H * p->W;
+    return p->padded_rows ? (n + 7) / 8 * 8 : n;
+}
+
 long long route_expand_workspace_bytes(const ss2d_expand_params* p) {
     if (!p || !dtype_ok(p->act_dtype) || p->B <= 0 || p->R <= 0 || p->N <= 0 || p->H <= 0 || p->W <= 0) return -1;
     if (!transpose_fits(p) || p->H == 1 || p->W == 1) return 0;
-    return 2 * (p->R + 2 * p->N) * p->B * p->H * p->W * (long long)dtype_size(p->act_dtype);
+    return 2 * (p->R + 2 * p->N) * expand_run(p) * (long long)dtype_size(p->act_dtype);
 }
 
 template <typename T>
@@ -411,9 +418,9 @@ static int launch_transpose(const ss2d_expand_params* p, cudaStream_t st) {
     t.xd = p->x_dbl; t.xt = p->workspace;
     t.xd_bs = p->x_dbl_batch_stride; t.xd_ks = p->x_dbl_route_stride; t.xd_rs = p->x_dbl_row_stride ? p->x_dbl_row_stride : p->H * p->W;
     t.C = (int)(p->R + 2 * p->N); t.B = (int)p->B; t.H = (int)p->H; t.W = (int)p->W; t.L = (int)(p->H * p->W);
-    t.planes = 2 * t.C * t.B;
+    t.planes = 2 * t.C * t.B; t.xt_rs = expand_run(p);
     const size_t pv = 16 / sizeof(T);
-    t.vec_ok = (t.xd_bs % pv) == 0 && (t.xd_ks % pv) == 0 && (t.xd_rs % pv) == 0 && aligned_to(p->x_dbl, 16) && aligned_to(p->workspace, 16);
+    t.vec_ok = (t.xt_rs % pv) == 0 && (t.xd_bs % pv) == 0 && (t.xd_ks % pv) == 0 && (t.xd_rs % pv) == 0 && aligned_to(p->x_dbl, 16) && aligned_to(p->workspace, 16);
     const size_t plane_bytes = ((size_t)t.H * (t.W + 1) * sizeof(T) + 15) / 16 * 16;
     int warps = (int)(32 * 1024 / plane_bytes);
     if (warps < 1) warps = 1;
@@ -449,9 +456,16 @@ int route_expand(const ss2d_expand_params* p, cudaStream_t st) {
     }
     // images adjacent in every tensor (channel-major maps): one run of B*L pixels per row, so that the
     // vector width does not depend on the size of a single map
-    bool flat = p->B > 1 && p->x_dbl_batch_stride == L;
+    const bool transposed = p->workspace && transpose_fits(p) && p->H > 1 && p->W > 1;
+    const bool pad = p->padded_rows && (transposed || p->H == 1 || p->W == 1);      // a gather could not tell the padding apart
+    bool flat = (p->B > 1 || pad) && p->x_dbl_batch_stride == L;
     for (int k = 0; k < 4; ++k) flat = flat && p->delta_batch_stride[k] == L && p->bc_batch_stride[k] == L;
-    const long long run = flat ? p->B * L : L;
+    const long long run = flat ? (pad ? expand_run(p) : p->B * L) : L;
+    if (flat && pad) {
+        if (xd_rs < run || p->x_dbl_route_stride < run) return SS2D_EINVAL_STRIDE;
+        for (int k = 0; k < 4; ++k)
+            if (p->delta_channel_stride[k] < run || p->bc_row_stride[k] < run) return SS2D_EINVAL_STRIDE;
+    }
     // widest pixel vector that keeps every row start aligned in every tensor
     int vec = 8;
     auto fit = [&](long long x) { if (x < 0) x = -x; while (vec > 1 && (x % vec) != 0) vec >>= 1; };
@@ -479,8 +493,8 @@ int route_expand(const ss2d_expand_params* p, cudaStream_t st) {
     a.xd_bs = p->x_dbl_batch_stride; a.xd_ks = p->x_dbl_route_stride; a.xd_rs = xd_rs;
     a.B = (int)p->B; a.D = (int)p->D; a.R = (int)p->R; a.N2 = (int)(2 * p->N); a.C = (int)C;
     a.H = (int)p->H; a.W = (int)p->W; a.L = (int)run; a.Limg = (int)L;
-    a.xt = nullptr; a.xt_rs = p->B * L;
-    if (p->workspace && transpose_fits(p) && p->H > 1 && p->W > 1) {
+    a.xt = nullptr; a.xt_rs = expand_run(p);
+    if (transposed) {
         if (p->workspace_bytes < route_expand_workspace_bytes(p)) return SS2D_EWORKSPACE;
         if (!aligned_to(p->workspace, 16)) return SS2D_EINVAL_ALIGN;
         int tr;

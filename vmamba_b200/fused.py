@@ -13,8 +13,6 @@ the per-route (delta, B, C) streams in the orientation order of each route.
 """
 from __future__ import annotations
 
-import ctypes
-import math
 from dataclasses import dataclass
 from typing import Optional
 
@@ -40,6 +38,15 @@ class CoreWeights:
     dt_rank: int
     d_inner: int
     eps: float = 1e-5
+    _native: object = None
+
+    @property
+    def native(self):
+        """The same weights as the host extension holds them."""
+        if self._native is None:
+            self._native = _host.CoreWeights(self.wx, self.wdt, self.A, self.Ds, self.dt_bias, self.ln_weight, self.ln_bias,
+                                             self.d_state, self.dt_rank, self.eps)
+        return self._native
 
     @staticmethod
     def build(x_proj_weight, dt_projs_weight, dt_projs_bias, A_logs, Ds, ln_weight, ln_bias, *,
@@ -66,48 +73,11 @@ def project(x: torch.Tensor, w: CoreWeights, channel_major: bool = False):
     all in the activation dtype (the dtype the projection produced them in, as in the reference under
     autocast).  One library GEMM (x_proj on the un-scanned map) and one `ss2d_route_expand` launch.
     """
-    if channel_major:
-        D, B, H, W = x.shape
-    else:
-        B, D, H, W = x.shape
-    L, R, N = H * W, w.dt_rank, w.d_state
-    C = R + 2 * N
-    p = _lib.ExpandParams()
-    if channel_major:
-        # one GEMM over the whole batch: (4C x D) . (D x B*L) -> rows (route, c), columns (b, l); the route
-        # streams keep that shape: delta (orientation, pair, D, B, L), B/C rows (orientation, pair, 2N, B, L)
-        if ops.linear_supported(K * C, D, B * L, x.dtype):
-            xd = ops.linear_cf(x.reshape(D, B * L), w.wx)             # x_proj on the tensor cores (ss2d_linear_fwd)
-        else:
-            xd = torch.matmul(w.wx, x.reshape(D, B * L))              # fp32 maps, odd widths: the library GEMM
-        p.x_dbl_batch_stride, p.x_dbl_route_stride, p.x_dbl_row_stride = L, C * B * L, B * L
-        delta = torch.empty((2, 2, D, B, L), device=x.device, dtype=x.dtype)
-        bc = torch.empty((2, 2, 2 * N, B, L), device=x.device, dtype=x.dtype)
-        for k in range(K):
-            j, i = k % 2, k // 2
-            p.delta[k], p.delta_batch_stride[k], p.delta_channel_stride[k] = delta[j, i].data_ptr(), L, B * L
-            p.bc[k], p.bc_batch_stride[k], p.bc_row_stride[k] = bc[j, i].data_ptr(), L, B * L
-    else:
-        xd = torch.matmul(w.wx, x.reshape(B, D, L))                   # (B, 4*C, L), route-major rows
-        p.x_dbl_batch_stride, p.x_dbl_route_stride, p.x_dbl_row_stride = xd.stride(0), C * L, L
-        delta = torch.empty((2, B, 2, D, L), device=x.device, dtype=x.dtype)   # [orientation][b][pair index]
-        bc = torch.empty((2, B, 2, 2 * N, L), device=x.device, dtype=x.dtype)
-        for k in range(K):
-            j, i = k % 2, k // 2
-            p.delta[k], p.delta_batch_stride[k] = delta[j, :, i].data_ptr(), delta.stride(1)
-            p.bc[k], p.bc_batch_stride[k] = bc[j, :, i].data_ptr(), bc.stride(1)
-    p.x_dbl, p.dt_weight = xd.data_ptr(), w.wdt.data_ptr()
-    p.B, p.D, p.R, p.N, p.H, p.W = B, D, R, N, H, W
-    p.act_dtype = ops.dtype_code(x)
-    need = int(lib().ss2d_route_expand_workspace_bytes(p))      # room for the transposed rows of the column-major routes
-    if need > 0:
-        ws = torch.empty(need, device=x.device, dtype=torch.uint8)
-        p.workspace, p.workspace_bytes = ws.data_ptr(), need
-    with torch.cuda.device(x.device):
-        check(lib().ss2d_route_expand(p, torch.cuda.current_stream(x.device).cuda_stream), "ss2d_route_expand")
+    bc, delta = _host.project(x.contiguous(), w.native, channel_major)
     if channel_major:       # (pair, rows, B, L) per orientation
-        return RouteStreams(bc[0], bc[1], delta[0], delta[1], True)
-    return RouteStreams(bc[0], bc[1], delta[0], delta[1], False)
+        D, B, H, W = x.shape
+        delta, bc = delta.view(2, 2, D, B, H * W), bc.view(2, 2, 2 * w.d_state, B, H * W)
+    return RouteStreams(bc[0], bc[1], delta[0], delta[1], channel_major)
 
 
 class RouteStreams(tuple):
@@ -181,28 +151,7 @@ def fused_supported(x_shape, d_state: int, dtype: torch.dtype = torch.bfloat16, 
     """True when `ss2d_core_fwd` takes the case itself.  Asks the library (`ss2d_core_supported`), which applies
     the rules of its launch planner to dense, 16-byte aligned streams of this shape, so the answer cannot drift
     from what the call will do."""
-    if channel_major:
-        D, B, H, W = x_shape
-    else:
-        B, D, H, W = x_shape
-    L = H * W
-    p = CoreParams()
-    fake = 4096                                   # an aligned address; the query dereferences nothing
-    p.x = p.A = p.Dskip = p.delta_bias = p.y = fake
-    for k in range(K):
-        p.delta[k] = p.Bm[k] = p.Cm[k] = fake
-        if channel_major:
-            p.delta_batch_stride[k], p.delta_channel_stride[k], p.bc_batch_stride[k] = L, B * L, L
-        else:
-            p.delta_batch_stride[k], p.delta_channel_stride[k], p.bc_batch_stride[k] = 2 * D * L, L, 4 * int(d_state) * L
-    p.B, p.D, p.H, p.W, p.N = B, D, H, W, int(d_state)
-    code = {torch.float32: _lib.SS2D_F32, torch.float16: _lib.SS2D_F16, torch.bfloat16: _lib.SS2D_BF16}[dtype]
-    p.act_dtype = p.y_dtype = code
-    p.with_norm = 1
-    if channel_major:
-        p.x_batch_stride = p.y_batch_stride = L
-        p.x_channel_stride = p.y_channel_stride = B * L
-    return int(lib().ss2d_core_supported(p)) == _lib.SS2D_OK
+    return _host.core_takes(list(x_shape), int(d_state), dtype, channel_major)
 
 
 def ss2d_core(x: torch.Tensor, w: CoreWeights, *, with_norm: bool = True, out_dtype=None,
@@ -217,60 +166,13 @@ def ss2d_core(x: torch.Tensor, w: CoreWeights, *, with_norm: bool = True, out_dt
     if x.shape[0 if channel_major else 1] != w.d_inner:
         raise RuntimeError(f"x has {x.shape[0 if channel_major else 1]} channels, weights were built for {w.d_inner}")
     out_dtype = out_dtype or (x.dtype if with_norm else torch.float32)
-    with torch.autocast("cuda", enabled=False):
-        def unfused():
-            if channel_major:
-                return _ss2d_core_unfused_cm(x, w, with_norm, out_dtype)
-            return _ss2d_core_unfused(x, w, with_norm, out_dtype)
-
-        if not fused_supported(x.shape, w.d_state, x.dtype, channel_major) or (channel_major and not with_norm):
-            return unfused()
-        try:
-            return scan_merge_norm(x, project(x, w, channel_major), w, with_norm=with_norm, out_dtype=out_dtype,
-                                   workspace=workspace, channel_major=channel_major)
-        except _lib.Ss2dError as e:        # refused before any launch (an alignment the query could not see)
-            if e.status != _lib.SS2D_ENOTSUP:
-                raise
-            return unfused()
+    return _host.ss2d_core(x, w.native, with_norm, out_dtype, workspace, channel_major)
 
 
-def _ss2d_core_unfused(x, w: CoreWeights, with_norm: bool, out_dtype, out_channel_major: bool = False):
+def _ss2d_core_unfused(x, w: CoreWeights, with_norm: bool, out_dtype):
     """Same mathematics through the operator-surface kernels (cross scan -> projections ->
     selective scan -> cross merge -> LayerNorm), the order of vmamba.py:1536-1571."""
-    B, D, H, W = x.shape
-    L, R, N = H * W, w.dt_rank, w.d_state
-    C = R + 2 * N
-    xs = ops.cross_scan_fwd(x, 0)                                        # (B, K, D, L)
-    x_dbl = torch.matmul(w.wx.view(K, C, D), xs)                         # (B, K, C, L)
-    dts = torch.matmul(w.wdt, x_dbl[:, :, :R]).reshape(B, K * D, L)
-    Bs = x_dbl[:, :, R:R + N]                                            # strided views: the scan takes batch / group / state strides
-    Cs = x_dbl[:, :, R + N:]
-    ys = ops.selective_scan_fwd(xs.view(B, K * D, L), dts, w.A, Bs, Cs, w.Ds, w.dt_bias, True, True)
-    y = ops.cross_merge_fwd(ys.view(B, K, D, H, W), 0).view(B, D, H, W)
-    if with_norm:
-        return ops.layer_norm_cf(y, w.ln_weight, w.ln_bias, w.eps, out_dtype, out_channel_major=out_channel_major)
-    return y.to(out_dtype)
-
-
-def _ss2d_core_unfused_cm(x, w: CoreWeights, with_norm: bool, out_dtype):
-    """The same chain on a channel-major map (D, B, H, W) without a layout copy: the batch is folded into the
-    plane count of CrossScan / CrossMerge (their routes stay per plane), each projection is one GEMM per route
-    over all images, and the selective scan reads and writes (route, channel, image) rows through its strides."""
-    D, B, H, W = x.shape
-    L, R, N = H * W, w.dt_rank, w.d_state
-    C = R + 2 * N
-    xs = ops.cross_scan_fwd(x.view(1, D * B, H, W), 0).view(K, D, B * L)         # route k: (D, B, L)
-    x_dbl = torch.bmm(w.wx.view(K, C, D), xs)                                    # (K, C, B*L)
-    dts = torch.bmm(w.wdt, x_dbl[:, :R])                                         # (K, D, B*L)
-    rows = lambda t: t.view(K * D, B, L).permute(1, 0, 2)                        # (B, K*D, L) view of (K, D, B, L)
-    bc = x_dbl.view(K, C, B, L).permute(2, 0, 1, 3)                              # (B, K, C, L) view
-    ys = torch.empty((K * D, B, L), device=x.device, dtype=torch.float32)
-    ops.selective_scan_fwd(rows(xs), rows(dts), w.A, bc[:, :, R:R + N], bc[:, :, R + N:], w.Ds, w.dt_bias, True, True,
-                           out=ys.permute(1, 0, 2))
-    y = ops.cross_merge_fwd(ys.view(1, K, D * B, H, W), 0).view(D, B, H, W)
-    if with_norm:
-        return ops.layer_norm_cf(y, w.ln_weight, w.ln_bias, w.eps, out_dtype, channel_major=True)
-    return y.to(out_dtype)
+    return _host.ss2d_core_by_operators(x.contiguous(), w.native, with_norm, out_dtype, False)
 
 
 def ss2d_core_autograd(x, x_proj_weight, dt_projs_weight, dt_projs_bias, A_logs, Ds, ln_weight, ln_bias, *,
