@@ -232,7 +232,13 @@ typedef struct ss2d_core_params {
     int64_t x_batch_stride, x_channel_stride;
     int64_t y_batch_stride, y_channel_stride;
     int64_t delta_channel_stride[SS2D_ROUTES];   /* 0 = L; (D, B, L) step-size maps: L as batch stride and B*L here */
+    int64_t stream_row;      /* 0 = L.  A multiple of 8 >= L: the delta, B and C rows have that many elements, those beyond L
+                              * finite in delta and zero in B (ss2d_route_expand writes them so with `image_row`) */
 } ss2d_core_params;
+
+/* 1 when rows padded to a multiple of 8 (`stream_row`) are the faster form for this problem: planes whose size no vector
+ * divides.  Reads the sizes, the dtype and the strides of x; stream_row and the streams' strides are ignored. */
+int ss2d_core_prefers_padded_rows(const ss2d_core_params *p);
 
 int64_t ss2d_core_workspace_bytes(const ss2d_core_params *p);
 int ss2d_core_fwd(const ss2d_core_params *p, void *cuda_stream);
@@ -299,6 +305,8 @@ typedef struct ss2d_expand_params {
                                            up to a multiple of 8 and may be read and written up to there */
     void *workspace;                    /* optional: ss2d_route_expand_workspace_bytes() bytes, 16-byte aligned */
     int64_t workspace_bytes;
+    int64_t image_row;                  /* non-zero: a multiple of 8 >= H * W; the rows of an image in delta and bc have that many
+                                           elements (their batch strides), the padding zero.  Needs the workspace */
 } ss2d_expand_params;
 
 /* With a workspace the projected rows of the two column-major routes are transposed once, plane by plane, by a

@@ -63,7 +63,7 @@ class CoreParams(ctypes.Structure):
                 ("B", _i64), ("D", _i64), ("H", _i64), ("W", _i64), ("N", _i64),
                 ("act_dtype", _i32), ("y_dtype", _i32), ("with_norm", _i32), ("ln_eps", _f32),
                 ("x_batch_stride", _i64), ("x_channel_stride", _i64), ("y_batch_stride", _i64), ("y_channel_stride", _i64),
-                ("delta_channel_stride", _i64 * ROUTES)]
+                ("delta_channel_stride", _i64 * ROUTES), ("stream_row", _i64)]
 
 
 class ExpandParams(ctypes.Structure):
@@ -72,7 +72,8 @@ class ExpandParams(ctypes.Structure):
                 ("delta_batch_stride", _i64 * ROUTES), ("bc_batch_stride", _i64 * ROUTES),
                 ("delta_channel_stride", _i64 * ROUTES), ("bc_row_stride", _i64 * ROUTES),
                 ("B", _i64), ("D", _i64), ("R", _i64), ("N", _i64), ("H", _i64), ("W", _i64),
-                ("act_dtype", _i32), ("padded_rows", _i32), ("workspace", _vp), ("workspace_bytes", _i64)]
+                ("act_dtype", _i32), ("padded_rows", _i32), ("workspace", _vp), ("workspace_bytes", _i64),
+                ("image_row", _i64)]
 
 
 class PointwiseParams(ctypes.Structure):
@@ -132,6 +133,7 @@ EXPORTS = {
     "ss2d_cross_merge_ex": (ctypes.c_int, [ctypes.POINTER(CrossExParams), _vp]),
     "ss2d_core_workspace_bytes": (_i64, [ctypes.POINTER(CoreParams)]),
     "ss2d_core_fwd": (ctypes.c_int, [ctypes.POINTER(CoreParams), _vp]),
+    "ss2d_core_prefers_padded_rows": (ctypes.c_int, [ctypes.POINTER(CoreParams)]),
     "ss2d_core_supported": (ctypes.c_int, [ctypes.POINTER(CoreParams)]),
     "ss2d_core_fwd_static": (ctypes.c_int, [ctypes.POINTER(CoreParams), _vp]),
     "ss2d_core_static_capacity": (_i64, []),

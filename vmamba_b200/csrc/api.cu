@@ -25,6 +25,7 @@ int layer_norm_cf(const ss2d_norm_params* p, cudaStream_t st);
 long long core_workspace_bytes(const ss2d_core_params* p);
 int core_fwd(const ss2d_core_params* p, cudaStream_t st);
 int core_supported(const ss2d_core_params* p);
+int core_prefers_padded_rows(const ss2d_core_params* p);
 int core_fwd_static(const ss2d_core_params* p, cudaStream_t st);
 long long core_static_capacity();
 int route_expand(const ss2d_expand_params* p, cudaStream_t st);
@@ -137,6 +138,7 @@ int ss2d_core_fwd(const ss2d_core_params* p, void* stream) {
     return ss2d::core_fwd(p, (cudaStream_t)stream);
 }
 int ss2d_core_supported(const ss2d_core_params* p) { return ss2d::core_supported(p); }
+int ss2d_core_prefers_padded_rows(const ss2d_core_params* p) { return ss2d::core_prefers_padded_rows(p); }
 int ss2d_core_fwd_static(const ss2d_core_params* p, void* stream) {
     ss2d::Range nvtx_("ss2d_core_fwd_static");
     if (p) SS2D_CHECK_PTRS(p->x, p->delta[0], p->delta[1], p->delta[2], p->delta[3], p->Bm[0], p->Bm[1], p->Bm[2], p->Bm[3], p->Cm[0], p->Cm[1],

@@ -492,7 +492,7 @@ static int launch_core_v(const CoreArgs& a, const PlaneConfig& c, unsigned grid,
 
 
 // ---- route-stream kernel (core_routes.cuh): which planes it takes, and its launch -----------------------------
-struct RoutePlan { int S, SV; size_t smem; };
+struct RoutePlan { int S, SV; size_t smem; bool pad; };
 
 // 0: choose by shape (default), 1: always the plane kernel, 2: the route-stream kernel wherever it applies.
 // Read once from SS2D_CORE_KERNEL = plane | routes (a switch for measurements; both kernels pass the same tests).
@@ -524,6 +524,23 @@ static bool plan_routes(const ss2d_core_params* p, RoutePlan& r) {
     r.S = vec;
     r.SV = (vec == 8 && p->W % 8 == 0) ? 8 : 4;
     r.smem = (size_t)L * (8 + s);
+    r.pad = false;
+    return r.smem <= 227 * 1024;
+}
+
+// Padded rows: chunks of 32 x 8 elements.
+static bool plan_padded(const ss2d_core_params* p, RoutePlan& r) {
+    const size_t s = dtype_size(p->act_dtype);
+    const long long Lp = p->stream_row;
+    if (Lp % 8 != 0 || Lp < p->H * p->W || Lp > 65536) return false;
+    for (int k = 0; k < 4; ++k) {
+        if (p->delta_batch_stride[k] % 8 != 0 || p->delta_channel_stride[k] % 8 != 0 || p->bc_batch_stride[k] % 8 != 0) return false;
+        if (!aligned_to(p->delta[k], 8 * s) || !aligned_to(p->Bm[k], 8 * s) || !aligned_to(p->Cm[k], 8 * s)) return false;
+    }
+    r.S = 8;
+    r.SV = 0;
+    r.smem = (size_t)Lp * (8 + 2 * s);
+    r.pad = true;
     return r.smem <= 227 * 1024;
 }
 
@@ -542,6 +559,15 @@ static int launch_routes_t(const RouteArgs& a, const RoutePlan& r, unsigned grid
     return launch_routes_k<T, 4, 4, MINB, 0>(a, r, grid, st);
 }
 
+template <typename T, int MINB>
+static int launch_pad(const RouteArgs& a, const RoutePlan& r, unsigned grid, cudaStream_t st) {
+    auto kern = core_route_pad_kernel<T, 8, MINB>;
+    if (ensure_dynamic_smem((const void*)kern, r.smem) != cudaSuccess) return SS2D_ECUDA;
+    kern<<<grid, 128, r.smem, st>>>(a);
+    count_launch();
+    return check_launch();
+}
+
 static int run_routes(const ss2d_core_params* p, const RoutePlan& r, float* merged, cudaStream_t st) {
     RouteArgs a;
     a.x = p->x;
@@ -555,25 +581,40 @@ static int run_routes(const ss2d_core_params* p, const RoutePlan& r, float* merg
     a.x_bs = p->x_batch_stride ? p->x_batch_stride : p->D * p->H * p->W;
     a.x_cs = p->x_channel_stride ? p->x_channel_stride : p->H * p->W;
     a.B = (int)p->B; a.D = (int)p->D; a.H = (int)p->H; a.W = (int)p->W; a.L = (int)(p->H * p->W);
-    a.magic_H = p->H > 1 ? (unsigned)(((1ULL << 32) + (unsigned long long)p->H - 1) / (unsigned long long)p->H) : 0;
+    auto magic = [](long long d) { return d > 1 ? (unsigned)(((1ULL << 32) + (unsigned long long)d - 1) / (unsigned long long)d) : 0u; };
+    a.magic_H = magic(p->H); a.magic_W = magic(p->W); a.plane = a.L;
     const long long grid = p->B * p->D;
     if (grid > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
+    if (r.pad) {
+        a.L = (int)p->stream_row;
+        if (p->act_dtype == SS2D_F32) return launch_pad<float, 4>(a, r, (unsigned)grid, st);
+        if (p->act_dtype == SS2D_BF16) return launch_pad<__nv_bfloat16, 7>(a, r, (unsigned)grid, st);
+        return launch_pad<__half, 7>(a, r, (unsigned)grid, st);
+    }
     if (p->act_dtype == SS2D_F32) return launch_routes_t<float, 4>(a, r, (unsigned)grid, st);
     if (p->act_dtype == SS2D_BF16) return launch_routes_t<__nv_bfloat16, 7>(a, r, (unsigned)grid, st);
     return launch_routes_t<__half, 7>(a, r, (unsigned)grid, st);
 }
 
-// The scan + merge kernel for this call.  Measured on B200 (bf16, scan + merge alone): the route-stream kernel wins
-// where its chunks are well filled and seven CTAs fit an SM (56 x 56: 0.223 against 0.267 ms at batch 128 x 96
-// channels; 32 x 32: 0.106 against 0.112 ms), and loses where a quarter of the last chunk's lanes idle (28 x 28:
-// 0.148 against 0.141 ms) or shared memory leaves five CTAs per SM (64 x 64: 0.231 against 0.219 ms).
+// The scan + merge kernel for this call.  Measured on B200 (bf16, whole core): the route-stream kernel wins where its chunks are
+// well filled and seven CTAs fit an SM (56 x 56: 0.223 against 0.267 ms at batch 128 x 96 channels; 36 x 36, fill 0.84: 189
+// against 204 us; 40 x 40: 122 against 129 us), and loses where a quarter of the last chunk's lanes idle (28 x 28: 77
+// against 72 us; 24 x 24: 107 against 94 us) or shared memory leaves five CTAs per SM (64 x 64: 0.231 against 0.219 ms) - but
+// wins again on planes of 4 608 pixels and more, where the plane kernel is one CTA of 600 threads and more per SM
+// (72 x 72: 220 against 238 us), and wherever that kernel has segments of at most two elements (27 x 40: 46 against
+// 61 us) or does not take the plane at all (54 x 80: 178 against 269 us through the operators, 96 x 96: 119 against 132 us;
+// 112 x 112, one CTA of four warps per SM: 298 against 219 us).
 static bool use_routes(const ss2d_core_params* p, RoutePlan& r) {
     const int choice = core_kernel_choice();
     if (choice == 1 || !plan_routes(p, r)) return false;
     if (choice == 2) return true;
+    if (r.S != 8) return false;
     const long long L = p->H * p->W, chunk = 32 * r.S;
     const long long chunks = (L + chunk - 1) / chunk;
-    return r.S == 8 && 10 * L >= 9 * chunks * chunk && r.smem <= 32 * 1024;
+    if (100 * L >= 82 * chunks * chunk && r.smem <= 32 * 1024) return true;
+    if (r.smem > 100 * 1024) return false;
+    PlaneConfig c;
+    return L >= 4608 || !plan_planes(p, c) || c.vec <= 2;
 }
 
 int layer_norm_cf(const ss2d_norm_params* p, cudaStream_t st);
@@ -614,6 +655,10 @@ long long core_workspace_bytes(const ss2d_core_params* p) {
 struct CorePlan { bool routes; RoutePlan r; PlaneConfig c; };
 
 static bool plan_core(const ss2d_core_params* p, CorePlan& plan) {
+    if (p->stream_row && p->stream_row != p->H * p->W) {
+        plan.routes = true;
+        return plan_padded(p, plan.r);
+    }
     plan.routes = use_routes(p, plan.r);
     return plan.routes || plan_planes(p, plan.c);
 }
@@ -673,6 +718,32 @@ static int prepare_core(const ss2d_core_params* p, CorePlan& plan, long long& ne
         if (p->y_batch_stride || p->y_channel_stride) return SS2D_ENOTSUP;     // the un-normalised fp32 map is written dense
     }
     return SS2D_OK;
+}
+
+// Padded rows pay where the plane kernel would run with short segments.  Whole core, bf16: two-element segments or one, from 128
+// pixels up (13 x 13, 64 x 192 planes: 94 -> 70 us; 17 x 17: 155 -> 92; 27 x 29, 17 x 456: 330 -> 142; 57 x 57, 16 x 192, which went
+// through the operators: 265 -> 184; but 9 x 9: 32 -> 37); seven-element ones from 200 pixels (35 x 35: 121 -> 80 us);
+// four-element ones of 16-bit maps from 480 (22 x 22: 99.5 -> 97; 54 x 54: 167 -> 147; but 18 x 18: 148 -> 154, and fp32 30 x 30:
+// 70 -> 81).  Above 76 KB of shared memory, two CTAs of four warps per SM, the operators are the faster form (91 x 91: 195
+// against 212 us).
+int core_prefers_padded_rows(const ss2d_core_params* p) {
+    if (!p || !dtype_ok(p->act_dtype) || p->N != 1 || p->B <= 0 || p->D <= 0 || p->H <= 0 || p->W <= 0 || p->H * p->W > 65536) return 0;
+    ss2d_core_params q = *p;
+    const long long L = p->H * p->W, cs = p->x_channel_stride ? p->x_channel_stride : L;
+    void* some = (void*)(uintptr_t)4096;
+    q.stream_row = 0;
+    for (int k = 0; k < 4; ++k) {
+        q.delta[k] = q.Bm[k] = q.Cm[k] = some;
+        q.delta_batch_stride[k] = p->x_batch_stride; q.delta_channel_stride[k] = cs; q.bc_batch_stride[k] = p->x_batch_stride;
+    }
+    RoutePlan r;
+    PlaneConfig c;
+    if (use_routes(&q, r)) return 0;
+    const bool plane = plan_planes(&q, c);
+    const size_t smem = (size_t)((L + 7) / 8 * 8) * (8 + 2 * dtype_size(p->act_dtype));
+    if (L < 128 || smem > 76 * 1024) return 0;
+    if (!plane) return 1;
+    return c.vec <= 2 || (c.vec == 7 && L >= 200) || (c.vec == 4 && L >= 480 && p->act_dtype != SS2D_F32);
 }
 
 int core_supported(const ss2d_core_params* p) {

@@ -41,37 +41,61 @@ static Tensor linear_cm(const Tensor& w, const Tensor& x, int64_t S) {      // x
 
 // -------------------------------------------------------------------------------------------- the core
 // Route streams: delta and B / C rows of the two orientations (even: routes 0, 2; odd: 1, 3) and two routes each.
-struct Streams { Tensor bc, delta; bool cm; };
+struct Streams { Tensor bc, delta; bool cm; int64_t pad; };      // pad: elements per image row, 0: dense
+
+// Whether the streams' rows are better padded (the library's planner decides).
+static bool prefers_padded(const CoreW& w, at::ScalarType type, bool cm, int64_t B, int64_t H, int64_t W, int64_t S) {
+    ss2d_core_params q = {};
+    q.x = (void*)(intptr_t)4096;                 // an aligned address: the query dereferences nothing
+    q.B = B; q.D = w.D; q.H = H; q.W = W; q.N = w.N; q.act_dtype = dtype_code(type);
+    q.x_batch_stride = cm ? H * W : w.D * H * W; q.x_channel_stride = cm ? S : H * W;
+    return ss2d_core_prefers_padded_rows(&q) != 0;
+}
 
 // x: channel-major, or (B, D, L) with S = L
-static Streams project(const Tensor& x, bool cm, int64_t B, int64_t H, int64_t W, int64_t S, const CoreW& w) {
+static Streams project(const Tensor& x, bool cm, int64_t B, int64_t H, int64_t W, int64_t S, const CoreW& w, bool padding) {
     const int64_t D = w.D, R = w.R, N = w.N, C = R + 2 * N, L = H * W;
     ss2d_expand_params p = {};
     Streams s;
     s.cm = cm;
+    s.pad = padding && prefers_padded(w, x.scalar_type(), cm, B, H, W, S) ? round8(L) : 0;
     Tensor xd;
     auto at_el = [](const Tensor& t, int64_t i) { return (char*)t.data_ptr() + i * t.element_size(); };
     if (cm) {
         xd = linear_cm(w.wx, x.view({D, S}), S);
         p.x_dbl_batch_stride = L; p.x_dbl_route_stride = C * S; p.x_dbl_row_stride = S;
-        s.delta = at::empty({2, 2, D, S}, x.options());
-        s.bc = at::empty({2, 2, 2 * N, S}, x.options());
-        for (int k = 0; k < 4; ++k) {
-            const int64_t i = (k % 2) * 2 + k / 2;
-            p.delta[k] = at_el(s.delta, i * D * S); p.delta_batch_stride[k] = L; p.delta_channel_stride[k] = S;
-            p.bc[k] = at_el(s.bc, i * 2 * N * S); p.bc_batch_stride[k] = L; p.bc_row_stride[k] = S;
+        if (!s.pad) {
+            s.delta = at::empty({2, 2, D, S}, x.options());
+            s.bc = at::empty({2, 2, 2 * N, S}, x.options());
+            for (int k = 0; k < 4; ++k) {
+                const int64_t i = (k % 2) * 2 + k / 2;
+                p.delta[k] = at_el(s.delta, i * D * S); p.delta_batch_stride[k] = L; p.delta_channel_stride[k] = S;
+                p.bc[k] = at_el(s.bc, i * 2 * N * S); p.bc_batch_stride[k] = L; p.bc_row_stride[k] = S;
+            }
+            p.padded_rows = S > B * L;
         }
-        p.padded_rows = S > B * L;
     } else {
         xd = at::matmul(w.wx, x.view({B, D, L}));
         p.x_dbl_batch_stride = 4 * C * L; p.x_dbl_route_stride = C * L; p.x_dbl_row_stride = L;
-        s.delta = at::empty({2, B, 2, D, L}, x.options());
-        s.bc = at::empty({2, B, 2, 2 * N, L}, x.options());
-        for (int k = 0; k < 4; ++k) {
-            const int64_t j = k % 2, i = k / 2;
-            p.delta[k] = at_el(s.delta, (j * B * 2 + i) * D * L); p.delta_batch_stride[k] = 2 * D * L;
-            p.bc[k] = at_el(s.bc, (j * B * 2 + i) * 2 * N * L); p.bc_batch_stride[k] = 4 * N * L;
+        if (!s.pad) {
+            s.delta = at::empty({2, B, 2, D, L}, x.options());
+            s.bc = at::empty({2, B, 2, 2 * N, L}, x.options());
+            for (int k = 0; k < 4; ++k) {
+                const int64_t j = k % 2, i = k / 2;
+                p.delta[k] = at_el(s.delta, (j * B * 2 + i) * D * L); p.delta_batch_stride[k] = 2 * D * L;
+                p.bc[k] = at_el(s.bc, (j * B * 2 + i) * 2 * N * L); p.bc_batch_stride[k] = 4 * N * L;
+            }
         }
+    }
+    if (s.pad) {            // rows of an image padded: one (route, channel, image, row) layout for either layout of x
+        const int64_t n = B * s.pad;
+        s.delta = at::empty({4, D, n}, x.options());
+        s.bc = at::empty({4, 2 * N, n}, x.options());
+        for (int k = 0; k < 4; ++k) {
+            p.delta[k] = at_el(s.delta, k * D * n); p.delta_batch_stride[k] = s.pad; p.delta_channel_stride[k] = n;
+            p.bc[k] = at_el(s.bc, k * 2 * N * n); p.bc_batch_stride[k] = s.pad; p.bc_row_stride[k] = n;
+        }
+        p.image_row = s.pad;
     }
     p.x_dbl = xd.data_ptr(); p.dt_weight = w.wdt.data_ptr();
     p.B = B; p.D = D; p.R = R; p.N = N; p.H = H; p.W = W; p.act_dtype = dtype_code(x);
@@ -88,7 +112,11 @@ static ss2d_core_params core_params(const Tensor& x, const Streams& s, const Cor
     p.x = x.data_ptr();
     for (int k = 0; k < 4; ++k) {
         const int64_t j = k % 2, i = k / 2;
-        if (s.cm) {
+        if (s.pad) {
+            const int64_t n = B * s.pad;
+            p.delta[k] = (char*)s.delta.data_ptr() + k * D * n * e; p.delta_batch_stride[k] = s.pad; p.delta_channel_stride[k] = n;
+            p.Bm[k] = (char*)s.bc.data_ptr() + k * 2 * N * n * e; p.Cm[k] = (char*)p.Bm[k] + N * n * e; p.bc_batch_stride[k] = s.pad;
+        } else if (s.cm) {
             p.delta[k] = (char*)s.delta.data_ptr() + (j * 2 + i) * D * S * e; p.delta_batch_stride[k] = L; p.delta_channel_stride[k] = S;
             p.Bm[k] = (char*)s.bc.data_ptr() + (j * 2 + i) * 2 * N * S * e; p.Cm[k] = (char*)p.Bm[k] + N * S * e; p.bc_batch_stride[k] = L;
         } else {
@@ -98,12 +126,14 @@ static ss2d_core_params core_params(const Tensor& x, const Streams& s, const Cor
     }
     p.A = w.A.data_ptr(); p.Dskip = w.Ds.data_ptr(); p.delta_bias = w.bias.data_ptr(); p.ln_weight = ptr(w.lnw); p.ln_bias = ptr(w.lnb);
     p.B = B; p.D = D; p.H = H; p.W = W; p.N = N; p.act_dtype = dtype_code(x); p.ln_eps = (float)w.eps;
+    p.stream_row = s.pad;
     if (s.cm) { p.x_batch_stride = p.y_batch_stride = L; p.x_channel_stride = p.y_channel_stride = S; }
     return p;
 }
 
-// Whether ss2d_core_fwd takes the map (its planner decides from sizes, strides and types).
-static bool core_takes(const CoreW& w, at::ScalarType type, bool cm, int64_t B, int64_t H, int64_t W, int64_t S) {
+// Whether ss2d_core_fwd takes the map (its planner decides from sizes, strides and types); `padding`: with padded rows too.
+static bool core_takes(const CoreW& w, at::ScalarType type, bool cm, int64_t B, int64_t H, int64_t W, int64_t S, bool padding) {
+    if (padding && prefers_padded(w, type, cm, B, H, W, S)) return true;
     const int64_t L = H * W;
     ss2d_core_params p = {};
     void* some = (void*)(intptr_t)4096;          // an aligned address: the query dereferences nothing
@@ -170,9 +200,9 @@ static Tensor core_by_operators(const Tensor& x, bool cm, int64_t B, int64_t H, 
 
 static Tensor core_run(const Tensor& x, bool cm, int64_t B, int64_t H, int64_t W, int64_t S, const CoreW& w, bool with_norm, at::ScalarType out_type,
                        Tensor workspace, Tensor out) {
-    if (!core_takes(w, x.scalar_type(), cm, B, H, W, S) || (cm && !with_norm))
+    if (!core_takes(w, x.scalar_type(), cm, B, H, W, S, true) || (cm && !with_norm))
         return core_by_operators(x, cm, B, H, W, S, w, with_norm, out_type, out);
-    const Streams s = project(x, cm, B, H, W, S, w);
+    const Streams s = project(x, cm, B, H, W, S, w, true);
     if (!out.defined()) out = at::empty_like(x, x.options().dtype(out_type));
     ss2d_core_params p = core_params(x, s, w, B, H, W, S);
     p.y = out.data_ptr(); p.y_dtype = dtype_code(out); p.with_norm = with_norm;
@@ -413,7 +443,7 @@ void bind_backbone(pybind11::module_& m) {
           [](const Tensor& x, const CoreW& w, bool cm) {
               const int64_t B = x.size(cm ? 1 : 0), H = x.size(2), W = x.size(3);
               const c10::cuda::OptionalCUDAGuard guard(x.device());
-              const Streams s = project(x, cm, B, H, W, cm ? B * H * W : H * W, w);
+              const Streams s = project(x, cm, B, H, W, cm ? B * H * W : H * W, w, false);
               return std::make_pair(s.bc, s.delta);
           }, release());
     m.def("core_takes",
@@ -421,7 +451,7 @@ void bind_backbone(pybind11::module_& m) {
               CoreW w;
               w.D = shape[cm ? 0 : 1]; w.N = d_state;
               const int64_t B = shape[cm ? 1 : 0], L = shape[2] * shape[3];
-              return core_takes(w, type, cm, B, shape[2], shape[3], cm ? B * L : L);
+              return core_takes(w, type, cm, B, shape[2], shape[3], cm ? B * L : L, false);      // of dense streams
           });
     py::class_<Backbone>(m, "Backbone")
         .def(py::init<>())

@@ -408,8 +408,58 @@ static long long expand_run(const ss2d_expand_params* p) {
 
 long long route_expand_workspace_bytes(const ss2d_expand_params* p) {
     if (!p || !dtype_ok(p->act_dtype) || p->B <= 0 || p->R <= 0 || p->N <= 0 || p->H <= 0 || p->W <= 0) return -1;
+    if (p->image_row) return 4 * (p->R + 2 * p->N) * p->B * p->image_row * (long long)dtype_size(p->act_dtype);
     if (!transpose_fits(p) || p->H == 1 || p->W == 1) return 0;
     return 2 * (p->R + 2 * p->N) * expand_run(p) * (long long)dtype_size(p->act_dtype);
+}
+
+// All projected rows in the orientation order of their route (pixel order for routes 0, 2, column-major for 1, 3), a row of an
+// image padded to `pad` elements with zeros: (4, C, B, pad).  A warp per plane; small next to what the expansion writes.
+template <typename T>
+__global__ void __launch_bounds__(256) orient_rows_kernel(const TransArgs a, const int pad) {
+    extern __shared__ __align__(16) unsigned char traw[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int P = a.W | 1;
+    T* tile = reinterpret_cast<T*>(traw) + (size_t)warp * a.H * P;
+    const T zero = from_f<T>(0.f);
+    for (int pid = blockIdx.x * nwarps + warp; pid < a.planes; pid += gridDim.x * nwarps) {
+        const int b = pid % a.B, kc = pid / a.B, k = kc / a.C, c = kc - k * a.C;
+        const T* __restrict__ src = (const T*)a.xd + k * a.xd_ks + b * a.xd_bs + c * a.xd_rs;
+        T* __restrict__ dst = (T*)a.xt + (long long)pid * pad;
+        if (k & 1) {
+#pragma unroll 4
+            for (int e = lane; e < a.L; e += 32) { const int h = e / a.W; tile[h * P + (e - h * a.W)] = src[e]; }
+            __syncwarp();
+#pragma unroll 4
+            for (int q = lane; q < pad; q += 32) { const int w = q / a.H; dst[q] = q < a.L ? tile[(q - w * a.H) * P + w] : zero; }
+            __syncwarp();
+        } else {
+#pragma unroll 4
+            for (int e = lane; e < pad; e += 32) dst[e] = e < a.L ? src[e] : zero;
+        }
+    }
+}
+
+template <typename T>
+static int launch_orient(const ss2d_expand_params* p, cudaStream_t st) {
+    TransArgs t;
+    t.xd = p->x_dbl; t.xt = p->workspace;
+    t.xd_bs = p->x_dbl_batch_stride; t.xd_ks = p->x_dbl_route_stride; t.xd_rs = p->x_dbl_row_stride ? p->x_dbl_row_stride : p->H * p->W;
+    t.C = (int)(p->R + 2 * p->N); t.B = (int)p->B; t.H = (int)p->H; t.W = (int)p->W; t.L = (int)(p->H * p->W); t.xt_rs = 0; t.vec_ok = 0;
+    if (4LL * t.C * t.B > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
+    t.planes = 4 * t.C * t.B;
+    const size_t plane_bytes = (size_t)t.H * (t.W | 1) * sizeof(T);
+    if (plane_bytes > 200 * 1024) return SS2D_ENOTSUP;
+    int warps = (int)(48 * 1024 / plane_bytes);
+    warps = warps < 1 ? 1 : warps > 8 ? 8 : warps;
+    auto kern = orient_rows_kernel<T>;
+    const size_t smem = plane_bytes * warps;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
+    long long ctas = (t.planes + warps - 1) / warps;
+    if (ctas > 148 * 16) ctas = 148 * 16;
+    kern<<<(unsigned)ctas, warps * 32, smem, st>>>(t, (int)p->image_row);
+    count_launch();
+    return check_launch();
 }
 
 template <typename T>
@@ -453,6 +503,21 @@ int route_expand(const ss2d_expand_params* p, cudaStream_t st) {
         if (!aligned_to(p->delta[k], s) || !aligned_to(p->bc[k], s)) return SS2D_EINVAL_ALIGN;
         if (p->B > 1 && (p->delta_batch_stride[k] < L || p->bc_batch_stride[k] < L)) return SS2D_EINVAL_STRIDE;
         if ((p->delta_channel_stride[k] && p->delta_channel_stride[k] < L) || (p->bc_row_stride[k] && p->bc_row_stride[k] < L)) return SS2D_EINVAL_STRIDE;
+    }
+    if (p->image_row) {
+        const long long Lp = p->image_row;
+        if (Lp % 8 != 0 || Lp < L || p->B * Lp > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
+        for (int k = 0; k < 4; ++k)
+            if (p->delta_batch_stride[k] != Lp || p->bc_batch_stride[k] != Lp || p->delta_channel_stride[k] < p->B * Lp || p->bc_row_stride[k] < p->B * Lp)
+                return SS2D_EINVAL_STRIDE;
+        if (!p->workspace || p->workspace_bytes < route_expand_workspace_bytes(p)) return SS2D_EWORKSPACE;
+        if (!aligned_to(p->workspace, 16)) return SS2D_EINVAL_ALIGN;
+        const int rc = p->act_dtype == SS2D_F32 ? launch_orient<float>(p, st) : p->act_dtype == SS2D_BF16 ? launch_orient<__nv_bfloat16>(p, st) : launch_orient<__half>(p, st);
+        if (rc != SS2D_OK) return rc;
+        ss2d_expand_params q = *p;        // the oriented rows as one long row per channel
+        q.x_dbl = p->workspace; q.x_dbl_batch_stride = Lp; q.x_dbl_row_stride = p->B * Lp; q.x_dbl_route_stride = C * p->B * Lp;
+        q.H = 1; q.W = Lp; q.image_row = 0; q.workspace = nullptr; q.workspace_bytes = 0; q.padded_rows = 0;
+        return route_expand(&q, st);
     }
     // images adjacent in every tensor (channel-major maps): one run of B*L pixels per row, so that the
     // vector width does not depend on the size of a single map
