@@ -19,6 +19,7 @@
 //
 // Every wait on an mbarrier is bounded: when one runs out the kernel raises an error flag in mapped host memory, every
 // role leaves its loop, TMEM is released and the kernel returns; the host reports SS2D_ECUDA on the next call.
+#include "linear_small.cuh"
 #include "tc05.cuh"
 
 namespace ss2d {
@@ -261,6 +262,7 @@ int linear_supported(const ss2d_linear_params* p) {
 int linear_fwd(const ss2d_linear_params* p, cudaStream_t st) {
     const int rc = linear_supported(p);
     if (rc != SS2D_OK) return rc;
+    if (linear_small_takes(p)) return p->dtype == SS2D_BF16 ? launch_linear_small<__nv_bfloat16>(p, st) : launch_linear_small<__half>(p, st);
     if (p->dtype == SS2D_BF16) return launch_linear<__nv_bfloat16>(p, st);
     return launch_linear<__half>(p, st);
 }

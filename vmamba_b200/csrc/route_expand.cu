@@ -299,7 +299,10 @@ static int launch_expand_mma(ExpandArgs a, cudaStream_t st) {
     // Eight pixel tiles per CTA: measured over the ten launches of the 14 x 14 and 7 x 7 stages of a batch-128
     // forward, 4 and 8 tiles are equal (253 / 255 us), 16 and more leave too few CTAs, 1 or 2 re-stage the weights
     // too often.
-    const int per = kMmaTilesPerCta;
+    // Fewer where that leaves SMs idle.
+    const long long slices = 4 * ((a.D + kDChunk - 1) / kDChunk);
+    int per = kMmaTilesPerCta;
+    while (per > 1 && a.B * ((tiles_per_run + per - 1) / per) * slices < 148 * 2) per /= 2;
     a.mma_tiles = per;
     const long long tiles = (long long)a.B * ((tiles_per_run + per - 1) / per);
     if (tiles > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
