@@ -4,12 +4,7 @@
 // to a multiple of eight elements, so that every projection is ONE GEMM with aligned rows for any batch and map size (14 x 14
 // and 7 x 7 maps of one image: 196 and 49 pixels per row sent the library to its unaligned kernels).  The padding takes
 // part in the projections and the elementwise kernels and is never looked at.
-#include <cublasLt.h>
-
-#include <array>
 #include <map>
-#include <memory>
-#include <mutex>
 
 #include "host_common.h"
 
@@ -17,73 +12,22 @@ namespace host {
 
 static int64_t round8(int64_t n) { return (n + 7) / 8 * 8; }
 
-// The library's GEMM of 16-bit maps through cublasLt, with the algorithm that its heuristics choose kept per shape: the choice
-// costs the host about 8 us on each cublasGemmEx or at::mm, more than many of a backbone's products run for.  The table is
-// bounded; an entry is a few hundred bytes.
-struct GemmPlan {
-    cublasLtMatmulDesc_t op = nullptr;
-    cublasLtMatrixLayout_t a = nullptr, b = nullptr, c = nullptr;
-    cublasLtMatmulAlgo_t algo;
-    size_t workspace = 0;
-    bool ok = false;
-    GemmPlan(cublasLtHandle_t handle, cudaDataType_t t, int64_t M, int64_t K, int64_t S) {
-        // row-major (M, S) = (M, K) . (K, S) as column-major (S, M) = (S, K) . (K, M)
-        if (cublasLtMatmulDescCreate(&op, CUBLAS_COMPUTE_32F, CUDA_R_32F) != CUBLAS_STATUS_SUCCESS) return;
-        if (cublasLtMatrixLayoutCreate(&a, t, S, K, S) != CUBLAS_STATUS_SUCCESS || cublasLtMatrixLayoutCreate(&b, t, K, M, K) != CUBLAS_STATUS_SUCCESS ||
-            cublasLtMatrixLayoutCreate(&c, t, S, M, S) != CUBLAS_STATUS_SUCCESS)
-            return;
-        cublasLtMatmulPreference_t pref = nullptr;
-        if (cublasLtMatmulPreferenceCreate(&pref) != CUBLAS_STATUS_SUCCESS) return;
-        const size_t most = 32 << 20;
-        cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &most, sizeof(most));
-        cublasLtMatmulHeuristicResult_t got;
-        int n = 0;
-        ok = cublasLtMatmulAlgoGetHeuristic(handle, op, a, b, c, c, pref, 1, &got, &n) == CUBLAS_STATUS_SUCCESS && n == 1;
-        if (ok) { algo = got.algo; workspace = got.workspaceSize; }
-        cublasLtMatmulPreferenceDestroy(pref);
-    }
-    GemmPlan(const GemmPlan&) = delete;
-    ~GemmPlan() {
-        if (a) cublasLtMatrixLayoutDestroy(a);
-        if (b) cublasLtMatrixLayoutDestroy(b);
-        if (c) cublasLtMatrixLayoutDestroy(c);
-        if (op) cublasLtMatmulDescDestroy(op);
-    }
-};
-
+// The library's GEMM as at::mm calls it (same handle, types, math mode), without at::mm: its dispatch and shape bookkeeping take
+// about 10 us, more than most of a backbone's products run for.
 Tensor matmul_rows(const Tensor& w, const Tensor& x) {
     const auto type = x.scalar_type();
     const auto& ctx = at::globalContext();
-    const auto any = at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK;      // torch's default; other choices: at::mm
-    const bool plain = type == at::kBFloat16 ? ctx.allowBF16ReductionCuBLAS() == any
-                       : type == at::kHalf   ? ctx.allowFP16ReductionCuBLAS() == any && !ctx.allowFP16AccumulationCuBLAS()
+    const bool plain = type == at::kBFloat16 ? ctx.allowBF16ReductionCuBLAS() == at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK
+                       : type == at::kHalf   ? ctx.allowFP16ReductionCuBLAS() == at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK
                                              : false;
+    if (!plain || !w.is_contiguous() || !x.is_contiguous()) return at::mm(w, x);
     const int64_t M = w.size(0), K = w.size(1), S = x.size(1);
-    auto aligned = [](const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 255) == 0; };
-    if (!plain || ctx.deterministicAlgorithms() || !w.is_contiguous() || !x.is_contiguous() || S % 8 != 0 || K % 8 != 0 || !aligned(w) || !aligned(x))
-        return at::mm(w, x);
+    Tensor y = at::empty({M, S}, x.options());
     const cudaDataType_t t = type == at::kBFloat16 ? CUDA_R_16BF : CUDA_R_16F;
-    cublasLtHandle_t handle = at::cuda::getCurrentCUDABlasLtHandle();
-    static std::mutex lock;
-    static std::map<std::array<int64_t, 5>, std::shared_ptr<GemmPlan>> plans;
-    std::shared_ptr<GemmPlan> plan;
-    {
-        const std::array<int64_t, 5> key = {x.get_device(), (int64_t)t, M, K, S};
-        std::lock_guard<std::mutex> hold(lock);
-        auto it = plans.find(key);
-        if (it == plans.end()) {
-            if (plans.size() >= 1024) plans.clear();
-            it = plans.emplace(key, std::make_shared<GemmPlan>(handle, t, M, K, S)).first;
-        }
-        plan = it->second;
-    }
-    if (!plan->ok) return at::mm(w, x);
-    Tensor y = at::empty({M, S}, x.options()), ws;
-    if (plan->workspace) ws = bytes((int64_t)plan->workspace, x);
     const float one = 1.f, zero = 0.f;
-    const cublasStatus_t rc = cublasLtMatmul(handle, plan->op, &one, x.data_ptr(), plan->a, w.data_ptr(), plan->b, &zero, y.data_ptr(), plan->c, y.data_ptr(), plan->c,
-                                             &plan->algo, ptr(ws), plan->workspace, (cudaStream_t)stream_of(x));
-    TORCH_CHECK(rc == CUBLAS_STATUS_SUCCESS, "cublasLtMatmul failed with status ", (int)rc);
+    const cublasStatus_t rc = cublasGemmEx(at::cuda::getCurrentCUDABlasHandle(), CUBLAS_OP_N, CUBLAS_OP_N, (int)S, (int)M, (int)K, &one, x.data_ptr(), t, (int)S,
+                                           w.data_ptr(), t, (int)K, &zero, y.data_ptr(), t, (int)S, CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT_TENSOR_OP);
+    TORCH_CHECK(rc == CUBLAS_STATUS_SUCCESS, "cublasGemmEx failed with status ", (int)rc);
     return y;
 }
 
