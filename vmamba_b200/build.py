@@ -72,7 +72,7 @@ def _link_host(objs):
     from torch.utils import cpp_extension
     libs = [f"-L{p}" for p in cpp_extension.library_paths()]
     cmd = ["g++", "-shared", "-o", HOST_PATH, *objs, f"-L{HERE}", "-l:libss2d_b200.so", "-Wl,-rpath,$ORIGIN", *libs,
-           "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda", "-lcublas"]
+           "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link of the host extension failed:\n{r.stdout}{r.stderr}")

@@ -12,25 +12,6 @@ namespace host {
 
 static int64_t round8(int64_t n) { return (n + 7) / 8 * 8; }
 
-// The library's GEMM as at::mm calls it (same handle, types, math mode), without at::mm: its dispatch and shape bookkeeping take
-// about 10 us, more than most of a backbone's products run for.
-Tensor matmul_rows(const Tensor& w, const Tensor& x) {
-    const auto type = x.scalar_type();
-    const auto& ctx = at::globalContext();
-    const bool plain = type == at::kBFloat16 ? ctx.allowBF16ReductionCuBLAS() == at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK
-                       : type == at::kHalf   ? ctx.allowFP16ReductionCuBLAS() == at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK
-                                             : false;
-    if (!plain || !w.is_contiguous() || !x.is_contiguous()) return at::mm(w, x);
-    const int64_t M = w.size(0), K = w.size(1), S = x.size(1);
-    Tensor y = at::empty({M, S}, x.options());
-    const cudaDataType_t t = type == at::kBFloat16 ? CUDA_R_16BF : CUDA_R_16F;
-    const float one = 1.f, zero = 0.f;
-    const cublasStatus_t rc = cublasGemmEx(at::cuda::getCurrentCUDABlasHandle(), CUBLAS_OP_N, CUBLAS_OP_N, (int)S, (int)M, (int)K, &one, x.data_ptr(), t, (int)S,
-                                           w.data_ptr(), t, (int)K, &zero, y.data_ptr(), t, (int)S, CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT_TENSOR_OP);
-    TORCH_CHECK(rc == CUBLAS_STATUS_SUCCESS, "cublasGemmEx failed with status ", (int)rc);
-    return y;
-}
-
 struct CoreW {
     Tensor wx, wdt, A, Ds, bias, lnw, lnb;       // (4 (R + 2N), D), (4, D, R), (4 D, N), (4 D), (4 D), (D), (D)
     int64_t N = 0, R = 0, D = 0;
@@ -55,7 +36,7 @@ static Tensor linear_cm(const Tensor& w, const Tensor& x, int64_t S) {      // x
             return y;
         }
     }
-    return matmul_rows(w, x);
+    return at::mm(w, x);
 }
 
 // -------------------------------------------------------------------------------------------- the core
@@ -323,7 +304,7 @@ private:
     static Map pw(const Tensor& w, const Map& x) {                    // 1 x 1 projection (vmamba.py:1060-1064)
         Map y = x;
         y.C = w.size(0);
-        y.t = matmul_rows(w, x.t);
+        y.t = at::mm(w, x.t);
         return y;
     }
     Map dwconv(const Map& x, const Tensor& w) const {

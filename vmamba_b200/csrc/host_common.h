@@ -1,7 +1,6 @@
 // Shared parts of the host extension (_host.so): the torch side of libss2d_b200.so.
 // Every function here only prepares arguments and launches; the kernels are behind the C interface of ss2d_b200.h.
 #pragma once
-#include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
@@ -57,9 +56,6 @@ std::vector<Tensor> scan_bwd_into(Tensor u, Tensor delta, Tensor A, Tensor B, Te
 Tensor cross_scan(const Tensor& x, int64_t scans);       // (B, C, H, W) -> (B, 4, C, L)
 Tensor cross_merge(const Tensor& ys, int64_t scans);     // (B, 4, C, H, W) -> (B, C, L)
 int64_t scan_ratio(const Tensor& u, const Tensor& delta);
-
-// host_backbone.cpp: w (M, K) . x (K, S), both dense, by the library
-Tensor matmul_rows(const Tensor& w, const Tensor& x);
 
 // host_core.cpp: CrossScan (op 0), CrossMerge (1), rows into (2) and out of (3) route order, rows of a route `stride` apart
 Tensor cross(const Tensor& in, Tensor out, int64_t B, int64_t C, int64_t H, int64_t W, int64_t stride, int op);
