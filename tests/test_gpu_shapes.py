@@ -87,8 +87,9 @@ def test_cross_padded_rows(vb, shape, scans, dt):
     assert np.array_equal(host(back[..., :L]), ys)
 
 
-@pytest.mark.parametrize("D,H,W,dt", [(6, 13, 13, "f32"), (5, 8, 17, "bf16"), (9, 27, 29, "f16"), (3, 57, 57, "bf16"), (4, 21, 21, "bf16"), (3, 54, 54, "f16"),
-                                      (3, 36, 29, "f32"), (2, 75, 75, "bf16"), (3, 54, 80, "bf16"), (2, 96, 96, "bf16"), (7, 9, 9, "bf16"), (2, 101, 97, "f32")])
+@pytest.mark.parametrize("D,H,W,dt", [(16, 13, 13, "f32"), (15, 8, 17, "bf16"), (19, 27, 29, "f16"), (13, 57, 57, "bf16"), (14, 21, 21, "bf16"),
+                                      (13, 54, 54, "f16"), (13, 36, 29, "f32"), (12, 75, 75, "bf16"), (13, 54, 80, "bf16"), (12, 96, 96, "bf16"),
+                                      (17, 9, 9, "bf16"), (12, 101, 97, "f32")])
 def test_core_any_plane_size(vb, D, H, W, dt):
     """The fused core on planes of any size (padded rows, both layouts) against the oracle."""
     c = _core_case(2, D, H, W, N=1, seed=H * W, Cmodel=24)
@@ -103,7 +104,7 @@ def test_core_any_plane_size(vb, D, H, W, dt):
     assert torch.equal(y, vb.ss2d_core(x, w))
 
 
-@pytest.mark.parametrize("D,N,H,W", [(6, 1, 14, 14), (7, 1, 13, 17), (4, 16, 5, 7), (3, 4, 33, 31), (2, 1, 1, 9)])
+@pytest.mark.parametrize("D,N,H,W", [(16, 1, 14, 14), (17, 1, 13, 17), (14, 16, 5, 7), (13, 4, 33, 31), (12, 1, 1, 9)])
 def test_core_training_node(vb, D, N, H, W):
     """The native node against the separate statements (fp32, which `oflex=False` still runs through)."""
     from vmamba_b200 import fused
@@ -118,7 +119,7 @@ def test_core_training_node(vb, D, N, H, W):
         assert a.shape == b.shape and O.max_rel_err(host(a), host(b)) <= 1e-4
 
 
-@pytest.mark.parametrize("B,D,L", [(1, 1, 1), (3, 96, 49), (2, 97, 64), (40, 96, 784), (2, 300, 33), (1, 1000, 130)])
+@pytest.mark.parametrize("B,D,L", [(1, 8, 1), (3, 96, 49), (2, 97, 64), (40, 96, 784), (2, 300, 33), (1, 1000, 130)])
 @pytest.mark.parametrize("dt", ["f32", "bf16"])
 def test_layer_norm_backward(B, D, L, dt):
     from vmamba_b200 import _lib

@@ -115,8 +115,8 @@ __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArg
         const int ig = first + i * kStep;
 #pragma unroll
         for (int j = 0; j < 3; ++j) racc[((i * kN1Warps + warp) * 3 + j) * 32 + lane] = 0.f;
-        if (ig < gs && ln == 0) {
-            const int64_t r = (int64_t)k * gs + ig;
+        if (ln == 0) {                                           // spare lanes of a shared warp: the group's last row
+            const int64_t r = (int64_t)k * gs + min(ig, gs - 1);
             const float An = __ldg(a.A + r);
             float e = 0.f;
             for (int j = a.S - 1; j > seg; --j)                  // what the segments behind leave
