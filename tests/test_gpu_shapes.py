@@ -87,6 +87,19 @@ def test_cross_padded_rows(vb, shape, scans, dt):
     assert np.array_equal(host(back[..., :L]), ys)
 
 
+@pytest.mark.parametrize("dt", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("scans", [0, 1, 2, 3])
+@pytest.mark.parametrize("H,W", [(48, 32), (40, 52), (32, 64), (64, 64), (66, 68), (130, 36), (72, 260)])
+def test_cross_merge_of_whole_planes(vb, H, W, scans, dt):
+    """Merge of planes with rows of whole vectors: one tile, several, ragged last ones, planes that do not fill a CTA."""
+    ys = np.random.default_rng(H * W).standard_normal((1, 4, 5, H, W), dtype=np.float32)
+    if dt != "f32":
+        ys = O._round_to(ys, dt)
+    got = host(vb.cross_merge_fn(dev(ys, TD[dt]), scans=scans)).reshape(1, 5, H * W)
+    want = O.cross_merge(ys, scans).reshape(1, 5, H * W)
+    assert np.abs(got - want).max() <= {"f32": 2e-6, "bf16": 0.1, "f16": 0.02}[dt]
+
+
 @pytest.mark.parametrize("D,H,W,dt", [(16, 13, 13, "f32"), (15, 8, 17, "bf16"), (19, 27, 29, "f16"), (13, 57, 57, "bf16"), (14, 21, 21, "bf16"),
                                       (13, 54, 54, "f16"), (13, 36, 29, "f32"), (12, 75, 75, "bf16"), (13, 54, 80, "bf16"), (12, 96, 96, "bf16"),
                                       (17, 9, 9, "bf16"), (12, 101, 97, "f32")])
