@@ -16,6 +16,9 @@
 // here), then thread (item, channel group) accumulates 4 channels x VEC pixels at a time with
 // the weights broadcast from shared memory; lanes of a warp hold consecutive items, so every
 // delta store is a full 512-byte line per channel.
+#include <algorithm>
+#include <cstring>
+
 #include "common.cuh"
 
 namespace ss2d {
@@ -140,100 +143,120 @@ __global__ void __launch_bounds__(kExpThreads) route_expand_kernel(const ExpandA
 }
 
 // ------------------------------------------------------------------------------------------------
-// Tensor-core variant for 16-bit maps: delta tile (128 channels x 64 pixels) = W (128 x R) . X (R x 64)
+// Tensor-core variant for 16-bit maps: delta tile (channels x pixels) = W (channels x R) . X (R x pixels)
 // with mma.sync m16n8k16 (fp32 accumulation, R zero-padded to a multiple of 16).  The contraction is
 // far too short for the tensor pipe to matter as arithmetic; what it buys is that the shared-memory
 // traffic and the issue slots of the FMA loop disappear, leaving the kernel with the write of delta.
-// Warp w owns channels [16 w, 16 w + 16) of the CTA's slice and all 64 pixels; the accumulators go
-// through a shared tile so that every channel row leaves as 16-byte vectors.
+//
+// A warp owns 16 channels and walks the pixels in blocks of 32.  The pixels of a block are dealt to the columns of the four
+// n8 operands so that a thread's accumulators are eight neighbouring pixels of two channels: column 2 t + e of operand n is pixel
+// 8 t + 2 n + e.  The results leave from registers as 16-byte vectors, 64 bytes of a row at a time, and a vector of x enters
+// shared memory as four words, 16 bytes apart; there is one barrier per tile of kMmaPix pixels.
+// Bound: HBM writes, and the bytes in flight: five CTAs of 256 threads to an SM where the contraction is short.  Against two
+// barriers a tile with the results through a shared tile: 64 x 192 planes of 28 x 28 28 -> 23 us (3.4 TB/s written), 15 launches
+// of 2 x 512 planes of 64 x 64 380 -> 311 us.
 constexpr int kMmaPix = 64;
-
 constexpr int kMmaTilesPerCta = 8;      // most pixel tiles per CTA: the staged weights then serve 512 pixels
 
-// PIX pixels per step.
-template <typename T, int KP, int PIX>
-__global__ void __launch_bounds__(256) route_expand_mma_kernel(const ExpandArgs a) {
-    constexpr int KPAD = KP + 8;                  // row pitch (elements) of the operand tiles: conflict-free fragment loads
-    constexpr int OPAD = PIX + 8;
+template <typename T> __device__ __forceinline__ uint32_t pack2(float x, float y) {
+    const T v[2] = {from_f<T>(x), from_f<T>(y)};
+    uint32_t w;
+    memcpy(&w, v, 4);
+    return w;
+}
+
+template <typename T, int KP>
+__global__ void __launch_bounds__(256, KP <= 32 ? 5 : 1) route_expand_mma_kernel(const ExpandArgs a) {
+    constexpr int PIX = kMmaPix;
+    constexpr int KPAD = KP + 8, XPAD = PIX + 8;       // pitches (elements): conflict-free fragment loads and vector stores
     __shared__ __align__(16) T Ws[kDChunk * KPAD];     // [channel][k]
-    __shared__ __align__(16) T Xt[PIX * KPAD];     // [pixel][k]
-    __shared__ __align__(16) T Os[kDChunk * OPAD];     // [channel][pixel]
+    __shared__ __align__(16) T Xs[2][KP * XPAD];       // [k][dealt pixel]
     const int k = blockIdx.y;
     const bool col = (k & 1) != 0 && a.H > 1 && a.W > 1;      // a single row or column: both orders are one
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, threads = blockDim.x, lane = tid & 31, warp = tid >> 5, slice = threads / 2;
     const int tiles_per_run = (a.L + PIX - 1) / PIX;
     const int groups_per_run = (tiles_per_run + a.mma_tiles - 1) / a.mma_tiles;
     const int b = blockIdx.x / groups_per_run;
     const int tile0 = (blockIdx.x - b * groups_per_run) * a.mma_tiles;
     const T* __restrict__ xd = (const T*)a.xd + (long long)k * a.xd_ks + (long long)b * a.xd_bs;
-    const int dc = blockIdx.z * kDChunk;
-    const int dn = min(kDChunk, a.D - dc);
+    const int dc = blockIdx.z * slice;
+    const int dn = min(slice, a.D - dc);
     const T zero = from_f<T>(0.f);
+
+    // one projected row of eight pixels, gathered column-major for the odd routes
+    auto fetch8 = [&](int row, int q) {
+        const T* rp = xd + (long long)row * a.xd_rs;
+        if (!col) return __ldg(reinterpret_cast<const uint4*>(rp + q));
+        if (a.xt)
+            return __ldg(reinterpret_cast<const uint4*>((const T*)a.xt + ((long long)(k >> 1) * a.C + row) * a.xt_rs + (long long)b * a.Limg + q));
+        __align__(16) T v[8];
+        const int img0 = (q / a.Limg) * a.Limg, qi = q - img0;
+        int w = qi / a.H, h = qi - w * a.H, base = img0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            v[j] = rp[base + h * a.W + w];
+            if (++h == a.H) { h = 0; if (++w == a.W) { w = 0; base += a.Limg; } }
+        }
+        return *reinterpret_cast<const uint4*>(v);
+    };
+    // The X tile is read into registers one step ahead: the loads of tile t + 1 are in flight while tile t is contracted,
+    // those of the first while the weights are staged.
+    constexpr int VR = PIX / 8;                        // vectors of a row
+    constexpr int NI = VR / 4;                         // of a thread: at least 4 KP threads
+    uint4 pre[NI];
+    auto load_tile = [&](int q0) {
+#pragma unroll
+        for (int n = 0; n < NI; ++n) {
+            const int i = tid + n * threads, r = i / VR, q = q0 + (i % VR) * 8;
+            if (r < a.R) pre[n] = q < a.L ? fetch8(r, q) : make_uint4(0u, 0u, 0u, 0u);      // L is a multiple of 8
+        }
+    };
+    auto store_tile = [&](T* xs) {
+#pragma unroll
+        for (int n = 0; n < NI; ++n) {
+            const int i = tid + n * threads, r = i / VR, c = i % VR;
+            if (r < a.R) {
+                uint32_t* x = reinterpret_cast<uint32_t*>(xs + r * XPAD + (c / 4) * 32) + c % 4;
+                x[0] = pre[n].x; x[4] = pre[n].y; x[8] = pre[n].z; x[12] = pre[n].w;
+            }
+        }
+    };
+    if (tile0 * PIX < a.L) load_tile(tile0 * PIX);
 
     // ---- weights of this channel slice, [channel][k], zero beyond R and beyond the slice ----------------
     const T* __restrict__ wk = (const T*)a.wdt + (long long)k * a.D * a.R;
     if ((a.R & 7) == 0 && (reinterpret_cast<uintptr_t>(wk) & 15) == 0) {       // rows of whole 16-byte pieces
-        for (int i = tid; i < kDChunk * (KP / 8); i += 256) {
+        for (int i = tid; i < slice * (KP / 8); i += threads) {
             const int dl = i / (KP / 8), r = (i - dl * (KP / 8)) * 8;
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
             if (dl < dn && r < a.R) v = __ldg(reinterpret_cast<const uint4*>(wk + (long long)(dc + dl) * a.R + r));
             *reinterpret_cast<uint4*>(&Ws[dl * KPAD + r]) = v;
         }
     } else {
-        for (int i = tid; i < kDChunk * KP; i += 256) {
+        for (int i = tid; i < slice * KP; i += threads) {
             const int dl = i / KP, r = i - dl * KP;
             Ws[dl * KPAD + r] = (dl < dn && r < a.R) ? wk[(long long)(dc + dl) * a.R + r] : zero;
         }
     }
-    // one projected row of eight pixels, gathered column-major for the odd routes
-    auto fetch8 = [&](int row, int q, T (&v)[8]) {
-        const T* rp = xd + (long long)row * a.xd_rs;
-        if (!col) {
-            *reinterpret_cast<uint4*>(v) = __ldg(reinterpret_cast<const uint4*>(rp + q));
-        } else if (a.xt) {
-            *reinterpret_cast<uint4*>(v) = __ldg(reinterpret_cast<const uint4*>(
-                (const T*)a.xt + ((long long)(k >> 1) * a.C + row) * a.xt_rs + (long long)b * a.Limg + q));
-        } else {
-            const int img0 = (q / a.Limg) * a.Limg, qi = q - img0;
-            int w = qi / a.H, h = qi - w * a.H, base = img0;
+    for (int i = tid; i < 2 * (KP - a.R) * XPAD; i += threads) {              // rows R .. KP - 1 are zero
+        const int s = i / ((KP - a.R) * XPAD);
+        Xs[s][a.R * XPAD + i - s * (KP - a.R) * XPAD] = zero;
+    }
+    if (tile0 * PIX < a.L) store_tile(Xs[0]);
+    __syncthreads();
+    const int g = lane >> 2, t4 = lane & 3, m0 = warp * 16;
+    uint32_t af[KP / 16][4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                v[j] = rp[base + h * a.W + w];
-                if (++h == a.H) { h = 0; if (++w == a.W) { w = 0; base += a.Limg; } }
-            }
-        }
-    };
-    const int g = lane >> 2, t4 = lane & 3;
-    const int m0 = warp * 16;
-    // X tile, transposed to [pixel][k]; rows R .. KP-1 are zero.  Consecutive threads take consecutive rows of the
-    // same eight pixels, so the transposed stores of a warp fall into consecutive words.  The tile is read from
-    // global memory into registers one step ahead: the loads of tile t+1 are in flight while tile t is contracted.
-    constexpr int NI = (KP * (PIX / 8) + 255) / 256;
-    T pre[NI][8];
-    auto load_tile = [&](int q0) {
-#pragma unroll
-        for (int n = 0; n < NI; ++n) {
-            const int i = tid + n * 256;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) pre[n][j] = zero;
-            if (i < KP * (PIX / 8)) {
-                const int p0 = (i / KP) * 8, r = i - (i / KP) * KP;
-                if (r < a.R && q0 + p0 < a.L) fetch8(r, q0 + p0, pre[n]);      // L is a multiple of 8: a chunk is wholly inside or outside
-            }
-        }
-    };
-    auto store_tile = [&]() {
-#pragma unroll
-        for (int n = 0; n < NI; ++n) {
-            const int i = tid + n * 256;
-            if (i < KP * (PIX / 8)) {
-                const int p0 = (i / KP) * 8, r = i - (i / KP) * KP;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) Xt[(p0 + j) * KPAD + r] = pre[n][j];
-            }
-        }
-    };
-    if (tile0 * PIX < a.L) { load_tile(tile0 * PIX); store_tile(); }
+    for (int k0 = 0; k0 < KP; k0 += 16) {
+        const T* w = Ws + (m0 + g) * KPAD + k0 + 2 * t4;
+        af[k0 / 16][0] = *reinterpret_cast<const uint32_t*>(w);
+        af[k0 / 16][1] = *reinterpret_cast<const uint32_t*>(w + 8 * KPAD);
+        af[k0 / 16][2] = *reinterpret_cast<const uint32_t*>(w + 8);
+        af[k0 / 16][3] = *reinterpret_cast<const uint32_t*>(w + 8 * KPAD + 8);
+    }
+    T* __restrict__ out = (T*)a.delta[k] + b * a.d_bs[k] + (long long)(dc + m0 + g) * a.d_cs[k] + t4 * 8;
+    const bool low = m0 + g < dn, high = m0 + g + 8 < dn;
+    const long long eight = 8 * a.d_cs[k];
     for (int tt = 0; tt < a.mma_tiles; ++tt) {
         const int q0 = (tile0 + tt) * PIX;
         if (q0 >= a.L) break;                        // uniform over the CTA
@@ -241,76 +264,65 @@ __global__ void __launch_bounds__(256) route_expand_mma_kernel(const ExpandArgs 
         if (has_next) load_tile(q0 + PIX);
         // ---- B / C rows pass through (first channel slice only) ---------------------------------------------
         if (blockIdx.z == 0) {
-            for (int i = tid; i < a.N2 * (PIX / 8); i += 256) {
-                const int n = i / (PIX / 8), p0 = (i - n * (PIX / 8)) * 8;
-                const int q = q0 + p0;
-                if (q >= a.L) continue;
-                T v[8];
-                fetch8(a.R + n, q, v);
-                *reinterpret_cast<uint4*>((T*)a.bc[k] + b * a.bc_bs[k] + (long long)n * a.bc_rs[k] + q) = *reinterpret_cast<const uint4*>(v);
+            for (int i = tid; i < a.N2 * VR; i += threads) {
+                const int n = i / VR, q = q0 + (i - n * VR) * 8;
+                if (q < a.L) *reinterpret_cast<uint4*>((T*)a.bc[k] + b * a.bc_bs[k] + (long long)n * a.bc_rs[k] + q) = fetch8(a.R + n, q);
             }
         }
-        __syncthreads();                             // X tile (and, first time, the weights) in place
-
-        // ---- 16 channels x 64 pixels per warp ---------------------------------------------------------------
-        float acc[PIX / 8][4];
+        const T* xs = Xs[tt & 1];
 #pragma unroll
-        for (int nt = 0; nt < PIX / 8; ++nt) { acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f; }
+        for (int p0 = 0; p0 < PIX; p0 += 32) {
+            float acc[4][4] = {};
 #pragma unroll
-        for (int k0 = 0; k0 < KP; k0 += 16) {
-            uint32_t af[4];
-            af[0] = *reinterpret_cast<const uint32_t*>(&Ws[(m0 + g) * KPAD + k0 + 2 * t4]);
-            af[1] = *reinterpret_cast<const uint32_t*>(&Ws[(m0 + g + 8) * KPAD + k0 + 2 * t4]);
-            af[2] = *reinterpret_cast<const uint32_t*>(&Ws[(m0 + g) * KPAD + k0 + 2 * t4 + 8]);
-            af[3] = *reinterpret_cast<const uint32_t*>(&Ws[(m0 + g + 8) * KPAD + k0 + 2 * t4 + 8]);
+            for (int k0 = 0; k0 < KP; k0 += 16) {
 #pragma unroll
-            for (int nt = 0; nt < PIX / 8; ++nt) {
-                uint32_t bf[2];
-                bf[0] = *reinterpret_cast<const uint32_t*>(&Xt[(nt * 8 + g) * KPAD + k0 + 2 * t4]);
-                bf[1] = *reinterpret_cast<const uint32_t*>(&Xt[(nt * 8 + g) * KPAD + k0 + 2 * t4 + 8]);
-                MmaK16<T>::run(acc[nt], af, bf);
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t f[4];
+                    const unsigned p = (unsigned)__cvta_generic_to_shared(xs + (k0 + (lane & 15)) * XPAD + p0 + h * 16 + (lane >> 4) * 8);
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                                 : "=r"(f[0]), "=r"(f[1]), "=r"(f[2]), "=r"(f[3]) : "r"(p) : "memory");
+                    const uint32_t f0[2] = {f[0], f[1]}, f1[2] = {f[2], f[3]};
+                    MmaK16<T>::run(acc[2 * h], af[k0 / 16], f0);
+                    MmaK16<T>::run(acc[2 * h + 1], af[k0 / 16], f1);
+                }
+            }
+            T* o = out + q0 + p0;
+            if (q0 + p0 + t4 * 8 < a.L) {
+                if (low)
+                    *reinterpret_cast<uint4*>(o) = make_uint4(pack2<T>(acc[0][0], acc[0][1]), pack2<T>(acc[1][0], acc[1][1]),
+                                                              pack2<T>(acc[2][0], acc[2][1]), pack2<T>(acc[3][0], acc[3][1]));
+                if (high)
+                    *reinterpret_cast<uint4*>(o + eight) = make_uint4(pack2<T>(acc[0][2], acc[0][3]), pack2<T>(acc[1][2], acc[1][3]),
+                                                                      pack2<T>(acc[2][2], acc[2][3]), pack2<T>(acc[3][2], acc[3][3]));
             }
         }
-        // ---- accumulators -> shared tile -> 16-byte stores along the pixels -----------------------------------
-#pragma unroll
-        for (int nt = 0; nt < PIX / 8; ++nt) {
-            T lo[2] = {from_f<T>(acc[nt][0]), from_f<T>(acc[nt][1])};
-            T hi[2] = {from_f<T>(acc[nt][2]), from_f<T>(acc[nt][3])};
-            *reinterpret_cast<uint32_t*>(&Os[(m0 + g) * OPAD + nt * 8 + 2 * t4]) = *reinterpret_cast<const uint32_t*>(lo);
-            *reinterpret_cast<uint32_t*>(&Os[(m0 + g + 8) * OPAD + nt * 8 + 2 * t4]) = *reinterpret_cast<const uint32_t*>(hi);
-        }
-        __syncthreads();                             // output tile complete; every read of the X tile is done
-        if (has_next) store_tile();                  // next X tile into the same buffer; the barrier at the top of the next step orders it
-        T* __restrict__ dout = (T*)a.delta[k] + b * a.d_bs[k] + q0;
-        for (int i = tid; i < kDChunk * (PIX / 8); i += 256) {
-            const int dl = i / (PIX / 8), p0 = (i - dl * (PIX / 8)) * 8;
-            if (dl < dn && q0 + p0 < a.L)
-                *reinterpret_cast<uint4*>(dout + (long long)(dc + dl) * a.d_cs[k] + p0) = *reinterpret_cast<const uint4*>(&Os[dl * OPAD + p0]);
-        }
-        // the barrier at the top of the next step orders the next writes of the output tile behind these reads
+        if (has_next) store_tile(Xs[(tt + 1) & 1]);  // its last readers passed the barrier of the step before
+        __syncthreads();
     }
 }
 
 template <typename T>
 static int launch_expand_mma(ExpandArgs a, cudaStream_t st) {
     const int kp = (a.R + 15) / 16 * 16;
-    const int pix = kMmaPix;          // 128 pixels per step were measured for the shortest contraction: 4 % slower
-    const long long tiles_per_run = (a.L + pix - 1) / pix;
+    const long long tiles_per_run = (a.L + kMmaPix - 1) / kMmaPix;
+    // equal slices of at most 128 channels, a warp for every 16 and threads enough for two vectors of the X tile each
+    const int cuts = (a.D + kDChunk - 1) / kDChunk;
+    const int threads = std::max(4 * kp, ((a.D + cuts - 1) / cuts + 15) / 16 * 32);
     // Eight pixel tiles per CTA: measured over the ten launches of the 14 x 14 and 7 x 7 stages of a batch-128
     // forward, 4 and 8 tiles are equal (253 / 255 us), 16 and more leave too few CTAs, 1 or 2 re-stage the weights
     // too often.
-    // Fewer where that leaves SMs idle.
-    const long long slices = 4 * ((a.D + kDChunk - 1) / kDChunk);
+    // Fewer where that leaves SMs idle; a run is cut into equal parts.
     int per = kMmaTilesPerCta;
-    while (per > 1 && a.B * ((tiles_per_run + per - 1) / per) * slices < 148 * 2) per /= 2;
-    a.mma_tiles = per;
-    const long long tiles = (long long)a.B * ((tiles_per_run + per - 1) / per);
+    while (per > 1 && a.B * ((tiles_per_run + per - 1) / per) * 4 * cuts < 148 * 2) per /= 2;
+    const long long parts = (tiles_per_run + per - 1) / per;
+    a.mma_tiles = (int)((tiles_per_run + parts - 1) / parts);
+    const long long tiles = (long long)a.B * ((tiles_per_run + a.mma_tiles - 1) / a.mma_tiles);
     if (tiles > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
-    const dim3 grid((unsigned)tiles, 4, (unsigned)((a.D + kDChunk - 1) / kDChunk));
-    if (kp == 16) route_expand_mma_kernel<T, 16, kMmaPix><<<grid, 256, 0, st>>>(a);
-    else if (kp == 32) route_expand_mma_kernel<T, 32, kMmaPix><<<grid, 256, 0, st>>>(a);
-    else if (kp == 48) route_expand_mma_kernel<T, 48, kMmaPix><<<grid, 256, 0, st>>>(a);
-    else if (kp == 64) route_expand_mma_kernel<T, 64, kMmaPix><<<grid, 256, 0, st>>>(a);
+    const dim3 grid((unsigned)tiles, 4, (unsigned)cuts);
+    if (kp == 16) route_expand_mma_kernel<T, 16><<<grid, threads, 0, st>>>(a);
+    else if (kp == 32) route_expand_mma_kernel<T, 32><<<grid, threads, 0, st>>>(a);
+    else if (kp == 48) route_expand_mma_kernel<T, 48><<<grid, threads, 0, st>>>(a);
+    else if (kp == 64) route_expand_mma_kernel<T, 64><<<grid, threads, 0, st>>>(a);
     else return SS2D_ENOTSUP;
     count_launch();
     return check_launch();
