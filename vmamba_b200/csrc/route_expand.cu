@@ -152,9 +152,9 @@ __global__ void __launch_bounds__(kExpThreads) route_expand_kernel(const ExpandA
 // n8 operands so that a thread's accumulators are eight neighbouring pixels of two channels: column 2 t + e of operand n is pixel
 // 8 t + 2 n + e.  The results leave from registers as 16-byte vectors, 64 bytes of a row at a time, and a vector of x enters
 // shared memory as four words, 16 bytes apart; there is one barrier per tile of kMmaPix pixels.
-// Bound: HBM writes, and the bytes in flight: five CTAs of 256 threads to an SM where the contraction is short.  Against two
-// barriers a tile with the results through a shared tile: 64 x 192 planes of 28 x 28 28 -> 23 us (3.4 TB/s written), 15 launches
-// of 2 x 512 planes of 64 x 64 380 -> 311 us.
+// Bound: HBM writes, and the warps that keep them coming: four CTAs of 256 threads to an SM (2 x 512 planes of 64 x 64: 12.9, 10.6,
+// 12.1 and 15.2 us with three to six).  Against two barriers a tile with the results through a shared tile: 64 x 192 planes
+// of 28 x 28 28 -> 22 us (3.4 TB/s written), 2 x 512 of 64 x 64 16.2 -> 10.6 us, 16 x 1024 of 16 x 16 21.7 -> 15.3 us.
 constexpr int kMmaPix = 64;
 constexpr int kMmaTilesPerCta = 8;      // most pixel tiles per CTA: the staged weights then serve 512 pixels
 
@@ -166,7 +166,7 @@ template <typename T> __device__ __forceinline__ uint32_t pack2(float x, float y
 }
 
 template <typename T, int KP>
-__global__ void __launch_bounds__(256, KP <= 32 ? 5 : 1) route_expand_mma_kernel(const ExpandArgs a) {
+__global__ void __launch_bounds__(256, 4) route_expand_mma_kernel(const ExpandArgs a) {
     constexpr int PIX = kMmaPix;
     constexpr int KPAD = KP + 8, XPAD = PIX + 8;       // pitches (elements): conflict-free fragment loads and vector stores
     __shared__ __align__(16) T Ws[kDChunk * KPAD];     // [channel][k]
