@@ -102,7 +102,7 @@ def test_cross_merge_of_whole_planes(vb, H, W, scans, dt):
 
 @pytest.mark.parametrize("D,H,W,dt", [(16, 13, 13, "f32"), (15, 8, 17, "bf16"), (19, 27, 29, "f16"), (13, 57, 57, "bf16"), (14, 21, 21, "bf16"),
                                       (13, 54, 54, "f16"), (13, 36, 29, "f32"), (12, 75, 75, "bf16"), (13, 54, 80, "bf16"), (12, 96, 96, "bf16"),
-                                      (17, 9, 9, "bf16"), (12, 101, 97, "f32")])
+                                      (17, 9, 9, "bf16"), (12, 101, 97, "f32"), (16, 7, 7, "bf16"), (40, 14, 14, "f16"), (24, 9, 11, "bf16")])
 def test_core_any_plane_size(vb, D, H, W, dt):
     """The fused core on planes of any size (padded rows, both layouts) against the oracle."""
     c = _core_case(2, D, H, W, N=1, seed=H * W, Cmodel=24)

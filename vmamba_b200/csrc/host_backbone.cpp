@@ -41,7 +41,7 @@ static Tensor linear_cm(const Tensor& w, const Tensor& x, int64_t S) {      // x
 
 // -------------------------------------------------------------------------------------------- the core
 // Route streams: delta and B / C rows of the two orientations (even: routes 0, 2; odd: 1, 3) and two routes each.
-struct Streams { Tensor bc, delta; bool cm; int64_t pad; };      // pad: elements per image row, 0: dense
+struct Streams { Tensor bc, delta; bool cm, x_cm; int64_t S, pad; };      // x_cm: x's own layout; pad: elements per image row, 0: dense
 
 // Whether the streams' rows are better padded (the library's planner decides).
 static bool prefers_padded(const CoreW& w, at::ScalarType type, bool cm, int64_t B, int64_t H, int64_t W, int64_t S) {
@@ -57,12 +57,30 @@ static Streams project(const Tensor& x, bool cm, int64_t B, int64_t H, int64_t W
     const int64_t D = w.D, R = w.R, N = w.N, C = R + 2 * N, L = H * W;
     ss2d_expand_params p = {};
     Streams s;
-    s.cm = cm;
+    s.x_cm = cm;
     s.pad = padding && prefers_padded(w, x.scalar_type(), cm, B, H, W, S) ? round8(L) : 0;
+    // 16-bit (B, D, L) maps whose planes are no whole vectors: a channel-major copy, so that the images of a row are one run and
+    // projection and expansion take the tensor-core kernels (whole core, 128 x 768 planes of 7 x 7 269 -> 109 us,
+    // 1 x 384 of 14 x 14 32 -> 25 us of kernels)
+    Tensor xc = x;
+    if (!cm && padding && !s.pad && L % 8 != 0 && R <= 64 && x.scalar_type() != at::kFloat) {
+        cm = true;
+        S = round8(B * L);
+        xc = at::empty({D, S}, x.options());
+        Tensor from = x.view({B, D, L}), to = xc.narrow(1, 0, B * L).view({D, B, L});
+        const int64_t e = L % 4 == 0 ? 4 : L % 2 == 0 ? 2 : 1;        // elements moved as one word
+        if (e > 1 && x.storage_offset() % e == 0 && (uintptr_t)x.data_ptr() % (2 * e) == 0) {
+            const auto word = e == 4 ? at::kLong : at::kInt;
+            from = from.view(word); to = to.view(word);
+        }
+        to.copy_(from.transpose(0, 1));
+    }
+    s.cm = cm;
+    s.S = S;
     Tensor xd;
     auto at_el = [](const Tensor& t, int64_t i) { return (char*)t.data_ptr() + i * t.element_size(); };
     if (cm) {
-        xd = linear_cm(w.wx, x.view({D, S}), S);
+        xd = linear_cm(w.wx, xc.view({D, S}), S);
         p.x_dbl_batch_stride = L; p.x_dbl_route_stride = C * S; p.x_dbl_row_stride = S;
         if (!s.pad) {
             s.delta = at::empty({2, 2, D, S}, x.options());
@@ -106,8 +124,8 @@ static Streams project(const Tensor& x, bool cm, int64_t B, int64_t H, int64_t W
     return s;
 }
 
-static ss2d_core_params core_params(const Tensor& x, const Streams& s, const CoreW& w, int64_t B, int64_t H, int64_t W, int64_t S) {
-    const int64_t L = H * W, D = w.D, N = w.N, e = x.element_size();
+static ss2d_core_params core_params(const Tensor& x, const Streams& s, const CoreW& w, int64_t B, int64_t H, int64_t W) {
+    const int64_t L = H * W, S = s.S, D = w.D, N = w.N, e = x.element_size();
     ss2d_core_params p = {};
     p.x = x.data_ptr();
     for (int k = 0; k < 4; ++k) {
@@ -127,7 +145,7 @@ static ss2d_core_params core_params(const Tensor& x, const Streams& s, const Cor
     p.A = w.A.data_ptr(); p.Dskip = w.Ds.data_ptr(); p.delta_bias = w.bias.data_ptr(); p.ln_weight = ptr(w.lnw); p.ln_bias = ptr(w.lnb);
     p.B = B; p.D = D; p.H = H; p.W = W; p.N = N; p.act_dtype = dtype_code(x); p.ln_eps = (float)w.eps;
     p.stream_row = s.pad;
-    if (s.cm) { p.x_batch_stride = p.y_batch_stride = L; p.x_channel_stride = p.y_channel_stride = S; }
+    if (s.x_cm) { p.x_batch_stride = p.y_batch_stride = L; p.x_channel_stride = p.y_channel_stride = S; }
     return p;
 }
 
@@ -204,7 +222,7 @@ static Tensor core_run(const Tensor& x, bool cm, int64_t B, int64_t H, int64_t W
         return core_by_operators(x, cm, B, H, W, S, w, with_norm, out_type, out);
     const Streams s = project(x, cm, B, H, W, S, w, true);
     if (!out.defined()) out = at::empty_like(x, x.options().dtype(out_type));
-    ss2d_core_params p = core_params(x, s, w, B, H, W, S);
+    ss2d_core_params p = core_params(x, s, w, B, H, W);
     p.y = out.data_ptr(); p.y_dtype = dtype_code(out); p.with_norm = with_norm;
     const int64_t need = ss2d_core_workspace_bytes(&p);
     TORCH_CHECK(need >= 0, "ss2d_core_workspace_bytes: invalid arguments");
