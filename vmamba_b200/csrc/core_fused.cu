@@ -443,6 +443,8 @@ static bool plan_planes(const ss2d_core_params* p, PlaneConfig& c) {
     // segments of at most four elements: two planes per thread (the kernel's NPL = 2), twice the planes per CTA
     // (677 -> 649 us for the eight 14 x 14 launches of a batch-128 VMamba-T forward)
     const int npl = (vec <= 4 && 2 * PP <= p->D) ? 2 : 1;
+    // few planes: fewer of them per CTA, so that every SM has one (1 x 384 planes of 14 x 14 7.3 -> 6.1 us)
+    while (PP > 1 && p->B * ((p->D + (PP * npl) - 1) / (PP * npl)) < 148) PP = (PP + 1) / 2;
     PP *= npl;
     const int Wp = (int)(p->W | 1);   // odd pitch spreads the transposed accesses over banks
     size_t smem = (size_t)PP * p->H * Wp * sizeof(float);
