@@ -16,6 +16,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "scan_row.cuh"
 
 namespace ss2d {
 
@@ -119,7 +120,7 @@ template <typename T, int RPW, int VW> struct StRaw {
             }
         });
     }
-    template <int E> __device__ __forceinline__ void get(int i, float (&v)[E]) const {
+    template <int E> __device__ __forceinline__ void get(int i, float (&v)[E], const T*, int64_t, int, int, int) const {
 #pragma unroll
         for (int h = 0; h < kVecs; ++h) {
             float x[VW];
@@ -127,6 +128,25 @@ template <typename T, int RPW, int VW> struct StRaw {
 #pragma unroll
             for (int e = 0; e < VW; ++e) v[h * VW + e] = x[e];
         }
+    }
+};
+// VW 0: rows of any alignment, runs of eight cut out of aligned pieces.  (Single elements, VW 1, cost the few-state kernels their
+// loads: 4 608 rows of 8 594 elements, 4 states, bf16 1021 -> 394 us.)
+template <typename T, int RPW> struct StRaw<T, RPW, 0> {
+    static constexpr int kRuns = RPW / 8;
+    Row8<T, 0> w[kRuns];
+    template <typename F> static __device__ __forceinline__ void for_each(int lane, F f) {
+#pragma unroll
+        for (int i = 0; i < kRuns; ++i) f(i, i * 8 + (lane >> 2), (lane & 3) * 8, std::integral_constant<int, 8>{});
+    }
+    __device__ __forceinline__ void load(const T* rows, int64_t stride, int count, int t0, int L, int lane) {
+        for_each(lane, [&](int i, int row, int el, auto) {
+            w[i] = {};
+            if (row < count) w[i].load(rows + row * stride, t0 + el, L);
+        });
+    }
+    __device__ __forceinline__ void get(int i, float (&v)[8], const T* rows, int64_t stride, int t0, int L, int lane) const {
+        w[i].get(rows + (i * 8 + (lane >> 2)) * stride, t0 + (lane & 3) * 8, L, v);
     }
 };
 // B or C of one chunk, spread over the threads of the CTA.
@@ -150,7 +170,7 @@ template <typename T, int NS, int VW, int WARPS> struct StRawBC {
             }
         }
     }
-    __device__ __forceinline__ void put(float* dst) const {
+    __device__ __forceinline__ void put(float* dst, const T*, int64_t, int, int) const {
 #pragma unroll
         for (int j = 0; j < kPer; ++j) {
             int n, el;
@@ -163,6 +183,31 @@ template <typename T, int NS, int VW, int WARPS> struct StRawBC {
 #pragma unroll
                     for (int e = 0; e < VW; ++e) dst[(el + h * VW + e) * StLayout<NS>::BCP + n] = x[e];
                 }
+            }
+        }
+    }
+};
+
+template <typename T, int NS, int WARPS> struct StRawBC<T, NS, 0, WARPS> {
+    static constexpr int kThreads = WARPS * 32, kItems = NS * 4, kPer = (kItems + kThreads - 1) / kThreads;
+    Row8<T, 0> w[kPer];
+    __device__ __forceinline__ void load(const T* src, int64_t state_stride, int N, int t0, int L) {
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int i = threadIdx.x + j * kThreads, n = i % NS, el = (i / NS) * 8;
+            w[j] = {};
+            if (n < N && el < kStChunk) w[j].load(src + n * state_stride, t0 + el, L);
+        }
+    }
+    __device__ __forceinline__ void put(float* dst, const T* src, int64_t state_stride, int t0, int L) const {
+#pragma unroll
+        for (int j = 0; j < kPer; ++j) {
+            const int i = threadIdx.x + j * kThreads, n = i % NS, el = (i / NS) * 8;
+            if (kItems % kThreads == 0 || i < kItems) {
+                float v[8];
+                w[j].get(src + n * state_stride, t0 + el, L, v);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) dst[(el + e) * StLayout<NS>::BCP + n] = v[e];
             }
         }
     }

@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(StLayout<NS>::kWarps * 32, 8 / StLayout<NS>::k
         {
             StRawBC<Tin, NS, VW, W> xb, xc;
             xb.load(Bm, a.B_ss, a.N, t0, L); xc.load(Cm, a.C_ss, a.N, t0, L);
-            xb.put(sB); xc.put(sC);
+            xb.put(sB, Bm, a.B_ss, t0, L); xc.put(sC, Cm, a.C_ss, t0, L);
         }
         // ---- stage the rows
         for (int s = 0; s < sets; ++s) {
@@ -146,7 +146,8 @@ __global__ void __launch_bounds__(StLayout<NS>::kWarps * 32, 8 / StLayout<NS>::k
             StRaw<Tin, RPW, VW>::for_each(lane, [&](int i, int rr, int el, auto n_el) {
                 constexpr int E = decltype(n_el)::value;
                 float uv[E], dv[E], gv[E];
-                xd.get(i, dv); xu.get(i, uv); xg.get(i, gv);
+                xd.get(i, dv, dt + o * a.d_ds, a.d_ds, t0, L, lane); xu.get(i, uv, u + o * a.u_ds, a.u_ds, t0, L, lane);
+                xg.get(i, gv, gp + o * a.g_ds, a.g_ds, t0, L, lane);
                 const float bs = __shfl_sync(0xffffffffu, bias_rl, rr * SL);
 #pragma unroll
                 for (int e = 0; e < E; ++e) {
@@ -411,11 +412,11 @@ __global__ void __launch_bounds__(StLayout<NS>::kWarps * 32) st_bwd_segments_ker
             xd.load(dt, a.d_ds, count, t0, L, lane);
             xg.load(gp, a.g_ds, count, t0, L, lane);
             __syncthreads();                         // the chunk in front is read
-            xc.put(sC);
+            xc.put(sC, Cm, a.C_ss, t0, L);
             StRaw<Tin, RPW, VW>::for_each(lane, [&](int i, int rr, int el, auto n_el) {
                 constexpr int E = decltype(n_el)::value;
                 float dv[E], gv[E];
-                xd.get(i, dv); xg.get(i, gv);
+                xd.get(i, dv, dt, a.d_ds, t0, L, lane); xg.get(i, gv, gp, a.g_ds, t0, L, lane);
                 const float bs = __shfl_sync(0xffffffffu, bias_rl, rr * SL);
 #pragma unroll
                 for (int j = 0; j < E; ++j) {

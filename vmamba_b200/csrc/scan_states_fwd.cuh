@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(StLayout<NS, R_>::kWarps * 32) st_fwd_kernel(c
     constexpr int RPW = Y::RPW, SL = Y::SL, R = Y::R, RL = Y::RL, P = kStPitch;
     constexpr int kRow = RPW * P, kBC = kStChunk * Y::BCP;
     using Raw = StRaw<Tin, RPW, VW>;
-    constexpr bool kPre = sizeof(Raw) <= 64;         // the next chunk is fetched into registers while this one is worked on
+    constexpr bool kPre = sizeof(Raw) <= (VW == 0 ? 128 : 64);         // the next chunk is fetched into registers while this one is worked on
     extern __shared__ __align__(16) float st_sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rl = lane / SL, sl = lane % SL, n0 = sl * 4;
     float* sd = st_sm + warp * 2 * kRow;             // step sizes of the warp's chunk
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(StLayout<NS, R_>::kWarps * 32) st_fwd_kernel(c
         Raw::for_each(lane, [&](int i, int rr, int el, auto n_el) {
             constexpr int E = decltype(n_el)::value;
             float uv[E], dv[E];
-            xu.get(i, uv); xd.get(i, dv);
+            xu.get(i, uv, u, a.u_ds, t0, L, lane); xd.get(i, dv, dt, a.d_ds, t0, L, lane);
             float bs = __shfl_sync(0xffffffffu, bias[0], (rr % RL) * SL);
             if constexpr (R == 2) {
                 const float b1 = __shfl_sync(0xffffffffu, bias[1], (rr % RL) * SL);
@@ -101,8 +101,8 @@ __global__ void __launch_bounds__(StLayout<NS, R_>::kWarps * 32) st_fwd_kernel(c
             st_put(sd + rr * P + el, dv);
             st_put(su + rr * P + el, uv);
         });
-        xb.put(sbc + buf * 2 * kBC);
-        if constexpr (kOut) xc.put(sbc + buf * 2 * kBC + kBC);
+        xb.put(sbc + buf * 2 * kBC, Bm, a.B_ss, t0, L);
+        if constexpr (kOut) xc.put(sbc + buf * 2 * kBC + kBC, Cm, a.C_ss, t0, L);
     };
     if (lo < hi) { fetch(lo); put(lo, 0); }
     __syncthreads();
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(StLayout<NS, R_>::kWarps * 32) st_fwd_kernel(c
         }
         __syncwarp();
         if constexpr (kOut) {
-            st_unstage<Tout, RPW, VW>(su, (Tout*)a.out + b * a.o_bs + r0 * a.o_ds, a.o_ds, count, t0, L, lane);
+            st_unstage<Tout, RPW, VW == 0 ? 1 : VW>(su, (Tout*)a.out + b * a.o_bs + r0 * a.o_ds, a.o_ds, count, t0, L, lane);
             __syncwarp();
         }
         if (more) {
@@ -249,7 +249,7 @@ static int st_rows_per_lane(const StFwdArgs& a, int64_t batch, cudaStream_t st) 
     return st_launch_fwd<Tin, Tout, NS, 1, VW, kOut>(a, batch, st);
 }
 
-// vw: vector width of the global accesses, 8, 4 or 1
+// vw: vector width of the global accesses, 8, 4 or less
 template <typename Tin, typename Tout, bool kOut>
 static int st_dispatch_fwd(const StFwdArgs& a, int64_t batch, int vw, cudaStream_t st) {
     const int NS = st_pad_states(a.N);
@@ -257,7 +257,7 @@ static int st_dispatch_fwd(const StFwdArgs& a, int64_t batch, int vw, cudaStream
     if (NS == NS_)                                                                              \
         return vw == 8   ? st_rows_per_lane<Tin, Tout, NS_, 8, kOut>(a, batch, st)              \
                : vw == 4 ? st_rows_per_lane<Tin, Tout, NS_, 4, kOut>(a, batch, st)              \
-                         : st_rows_per_lane<Tin, Tout, NS_, 1, kOut>(a, batch, st);
+                         : st_rows_per_lane<Tin, Tout, NS_, 0, kOut>(a, batch, st);
     SS2D_ST(4)
     SS2D_ST(8)
     SS2D_ST(16)
