@@ -364,7 +364,7 @@ typedef struct ss2d_linear_params {
     int64_t M, K, N;
     int64_t x_row_stride, out_row_stride;
     int32_t dtype;
-    int32_t reserved0;
+    int32_t act;            /* 0: none, 1: GELU (erf form) after the bias; small maps only, with M up to 2^20 */
 } ss2d_linear_params;
 
 int ss2d_linear_supported(const ss2d_linear_params *p);

@@ -162,3 +162,17 @@ def test_linear_few_pixels(M, K, N, dt):
     want = w.double() @ x.double() + b.double()[:, None]
     got = ops.linear_cf(x, w, bias=b)
     assert O.max_rel_err(host(got), want.float().cpu().numpy()) <= TOL_BF16
+
+
+@pytest.mark.parametrize("M,K,N", [(8, 32, 8), (40, 64, 72), (1536, 384, 200), (768, 192, 784), (96, 768, 56)])
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+def test_linear_few_pixels_gelu(M, K, N, dt):
+    """Projection, bias and GELU in one launch: tiles of 32 rows and 64 pixels, whole and ragged."""
+    from vmamba_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    w, x = (torch.randn(s, device="cuda", generator=g).mul_(k).to(TD[dt]) for s, k in (((M, K), K ** -0.5), ((K, N), 1.0)))
+    bias, out = torch.randn(M, device="cuda", generator=g), torch.empty(M, N, device="cuda", dtype=TD[dt])
+    p = _lib.LinearParams(x.data_ptr(), w.data_ptr(), bias.data_ptr(), out.data_ptr(), M, K, N, 0, 0, {"bf16": _lib.SS2D_BF16, "f16": _lib.SS2D_F16}[dt], 1)
+    assert _lib.lib().ss2d_linear_fwd(p, torch.cuda.current_stream().cuda_stream) == _lib.SS2D_OK
+    ref = torch.nn.functional.gelu(w.double() @ x.double() + bias.double()[:, None])
+    assert (out.double() - ref).abs().max() <= (2e-2 if dt == "bf16" else 3e-3)

@@ -113,7 +113,7 @@ class MlpParams(ctypes.Structure):
 
 class LinearParams(ctypes.Structure):
     _fields_ = [(n, _vp) for n in ("x", "w", "bias", "out")] + \
-               [(n, _i64) for n in ("M", "K", "N", "x_row_stride", "out_row_stride")] + [("dtype", _i32), ("reserved0", _i32)]
+               [(n, _i64) for n in ("M", "K", "N", "x_row_stride", "out_row_stride")] + [("dtype", _i32), ("act", _i32)]
 
 
 EXPORTS = {

@@ -344,6 +344,16 @@ private:
                 return y;
             }
         }
+        if (type != at::kFloat) {                                     // few pixels: bias and GELU in the projection's epilogue
+            ss2d_linear_params p = {};
+            Map h = x.like(b.w1.size(0));
+            p.x = x.t.data_ptr(); p.w = b.w1.data_ptr(); p.bias = b.b1.data_ptr(); p.out = h.t.data_ptr();
+            p.M = h.C; p.K = x.C; p.N = x.S; p.dtype = dtype_code(x.t); p.act = 1;
+            if (ss2d_linear_supported(&p) == SS2D_OK) {
+                check(ss2d_linear_fwd(&p, stream_of(x.t)), "ss2d_linear_fwd");
+                return pw(b.w2, h);
+            }
+        }
         const Map h = pw(b.w1, x);
         ss2d_pointwise_params p = {};
         p.x = p.y = h.t.data_ptr(); p.bias = b.b1.data_ptr();

@@ -249,8 +249,11 @@ int linear_supported(const ss2d_linear_params* p) {
     if (!p->x || !p->w || !p->out) return SS2D_EINVAL_NULL;
     if (p->dtype != SS2D_BF16 && p->dtype != SS2D_F16) return SS2D_ENOTSUP;     // fp32 maps: the library GEMM
     if (p->M <= 0 || p->K <= 0 || p->N <= 0) return SS2D_EINVAL_SHAPE;
-    if (p->M > 256 || p->M % 8 != 0 || p->K % 32 != 0) return SS2D_ENOTSUP;
-    { LinearArgs g; if (!plan_linear(p->M, p->K, g)) return SS2D_ENOTSUP; }      // W must leave room for the ring
+    if (p->act < 0 || p->act > 1 || p->M % 8 != 0 || p->K % 32 != 0) return SS2D_ENOTSUP;
+    if (p->act) {        // an epilogue of the few-pixel kernel alone
+        if (p->M > (1 << 20) || p->N > 0x7fffff00LL || !linear_small_takes(p)) return SS2D_ENOTSUP;
+    } else if (p->M > 256) return SS2D_ENOTSUP;
+    else { LinearArgs g; if (!plan_linear(p->M, p->K, g)) return SS2D_ENOTSUP; }      // W must leave room for the ring
     const long long xs = p->x_row_stride ? p->x_row_stride : p->N, os = p->out_row_stride ? p->out_row_stride : p->N;
     if (xs < p->N || os < p->N) return SS2D_EINVAL_STRIDE;
     if (xs % 8 != 0 || os % 2 != 0 || p->N % 8 != 0 || p->N > 0x7fffff00LL) return SS2D_ENOTSUP;   // 16-byte row pitch for TMA, paired stores

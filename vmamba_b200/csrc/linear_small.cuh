@@ -4,8 +4,11 @@
 // A CTA of four warps computes a tile of 32 rows x 64 pixels.  Everything it needs (32 rows of W, 64 pixels of all K rows of x) is
 // requested at once with cp.async, so that the whole load is one memory latency; the warps then split K between them
 // (mma.sync m16n8k16, x through ldmatrix.trans) and meet in shared memory.  x is read once per 32 rows of W, from L2.
+// With GELU it is the first half of an MLP block (the result stays fp32 until then), one launch instead of a library GEMM and a pass
+// over its result.
 // Bound: latency (two round trips to L2 and a launch).
 #pragma once
+#include "activations.cuh"
 #include "common.cuh"
 
 namespace ss2d {
@@ -16,7 +19,7 @@ struct LinearSmallArgs {
     const void *x, *w;
     const float* bias;
     void* out;
-    int M, K, N;
+    int M, K, N, act;
     long long x_rs, out_rs;
 };
 
@@ -107,6 +110,13 @@ __global__ void __launch_bounds__(kLsWarps * 32) linear_small_kernel(const Linea
             const float4 x = q[0], y = q[1];
             v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w; v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
         }
+        if (a.act) {
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+                const float2 r = gelu_pair_poly(make_float2(v[e], v[e + 1]));
+                v[e] = r.x; v[e + 1] = r.y;
+            }
+        }
         Vec<T, 8>::store((T*)a.out + (m0 + m) * a.out_rs + n0 + c, v);
     }
 }
@@ -120,7 +130,7 @@ inline bool linear_small_takes(const ss2d_linear_params* p) {
 }
 
 template <typename T> static int launch_linear_small(const ss2d_linear_params* p, cudaStream_t st) {
-    LinearSmallArgs a = {p->x, p->w, (const float*)p->bias, p->out, (int)p->M, (int)p->K, (int)p->N, p->x_row_stride ? p->x_row_stride : p->N,
+    LinearSmallArgs a = {p->x, p->w, (const float*)p->bias, p->out, (int)p->M, (int)p->K, (int)p->N, p->act, p->x_row_stride ? p->x_row_stride : p->N,
                          p->out_row_stride ? p->out_row_stride : p->N};
     const size_t smem = linear_small_smem(p->K);
     auto kern = linear_small_kernel<T>;
