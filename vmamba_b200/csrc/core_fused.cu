@@ -657,9 +657,10 @@ long long core_workspace_bytes(const ss2d_core_params* p) {
 struct CorePlan { bool routes; RoutePlan r; PlaneConfig c; };
 
 static bool plan_core(const ss2d_core_params* p, CorePlan& plan) {
-    if (p->stream_row && p->stream_row != p->H * p->W) {
+    if (p->stream_row) {         // a stream_row of L, a multiple of 8, is a row with nothing to pad
         plan.routes = true;
-        return plan_padded(p, plan.r);
+        if (plan_padded(p, plan.r)) return true;
+        if (p->stream_row != p->H * p->W) return false;
     }
     plan.routes = use_routes(p, plan.r);
     return plan.routes || plan_planes(p, plan.c);

@@ -551,7 +551,8 @@ int cross_scan(const ss2d_cross_params* p, cudaStream_t st) {
         const bool f32 = p->dtype == SS2D_F32, plane = f32 ? plan_plane<float>(p, 1, pa, pv, smem) : plan_plane<uint16_t>(p, 1, pa, pv, smem);
         if (!plane || pv < 2) {      // with pairs the plane kernel is the faster one (57 x 58 maps: 15 against 18 us)
             FlatArgs fa; int threads; size_t fs;
-            if (plan_flat(p, f32 ? 4 : 2, 1, fa, threads, fs) && (plane || !f32))
+            // a plane that leaves one CTA on an SM is faster in tiles (192 planes of 247 x 256: 133 against 49 us)
+            if (plan_flat(p, f32 ? 4 : 2, 1, fa, threads, fs) && (plane || !f32) && fs <= 100 * 1024)
                 return f32 ? launch_scan_flat<float>(fa, p->B, threads, fs, st) : launch_scan_flat<uint16_t>(fa, p->B, threads, fs, st);
         }
         if (plane) return f32 ? scan_plane_v<float>(pa, pv, smem, st) : scan_plane_v<uint16_t>(pa, pv, smem, st);

@@ -432,11 +432,14 @@ long long route_expand_workspace_bytes(const ss2d_expand_params* p) {
 }
 
 // All projected rows in the orientation order of their route (pixel order for routes 0, 2, column-major for 1, 3), a row of an
-// image padded to `pad` elements with zeros: (4, C, B, pad).  A warp per plane; small next to what the expansion writes.
-template <typename T>
+// image padded to `pad` elements with zeros: (4, C, B, pad).  Small next to what the expansion writes.  A warp per plane, or, where
+// that leaves SMs idle, a CTA (104 planes of 62 x 64: 28 us with warps).
+template <typename T, bool kCta>
 __global__ void __launch_bounds__(256) orient_rows_kernel(const TransArgs a, const int pad) {
     extern __shared__ __align__(16) unsigned char traw[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int step = kCta ? blockDim.x : 32, lane = kCta ? threadIdx.x : threadIdx.x & 31;
+    const int warp = kCta ? 0 : threadIdx.x >> 5, nwarps = kCta ? 1 : blockDim.x >> 5;
+    const auto sync = [] { if constexpr (kCta) __syncthreads(); else __syncwarp(); };
     const int P = a.W | 1;
     T* tile = reinterpret_cast<T*>(traw) + (size_t)warp * a.H * P;
     const T zero = from_f<T>(0.f);
@@ -446,14 +449,14 @@ __global__ void __launch_bounds__(256) orient_rows_kernel(const TransArgs a, con
         T* __restrict__ dst = (T*)a.xt + (long long)pid * pad;
         if (k & 1) {
 #pragma unroll 4
-            for (int e = lane; e < a.L; e += 32) { const int h = e / a.W; tile[h * P + (e - h * a.W)] = src[e]; }
-            __syncwarp();
+            for (int e = lane; e < a.L; e += step) { const int h = e / a.W; tile[h * P + (e - h * a.W)] = src[e]; }
+            sync();
 #pragma unroll 4
-            for (int q = lane; q < pad; q += 32) { const int w = q / a.H; dst[q] = q < a.L ? tile[(q - w * a.H) * P + w] : zero; }
-            __syncwarp();
+            for (int q = lane; q < pad; q += step) { const int w = q / a.H; dst[q] = q < a.L ? tile[(q - w * a.H) * P + w] : zero; }
+            sync();
         } else {
 #pragma unroll 4
-            for (int e = lane; e < pad; e += 32) dst[e] = e < a.L ? src[e] : zero;
+            for (int e = lane; e < pad; e += step) dst[e] = e < a.L ? src[e] : zero;
         }
     }
 }
@@ -468,14 +471,15 @@ static int launch_orient(const ss2d_expand_params* p, cudaStream_t st) {
     t.planes = 4 * t.C * t.B;
     const size_t plane_bytes = (size_t)t.H * (t.W | 1) * sizeof(T);
     if (plane_bytes > 200 * 1024) return SS2D_ENOTSUP;
-    int warps = (int)(48 * 1024 / plane_bytes);
+    const bool cta = t.planes < 148 * 8;
+    int warps = cta ? 1 : (int)(48 * 1024 / plane_bytes);
     warps = warps < 1 ? 1 : warps > 8 ? 8 : warps;
-    auto kern = orient_rows_kernel<T>;
+    auto kern = cta ? orient_rows_kernel<T, true> : orient_rows_kernel<T, false>;
     const size_t smem = plane_bytes * warps;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
     long long ctas = (t.planes + warps - 1) / warps;
     if (ctas > 148 * 16) ctas = 148 * 16;
-    kern<<<(unsigned)ctas, warps * 32, smem, st>>>(t, (int)p->image_row);
+    kern<<<(unsigned)ctas, cta ? 256 : warps * 32, smem, st>>>(t, (int)p->image_row);
     count_launch();
     return check_launch();
 }
