@@ -6,9 +6,9 @@ CrossMerge -> out_norm -> cast, without ever materialising the (B, 4, D, L) scan
 per-route outputs.
 
 Because a 1x1 projection commutes with a permutation of the pixels, the x_proj contraction is done
-once on x in its native layout (one library GEMM, (4(R+2N) x D) . (D x L) per image); the rows of
+once on x in its native layout ((4(R+2N) x D) . (D x L) per image); the rows of
 the two column-major routes are then transposed (they are (R+2N)/D of the size of x), the step
-sizes are expanded per route (R -> D, a batched library GEMM) and the CUDA kernel consumes x plus
+sizes are expanded per route (R -> D, `ss2d_route_expand`) and the CUDA kernel consumes x plus
 the per-route (delta, B, C) streams in the orientation order of each route.
 """
 from __future__ import annotations

@@ -6,7 +6,7 @@ Mirrors, name for name, what MzeroMiko/VMamba's modules resolve at call time:
                                                                        vmamba.py:837-885
   cross_scan_fn, cross_merge_fn, CrossScanF, CrossMergeF (+ aliases)  classification/models/csm_triton.py:182-273,
                                                                        403-517; vmamba.py:254-345, 481-601
-Forward (inference) only.  Tensors must live on a CUDA device; there is no torch/CPU path here
+Forward and backward.  Tensors must live on a CUDA device; there is no torch/CPU path here
 (`backend="torch"` raises).  Argument meaning, output shapes/dtypes and the error behaviour on bad
 shapes follow the reference.
 """
