@@ -437,7 +437,9 @@ static bool plan_planes(const ss2d_core_params* p, PlaneConfig& c) {
     if (G > 1024) return false;
     // ~14 warps per CTA, two CTAs per SM; seven-thread planes (7 x 7) in CTAs of seven warps, four per SM: 61.6 -> 51.4 us
     // per launch at 128 x 768 planes (the 14 x 14 launch takes 84 us with 448, 224 or 160 threads and 98 us with 320)
-    int PP = (int)((G <= 8 ? 224 : 448) / G);
+    // Seven warps and four CTAs too where at least two planes of 28 x 28 and less go into them: barriers of fewer warps (64 x 192
+    // planes of 28 x 28, whole core: 127 -> 121 us; ten warps 135, four 125).
+    int PP = (int)((G <= 8 || (G > 56 && G <= 112) ? 224 : 448) / G);
     if (PP < 1) PP = 1;
     if (PP > p->D) PP = (int)p->D;
     // segments of at most four elements: two planes per thread (the kernel's NPL = 2), twice the planes per CTA
