@@ -1,0 +1,88 @@
+"""What the state of the calling program must not change: autocast regions, copies of a model, what a training step keeps.
+Needs a GPU."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def vb():
+    import vmamba_b200
+    return vmamba_b200
+
+
+def state_dict(dims=(32, 64, 128, 256), depths=(1, 1, 1, 1), classes=10, seed=0):
+    """Random weights of a small backbone with a classifier and the feature norms, in the key layout of its checkpoints."""
+    g = torch.Generator().manual_seed(seed)
+    rnd = lambda *s: torch.randn(s, generator=g) * math.prod(s[1:]) ** -0.5      # noqa: E731
+    sd = {}
+
+    def norm(name, n):
+        sd[name + ".weight"], sd[name + ".bias"] = torch.ones(n), torch.zeros(n)
+
+    def conv(name, out, inn):
+        sd[name + ".weight"], sd[name + ".bias"] = rnd(out, inn, 3, 3), torch.zeros(out)
+
+    conv("patch_embed.0", dims[0] // 2, 3)
+    norm("patch_embed.2", dims[0] // 2)
+    conv("patch_embed.5", dims[0], dims[0] // 2)
+    norm("patch_embed.7", dims[0])
+    for i, d in enumerate(dims):
+        R = math.ceil(d / 16)
+        for j in range(depths[i]):
+            p = f"layers.{i}.blocks.{j}."
+            norm(p + "norm", d)
+            norm(p + "norm2", d)
+            norm(p + "op.out_norm", d)
+            for name, shape in (("op.in_proj", (d, d)), ("op.out_proj", (d, d)), ("mlp.fc1", (4 * d, d)), ("mlp.fc2", (d, 4 * d)),
+                                ("op.conv2d", (d, 1, 3, 3)), ("op.x_proj", (4 * (R + 2), d)), ("op.dt_projs", (4 * d, R))):
+                sd[p + name + ".weight"] = rnd(*shape)
+            sd[p + "mlp.fc1.bias"], sd[p + "mlp.fc2.bias"] = torch.zeros(4 * d), torch.zeros(d)
+            sd[p + "op.dt_projs_bias"], sd[p + "op.A_logs"], sd[p + "op.Ds"] = torch.full((4, d), -3.0), torch.zeros(4 * d, 1), torch.ones(4 * d)
+        norm(f"outnorm{i}", d)
+        if i + 1 < len(dims):
+            conv(f"layers.{i}.downsample.1", dims[i + 1], d)
+            norm(f"layers.{i}.downsample.3", dims[i + 1])
+    norm("classifier.norm", dims[-1])
+    sd["classifier.head.weight"], sd["classifier.head.bias"] = rnd(classes, dims[-1]), torch.zeros(classes)
+    return sd
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("region", [torch.float16, torch.bfloat16])
+def test_backbone_under_autocast(vb, dtype, region):
+    """A model computes in its own type, inside an autocast region as outside: same bits."""
+    m = vb.VSSMInfer.from_state_dict(state_dict(), dtype=dtype)
+    x = torch.randn(2, 3, 64, 96, device="cuda").to(dtype)
+    want, maps = m(x), m.features(x)
+    with torch.autocast("cuda", dtype=region):
+        got, inside = m(x), m.features(x)
+    assert got.dtype == want.dtype and torch.equal(got, want)
+    for a, b in zip(inside, maps):
+        assert a.dtype == b.dtype and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_core_under_autocast(vb, dtype):
+    """The core, its projections and the gradients of a step whose backward pass alone lies in the region."""
+    from vmamba_b200 import fused
+    D, R = 32, 2
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=g)      # noqa: E731
+    par = [rnd(4 * (R + 2), D) * D ** -0.5, rnd(4 * D, R) * R ** -0.5, torch.full((4, D), -3.0, device="cuda"), torch.zeros(4 * D, 1, device="cuda"),
+           torch.ones(4 * D, device="cuda"), torch.ones(D, device="cuda"), torch.zeros(D, device="cuda")]
+    x, gy = rnd(2, D, 9, 10).to(dtype), rnd(2, D, 9, 10).to(dtype)
+    w = vb.CoreWeights.build(*par, d_state=1, dt_rank=R, dtype=dtype)
+    leaves = [t.requires_grad_(True) for t in [x, *par]]
+
+    def step(region):
+        with torch.no_grad(), torch.autocast("cuda", enabled=region):
+            outs = [vb.ss2d_core(x, w), *fused.project(x, w)]
+        y = vb.ss2d_core_autograd(*leaves, d_state=1, dt_rank=R)
+        with torch.autocast("cuda", enabled=region):
+            return [*outs, y, *torch.autograd.grad(y, leaves, gy)]
+    for a, b in zip(step(False), step(True)):
+        assert a.dtype == b.dtype and torch.equal(a, b)

@@ -280,13 +280,13 @@ public:
     Tensor forward(const Tensor& img) {
         TORCH_CHECK(!head.empty(), "this model was built without a classifier");
         at::NoGradGuard no_grad;
-        const c10::cuda::OptionalCUDAGuard guard(img.device());
+        const CallGuard guard(img);
         const Tensor x = run(img, nullptr);
         return at::linear(x.mean({2, 3}).to(type), head[2], head[3]);
     }
     std::vector<Tensor> features(const Tensor& img, const std::vector<int64_t>& which) {
         at::NoGradGuard no_grad;
-        const c10::cuda::OptionalCUDAGuard guard(img.device());
+        const CallGuard guard(img);
         std::vector<Map> maps;
         run(img, &maps);
         std::vector<Tensor> out;
@@ -456,21 +456,20 @@ void bind_backbone(pybind11::module_& m) {
     m.def("ss2d_core",
           [](const Tensor& x, const CoreW& w, bool with_norm, at::ScalarType out_type, const OptT& workspace, bool cm) {
               const int64_t B = x.size(cm ? 1 : 0), H = x.size(2), W = x.size(3);
-              const c10::cuda::OptionalCUDAGuard guard(x.device());
-              c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
+              const CallGuard guard(x);
               at::NoGradGuard no_grad;
               return core_run(x, cm, B, H, W, cm ? B * H * W : H * W, w, with_norm, out_type, opt(workspace), Tensor());
           }, release());
     m.def("ss2d_core_by_operators",
           [](const Tensor& x, const CoreW& w, bool with_norm, at::ScalarType out_type, bool cm) {
               const int64_t B = x.size(cm ? 1 : 0), H = x.size(2), W = x.size(3);
-              const c10::cuda::OptionalCUDAGuard guard(x.device());
+              const CallGuard guard(x);
               return core_by_operators(x, cm, B, H, W, cm ? B * H * W : H * W, w, with_norm, out_type, Tensor());
           }, release());
     m.def("project",
           [](const Tensor& x, const CoreW& w, bool cm) {
               const int64_t B = x.size(cm ? 1 : 0), H = x.size(2), W = x.size(3);
-              const c10::cuda::OptionalCUDAGuard guard(x.device());
+              const CallGuard guard(x);
               const Streams s = project(x, cm, B, H, W, cm ? B * H * W : H * W, w, false);
               return std::make_pair(s.bc, s.delta);
           }, release());

@@ -46,6 +46,14 @@ inline Tensor f32(const Tensor& t) {
 inline Tensor rows(const Tensor& t) { return t.stride(-1) == 1 ? t : t.contiguous(); }
 inline Tensor bytes(int64_t n, const Tensor& like) { return at::empty({n}, like.options().dtype(at::kByte)); }
 
+// The caller's state as a call on raw pointers needs it: x's device, no autocast (a library product inside would return another
+// type than the one whose code goes to the kernels behind it).
+struct CallGuard {
+    explicit CallGuard(const Tensor& x) : device(x.device()), no_autocast(c10::autocast_dispatch_keyset) {}
+    c10::cuda::OptionalCUDAGuard device;
+    c10::impl::ExcludeDispatchKeyGuard no_autocast;
+};
+
 // host_ops.cpp
 std::pair<Tensor, Tensor> scan_fwd(Tensor u, Tensor delta, Tensor A, Tensor B, Tensor C, Tensor D, Tensor bias, bool softplus, bool out_float,
                                    int64_t every, Tensor out);

@@ -64,7 +64,7 @@ struct CoreNode : public torch::autograd::Function<CoreNode> {
     static Tensor forward(AutogradContext* ctx, const Tensor& x_, const Tensor& x_proj, const Tensor& dt_projs, const Tensor& dt_bias,
                           const Tensor& A_logs, const Tensor& Ds, const Tensor& ln_w, const Tensor& ln_b, int64_t N, int64_t R, double eps) {
         const Tensor x = x_.contiguous();
-        const c10::cuda::OptionalCUDAGuard guard(x.device());
+        const CallGuard guard(x);
         const int64_t B = x.size(0), D = x.size(1), H = x.size(2), W = x.size(3), L = H * W, C = R + 2 * N, S = padded_row(B, D, H, W);
         const auto of = x.options();
         const Tensor wx = x_proj.reshape({4 * C, D}).to(x.scalar_type()), wdt = dt_projs.reshape({4, D, R}).to(x.scalar_type()).contiguous();
@@ -102,7 +102,7 @@ struct CoreNode : public torch::autograd::Function<CoreNode> {
         const auto sz = ctx->saved_data["n"].toIntVector();
         const Tensor &xs = t[0], &xd = t[1], &dts = t[2], &bc = t[3], &states = t[4], &y = t[5], &wx = t[6], &wdt = t[7], &A = t[8];
         const int64_t B = sz[0], D = sz[1], H = sz[2], W = sz[3], N = sz[4], R = sz[5], S = sz[6], L = H * W, C = R + 2 * N;
-        const c10::cuda::OptionalCUDAGuard guard(xs.device());
+        const CallGuard guard(xs);                // backward() may be called inside an autocast region that the forward was not in
         const auto of = xs.options(), of32 = of.dtype(at::kFloat);
         const Tensor g = grads[0].contiguous(), lw = f32(in[6]);
         Tensor dy = at::empty({B, D, L}, of32), dlw = at::empty({D}, of32), dlb = at::empty({D}, of32);
