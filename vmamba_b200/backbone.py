@@ -78,7 +78,11 @@ class VSSMInfer:
         self.outnorm: Dict[int, tuple] = {}
         self.dtype = torch.bfloat16
         self.device = torch.device("cuda")
-        self._native = None
+
+    _native = None
+
+    def __getstate__(self):         # copies and pickles hold the tensors; a copy makes its own `native`
+        return {**self.__dict__, "_native": None}
 
     # ------------------------------------------------------------------ construction
     @staticmethod

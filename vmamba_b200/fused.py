@@ -38,7 +38,11 @@ class CoreWeights:
     dt_rank: int
     d_inner: int
     eps: float = 1e-5
-    _native: object = None
+
+    _native = None              # no field: what `native` made of the fields above
+
+    def __getstate__(self):     # copies and pickles hold the tensors; a copy makes its own `native`
+        return {**self.__dict__, "_native": None}
 
     @property
     def native(self):
