@@ -1,5 +1,6 @@
 """What the state of the calling program must not change: autocast regions, copies of a model, what a training step keeps.
 Needs a GPU."""
+import copy
 import math
 
 import pytest
@@ -86,3 +87,21 @@ def test_core_under_autocast(vb, dtype):
             return [*outs, y, *torch.autograd.grad(y, leaves, gy)]
     for a, b in zip(step(False), step(True)):
         assert a.dtype == b.dtype and torch.equal(a, b)
+
+
+def test_parts_replaced_after_the_first_call(vb):
+    """A model whose parts are replaced gives what one built with them gives, and a copy is a model of its own."""
+    sd, x = state_dict(), torch.randn(2, 3, 64, 64, device="cuda").bfloat16()
+    m = vb.VSSMInfer.from_state_dict(sd)
+    first = m(x)
+    twin = copy.deepcopy(m)
+    sd["classifier.head.bias"], sd["layers.2.blocks.0.op.Ds"] = torch.ones(10), sd["layers.2.blocks.0.op.Ds"] * 2
+    other = vb.VSSMInfer.from_state_dict(sd)
+    m.head["b"], m.blocks[2][0].core.Ds = other.head["b"], other.blocks[2][0].core.Ds
+    assert torch.equal(m(x), other(x)) and not torch.equal(m(x), first)
+    assert torch.equal(twin(x), first)
+    w = vb.CoreWeights(*(getattr(m.blocks[0][0].core, k) for k in ("wx", "wdt", "A", "Ds", "dt_bias", "ln_weight", "ln_bias", "d_state", "dt_rank", "d_inner")))
+    y = torch.randn(1, w.d_inner, 8, 8, device="cuda").bfloat16()
+    one = vb.ss2d_core(y, w)
+    w.ln_bias = w.ln_bias + 1
+    assert ((vb.ss2d_core(y, w) - one).float() - 1).abs().max() < 0.05      # bf16: half a unit in the last place of values below 8

@@ -32,3 +32,47 @@ def test_core_weights_are_a_plain_dataclass(model):
     names = [f.name for f in dataclasses.fields(w)]
     assert names[0] == "wx" and names[-1] == "eps" and set(dataclasses.asdict(w)) == set(names)
     assert dataclasses.replace(w, eps=1e-6).native is not w.native
+
+
+def _replace_head(m):
+    m.head["b"] = torch.ones_like(m.head["b"])
+
+
+def _replace_core_field(m):
+    m.blocks[1][0].core.Ds = m.blocks[1][0].core.Ds * 2
+
+
+def _drop_a_block(m):
+    m.blocks[3] = []
+
+
+CHANGES = {
+    "dtype": lambda m: setattr(m, "dtype", torch.float16),
+    "stem": lambda m: m.stem.update(b0=m.stem["b0"] + 1),
+    "block": lambda m: setattr(m.blocks[0][0], "w_in", m.blocks[0][0].w_in * 2),
+    "core": _replace_core_field,
+    "eps": lambda m: setattr(m.blocks[0][0].core, "eps", 1e-3),
+    "blocks": _drop_a_block,
+    "down": lambda m: m.down[0].update(bf=m.down[0]["bf"] + 1),
+    "outnorm": lambda m: m.outnorm.update({2: (m.outnorm[2][0] * 2, m.outnorm[2][1])}),
+    "head": _replace_head,
+    "no head": lambda m: setattr(m, "head", None),
+}
+
+
+@pytest.mark.parametrize("what", CHANGES)
+def test_changes_after_the_first_call_count(model, what):
+    before = model.native
+    CHANGES[what](model)
+    after = model.native
+    assert after is not before and after is model.native
+    assert after.dtype == model.dtype and len(after.head) == (0 if model.head is None else 4)
+    if model.head is not None:
+        assert torch.equal(after.head[3], model.head["b"])
+
+
+def test_core_weight_changes_count(model):
+    w = model.blocks[0][0].core
+    before = w.native
+    w.eps = 1e-3
+    assert w.native is not before and w.native is w.native

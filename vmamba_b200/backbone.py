@@ -15,6 +15,7 @@ the scan.
 from __future__ import annotations
 
 import re
+from operator import attrgetter, is_, itemgetter
 from typing import Dict, List, Optional, Sequence
 
 import torch
@@ -32,6 +33,13 @@ CONFIGS = dict(
 
 class _Block:
     __slots__ = ("n1w", "n1b", "w_in", "w_dw", "core", "w_out", "n2w", "n2b", "w1", "b1f", "w2", "b2f", "D")
+
+
+# what the host extension holds of a model, part by part
+_STEM = itemgetter("w0", "b0", "n0w", "n0b", "w1", "b1", "n1w", "n1b")
+_BLOCK = attrgetter("n1w", "n1b", "n2w", "n2b", "w_in", "w_dw", "w_out", "w1", "b1f", "w2", "b2f", "core.native")
+_DOWN = itemgetter("w", "bf", "nw", "nb")
+_HEAD = itemgetter("nw", "nb", "w", "b")
 
 
 def normalize_state_dict(sd: dict) -> dict:
@@ -150,25 +158,37 @@ class VSSMInfer:
     # ------------------------------------------------------------------ public
     # The forward itself (patch embedding, blocks, downsampling, norms) runs in the host extension: a forward is 120 to 300
     # launches, which Python issues more slowly than the GPU runs them (csrc/host_backbone.cpp).
+    def _parts(self) -> list:
+        parts = [self.dtype, *_STEM(self.stem), *(() if self.head is None else _HEAD(self.head))]
+        for stage, down in zip(self.blocks, self.down):
+            for b in stage:
+                parts += _BLOCK(b)
+            parts += (None,) if down is None else _DOWN(down)
+        for i, (w, b) in self.outnorm.items():
+            parts += (i, w, b)
+        return parts
+
     @property
     def native(self):
-        if self._native is None:
-            n = _host.Backbone()
-            n.dtype = self.dtype
-            s = self.stem
-            n.stem = [s["w0"], s["b0"], s["n0w"], s["n0b"], s["w1"], s["b1"], s["n1w"], s["n1b"]]
-            for stage, down in zip(self.blocks, self.down):
-                for j, b in enumerate(stage):
-                    c = b.core
-                    n.add_block(j == 0, [b.n1w, b.n1b, b.n2w, b.n2b, b.w_in, b.w_dw, b.w_out, b.w1, b.b1f, b.w2, b.b2f,
-                                         c.wx, c.wdt, c.A, c.Ds, c.dt_bias], [c.ln_weight, c.ln_bias], c.d_state, c.dt_rank, c.eps)
-                n.add_down([] if down is None else [down["w"], down["bf"], down["nw"], down["nb"]])
-            if self.head is not None:
-                n.head = [self.head["nw"], self.head["nb"], self.head["w"], self.head["b"]]
-            for i, (w, b) in self.outnorm.items():
-                n.add_outnorm(i, w, b)
-            self._native = n
-        return self._native
+        """The model as the host extension holds it, made anew when a part of this one has been replaced since.  The parts it was
+        made from are kept with it, so that `is` cannot mistake a new tensor for one of them."""
+        parts, made = self._parts(), self._native
+        if made is not None and len(made[0]) == len(parts) and all(map(is_, made[0], parts)):
+            return made[1]
+        n = _host.Backbone()
+        n.dtype = self.dtype
+        n.stem = list(_STEM(self.stem))
+        for stage, down in zip(self.blocks, self.down):
+            for j, b in enumerate(stage):
+                *tensors, core = _BLOCK(b)
+                n.add_block(j == 0, tensors, core)
+            n.add_down([] if down is None else list(_DOWN(down)))
+        if self.head is not None:
+            n.head = list(_HEAD(self.head))
+        for i, (w, b) in self.outnorm.items():
+            n.add_outnorm(i, w, b)
+        self._native = parts, n
+        return n
 
     def __call__(self, img: torch.Tensor) -> torch.Tensor:
         """VSSM.forward (vmamba.py:2027-2035): (B, 3, H, W) -> (B, num_classes) logits."""

@@ -263,11 +263,11 @@ public:
     std::map<int64_t, Norm> outnorm;
     at::ScalarType type = at::kBFloat16;
 
-    void add_block(bool first, std::vector<Tensor> t, std::vector<OptT> ln, int64_t N, int64_t R, double eps) {
+    void add_block(bool first, std::vector<Tensor> t, const CoreW& core) {
         Block b;
         b.n1 = {t[0], t[1]}; b.n2 = {t[2], t[3]};
         b.w_in = t[4]; b.w_dw = t[5]; b.w_out = t[6]; b.w1 = t[7]; b.b1 = t[8]; b.w2 = t[9]; b.b2 = t[10];
-        b.core = core_weights(t[11], t[12], t[13], t[14], t[15], ln[0], ln[1], N, R, eps);
+        b.core = core;
         if (first) stages.emplace_back();
         stages.back().push_back(std::move(b));
     }

@@ -44,6 +44,11 @@ class CoreWeights:
     def __getstate__(self):     # copies and pickles hold the tensors; a copy makes its own `native`
         return {**self.__dict__, "_native": None}
 
+    def __setattr__(self, name, value):
+        super().__setattr__(name, value)
+        if name != "_native":
+            super().__setattr__("_native", None)
+
     @property
     def native(self):
         """The same weights as the host extension holds them."""
