@@ -5,6 +5,7 @@ import math
 
 import pytest
 import torch
+import torch.utils.checkpoint
 
 pytestmark = pytest.mark.gpu
 
@@ -105,3 +106,51 @@ def test_parts_replaced_after_the_first_call(vb):
     one = vb.ss2d_core(y, w)
     w.ln_bias = w.ln_bias + 1
     assert ((vb.ss2d_core(y, w) - one).float() - 1).abs().max() < 0.05      # bf16: half a unit in the last place of values below 8
+
+
+def _core_step(vb, dtype=torch.bfloat16):
+    D, R = 64, 4
+    g = torch.Generator(device="cuda").manual_seed(2)
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=g)      # noqa: E731
+    leaves = [rnd(2, D, 24, 24).to(dtype), rnd(4 * (R + 2), D) * D ** -0.5, rnd(4 * D, R) * R ** -0.5, torch.full((4, D), -3.0, device="cuda"),
+              torch.zeros(4 * D, 1, device="cuda"), torch.ones(4 * D, device="cuda"), torch.ones(D, device="cuda"), torch.zeros(D, device="cuda")]
+    return [t.requires_grad_(True) for t in leaves], lambda *t: vb.ss2d_core_autograd(*t, d_state=1, dt_rank=R)
+
+
+def _scan_step(vb):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=g)      # noqa: E731
+    leaves = [rnd(2, 64, 600), rnd(2, 64, 600) - 3, -torch.ones(64, 1, device="cuda"), rnd(2, 4, 1, 600), rnd(2, 4, 1, 600)]
+    return [t.requires_grad_(True) for t in leaves], vb.selective_scan_fn
+
+
+# what a step keeps between its passes, in units of its largest input: the core four routes of x and of the step sizes, the states
+# (four routes, fp32, one of eight elements) and the merged map (fp32); the scan u, delta and the states
+@pytest.mark.parametrize("step,kept", [(_core_step, 4 + 4 + 1 + 2), (_scan_step, 2 + 1 / 8)])
+def test_what_a_training_step_keeps(vb, step, kept):
+    """Tensors kept for the backward pass go through saved-tensor hooks and are freed by it, though the result lives on."""
+    leaves, fn = step(vb)
+    size = leaves[0].numel() * leaves[0].element_size()
+    seen = []
+
+    def pack(t):
+        seen.append(t.numel() * t.element_size())
+        return t.cpu()
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()):
+        y = fn(*leaves)
+    assert sum(seen) >= kept * size
+    gy = torch.ones_like(y)
+    from_host = torch.autograd.grad(y, leaves, gy)
+    y = fn(*leaves)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    grads = torch.autograd.grad(y, leaves, gy)
+    torch.cuda.synchronize()
+    held = sum(t.numel() * t.element_size() for t in grads)
+    own = 0 if step is _core_step else 2             # the scan keeps its caller's u and delta
+    assert torch.cuda.memory_allocated() <= before + held - 0.9 * (kept - own) * size
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(y, leaves, gy)
+    again = torch.autograd.grad(torch.utils.checkpoint.checkpoint(fn, *leaves, use_reentrant=False), leaves, gy)
+    for a, b, c in zip(grads, from_host, again):
+        assert torch.equal(a, b) and torch.equal(a, c)

@@ -89,8 +89,8 @@ struct CoreNode : public torch::autograd::Function<CoreNode> {
         n.in = y.data_ptr(); n.weight = lw.data_ptr(); n.bias = lb.data_ptr(); n.out = out.data_ptr();
         n.B = B; n.D = D; n.L = L; n.io_dtype = dtype_code(x); n.eps = (float)eps;
         check(ss2d_layer_norm_cf(&n, stream_of(x)), "ss2d_layer_norm_cf");
-        ctx->save_for_backward({x_, x_proj, dt_projs, dt_bias, A_logs, Ds, ln_w, ln_b});
-        ctx->saved_data["t"] = std::vector<Tensor>{xs, xd, dts, bc, states, y, wx, wdt, A};
+        // all tensors as saved variables: saved-tensor hooks see them, and they are freed as the backward pass advances
+        ctx->save_for_backward({x_, x_proj, dt_projs, dt_bias, A_logs, Ds, ln_w, ln_b, xs, xd, dts, bc, states, y, wx, wdt, A});
         ctx->saved_data["n"] = std::vector<int64_t>{B, D, H, W, N, R, S};
         ctx->saved_data["eps"] = eps;
         return out;
@@ -98,9 +98,8 @@ struct CoreNode : public torch::autograd::Function<CoreNode> {
 
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         const auto in = ctx->get_saved_variables();
-        const auto t = ctx->saved_data["t"].toTensorVector();
         const auto sz = ctx->saved_data["n"].toIntVector();
-        const Tensor &xs = t[0], &xd = t[1], &dts = t[2], &bc = t[3], &states = t[4], &y = t[5], &wx = t[6], &wdt = t[7], &A = t[8];
+        const Tensor &xs = in[8], &xd = in[9], &dts = in[10], &bc = in[11], &states = in[12], &y = in[13], &wx = in[14], &wdt = in[15], &A = in[16];
         const int64_t B = sz[0], D = sz[1], H = sz[2], W = sz[3], N = sz[4], R = sz[5], S = sz[6], L = H * W, C = R + 2 * N;
         const CallGuard guard(xs);                // backward() may be called inside an autocast region that the forward was not in
         const auto of = xs.options(), of32 = of.dtype(at::kFloat);

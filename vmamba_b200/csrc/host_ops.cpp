@@ -115,14 +115,13 @@ struct ScanNode : public torch::autograd::Function<ScanNode> {
         const Tensor D = opt(D_), bias = opt(bias_);
         const int64_t ratio = u.dim() == 3 && delta.dim() == 3 && delta.size(1) ? scan_ratio(u, delta) : 1;
         auto [out, ckpt] = scan_fwd(u, delta, A, B, C, D, bias, softplus, out_float, ss2d_selective_scan_checkpoint_every(A.size(-1), ratio), Tensor());
-        ctx->save_for_backward({u, delta, A, B, C, D, bias});
-        ctx->saved_data["states"] = ckpt;
+        ctx->save_for_backward({u, delta, A, B, C, D, bias, ckpt});
         ctx->saved_data["softplus"] = softplus;
         return out;
     }
     static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list g) {
         const auto s = ctx->get_saved_variables();
-        auto r = scan_bwd(s[0], s[1], s[2], s[3], s[4], s[5], s[6], g[0], ctx->saved_data["softplus"].toBool(), ctx->saved_data["states"].toTensor());
+        auto r = scan_bwd(s[0], s[1], s[2], s[3], s[4], s[5], s[6], g[0], ctx->saved_data["softplus"].toBool(), s[7]);
         auto as = [](const Tensor& x, const Tensor& like) { return x.defined() && x.scalar_type() != like.scalar_type() ? x.to(like.scalar_type()) : x; };
         return {r[0], r[1], as(r[2], s[2]), r[3], r[4], as(r[5], s[5]), as(r[6], s[6]), Tensor(), Tensor()};
     }
