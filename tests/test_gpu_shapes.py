@@ -176,3 +176,29 @@ def test_linear_few_pixels_gelu(M, K, N, dt):
     assert _lib.lib().ss2d_linear_fwd(p, torch.cuda.current_stream().cuda_stream) == _lib.SS2D_OK
     ref = torch.nn.functional.gelu(w.double() @ x.double() + bias.double()[:, None])
     assert (out.double() - ref).abs().max() <= (2e-2 if dt == "bf16" else 3e-3)
+
+
+@pytest.mark.parametrize("at", [(0, 0, 0, 0), (1, 3, 5, 7), (6, 2, 1, 4)])
+@pytest.mark.parametrize("N,K,Cd,L,dt", [(1, 3, 3, 5, "bf16"), (1, 1, 1, 1, "f32"), (1, 3, 5, 49, "f16"), (1, 1, 3, 131, "f32"), (1, 3, 7, 1001, "bf16"),
+                                         (1, 1, 9, 4099, "bf16"), (1, 3, 1100, 33, "f32"), (2, 3, 5, 67, "f32"), (4, 1, 33, 131, "bf16"), (16, 3, 3, 35, "f16")])
+def test_scan_tensors_off_16_byte_boundaries(vb, N, K, Cd, L, dt, at):
+    """Tensors that do not start or end on 16-byte boundaries, of odd row lengths and counts, in the middle of NaN: forward, states and
+    gradients."""
+    u, delta, A, B, C, D, bias, dout = _random_case(1, K, Cd, N, L, seed=L + N)
+    td = TD[dt]
+
+    def put(a, offset, type=td):
+        flat = torch.full((a.size + 32,), float("nan"), device="cuda", dtype=type)
+        view = flat[8 + offset:8 + offset + a.size].view(a.shape)
+        view.copy_(dev(a, type))
+        return view
+    if dt != "f32":
+        u, delta, B, C = (O._round_to(a, dt) for a in (u, delta, B, C))
+    ts = [put(a, o) for a, o in zip((u, delta, B, C), at)]
+    y, states = vb.selective_scan_fwd(ts[0], ts[1], dev(A), ts[2], ts[3], dev(D), dev(bias), True, True, return_checkpoints="grad")
+    assert O.max_rel_err(host(y), CO.selective_scan(u, delta, A, B, C, D, bias, True)) <= TOL_F32
+    ref = O.selective_scan_bwd(u, delta, A, B, C, D, bias, dout, True, dt)
+    for ck in (states, None):
+        got = vb.selective_scan_bwd(ts[0], ts[1], dev(A), ts[2], ts[3], dev(D), dev(bias), put(dout, at[0], torch.float32), True, ck)
+        for name, x, r in zip(NAMES, got, ref):
+            assert O.max_rel_err(host(x), r) <= TOL[dt], name

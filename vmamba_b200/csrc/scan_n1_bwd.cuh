@@ -12,6 +12,8 @@
 //
 // Bound: instruction issue (about 45 per element, four of them on the MUFU pipe).
 #pragma once
+#include <type_traits>
+
 #include "scan_row.cuh"
 
 namespace ss2d {
@@ -29,12 +31,15 @@ struct N1BwdArgs {
     int64_t dim, group_size, batch, dratio;
     int64_t u_bs, u_ds, d_bs, d_ds, g_bs, g_ds, B_bs, B_gs, C_bs, C_gs;
     int L, Lp, n_groups, parts, R, S, seg_len, softplus;
+    // AL = 0: B and C start and end on 16-byte boundaries; else their elements are loaded one by one (32 x 384 rows of 3 137
+    // elements, bf16: the choice costs 257 -> 265 us of the gradients, always one by one 277)
+    int bc_pieces;
 };
 
 template <typename T, int AL>
 __device__ __forceinline__ void row8_pairs(const Row8<T, AL>& w, const T* row, int pos, int L, float2 (&v)[4]) {
     float x[8];
-    w.get(row, pos, L, x);
+    w.get(row, pos, 0, L, x);
 #pragma unroll
     for (int i = 0; i < 4; ++i) v[i] = make_float2(x[2 * i], x[2 * i + 1]);
 }
@@ -133,7 +138,7 @@ __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArg
     auto delta_row = [&](int64_t r) { return dt + (a.dratio == 1 ? r : r / a.dratio) * a.d_ds; };
     auto fetch = [&](int i, int pos) {
         const int64_t r = row_of(i);
-        nu.load(u + r * a.u_ds, pos, L); nd.load(delta_row(r), pos, L); ng.load(gp + r * a.g_ds, pos, L);
+        nu.load(u + r * a.u_ds, pos, 0, L); nd.load(delta_row(r), pos, 0, L); ng.load(gp + r * a.g_ds, pos, 0, L);
         nh = pos < L ? __ldg(a.ckpt + (out0 + r) * nck + (pos >> 3)) : 0.f;
     };
     int buf = 0;
@@ -142,11 +147,13 @@ __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArg
         const int pos = c * kChunk + ln * 8;
         float2 bv[4], cv[4], accB[4], accC[4];
         if (mine) fetch(0, pos);
-        {
-            Row8<Tin, AL> rb, rc;
-            rb.load(Bm, pos, L); rc.load(Cm, pos, L);
+        auto load_bc = [&](auto al) {
+            Row8<Tin, decltype(al)::value> rb, rc;
+            rb.load(Bm, pos, 0, L); rc.load(Cm, pos, 0, L);
             row8_pairs(rb, Bm, pos, L, bv); row8_pairs(rc, Cm, pos, L, cv);
-        }
+        };
+        if (AL == 0 && !a.bc_pieces) load_bc(std::integral_constant<int, 1>{});
+        else load_bc(std::integral_constant<int, AL>{});
 #pragma unroll
         for (int i = 0; i < 4; ++i) accB[i] = accC[i] = pk(0.f);
 #pragma unroll 1
@@ -293,10 +300,17 @@ __global__ void __launch_bounds__(kN1Warps * 32) n1_bwd_segments_kernel(const N1
         const int pos = c * kN1Chunk + lane * 8;
         float2 d[4], g[4], cv[4];
         {
-            Row8<Tin, AL> xd, xc;
+            Row8<Tin, AL> xd;
             Row8<Tg, AL> xg;
-            xd.load(dt, pos, L); xg.load(gp, pos, L); xc.load(Cm, pos, L);
-            row8_pairs(xd, dt, pos, L, d); row8_pairs(xg, gp, pos, L, g); row8_pairs(xc, Cm, pos, L, cv);
+            xd.load(dt, pos, 0, L); xg.load(gp, pos, 0, L);
+            auto load_c = [&](auto al) {
+                Row8<Tin, decltype(al)::value> xc;
+                xc.load(Cm, pos, 0, L);
+                row8_pairs(xc, Cm, pos, L, cv);
+            };
+            if (AL == 0 && !a.bc_pieces) load_c(std::integral_constant<int, 1>{});
+            else load_c(std::integral_constant<int, AL>{});
+            row8_pairs(xd, dt, pos, L, d); row8_pairs(xg, gp, pos, L, g);
         }
         float le = 0.f, ls = 0.f;
 #pragma unroll

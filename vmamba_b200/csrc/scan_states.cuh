@@ -130,7 +130,7 @@ template <typename T, int RPW, int VW> struct StRaw {
         }
     }
 };
-// VW 0: rows of any alignment, runs of eight cut out of aligned pieces.  (Single elements, VW 1, cost the few-state kernels their
+// VW 0: rows of any alignment in tensors that start and end on 16-byte boundaries, runs of eight cut out of aligned pieces.  (Single elements, VW 1, cost the few-state kernels their
 // loads: 4 608 rows of 8 594 elements, 4 states, bf16 1021 -> 394 us.)
 template <typename T, int RPW> struct StRaw<T, RPW, 0> {
     static constexpr int kRuns = RPW / 8;
@@ -142,11 +142,11 @@ template <typename T, int RPW> struct StRaw<T, RPW, 0> {
     __device__ __forceinline__ void load(const T* rows, int64_t stride, int count, int t0, int L, int lane) {
         for_each(lane, [&](int i, int row, int el, auto) {
             w[i] = {};
-            if (row < count) w[i].load(rows + row * stride, t0 + el, L);
+            if (row < count) w[i].load(rows + row * stride, t0 + el, 0, L);
         });
     }
     __device__ __forceinline__ void get(int i, float (&v)[8], const T* rows, int64_t stride, int t0, int L, int lane) const {
-        w[i].get(rows + (i * 8 + (lane >> 2)) * stride, t0 + (lane & 3) * 8, L, v);
+        w[i].get(rows + (i * 8 + (lane >> 2)) * stride, t0 + (lane & 3) * 8, 0, L, v);
     }
 };
 // B or C of one chunk, spread over the threads of the CTA.
@@ -196,7 +196,7 @@ template <typename T, int NS, int WARPS> struct StRawBC<T, NS, 0, WARPS> {
         for (int j = 0; j < kPer; ++j) {
             const int i = threadIdx.x + j * kThreads, n = i % NS, el = (i / NS) * 8;
             w[j] = {};
-            if (n < N && el < kStChunk) w[j].load(src + n * state_stride, t0 + el, L);
+            if (n < N && el < kStChunk) w[j].load(src + n * state_stride, t0 + el, 0, L);
         }
     }
     __device__ __forceinline__ void put(float* dst, const T* src, int64_t state_stride, int t0, int L) const {
@@ -205,7 +205,7 @@ template <typename T, int NS, int WARPS> struct StRawBC<T, NS, 0, WARPS> {
             const int i = threadIdx.x + j * kThreads, n = i % NS, el = (i / NS) * 8;
             if (kItems % kThreads == 0 || i < kItems) {
                 float v[8];
-                w[j].get(src + n * state_stride, t0 + el, L, v);
+                w[j].get(src + n * state_stride, t0 + el, 0, L, v);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) dst[(el + e) * StLayout<NS>::BCP + n] = v[e];
             }

@@ -249,8 +249,8 @@ static int st_rows_per_lane(const StFwdArgs& a, int64_t batch, cudaStream_t st) 
     return st_launch_fwd<Tin, Tout, NS, 1, VW, kOut>(a, batch, st);
 }
 
-// vw: vector width of the global accesses, 8, 4 or less.  Rows without vectors: pieces of 16-bit rows (above), but single elements
-// of fp32 rows where a warp holds no more than 16 of them (4 608 rows of 8 593, 16 states: 0.82 against 1.36 ms with pieces; 4 states:
+// vw: vector width of the global accesses, 8, 4, 1, or 0 for rows without vectors in tensors that start and end on 16-byte
+// boundaries (no piece reaches beyond them then): pieces of 16-bit rows (above), but single elements of fp32 rows where a warp holds no more than 16 of them (4 608 rows of 8 593, 16 states: 0.82 against 1.36 ms with pieces; 4 states:
 // 508 against 445 us).
 template <typename Tin, typename Tout, bool kOut>
 static int st_dispatch_fwd(const StFwdArgs& a, int64_t batch, int vw, cudaStream_t st) {
@@ -259,7 +259,8 @@ static int st_dispatch_fwd(const StFwdArgs& a, int64_t batch, int vw, cudaStream
     if (NS == NS_)                                                                              \
         return vw == 8   ? st_rows_per_lane<Tin, Tout, NS_, 8, kOut>(a, batch, st)              \
                : vw == 4 ? st_rows_per_lane<Tin, Tout, NS_, 4, kOut>(a, batch, st)              \
-                         : st_rows_per_lane<Tin, Tout, NS_, (sizeof(Tin) == 2 || NS_ == 4 ? 0 : 1), kOut>(a, batch, st);
+               : vw == 0 ? st_rows_per_lane<Tin, Tout, NS_, (sizeof(Tin) == 2 || NS_ == 4 ? 0 : 1), kOut>(a, batch, st) \
+                         : st_rows_per_lane<Tin, Tout, NS_, 1, kOut>(a, batch, st);
     SS2D_ST(4)
     SS2D_ST(8)
     SS2D_ST(16)

@@ -19,6 +19,7 @@ struct ScanArgs {
     int64_t rows, dim, dstate, seqlen, group_size;
     int64_t u_bs, u_ds, d_bs, d_ds, o_bs, o_ds;
     int64_t B_bs, B_gs, B_ss, C_bs, C_gs, C_ss;
+    ScanSpans span;
     int softplus;
     int64_t dratio;   // channels per delta row
     float* ckpt;      // (rows, nck, dstate) or null
@@ -35,11 +36,13 @@ constexpr int kWarpsPerCta = 4;
 // fill the chip; fewer rows get the more warps (up to 24 per SM).
 // AL is the vector width of every access (8 or 4 elements), or 0 for rows of any alignment: a row is then walked from
 // the 16-byte boundary in front of its result, so that the results leave as vectors, and the inputs are cut out of the
-// aligned pieces around them.
+// aligned pieces around them.  Elements of the tensors' first and last rows whose pieces would reach beyond a tensor (at most
+// seven at either end) are taken one by one in front of the walk and behind it.
 // `every` (a multiple of 8): spacing of the states kept for the backward pass.
 // Rows of at most 128 (64) elements share a warp, two (four) at a time, LPR = 16 (8) lanes each.
+// fp32 rows of any alignment are held to 128 registers, four CTAs per SM (12 288 rows of 3 137 elements: 170 -> 132 us).
 template <typename Tin, typename Tout, int AL, int W, int LPR>
-__global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32) selscan_fwd_n1_kernel(const ScanArgs a) {
+__global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32, W == 1 && AL == 0 && sizeof(Tin) == 4 ? 4 : 0) selscan_fwd_n1_kernel(const ScanArgs a) {
     static_assert(W == 1 || LPR == 32, "rows of several warps take whole warps");
     constexpr int VEC = 8, WSTEP = LPR * VEC, STEP = W * WSTEP;
     __shared__ AB agg[2][W];
@@ -63,15 +66,31 @@ __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32) selscan_f
     constexpr int OV = 16 / (int)sizeof(Tout);       // elements per 16-byte store
     const int ph = AL ? 0 : (int)((reinterpret_cast<uintptr_t>(out) / sizeof(Tout)) & (OV - 1));
     constexpr int ph_max = AL ? 0 : OV - 1;
+    Inner in = {0, L};
+    if constexpr (AL == 0)
+        in = both(both(inner_of(u, L, a.span.u), inner_of(dt, L, a.span.delta), L), both(inner_of(Bm, L, a.span.B), inner_of(Cm, L, a.span.C), L), L);
+    const int l0 = in.from, l1 = in.to;              // the elements of the walk
     Row8<Tin, AL> ru, rd, rb, rc;
-    auto fetch = [&](int at) { ru.load(u, at, L); rd.load(dt, at, L); rb.load(Bm, at, L); rc.load(Cm, at, L); };
+    auto fetch = [&](int at) { ru.load(u, at, l0, l1); rd.load(dt, at, l0, l1); rb.load(Bm, at, l0, l1); rc.load(Cm, at, l0, l1); };
     int pos = wi * WSTEP + lane * VEC - ph;
     fetch(pos);
     float hc = 0.f;                                  // state entering this step
-    // rows that share a warp may start at different phases: they take the same number of steps
-    for (int base = LPR < 32 ? -ph_max : -ph, it = 0; base < L; base += STEP, ++it) {
+    auto one_by_one = [&](int l, int to) {           // by all lanes of the row alike
+        for (; l < to; ++l) {
+            const float ul = to_f<Tin>(u[l]);
+            float dl = to_f<Tin>(dt[l]) + bias;
+            if (sp) dl = softplus_fast(dl);
+            const bool writes = real && lane == 0 && wi == 0;
+            if (a.ckpt && writes && l % a.every == 0) a.ckpt[row * a.nck + l / a.every] = hc;
+            hc = fmaf(decay_fast(dl, A2), hc, dl * to_f<Tin>(Bm[l]) * ul);
+            if (!a.states_only && writes) out[l] = from_f<Tout>(fmaf(Dv, ul, to_f<Tin>(Cm[l]) * hc));
+        }
+    };
+    if constexpr (AL == 0) one_by_one(0, l0);
+    // rows that share a warp may start at different phases and end at different elements: they take the same number of steps
+    for (int base = LPR < 32 ? -ph_max : -ph, it = 0; base < (LPR < 32 ? L : l1); base += STEP, ++it) {
         float uv[VEC], dv[VEC], bv[VEC], cv[VEC], P[VEC], hl[VEC];
-        ru.get(u, pos, L, uv); rd.get(dt, pos, L, dv); rb.get(Bm, pos, L, bv); rc.get(Cm, pos, L, cv);
+        ru.get(u, pos, l0, l1, uv); rd.get(dt, pos, l0, l1, dv); rb.get(Bm, pos, l0, l1, bv); rc.get(Cm, pos, l0, l1, cv);
         fetch(pos + STEP);
         float p = 1.f, h = 0.f;
 #pragma unroll
@@ -79,7 +98,7 @@ __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32) selscan_f
             float dl = dv[i] + bias;
             if (sp) dl = softplus_fast(dl);
             // outside the row: a step of zero leaves the state as it is (whole vectors are tested once below)
-            if constexpr (AL != 8) dl = pos + (AL ? i / (AL ? AL : 1) * AL : i) < L && (AL || pos + i >= 0) ? dl : 0.f;
+            if constexpr (AL != 8) dl = pos + (AL ? i / (AL ? AL : 1) * AL : i) < l1 && (AL || pos + i >= l0) ? dl : 0.f;
             const float aa = decay_fast(dl, A2);
             h = fmaf(aa, h, dl * bv[i] * uv[i]);
             p *= aa;
@@ -116,7 +135,7 @@ __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32) selscan_f
             } else {
 #pragma unroll
                 for (int i = 0; i < VEC; ++i)
-                    if (pos + i >= 0 && pos + i < L && (pos + i) % a.every == 0)
+                    if (pos + i >= l0 && pos + i < l1 && (pos + i) % a.every == 0)
                         a.ckpt[row * a.nck + (pos + i) / a.every] = i == 0 ? hin : fmaf(P[i > 0 ? i - 1 : 0], hin, hl[i > 0 ? i - 1 : 0]);
             }
         }
@@ -128,7 +147,7 @@ __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32) selscan_f
 #pragma unroll
             for (int j = 0; j < VEC; j += SV) {
                 const int q = pos + j;
-                if (AL != 0 ? q < L : (q >= 0 && q + SV <= L)) {
+                if (AL != 0 ? q < L : (q >= l0 && q + SV <= l1)) {
                     float o[SV];
 #pragma unroll
                     for (int e = 0; e < SV; ++e) o[e] = ov[j + e];
@@ -136,12 +155,13 @@ __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32) selscan_f
                 } else if (AL == 0) {
 #pragma unroll
                     for (int e = 0; e < SV; ++e)
-                        if (q + e >= 0 && q + e < L) out[q + e] = from_f<Tout>(ov[j + e]);
+                        if (q + e >= l0 && q + e < l1) out[q + e] = from_f<Tout>(ov[j + e]);
                 }
             }
         }
         pos += STEP;
     }
+    if constexpr (AL == 0) one_by_one(max(l0, l1), L);
 }
 
 // d_state > 1: the carry of each state lives in shared memory (one slot per warp and state).
@@ -375,7 +395,10 @@ static int selective_scan_states(const ss2d_scan_params* p, cudaStream_t st) {
     a.S = s.count; a.seg_len = s.len;
     a.ends = floats ? (float*)p->workspace : nullptr;
     a.sums = floats ? a.ends + p->batch * p->dim * s.count * st_pad_states(p->dstate) : nullptr;
-    const int v = fwd_vec(p), vw = v >= 8 ? 8 : v >= 4 ? 4 : 1;
+    // 0: no vectors, but pieces (16-byte boundaries at the tensors' ends)
+    const ScanSpans s4 = scan_spans(*p, dtype_size(p->in_dtype));
+    const bool pieces = whole_pieces(s4.u) && whole_pieces(s4.delta) && whole_pieces(s4.B) && whole_pieces(s4.C);
+    const int v = fwd_vec(p), vw = v >= 8 ? 8 : v >= 4 ? 4 : pieces ? 0 : 1;
     const bool of32 = p->out_dtype == SS2D_F32;
     if (p->in_dtype == SS2D_F32) return states_fwd<float, float>(a, p, vw, st);
     if (p->in_dtype == SS2D_BF16) return of32 ? states_fwd<__nv_bfloat16, float>(a, p, vw, st) : states_fwd<__nv_bfloat16, __nv_bfloat16>(a, p, vw, st);
@@ -398,6 +421,7 @@ int selective_scan_fwd(const ss2d_scan_params* p, cudaStream_t st) {
     a.o_bs = p->out_batch_stride; a.o_ds = p->out_dim_stride;
     a.B_bs = p->B_batch_stride; a.B_gs = p->B_group_stride; a.B_ss = p->B_state_stride;
     a.C_bs = p->C_batch_stride; a.C_gs = p->C_group_stride; a.C_ss = p->C_state_stride;
+    a.span = scan_spans(*p, dtype_size(p->in_dtype));
     a.softplus = p->delta_softplus;
     a.dratio = p->delta_ratio > 1 ? p->delta_ratio : 1;
     a.ckpt = (float*)p->checkpoints;

@@ -157,9 +157,17 @@ static int dispatch_grad(const ss2d_scan_bwd_params* p, const GradPlan& c, float
         a.u_bs = p->u_batch_stride; a.u_ds = p->u_dim_stride; a.d_bs = p->delta_batch_stride; a.d_ds = p->delta_dim_stride;
         a.g_bs = p->dout_batch_stride; a.g_ds = p->dout_dim_stride;
         a.B_bs = p->B_batch_stride; a.B_gs = p->B_group_stride; a.C_bs = p->C_batch_stride; a.C_gs = p->C_group_stride;
+        const ScanSpans s = scan_spans(*p, dtype_size(p->in_dtype));
         a.L = (int)p->seqlen; a.Lp = c.Lp; a.n_groups = (int)p->n_groups; a.parts = c.parts; a.R = c.sets; a.S = c.S; a.seg_len = c.seg_len;
         a.softplus = p->delta_softplus;
-        return c.vw == 8 ? launch_n1_bwd<Tin, Tg, 8>(a, st) : c.vw == 4 ? launch_n1_bwd<Tin, Tg, 4>(a, st) : launch_n1_bwd<Tin, Tg, 0>(a, st);
+        a.bc_pieces = whole_pieces(s.B) && whole_pieces(s.C);
+        // rows without vectors: pieces, if the large tensors start and end on 16-byte boundaries; else single elements
+        const Span g = span_of(p->dout, dtype_size(p->dout_dtype), (p->batch - 1) * p->dout_batch_stride + (p->dim - 1) * p->dout_dim_stride + p->seqlen);
+        const bool pieces = whole_pieces(s.u) && whole_pieces(s.delta) && whole_pieces(g);
+        return c.vw == 8   ? launch_n1_bwd<Tin, Tg, 8>(a, st)
+               : c.vw == 4 ? launch_n1_bwd<Tin, Tg, 4>(a, st)
+               : pieces    ? launch_n1_bwd<Tin, Tg, 0>(a, st)
+                           : launch_n1_bwd<Tin, Tg, 1>(a, st);
     }
     StBwdArgs a = {};
     a.u = p->u; a.delta = p->delta; a.B = p->B; a.C = p->C; a.dout = p->dout;
