@@ -55,15 +55,16 @@ template <typename T> long wrong() {                  // T: 16-bit or 32-bit val
                     for (int pos = -9; pos < L + 9; ++pos) {
                         const T* row = t + r * stride;
                         float x[8];
-                        if (pieces && pos % 2) {
-                            ss2d::Row8<T, 0> v;
-                            v.load(row, pos, 0, L);
-                            v.get(row, pos, 0, L, x);
-                        } else ss2d::row8_now<T, 0>(row, pos, L, s, x);
+                        const ss2d::Inner in = ss2d::inner_of(row, L, s);
+                        if (pieces) bad += in.from != 0 || in.to != L;
+                        ss2d::Row8<T, 0> v;
+                        v.load(row, pos, in.from, in.to);
+                        v.get(row, pos, in.from, in.to, x);
                         for (int e = 0; e < 8; ++e) {
-                            const uint32_t want = pos + e >= 0 && pos + e < L ? t[r * stride + pos + e] : 0;
+                            const uint32_t want = pos + e >= in.from && pos + e < in.to ? t[r * stride + pos + e] : 0;
                             float w = (float)want;
                             if (sizeof(T) == 4) memcpy(&w, &want, 4);
+                            if (in.from < in.to) bad += in.from > 7 || L - in.to > 7;       // what is left for single elements
                             bad += memcmp(&w, &x[e], 4) != 0;
                         }
                     }
