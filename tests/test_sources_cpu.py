@@ -1,0 +1,16 @@
+"""Rules of the kernel sources that no compiler checks."""
+import glob
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "vmamba_b200", "csrc")
+
+
+def test_dynamic_shared_memory_declares_its_alignment():
+    """Parts of it are read and written as 16-byte vectors: its start has to be aligned by declaration, not by chance."""
+    found = 0
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+        for line in re.findall(r"extern\s+__shared__[^;]*;", open(path).read()):
+            assert re.search(r"__align__\((16|32|64|128|1024)\)", line), (os.path.basename(path), line)
+            found += 1
+    assert found > 10

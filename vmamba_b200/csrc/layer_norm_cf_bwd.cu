@@ -26,7 +26,7 @@ struct NormBwdArgs {
 // PV: pixels per lane (neighbours, one access).  IT > 0: a warp's IT groups of channels stay in registers (D <= 32 * IT).
 template <typename Tg, int PV, int IT>
 __global__ void __launch_bounds__(kLnbWarps * 32, 3) layer_norm_cf_bwd_kernel(const NormBwdArgs a) {
-    extern __shared__ float lnb_sm[];                // [2][D] sums of dw, db
+    extern __shared__ __align__(16) float lnb_sm[];                // [2][D] sums of dw, db
     __shared__ float red[3][kLnbWarps][32 * PV];
     using VY = Vec<float, PV>;
     using VG = Vec<Tg, PV>;

@@ -51,7 +51,7 @@ struct LinearArgs {
 template <typename T, bool kBias>
 __global__ void __launch_bounds__(kThreads, 1)
 linear_cf_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const LinearArgs a) {
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* ring = sm + a.w_bytes;                      // W first: [K / 32][Mpad rows][64 B], 64-byte swizzle
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm + kSmemBudget);

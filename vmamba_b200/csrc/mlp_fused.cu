@@ -71,7 +71,7 @@ mlp_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
     constexpr int kTmemCols = 512;
     constexpr int kColH = 0, kColY = 2 * kHC;                  // TMEM columns: two H chunks, then two Y tiles of C columns
     static_assert(kColY + 2 * C <= kTmemCols, "TMEM holds two H chunks and two Y tiles");
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm + S::kBars);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + BAR_COUNT);

@@ -92,7 +92,7 @@ __device__ __forceinline__ void softplus_pair(float2 x, float2& sp, float2& dsp)
 // LPR: lanes per row.  Rows of at most 128 (64) elements share a warp, two (four) at a time.
 template <typename Tin, typename Tg, int AL, int LPR>
 __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArgs a) {
-    extern __shared__ float n1_sm[];
+    extern __shared__ __align__(16) float n1_sm[];
     constexpr int G = 32 / LPR, kChunk = LPR * 8, kStep = kN1Warps * G;     // kStep: rows of the CTA that are worked on at a time
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, R = a.R, L = a.L, ln = lane & (LPR - 1), wr = warp * G + lane / LPR;
     float* red = n1_sm;                                          // [2][warp][2][256]

@@ -46,7 +46,7 @@ struct BwdArgs {
 
 template <typename Tin, typename Tg, int VEC>
 __global__ void __launch_bounds__(256) selscan_bwd_kernel(const BwdArgs a) {
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     constexpr int STEP = 32 * VEC;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, RW = blockDim.x >> 5;
     const int N = a.N, L = (int)a.seqlen, nsteps = a.nsteps;
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(256) selscan_bwd_kernel(const BwdArgs a) {
 // row's u / delta / dout vectors are fetched before the current row's arithmetic.
 template <typename Tin, typename Tg, int VEC>
 __global__ void __launch_bounds__(256) selscan_bwd_n1_kernel(const BwdArgs a, const int R) {
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     constexpr int STEP = 32 * VEC;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, RW = blockDim.x >> 5;
     const int L = (int)a.seqlen, nsteps = a.nsteps;
@@ -452,7 +452,7 @@ constexpr int kBwdFloatsPerWarp = 4 * kBwdTile * kBwdPitch + 8 * 32 + 2 * kBwdTi
 
 template <typename Tin, typename Tg>
 __global__ void __launch_bounds__(kBwdRowsWarps * 32, 4) selscan_bwd_rows_kernel(const BwdArgs a) {
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     constexpr int T = kBwdTile, P = kBwdPitch, PE = 4;         // PE: elements per piece (8 bytes of a 16-bit tensor)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* su = sm + (size_t)warp * kBwdFloatsPerWarp;         // u, then du
@@ -625,7 +625,7 @@ template <int NS> struct BwdRowsN {
 
 template <typename Tin, typename Tg, int NS>
 __global__ void __launch_bounds__(kBwdRowsWarps * 32, 2) selscan_bwd_rows_nx_kernel(const BwdArgs a) {
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     constexpr int T = kBwdTile, P = kBwdPitch, PE = 4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* su = sm + (size_t)warp * BwdRowsN<NS>::kFloatsPerWarp;   // u, then du

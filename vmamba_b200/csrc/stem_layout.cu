@@ -374,7 +374,7 @@ struct RowsArgs {
 
 template <typename Tin, typename Tout, int TP>
 __global__ void __launch_bounds__(256) pixels_norm_to_planes_kernel(const RowsArgs a) {
-    extern __shared__ float tile[];                       // [TP][C + 1], then part[256 / TP][TP], scale[TP], shift[TP]
+    extern __shared__ __align__(16) float tile[];                       // [TP][C + 1], then part[256 / TP][TP], scale[TP], shift[TP]
     const long long n0 = (long long)blockIdx.x * TP;
     const int C = a.C, P = C + 1;
     float* part = tile + TP * P;
@@ -499,7 +499,7 @@ struct PlanesArgs {
 
 template <typename T, int TP>
 __global__ void __launch_bounds__(256) planes_to_pixels_kernel(const PlanesArgs a) {
-    extern __shared__ float tile[];                       // [TP][C + 1]
+    extern __shared__ __align__(16) float tile[];                       // [TP][C + 1]
     const long long n0 = (long long)blockIdx.x * TP;
     const int C = a.C, P = C + 1;
     if (a.quads) {
