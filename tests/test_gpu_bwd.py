@@ -303,3 +303,39 @@ def test_backward_with_and_without_forward_checkpoints(vb, N, L):
             want[:, :, i // 128] = h
         h = np.exp(dl[:, :, i, None] * A[None]) * h + (dl[:, :, i] * u[:, :, i])[:, :, None] * Bx[..., i]
     assert O.max_rel_err(host(ck), want) <= 1e-4
+
+
+# (images, groups, channels, states, length, type, states of the forward call): a kernel of selective_scan_bwd.cu each
+@pytest.mark.parametrize("Bt,K,Cd,N,L,dt,ckpt", [
+    (27, 4, 320, 1, 200, "bf16", True), (27, 4, 320, 1, 36, "f32", True),             # 34 560 rows of one state: lanes are rows
+    (2, 4, 9, 1, 197, "f32", False), (1, 2, 7, 1, 784, "bf16", True),                 # few rows of one state
+    (2, 4, 608, 16, 20, "f32", True), (2, 4, 608, 8, 140, "bf16", True), (2, 4, 608, 4, 132, "f16", True),      # 4 864 rows: lanes are rows
+    (2, 2, 5, 16, 130, "f32", True), (1, 2, 3, 3, 140, "bf16", False)])               # a warp per row
+def test_scan_gradients_of_the_c_interface_by_default(vb, Bt, K, Cd, N, L, dt, ckpt):
+    """checkpoint_every = 0: states every 128 elements, or none, and the kernels that go with them."""
+    from vmamba_b200 import _lib
+    u, delta, A, B, C, D, bias, dout = _random_case(Bt, K, Cd, N, L, seed=L + N)
+    if dt != "f32":
+        u, delta, B, C = (O._round_to(a, dt) for a in (u, delta, B, C))
+    td, code = TD[dt], {"f32": _lib.SS2D_F32, "bf16": _lib.SS2D_BF16, "f16": _lib.SS2D_F16}[dt]
+    ts = dict(u=dev(u, td), delta=dev(delta, td), A=dev(A), B=dev(B, td), C=dev(C, td), D=dev(D), delta_bias=dev(bias))
+    out = dict(du=torch.empty_like(ts["u"]), ddelta=torch.empty_like(ts["u"]), dA=torch.empty_like(ts["A"]), dB=torch.empty_like(ts["B"]),
+               dC=torch.empty_like(ts["C"]), dD=torch.empty_like(ts["D"]), ddelta_bias=torch.empty_like(ts["D"]))
+    g = dev(dout)
+    p = _lib.ScanBwdParams(dout=g.data_ptr(), in_dtype=code, dout_dtype=_lib.SS2D_F32, delta_softplus=1, batch=Bt, dim=K * Cd, dstate=N, seqlen=L,
+                           n_groups=K, **{k: t.data_ptr() for k, t in {**ts, **out}.items()})
+    for name in ("u", "delta", "dout"):
+        setattr(p, name + "_batch_stride", K * Cd * L)
+        setattr(p, name + "_dim_stride", L)
+    for name in ("B", "C"):
+        setattr(p, name + "_batch_stride", K * N * L)
+        setattr(p, name + "_group_stride", N * L)
+        setattr(p, name + "_state_stride", L)
+    if ckpt:
+        states = vb.selective_scan_fwd(*ts.values(), True, True, return_checkpoints=True)[1]
+        p.checkpoints = states.data_ptr()
+    ws = torch.empty(_lib.lib().ss2d_selective_scan_bwd_workspace_bytes(p), device="cuda", dtype=torch.uint8)
+    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
+    assert _lib.lib().ss2d_selective_scan_bwd(p, torch.cuda.current_stream().cuda_stream) == _lib.SS2D_OK
+    for (name, x), r in zip(out.items(), O.selective_scan_bwd(u, delta, A, B, C, D, bias, dout, True, dt)):
+        assert O.max_rel_err(host(x), r) <= TOL[dt], name
