@@ -191,17 +191,6 @@ __device__ __forceinline__ void unpack_pairs(const typename SegVec<T, VEC>::type
     for (int j = 0; j < VEC / 2; ++j) v[j] = make_float2(f[2 * j], f[2 * j + 1]);
     if constexpr (VEC & 1) v[VEC / 2] = make_float2(f[VEC - 1], 0.f);
 }
-template <int VEC>
-__device__ __forceinline__ void load_pairs(const float* p, float2 (&v)[(VEC + 1) / 2]) {
-    float f[VEC];
-    Vec<float, VEC>::load(p, f);
-    if constexpr (VEC == 1) v[0] = make_float2(f[0], 0.f);
-    else {
-#pragma unroll
-        for (int j = 0; j < VEC / 2; ++j) v[j] = make_float2(f[2 * j], f[2 * j + 1]);
-    }
-}
-
 // Shared-memory words of a VEC-segment of a plane walked with one index fastest ("minor", line
 // length n_minor).  The host picks VEC so that VEC/2 divides n_minor: a segment then either lies
 // in one line or wraps exactly at its middle, so the first half is affine from `lo` and the second

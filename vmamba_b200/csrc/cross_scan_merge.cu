@@ -204,18 +204,6 @@ __device__ __forceinline__ int mdiv_u(int n, unsigned magic) { return magic ? (i
 struct RouteMapI { int base, sh, sw, col_like; };
 __device__ __forceinline__ RouteMapI narrow(const RouteMap& m) { return RouteMapI{(int)m.base, (int)m.sh, (int)m.sw, (int)m.col_like}; }
 
-// source position (flat h*W + w) read by step l of a route
-__device__ __forceinline__ int route_src(const RouteMapI& m, int l, int H, int W, unsigned magic_H) {
-    if (!m.col_like) return m.sw > 0 ? l : (int)m.base - l;            // row-major, forward or reversed
-    // l = base + sh*h + sw*w with |sh| = 1, |sw| = H: recover (h, w)
-    const int t = (int)(m.sw > 0 ? 0 : -m.sw * (W - 1));                // offset so that the w term is non-negative
-    int r = l - (int)m.base + t + (m.sh < 0 ? (H - 1) : 0);            // = hh + H * ww with hh, ww in range
-    const int ww = mdiv_u(r, magic_H), hh = r - ww * H;
-    const int h = m.sh > 0 ? hh : H - 1 - hh;
-    const int w = m.sw > 0 ? ww : W - 1 - ww;
-    return h * W + w;
-}
-
 // Shared-memory planes have an odd line pitch (W | 1 for a row-major plane, H | 1 for a column-major one): the gathers of
 // the permutation then walk down a line with consecutive lanes in different banks.  With the natural pitch (56 for a
 // 56 x 56 map) 32 lanes fell into 4 banks and the kernels ran at a third of the copy bandwidth.

@@ -1,4 +1,4 @@
-// Shared parts of the selective-scan kernels for 2 .. 16 states (scan_states_fwd.cu, scan_states_bwd.cu).
+// Shared parts of the selective-scan kernels for 2 .. 16 states (scan_states_fwd.cuh, scan_states_bwd.cuh).
 //
 // Mapping.  The NS = 4, 8 or 16 states of a row (a smaller state count is padded with states whose A, B and C are zero)
 // are split over SL = NS / 4 neighbouring lanes, four states per lane, so that a warp holds 32 / SL rows and the chip is
@@ -37,21 +37,6 @@ template <int NS, int R_ = 1> struct StLayout {
 
 __device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
 
-// Eight consecutive elements of a row from element t, in vectors of VW (8 or 4); elements beyond L read as zero.
-template <typename T, int VW>
-__device__ __forceinline__ void st_load8(const T* row, int t, int L, bool ok, float (&v)[8]) {
-#pragma unroll
-    for (int h = 0; h < 8; h += VW) {
-        float x[VW];
-        if (ok && t + h < L) Vec<T, VW>::load(row + t + h, x);
-        else {
-#pragma unroll
-            for (int e = 0; e < VW; ++e) x[e] = 0.f;
-        }
-#pragma unroll
-        for (int e = 0; e < VW; ++e) v[h + e] = x[e];
-    }
-}
 __device__ __forceinline__ void st_put8(float* dst, const float (&v)[8]) {
     float4* q = reinterpret_cast<float4*>(dst);
     q[0] = make_float4(v[0], v[1], v[2], v[3]);
