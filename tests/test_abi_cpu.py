@@ -298,3 +298,25 @@ def test_accelerate_refuses_modules_that_are_not_on_a_gpu():
     import vmamba_b200 as vb
     with pytest.raises(RuntimeError, match="CUDA"):
         vb.accelerate(torch.nn.Linear(4, 4))
+
+
+def test_gradient_planner_deals_rows_while_two_ctas_per_sm_are_left():
+    """One state: the workspace holds a dB / dC partial per CTA, four warps of R rows; R doubles as long as 296 CTAs are left."""
+    L = _lib.lib()
+
+    def parts(batch, group, seqlen):
+        p = _lib.ScanBwdParams(**{k: 0x10000 for k in ("u", "delta", "A", "B", "C", "dout", "du", "ddelta", "dA", "dB", "dC", "checkpoints")})
+        dim, p.checkpoint_every = 4 * group, L.ss2d_selective_scan_checkpoint_every(1, 1)
+        p.in_dtype, p.dout_dtype, p.delta_softplus = 2, 0, 1
+        p.batch, p.dim, p.dstate, p.seqlen, p.n_groups = batch, dim, 1, seqlen, 4
+        p.u_batch_stride = p.delta_batch_stride = p.dout_batch_stride = dim * seqlen
+        p.u_dim_stride = p.delta_dim_stride = p.dout_dim_stride = seqlen
+        p.B_batch_stride = p.C_batch_stride = 4 * seqlen
+        p.B_group_stride = p.C_group_stride = p.B_state_stride = p.C_state_stride = seqlen
+        floats = L.ss2d_selective_scan_bwd_workspace_bytes(p) // 4 - batch * dim * 3
+        return floats / (batch * 4 * 2 * ((seqlen + 31) // 32 * 32))
+
+    assert parts(32, 96, 3136) == 3                                # 384 CTAs of 8 rows per warp
+    assert parts(8, 96, 3136) == 12                                # 384 of 2; 4 would leave 192
+    assert parts(16, 192, 784) == 6                                # 384 of 8
+    assert parts(4, 96, 3136) == 24                                # 384 of 1

@@ -58,11 +58,14 @@ static int plan_grad(const ss2d_scan_bwd_params* p, GradPlan& c) {
     const int64_t groups = p->batch * p->n_groups;
     if (N == 1) {
         c.NS = 1;
-        // rows per warp: as many as leave four CTAs per SM (the sums over rows of a chunk are then formed once for all of them)
+        // rows per warp: as many as leave two CTAs per SM (the sums over rows of a chunk are then formed once for all of them; three
+        // CTAs are resident, 153 to 168 registers).  us with one, two, three, four and six left, bf16: 32 x 384 rows of 3 136 elements
+        // 170, 167, 177, 181, 199; 8 x 384 of 3 136 81, 61, 75, 75, 75; 8 x 768 of 784 50, 38, 45, 53, 54; 16 x 768 of 784 63, 63,
+        // 65, 65, 73; 4 x 384 of 3 136 54, 44, 44, 44, 44
         const int64_t step = kN1Warps * (32 / n1_lanes(L));
         auto parts_of = [&](int64_t R) { return (gs + step * R - 1) / (step * R); };
         c.sets = 1;
-        while (c.sets < kN1MaxR && step * c.sets < gs && groups * parts_of(c.sets * 2) >= 148 * 4) c.sets *= 2;
+        while (c.sets < kN1MaxR && step * c.sets < gs && groups * parts_of(c.sets * 2) >= 148 * 2) c.sets *= 2;
         c.parts = (int)parts_of(c.sets);
         const int64_t ctas = groups * c.parts;
         c.S = 1; c.seg_len = (int)((L + kN1Chunk - 1) / kN1Chunk * kN1Chunk);
