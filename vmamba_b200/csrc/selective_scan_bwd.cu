@@ -946,11 +946,11 @@ static int plan_bwd(const ss2d_scan_bwd_params* p, BwdPlan& c) {
     // (measured crossover against the warp-per-row kernel, bf16 with checkpoints: 24 576 rows 0.96 against 0.74 ms at
     // L = 3136, 36 864 rows 0.99 against 1.11 ms; 49 152 rows of 196 elements 0.095 against 0.158 ms)
     c.rows = p->dstate == 1 && p->checkpoints != nullptr && gs % 32 == 0 && p->delta_ratio <= 1 && c.vec >= 4 &&
-             p->batch * p->dim >= 32LL * 148 * 7 && rows_kernels_enabled();
+             p->batch * p->dim >= 32LL * 148 * 7;
     // the same form for d_state 4 / 8 / 16.  Measured (d_state 16, bf16): 15-20 ms against 35-47 ms of the warp-per-row kernel
     // on 2 GB of rows; 57 against 115 ms on 6 528 rows of 65 536 elements, where 1.4 warps per SM walk at their own latency
     const bool rows_nx = (p->dstate == 4 || p->dstate == 8 || p->dstate == 16) && p->checkpoints != nullptr && gs % 32 == 0 &&
-                         p->delta_ratio <= 1 && c.vec >= 4 && p->batch * p->dim >= 32LL * 148 && rows_kernels_enabled();
+                         p->delta_ratio <= 1 && c.vec >= 4 && p->batch * p->dim >= 32LL * 148;
     if (c.rows) {
         c.parts = (int)(gs / 32);
         c.smem = (size_t)kBwdRowsWarps * kBwdFloatsPerWarp * sizeof(float);
