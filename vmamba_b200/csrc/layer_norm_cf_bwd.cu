@@ -3,10 +3,10 @@
 //   xhat = (y - mean) rstd,  dy = rstd (g w - mean_D(g w) - xhat mean_D(g w xhat)),  dw = sum g xhat,  db = sum g
 //
 // A CTA of eight warps takes tiles of 32 pixels (or pixel pairs) of one image: a lane is a pixel, a warp every eighth group of four channels.
-// Three passes over the tile (mean; squares and the two sums of g w; results), of which the first reads memory and the
-// others the caches.  dw / db: the eight values of a warp's four channels are summed over its pixels by halving exchanges
+// Three passes over the tile (mean; squares and the two sums of g w; results).  Up to 96 channels they work on registers; wider
+// maps read the tile again from the caches.  dw / db: the eight values of a warp's four channels are summed over its pixels by halving exchanges
 // (nine shuffles) and kept per CTA in shared memory over all its tiles; a second kernel folds the CTAs in a fixed order.
-// Bound: HBM, 6 + 4 bytes per value in 16 bits (32 x 96 x 3 136: 21 us, 0.7 of the copy bandwidth; a pixel per lane, the tile
+// Bound of the register form: HBM, 6 + 4 bytes per value in 16 bits (32 x 96 x 3 136: 21 us, 0.7 of the copy bandwidth; a pixel per lane, the tile
 // read three times and 64-bit addresses for each value took 91 us).
 #include "common.cuh"
 
@@ -164,6 +164,9 @@ __global__ void __launch_bounds__(kLnbWarps * 32, 3) layer_norm_cf_bwd_kernel(co
     for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) a.part[(long long)blockIdx.x * 2 * D + i] = lnb_sm[i];
 }
 
+// The tile in registers up to 96 channels, three groups of four per warp: 32 x 96 x 3 136, both launches on cold caches, 38 us against 54
+// with three reads.  Six groups spill (80 registers, 1 KB of stack): 32 x 128 x 3 136 124 us against 69 (1.9 TB/s) with three
+// reads, 32 x 192 x 3 136 140 against 93 (2.1 TB/s); 16 x 384 x 3 136 runs at 1.9, 32 x 768 x 196 at 0.8 TB/s.
 template <typename Tg>
 static void launch_lnb(const NormBwdArgs& a, int pv, unsigned ctas, cudaStream_t st) {
     const size_t smem = (size_t)2 * a.D * sizeof(float);

@@ -10,7 +10,9 @@
 // Segments: where the rows do not fill the chip they are cut into S segments; a first kernel leaves each segment's
 // effect on e (its value from zero, and the sum of its step sizes), and a segment starts from the fold of those behind it.
 //
-// Bound: instruction issue (about 45 per element, four of them on the MUFU pipe).
+// Bound: latency at three CTAs of four warps per SM (153 to 168 registers).  32 x 384 rows of 3 136 elements, bf16, 150 us: an SM issues
+// in half of its cycles with 2.5 warps per scheduler, 0.7 of them eligible; the arithmetic alone (about 45 instructions per
+// element, four on the MUFU pipe) is 47 us, the bytes 74 us at the copy rate (38 % of the DRAM rate).
 #pragma once
 #include <type_traits>
 

@@ -11,7 +11,9 @@
 //
 // Rows too few for the chip are cut into segments: st_bwd_segments_kernel leaves what a segment does to the reverse state.
 //
-// Bound: instruction issue, about 11 per (element, state), and 1.75 exponentials per (element, state).
+// Bound: latency at eight warps per SM (254 registers).  4 x 1 536 rows of 1 001 elements, 16 states, fp32, 196 us: an SM issues in 47 %
+// of its cycles with 1.8 warps per scheduler, 0.6 of them eligible, its shared memory at 52 %, DRAM at 8 %.  The
+// instructions (about 11 per element and state) are 29 us at full rate, the exponentials (1.75) 37 us.
 #pragma once
 #include "scan_n1_bwd.cuh"
 #include "scan_states_fwd.cuh"

@@ -1,12 +1,9 @@
-// Selective-scan forward, the operator-surface kernel (one tensor in, one tensor out per row).
+// Selective-scan forward, the operator surface: planner, launches, and the kernels for one state and for many.
 //
-// Mapping: one warp owns one row (b, r) of length L.  Per step a lane takes VEC consecutive
-// elements (one 16-byte load per tensor when alignment allows), runs the recurrence over them
-// in registers, the 32 lane aggregates are combined with a shuffle scan of the associative pair
-// (a, b) o (a', b') = (a a', a' b + b'), and the carry into the next 32*VEC-element step stays in
-// a register (d_state 1) or in shared memory (d_state > 1).  The next step's vectors are
-// fetched before the current step's arithmetic.  Traffic per row: u and delta read once, out
-// written once; B/C rows are shared by all channels of a group and come from L2.
+// One state (every VMamba backbone): selscan_fwd_n1_kernel.  2 .. 16 states: scan_states_fwd.cuh.  More than 16 states, and more than
+// one where channels share a row of step sizes: selscan_fwd_nx_kernel, a warp per row, the carry of every state in shared memory.
+// In all of them u and delta are read once and the result is written once; the B / C rows, shared by the channels of a
+// group, come from the caches.
 #include "scan_row.cuh"
 #include "scan_states_fwd.cuh"
 
@@ -32,8 +29,10 @@ constexpr int kWarpsPerCta = 4;
 
 // d_state 1: W warps per row (1: four rows per CTA; 2 .. 8: the CTA is one row).  Per step a warp takes 256 elements, eight
 // per lane, and scans its lanes' (a, b) pairs by shuffle; with several warps per row their totals meet in shared memory
-// (one barrier per step) and every warp folds the ones in front of it.  One warp per row is the faster form where the rows
-// fill the chip; fewer rows get the more warps (up to 24 per SM).
+// (one barrier per step) and every warp folds the ones in front of it.  How many: n1_warps.  The next step's vectors are
+// fetched in front of this one's arithmetic.
+// Bound, 1 024 rows of 16 385 elements (four warps each, 51 us, 20 % of the DRAM rate): instruction issue, 72 % of the slots of an SM
+// that has work, and 1 024 CTAs on the 740 places that 91 registers leave, so that the second wave is a third full.
 // AL is the vector width of every access (8 or 4 elements), or 0 for rows of any alignment: a row is then walked from
 // the 16-byte boundary in front of its result, so that the results leave as vectors, and the inputs are cut out of the
 // aligned pieces around them.  Elements of the tensors' first and last rows whose pieces would reach beyond a tensor (at most
@@ -242,8 +241,18 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) selscan_fwd_nx_kernel(const
     }
 }
 
-// d_state 1: warps per row.  Rows that fill the chip (24 warps on each of 148 SMs) get one; fewer rows more, as long as a
-// step of all of them is not longer than the row.
+// d_state 1: warps per row.  One where the rows alone are 24 warps for each of 148 SMs; fewer rows get more, as long as a step of
+// all warps but half is shorter than the row.  The rule counts warps, not the CTAs that are resident at once (aligned rows: 4, 8
+// and 16 CTAs per SM of eight, four and two warps; unaligned ones 2, 5 and 10), because long rows gain from more warps in a
+// second wave too.  us with 1 / 2 / 4 / 8 warps, bf16, the rule's in brackets:
+//   rows    L = 3 136 (aligned)        L = 3 137                  L = 16 385
+//   256     16.4  12.3  11.0 [10.2]    19.2  14.4  12.4 [12.3]    61.4  37.9  25.6 [22.5]
+//   740     16.4  14.4  12.3 [14.3]    20.5  18.4  17.3 [20.5]    69.6  47.1  38.9 [48.1]
+//   1 024   17.5  14.4 [14.4] 16.4     21.4  20.5 [22.6] 24.6     70.8  55.3 [53.3] 62.5
+//   2 048   20.5 [18.5] 20.5  23.5     26.7 [28.7] 32.8  43.0
+//   3 584  [26.6] 27.5  30.7  34.8    [43.0] 43.0  51.2  69.7
+// It is within 3 % of the best but where CTAs of eight warps do not fit at once (444 to 740 rows, up to 24 %) and at its steps
+// (1 536 and 3 072 rows, up to 13 %).
 static int n1_warps(int64_t rows, int64_t L) {
     int w = 1;
     while (w < 8 && rows * w < 148 * 24 && (int64_t)w * 256 < L) w *= 2;

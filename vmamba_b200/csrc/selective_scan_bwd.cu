@@ -9,15 +9,20 @@
 //     dd'_l = sum_n dh_l (B_l u_l + A a_l h_{l-1})  dA_n  = sum_{b,l} dh_l d'_l a_l h_{l-1}
 //     ddelta_l = dd'_l * sigmoid(delta_l + bias) (1 above softplus' threshold 20),  dbias = sum_{b,l} ddelta_l
 //
-// Mapping: as in the forward kernel one warp owns one row (b, r) and walks it in steps of 32*VEC
-// elements, a lane holding VEC consecutive elements.  The warps of a CTA own rows of the SAME
-// (image, group), so that their contributions to dB / dC (which are shared by the channels of a
-// group) are summed inside the CTA, in a fixed order, through shared memory.
-//   pass 1 (forward over the row): the state entering every step is recomputed and kept in shared
-//           memory (nothing is saved by the forward kernel);
-//   pass 2 (backward over the steps): within a step the states h come from a forward shuffle scan
-//           started at the saved state, e from a backward shuffle scan started at the carry of the
-//           step after; every gradient of the step follows elementwise.
+// Calls with 1 .. 16 states that give the spacing of their states (every call of the package) go to scan_n1_bwd.cuh and
+// scan_states_bwd.cuh (planner: selective_scan_grad.cu); this file keeps the entry point, the fold, and
+//   selscan_bwd_kernel           more than 16 states, or more than one where channels share a row of step sizes
+//   selscan_bwd_n1_kernel        checkpoint_every = 0 (the C interface's default), one state, few rows
+//   selscan_bwd_rows_kernel      the same, one state and many rows; selscan_bwd_rows_nx_kernel: 4, 8 or 16 states and many rows
+//
+// selscan_bwd_kernel: one warp owns one row (b, r) and walks it in steps of 32 * VEC elements, a lane holding VEC consecutive
+// ones.  The warps of a CTA own rows of the SAME (image, group), so that their contributions to dB / dC (which are shared
+// by the channels of a group) are summed inside the CTA, in a fixed order, through shared memory.
+//   pass 1 (forward over the row): the state entering every step is recomputed and kept in shared memory, or taken from the
+//           forward call's states where the steps line up;
+//   pass 2 (backward over the steps): within a step the states h come from a forward shuffle scan started at the saved state,
+//           e from a backward shuffle scan started at the carry of the step after; every gradient of the step follows
+//           elementwise.
 // Sums that cross CTAs (dB / dC over the CTAs of a group, dA / dD / dbias over the batch) go to an
 // fp32 workspace as partials and are folded by a second kernel in a fixed order: no atomics, the
 // result is bit-identical from run to run.
