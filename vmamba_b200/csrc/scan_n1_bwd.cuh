@@ -14,8 +14,6 @@
 // in half of its cycles with 2.5 warps per scheduler, 0.7 of them eligible; the arithmetic alone (about 45 instructions per
 // element, four on the MUFU pipe) is 47 us, the bytes 74 us at the copy rate (38 % of the DRAM rate).
 #pragma once
-#include <type_traits>
-
 #include "scan_row.cuh"
 
 namespace ss2d {
@@ -33,9 +31,6 @@ struct N1BwdArgs {
     int64_t dim, group_size, batch, dratio;
     int64_t u_bs, u_ds, d_bs, d_ds, g_bs, g_ds, B_bs, B_gs, C_bs, C_gs;
     int L, Lp, n_groups, parts, R, S, seg_len, softplus;
-    // AL = 0: B and C start and end on 16-byte boundaries; else their elements are loaded one by one (32 x 384 rows of 3 137
-    // elements, bf16: the choice costs 257 -> 265 us of the gradients, always one by one 277)
-    int bc_pieces;
 };
 
 template <typename T, int AL>
@@ -92,7 +87,9 @@ __device__ __forceinline__ void softplus_pair(float2 x, float2& sp, float2& dsp)
 }
 
 // LPR: lanes per row.  Rows of at most 128 (64) elements share a warp, two (four) at a time.
-template <typename Tin, typename Tg, int AL, int LPR>
+// BC: vectors of B and C; AL, or 1 with AL 0 where they do not start and end on 16-byte boundaries.  (32 x 384 rows of 3 137 elements,
+// bf16, all gradients: 245 us with pieces; single elements cost 9 %, the choice inside one kernel 4 %.)
+template <typename Tin, typename Tg, int AL, int LPR, int BC>
 __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArgs a) {
     extern __shared__ __align__(16) float n1_sm[];
     constexpr int G = 32 / LPR, kChunk = LPR * 8, kStep = kN1Warps * G;     // kStep: rows of the CTA that are worked on at a time
@@ -149,13 +146,11 @@ __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArg
         const int pos = c * kChunk + ln * 8;
         float2 bv[4], cv[4], accB[4], accC[4];
         if (mine) fetch(0, pos);
-        auto load_bc = [&](auto al) {
-            Row8<Tin, decltype(al)::value> rb, rc;
+        {
+            Row8<Tin, BC> rb, rc;
             rb.load(Bm, pos, 0, L); rc.load(Cm, pos, 0, L);
             row8_pairs(rb, Bm, pos, L, bv); row8_pairs(rc, Cm, pos, L, cv);
-        };
-        if (AL == 0 && !a.bc_pieces) load_bc(std::integral_constant<int, 1>{});
-        else load_bc(std::integral_constant<int, AL>{});
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i) accB[i] = accC[i] = pk(0.f);
 #pragma unroll 1
@@ -284,7 +279,7 @@ __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArg
 }
 
 // What a segment does to e: a warp per (row, segment), chunks of 256 elements from the segment's end.
-template <typename Tin, typename Tg, int AL>
+template <typename Tin, typename Tg, int AL, int BC>
 __global__ void __launch_bounds__(kN1Warps * 32) n1_bwd_segments_kernel(const N1BwdArgs a) {
     const int lane = threadIdx.x & 31, L = a.L;
     const int64_t w = (int64_t)blockIdx.x * kN1Warps + (threadIdx.x >> 5);
@@ -303,16 +298,10 @@ __global__ void __launch_bounds__(kN1Warps * 32) n1_bwd_segments_kernel(const N1
         float2 d[4], g[4], cv[4];
         {
             Row8<Tin, AL> xd;
+            Row8<Tin, BC> xc;
             Row8<Tg, AL> xg;
-            xd.load(dt, pos, 0, L); xg.load(gp, pos, 0, L);
-            auto load_c = [&](auto al) {
-                Row8<Tin, decltype(al)::value> xc;
-                xc.load(Cm, pos, 0, L);
-                row8_pairs(xc, Cm, pos, L, cv);
-            };
-            if (AL == 0 && !a.bc_pieces) load_c(std::integral_constant<int, 1>{});
-            else load_c(std::integral_constant<int, AL>{});
-            row8_pairs(xd, dt, pos, L, d); row8_pairs(xg, gp, pos, L, g);
+            xd.load(dt, pos, 0, L); xg.load(gp, pos, 0, L); xc.load(Cm, pos, 0, L);
+            row8_pairs(xd, dt, pos, L, d); row8_pairs(xg, gp, pos, L, g); row8_pairs(xc, Cm, pos, L, cv);
         }
         float le = 0.f, ls = 0.f;
 #pragma unroll

@@ -112,16 +112,16 @@ long long selective_scan_grad_workspace_bytes(const ss2d_scan_bwd_params* p) {
     return plan_grad(p, c) == SS2D_OK ? (long long)c.total * 4 : -1;
 }
 
-template <typename Tin, typename Tg, int AL>
+template <typename Tin, typename Tg, int AL, int BC>
 static int launch_n1_bwd(const N1BwdArgs& a, cudaStream_t st) {
     const size_t smem = sizeof(float) * (2 * kN1Warps * 2 * kN1Chunk + (size_t)kN1Warps * a.R * (4 * (32 / n1_lanes(a.L)) + 96) + (AL ? 0 : kN1Warps * 264));
     const int lpr = n1_lanes(a.L);
-    auto kern = lpr == 8 ? n1_bwd_kernel<Tin, Tg, AL, 8> : lpr == 16 ? n1_bwd_kernel<Tin, Tg, AL, 16> : n1_bwd_kernel<Tin, Tg, AL, 32>;
+    auto kern = lpr == 8 ? n1_bwd_kernel<Tin, Tg, AL, 8, BC> : lpr == 16 ? n1_bwd_kernel<Tin, Tg, AL, 16, BC> : n1_bwd_kernel<Tin, Tg, AL, 32, BC>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
     const int64_t ctas = a.batch * a.n_groups * a.parts * a.S, seg_ctas = (a.batch * a.dim * (a.S - 1) + kN1Warps - 1) / kN1Warps;
     if (ctas > 0x7fffffffLL || seg_ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
     if (a.S > 1) {
-        n1_bwd_segments_kernel<Tin, Tg, AL><<<(unsigned)seg_ctas, kN1Warps * 32, 0, st>>>(a);
+        n1_bwd_segments_kernel<Tin, Tg, AL, BC><<<(unsigned)seg_ctas, kN1Warps * 32, 0, st>>>(a);
         count_launch();
     }
     kern<<<(unsigned)ctas, kN1Warps * 32, smem, st>>>(a);
@@ -163,14 +163,14 @@ static int dispatch_grad(const ss2d_scan_bwd_params* p, const GradPlan& c, float
         const ScanSpans s = scan_spans(*p, dtype_size(p->in_dtype));
         a.L = (int)p->seqlen; a.Lp = c.Lp; a.n_groups = (int)p->n_groups; a.parts = c.parts; a.R = c.sets; a.S = c.S; a.seg_len = c.seg_len;
         a.softplus = p->delta_softplus;
-        a.bc_pieces = whole_pieces(s.B) && whole_pieces(s.C);
-        // rows without vectors: pieces, if the large tensors start and end on 16-byte boundaries; else single elements
+        // rows without vectors: pieces of the tensors that start and end on 16-byte boundaries; else single elements
         const Span g = span_of(p->dout, dtype_size(p->dout_dtype), (p->batch - 1) * p->dout_batch_stride + (p->dim - 1) * p->dout_dim_stride + p->seqlen);
         const bool pieces = whole_pieces(s.u) && whole_pieces(s.delta) && whole_pieces(g);
-        return c.vw == 8   ? launch_n1_bwd<Tin, Tg, 8>(a, st)
-               : c.vw == 4 ? launch_n1_bwd<Tin, Tg, 4>(a, st)
-               : pieces    ? launch_n1_bwd<Tin, Tg, 0>(a, st)
-                           : launch_n1_bwd<Tin, Tg, 1>(a, st);
+        return c.vw == 8                                        ? launch_n1_bwd<Tin, Tg, 8, 8>(a, st)
+               : c.vw == 4                                      ? launch_n1_bwd<Tin, Tg, 4, 4>(a, st)
+               : !pieces                                        ? launch_n1_bwd<Tin, Tg, 1, 1>(a, st)
+               : whole_pieces(s.B) && whole_pieces(s.C)         ? launch_n1_bwd<Tin, Tg, 0, 0>(a, st)
+                                                                : launch_n1_bwd<Tin, Tg, 0, 1>(a, st);
     }
     StBwdArgs a = {};
     a.u = p->u; a.delta = p->delta; a.B = p->B; a.C = p->C; a.dout = p->dout;
