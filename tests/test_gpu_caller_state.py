@@ -154,3 +154,26 @@ def test_what_a_training_step_keeps(vb, step, kept):
     again = torch.autograd.grad(torch.utils.checkpoint.checkpoint(fn, *leaves, use_reentrant=False), leaves, gy)
     for a, b, c in zip(grads, from_host, again):
         assert torch.equal(a, b) and torch.equal(a, c)
+
+
+def test_core_refuses_what_does_not_fit(vb):
+    """Types and sizes that a library product or layer_norm refused are still refused where kernels take their place."""
+    from vmamba_b200 import fused
+    D, R = 32, 2
+    par = [torch.randn(4 * (R + 2), D), torch.randn(4 * D, R), torch.zeros(4, D), torch.zeros(4 * D, 1), torch.ones(4 * D), torch.ones(D), torch.zeros(D)]
+    par = [t.cuda() for t in par]
+    w = vb.CoreWeights.build(*par, d_state=1, dt_rank=R, dtype=torch.bfloat16)
+    for shape, cm in (((2, D, 8, 8), False), ((2, D, 7, 7), False), ((D, 2, 8, 8), True)):
+        for other in (torch.float16, torch.float32):
+            with pytest.raises(RuntimeError):
+                vb.ss2d_core(torch.randn(shape, device="cuda", dtype=other), w, channel_major=cm)
+            with pytest.raises(RuntimeError):
+                fused.project(torch.randn(shape, device="cuda", dtype=other), w, cm)
+    with pytest.raises(RuntimeError):
+        fused.project(torch.randn(2, D + 8, 8, 8, device="cuda", dtype=torch.bfloat16), w)
+    x = torch.randn(2, D, 8, 8, device="cuda")
+    for i in (5, 6):                                     # the LayerNorm's weight and bias
+        wrong = list(par)
+        wrong[i] = wrong[i][:D // 2]
+        with pytest.raises(RuntimeError):
+            vb.ss2d_core_autograd(x, *wrong, d_state=1, dt_rank=R)

@@ -76,3 +76,10 @@ def test_core_weight_changes_count(model):
     before = w.native
     w.eps = 1e-3
     assert w.native is not before and w.native is w.native
+
+
+def test_a_model_refuses_host_images(model):
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        model(torch.zeros(1, 3, 64, 64))
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        model.features(torch.zeros(1, 3, 64, 64))

@@ -244,6 +244,13 @@ static CoreW core_weights(const Tensor& wx, const Tensor& wdt, const Tensor& A, 
     return w;
 }
 
+static void check_core(const Tensor& x, const CoreW& w, bool cm) {
+    require_on(x, {&w.wx, &w.wdt, &w.A, &w.Ds, &w.bias, &w.lnw, &w.lnb});
+    TORCH_CHECK(x.dim() == 4 && x.size(cm ? 0 : 1) == w.D, "x must be a 4-d map of ", w.D, " channels, got ", x.sizes());
+    TORCH_CHECK(x.scalar_type() == w.wx.scalar_type() && x.scalar_type() == w.wdt.scalar_type(), "x is ", x.scalar_type(),
+                ", the weights were built for ", w.wx.scalar_type(), " and ", w.wdt.scalar_type());
+}
+
 // -------------------------------------------------------------------------------------------- the backbone
 struct Norm { Tensor w, b; };
 struct Block {
@@ -280,12 +287,14 @@ public:
     Tensor forward(const Tensor& img) {
         TORCH_CHECK(!head.empty(), "this model was built without a classifier");
         at::NoGradGuard no_grad;
+        require_on(img, {&stem.at(0)});
         const CallGuard guard(img);
         const Tensor x = run(img, nullptr);
         return at::linear(x.mean({2, 3}).to(type), head[2], head[3]);
     }
     std::vector<Tensor> features(const Tensor& img, const std::vector<int64_t>& which) {
         at::NoGradGuard no_grad;
+        require_on(img, {&stem.at(0)});
         const CallGuard guard(img);
         std::vector<Map> maps;
         run(img, &maps);
@@ -455,6 +464,7 @@ void bind_backbone(pybind11::module_& m) {
     // x: contiguous (D, B, H, W) with channel_major, else (B, D, H, W)
     m.def("ss2d_core",
           [](const Tensor& x, const CoreW& w, bool with_norm, at::ScalarType out_type, const OptT& workspace, bool cm) {
+              check_core(x, w, cm);
               const int64_t B = x.size(cm ? 1 : 0), H = x.size(2), W = x.size(3);
               const CallGuard guard(x);
               at::NoGradGuard no_grad;
@@ -462,12 +472,14 @@ void bind_backbone(pybind11::module_& m) {
           }, release());
     m.def("ss2d_core_by_operators",
           [](const Tensor& x, const CoreW& w, bool with_norm, at::ScalarType out_type, bool cm) {
+              check_core(x, w, cm);
               const int64_t B = x.size(cm ? 1 : 0), H = x.size(2), W = x.size(3);
               const CallGuard guard(x);
               return core_by_operators(x, cm, B, H, W, cm ? B * H * W : H * W, w, with_norm, out_type, Tensor());
           }, release());
     m.def("project",
           [](const Tensor& x, const CoreW& w, bool cm) {
+              check_core(x, w, cm);
               const int64_t B = x.size(cm ? 1 : 0), H = x.size(2), W = x.size(3);
               const CallGuard guard(x);
               const Streams s = project(x, cm, B, H, W, cm ? B * H * W : H * W, w, false);

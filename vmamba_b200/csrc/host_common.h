@@ -36,6 +36,12 @@ inline void require_cuda(std::initializer_list<const Tensor*> ts) {
         TORCH_CHECK(!t->defined() || t->is_cuda(),
                     "vmamba_b200 operators run on CUDA tensors only (no CPU fallback); use the oracle under oracle/ for CPU reference values");
 }
+// what library products between raw-pointer calls would have checked
+inline void require_on(const Tensor& x, std::initializer_list<const Tensor*> ts) {
+    require_cuda({&x});
+    for (const Tensor* t : ts)
+        TORCH_CHECK(!t->defined() || t->device() == x.device(), "expected all tensors on ", x.device(), ", got one on ", t->device());
+}
 inline void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 inline Tensor opt(const OptT& t) { return t.has_value() ? *t : Tensor(); }
 inline void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }

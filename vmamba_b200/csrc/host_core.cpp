@@ -63,9 +63,12 @@ Tensor expand_rows(const Tensor& xd, const Tensor& wdt, Tensor dts, int64_t B, i
 struct CoreNode : public torch::autograd::Function<CoreNode> {
     static Tensor forward(AutogradContext* ctx, const Tensor& x_, const Tensor& x_proj, const Tensor& dt_projs, const Tensor& dt_bias,
                           const Tensor& A_logs, const Tensor& Ds, const Tensor& ln_w, const Tensor& ln_b, int64_t N, int64_t R, double eps) {
+        require_on(x_, {&x_proj, &dt_projs, &dt_bias, &A_logs, &Ds, &ln_w, &ln_b});
         const Tensor x = x_.contiguous();
         const CallGuard guard(x);
         const int64_t B = x.size(0), D = x.size(1), H = x.size(2), W = x.size(3), L = H * W, C = R + 2 * N, S = padded_row(B, D, H, W);
+        TORCH_CHECK(ln_w.numel() == D && ln_b.numel() == D, "the LayerNorm's weight and bias must have ", D, " elements, got ", ln_w.numel(), " and ",
+                    ln_b.numel());
         const auto of = x.options();
         const Tensor wx = x_proj.reshape({4 * C, D}).to(x.scalar_type()), wdt = dt_projs.reshape({4, D, R}).to(x.scalar_type()).contiguous();
         const Tensor A = A_logs.to(at::kFloat).exp().neg().contiguous(), bias = f32(dt_bias.reshape(-1)), Dp = f32(Ds.reshape(-1));
