@@ -13,7 +13,7 @@ from vmamba_b200.backbone import AcceleratedVSSM
 
 @pytest.fixture()
 def model():
-    m = vb.VSSMInfer.from_state_dict(state_dict(), device="cpu")
+    m = vb.VSSMInfer.from_state_dict(state_dict(depths=(1, 1, 2, 1)), device="cpu")
     assert m.native is m.native and m.blocks[0][0].core.native is not None       # as after a first call
     return m
 
@@ -43,11 +43,10 @@ def _replace_core_field(m):
 
 
 def _drop_a_block(m):
-    m.blocks[3] = []
+    m.blocks[2] = m.blocks[2][:-1]
 
 
 CHANGES = {
-    "dtype": lambda m: setattr(m, "dtype", torch.float16),
     "stem": lambda m: m.stem.update(b0=m.stem["b0"] + 1),
     "block": lambda m: setattr(m.blocks[0][0], "w_in", m.blocks[0][0].w_in * 2),
     "core": _replace_core_field,
@@ -69,6 +68,28 @@ def test_changes_after_the_first_call_count(model, what):
     assert after.dtype == model.dtype and len(after.head) == (0 if model.head is None else 4)
     if model.head is not None:
         assert torch.equal(after.head[3], model.head["b"])
+
+
+WRONG = {
+    "type": lambda m: setattr(m, "dtype", torch.float16),
+    "depthwise kernel": lambda m: setattr(m.blocks[0][0], "w_dw", torch.zeros(32, 1, 5, 5, dtype=m.dtype)),
+    "norm": lambda m: setattr(m.blocks[1][0], "n2w", m.blocks[1][0].n2w[:8]),
+    "out_proj": lambda m: setattr(m.blocks[0][0], "w_out", m.blocks[0][0].w_out[:16]),
+    "layout": lambda m: setattr(m.blocks[0][0], "w_in", m.blocks[0][0].w_in.t()),
+    "bias type": lambda m: setattr(m.blocks[0][0], "b1f", m.blocks[0][0].b1f.bfloat16()),
+    "core": lambda m: setattr(m.blocks[0][0], "core", m.blocks[1][0].core),
+    "core field": lambda m: setattr(m.blocks[0][0].core, "Ds", m.blocks[0][0].core.Ds[:8]),
+    "outnorm": lambda m: m.outnorm.update({0: m.outnorm[1]}),
+    "head": lambda m: m.head.update(nw=m.head["nw"][:8]),
+    "stem": lambda m: m.stem.update(w0=torch.zeros(16, 3, 4, 4, dtype=m.dtype)),
+}
+
+
+@pytest.mark.parametrize("what", WRONG)
+def test_parts_that_do_not_fit_are_refused(model, what):
+    WRONG[what](model)
+    with pytest.raises(RuntimeError):
+        model.native
 
 
 def test_core_weight_changes_count(model):

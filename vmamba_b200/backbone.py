@@ -187,6 +187,7 @@ class VSSMInfer:
             n.head = list(_HEAD(self.head))
         for i, (w, b) in self.outnorm.items():
             n.add_outnorm(i, w, b)
+        n.validate()
         self._native = parts, n
         return n
 

@@ -236,11 +236,26 @@ static Tensor core_run(const Tensor& x, bool cm, int64_t B, int64_t H, int64_t W
     return out;
 }
 
+// Weights whose data the kernels read by address: of the stated size and type, in one piece.
+static void expect(const char* name, const Tensor& t, std::vector<int64_t> sizes, at::ScalarType type) {
+    TORCH_CHECK(t.defined() && t.sizes() == at::IntArrayRef(sizes), name, " must be ", at::IntArrayRef(sizes), ", got ", t.sizes());
+    TORCH_CHECK(t.scalar_type() == type, name, " must be ", type, ", got ", t.scalar_type());
+    TORCH_CHECK(t.is_contiguous(), name, " must be contiguous");
+}
+
 static CoreW core_weights(const Tensor& wx, const Tensor& wdt, const Tensor& A, const Tensor& Ds, const Tensor& bias, const OptT& lnw, const OptT& lnb,
                           int64_t N, int64_t R, double eps) {
     CoreW w;
     w.wx = wx; w.wdt = wdt; w.A = A; w.Ds = Ds; w.bias = bias; w.lnw = opt(lnw); w.lnb = opt(lnb);
-    w.N = N; w.R = R; w.D = wx.size(1); w.eps = eps;
+    w.N = N; w.R = R; w.D = wx.size(-1); w.eps = eps;
+    const int64_t K = 4;
+    expect("wx", wx, {K * (R + 2 * N), w.D}, wx.scalar_type());
+    expect("wdt", wdt, {K, w.D, R}, wx.scalar_type());
+    expect("A", A, {K * w.D, N}, at::kFloat);
+    expect("Ds", Ds, {K * w.D}, at::kFloat);
+    expect("dt_bias", bias, {K * w.D}, at::kFloat);
+    for (const Tensor* t : {&w.lnw, &w.lnb})
+        if (t->defined()) expect("ln_weight / ln_bias", *t, {w.D}, at::kFloat);
     return w;
 }
 
@@ -284,6 +299,46 @@ public:
         downs.push_back(d);
     }
 
+    // every part of the size that the parts around it ask for, once per model
+    void validate() const {
+        auto norm_of = [](const char* name, const Norm& n, int64_t C) {
+            expect(name, n.w, {C}, at::kFloat);
+            expect(name, n.b, {C}, at::kFloat);
+        };
+        TORCH_CHECK(stem.size() == 8 && stages.size() == downs.size() && !stages.empty(), "a backbone needs a stem and stages");
+        const int64_t C0 = stem[0].size(0);
+        int64_t C = stem[4].size(0);
+        expect("patch_embed.0.weight", stem[0], {C0, stem[0].size(1), 3, 3}, type);
+        expect("patch_embed.0.bias", stem[1], {C0}, at::kFloat);
+        norm_of("patch_embed.2", {stem[2], stem[3]}, C0);
+        expect("patch_embed.5.bias", stem[5], {C}, at::kFloat);
+        norm_of("patch_embed.7", {stem[6], stem[7]}, C);
+        for (size_t i = 0; i < stages.size(); ++i) {
+            for (const Block& b : stages[i]) {
+                const int64_t D = b.w_in.size(0), hidden = b.w1.size(0);
+                norm_of("norm", b.n1, C);
+                norm_of("norm2", b.n2, C);
+                expect("op.in_proj", b.w_in, {D, C}, type);
+                TORCH_CHECK(b.w_dw.numel() == 9 * D, "op.conv2d must have 3 x 3 weights for ", D, " channels, got ", b.w_dw.sizes());
+                expect("op.conv2d", b.w_dw.view({D, 9}), {D, 9}, type);
+                expect("op.out_proj", b.w_out, {C, D}, type);
+                expect("mlp.fc1", b.w1, {hidden, C}, type);
+                expect("mlp.fc1.bias", b.b1, {hidden}, at::kFloat);
+                expect("mlp.fc2", b.w2, {C, hidden}, type);
+                expect("mlp.fc2.bias", b.b2, {C}, at::kFloat);
+                TORCH_CHECK(b.core.D == D && b.core.wx.scalar_type() == type, "the core must have ", D, " channels of ", type);
+                TORCH_CHECK(b.core.lnw.defined() && b.core.lnb.defined(), "the core needs its LayerNorm");
+            }
+            const auto it = outnorm.find((int64_t)i);
+            if (it != outnorm.end()) norm_of("outnorm", it->second, C);
+            if (downs[i].there) {
+                C = downs[i].w.size(0);
+                expect("downsample bias", downs[i].b, {C}, at::kFloat);
+                norm_of("downsample norm", downs[i].n, C);
+            }
+        }
+        if (!head.empty()) norm_of("classifier.norm", {head[0], head[1]}, C);
+    }
     Tensor forward(const Tensor& img) {
         TORCH_CHECK(!head.empty(), "this model was built without a classifier");
         at::NoGradGuard no_grad;
@@ -499,6 +554,7 @@ void bind_backbone(pybind11::module_& m) {
         .def_readwrite("dtype", &Backbone::type)
         .def("add_block", &Backbone::add_block)
         .def("add_down", &Backbone::add_down)
+        .def("validate", &Backbone::validate)
         .def("add_outnorm", [](Backbone& b, int64_t i, const Tensor& w, const Tensor& bias) { b.outnorm[i] = {w, bias}; })
         .def("forward", &Backbone::forward, release())
         .def("features", &Backbone::features, release());
