@@ -308,14 +308,15 @@ def op_sweep(args):
                 # gradients of the same cell: reads u, delta, dout (fp32), B, C; writes du, ddelta, dB, dC
                 from vmamba_b200 import ops as _ops
                 dout = torch.randn((Bt, K * D, L), device="cuda", generator=g)
-                _, ck = _ops.selective_scan_fwd(u, delta, A, Bm, Cm, Dp, bias, True, True, return_checkpoints=True)
+                # with the states that a training step's forward call leaves
+                _, ck = _ops.selective_scan_fwd(u, delta, A, Bm, Cm, Dp, bias, True, True, return_checkpoints="grad")
                 ms = time_events(lambda: _ops.selective_scan_bwd(u, delta, A, Bm, Cm, Dp, bias, dout, True, ck), args.steps)
                 nbytes = Bt * L * (K * D * (2 * 2 + 4 + 2 * 2) + 4 * K * N * 2) + 4 * (2 * K * D * N + 4 * K * D)
                 gbs = nbytes / (ms * 1e-3) / 1e9
                 print(json.dumps({"op": "selective_scan_bwd", "dtype": "bf16, dout f32", "d_state": N, "D": D, "L": L, "batch": Bt,
                                   "ms": ms, "algorithmic_bytes": nbytes, "achieved_gbs": gbs, "frac": gbs / peak,
                                   "peak_gbs": peak, "peak_kind": f"of {kind}"}), flush=True)
-                del u, delta, Bm, Cm, dout
+                del u, delta, Bm, Cm, dout, ck
     for (D, H) in ((96, 56), (384, 14), (96, 256)):
         Bt = max(1, int(min(args.sweep_gb, 8.0) * 1e9 / (10 * D * H * H)))
         x = torch.randn((Bt, D, H, H), device="cuda", generator=g).to(torch.bfloat16)

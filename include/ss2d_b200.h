@@ -54,6 +54,7 @@ typedef enum ss2d_status {
  * A: (dim, dstate) fp32 contiguous.  B, C: (batch, n_groups, dstate, seqlen), last dimension
  * contiguous.  D, delta_bias: (dim) fp32 or NULL.  in_dtype is the type of u, delta, B, C;
  * out_dtype is SS2D_F32 ("oflex") or equal to in_dtype.  State and arithmetic are fp32.
+ * Tensors need no alignment beyond their element's, and nothing outside them is read.
  * -------------------------------------------------------------------------------- */
 typedef struct ss2d_scan_params {
     const void *u, *delta, *A, *B, *C, *D, *delta_bias;
