@@ -92,9 +92,9 @@ def test_selective_scan_bwd_fp32_vs_oracle(vb, Bt, K, Cd, N, L):
 @pytest.mark.parametrize("L,dt,oflex,opt", [(200, "f32", True, True), (392, "bf16", True, True), (136, "bf16", False, True),
                                             (196, "f16", True, False), (16, "f32", True, True)])
 def test_selective_scan_bwd_many_rows(vb, L, dt, oflex, opt):
-    """d_state 1 with enough rows (26 x 4 x 384 = 39 936) for the lanes-are-rows backward kernel: rows of one chunk and a
+    """d_state 1 with many rows (26 x 4 x 384 = 39 936, several per warp): rows of one chunk and a
     ragged second one (L = 200), several chunks (392), a 14 x 14 map (196), a single tile; every gradient against
-    the oracle, and against the warp-per-row kernel on the first two images (too few rows for this one)."""
+    the oracle, and against the call on the first two images (fewer rows per warp)."""
     Bt, K, Cd = 26, 4, 384
     u, delta, A, B, C, D, bias, dout = _random_case(Bt, K, Cd, 1, L, seed=L, with_D=opt, with_bias=opt)
     if dt != "f32":
@@ -122,8 +122,8 @@ def test_selective_scan_bwd_many_rows(vb, L, dt, oflex, opt):
                                               (4, 16, "f32", True, True), (16, 72, "f32", True, False),
                                               (16, 3136, "bf16", True, True)])
 def test_selective_scan_bwd_many_rows_states(vb, N, L, dt, oflex, opt):
-    """d_state 4 / 8 / 16 with enough rows (3 x 4 x 800 = 9 600) for the lanes-are-rows backward kernel of those state
-    counts: every gradient against the oracle (short rows) and against the warp-per-row kernel run image by image (too
+    """d_state 4 / 8 / 16 with many rows (3 x 4 x 800 = 9 600): every gradient against the oracle (short rows) and against
+    calls image by image (rows cut otherwise; too
     few rows for this one); one case without D and delta_bias."""
     Bt, K, Cd = 3, 4, 800
     u, delta, A, B, C, D, bias, dout = _random_case(Bt, K, Cd, N, L, seed=L + N, with_D=opt, with_bias=opt)
@@ -282,7 +282,7 @@ def test_shared_delta_rows_forward_and_backward(vb, ratio):
 @pytest.mark.parametrize("N,L", [(1, 3136), (1, 200), (3, 300), (1, 90)])
 def test_backward_with_and_without_forward_checkpoints(vb, N, L):
     """The step states written by the forward call give the same gradients as recomputing them (to fp32 rounding: the
-    forward kernel composes the recurrence in 256-element steps, the recomputation in 128-element steps), and the
+    gradient kernels form their own states where these are 128 elements apart), and the
     checkpoints are the oracle's states in front of every 128th element."""
     from vmamba_b200 import ops
     u, delta, A, B, C, D, bias, dout = _random_case(2, 2, 3, N, L, seed=L)

@@ -155,7 +155,7 @@ def test_selective_scan_dstate16_sweep_shapes(vb, L, KD, dtype):
                                            (4, 32, "f32", False), (16, 392, "f16", True), (16, 196, "bf16", True),
                                            (1, 196, "bf16", True), (1, 64, "f32", False)])
 def test_selective_scan_many_rows_small_state(vb, N, L, dtype, opt):
-    """d_state 4 / 8 / 16 (and 1 on short rows) with enough rows (B x 4 x 384 = 39 936) for the lanes-are-rows kernel: whole and ragged tiles
+    """d_state 4 / 8 / 16 (and 1 on short rows) with many rows (B x 4 x 384 = 39 936, two per lane): whole and ragged chunks
     (L = 200 = 12 x 16 + 8; L = 196, a 14 x 14 map, whose 16-bit rows allow 8-byte pieces only), 16-bit and fp32 tensors, with and without D / bias / softplus, A drawn per row, against the
     C oracle; the states it leaves for the backward pass against the forward kernel for fewer rows."""
     rng = np.random.default_rng(N * 100 + L)
@@ -183,7 +183,7 @@ def test_selective_scan_many_rows_small_state(vb, N, L, dtype, opt):
     assert _lib.launch_count() == n0 + 1
     assert y.dtype == torch.float32 and O.max_rel_err(host(y), ref) <= TOL_F32
     assert torch.equal(y, vb.selective_scan_fn(*args)), "results must be bit-identical run to run"
-    # same values as the warp-per-row kernel gives for a slice with too few rows for this one
+    # same values as the call on a slice gives (one row per lane)
     few = tuple(t[:2] if isinstance(t, torch.Tensor) and t.dim() >= 3 else t for t in args)
     assert O.max_rel_err(host(vb.selective_scan_fn(*few)), ref[:2]) <= TOL_F32
     assert O.max_rel_err(host(y[:2]), host(vb.selective_scan_fn(*few))) <= 2e-6
