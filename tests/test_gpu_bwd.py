@@ -123,8 +123,7 @@ def test_selective_scan_bwd_many_rows(vb, L, dt, oflex, opt):
                                               (16, 3136, "bf16", True, True)])
 def test_selective_scan_bwd_many_rows_states(vb, N, L, dt, oflex, opt):
     """d_state 4 / 8 / 16 with many rows (3 x 4 x 800 = 9 600): every gradient against the oracle (short rows) and against
-    calls image by image (rows cut otherwise; too
-    few rows for this one); one case without D and delta_bias."""
+    calls image by image (other row sets and segments); one case without D and delta_bias."""
     Bt, K, Cd = 3, 4, 800
     u, delta, A, B, C, D, bias, dout = _random_case(Bt, K, Cd, N, L, seed=L + N, with_D=opt, with_bias=opt)
     if dt != "f32":

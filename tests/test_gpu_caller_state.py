@@ -7,6 +7,8 @@ import pytest
 import torch
 import torch.utils.checkpoint
 
+from vmamba_b200.backbone import AcceleratedVSSM
+
 pytestmark = pytest.mark.gpu
 
 
@@ -177,3 +179,20 @@ def test_core_refuses_what_does_not_fit(vb):
         wrong[i] = wrong[i][:D // 2]
         with pytest.raises(RuntimeError):
             vb.ss2d_core_autograd(x, *wrong, d_state=1, dt_rank=R)
+
+
+def test_a_captured_graph_keeps_its_weights(vb):
+    """Parts replaced after the capture count in eager calls; the graph goes on with those it was captured with, which stay allocated."""
+    m = vb.VSSMInfer.from_state_dict(state_dict())
+    x = torch.randn(2, 3, 64, 64, device="cuda").bfloat16()
+    for model in (m, AcceleratedVSSM(m, False, ())):
+        runner = vb.GraphedBackbone(model, tuple(x.shape), dtype=torch.bfloat16)
+        first = runner(x).clone()
+        torch.cuda.synchronize()
+        for stage in m.blocks:
+            for b in stage:
+                for name in ("w_in", "w_dw", "w_out", "w1", "w2"):
+                    setattr(b, name, getattr(b, name) * 2)
+        assert not torch.equal(m(x), first)              # the model's own object is made anew, and the old one let go
+        junk = [torch.full_like(t, float("nan")) for stage in m.blocks for b in stage for t in (b.w_in, b.w_dw, b.w_out, b.w1, b.w2)]
+        assert torch.equal(runner(x), first) and len(junk) == 20

@@ -32,6 +32,8 @@ class GraphedBackbone:
         self.model = model
         self.device = torch.device(device) if device is not None else torch.device("cuda", torch.cuda.current_device())
         self.dtype = dtype or getattr(model, "dtype", torch.bfloat16)
+        # the graph reads the weights by address: they stay, whatever becomes of the model's parts
+        self._weights = getattr(getattr(model, "fast", model), "native", None)
         fn: Callable = (lambda x: model.features(x, out_indices)) if features else model
         with torch.cuda.device(self.device):
             self.input = torch.zeros(tuple(batch_shape), device=self.device, dtype=self.dtype)
