@@ -202,3 +202,32 @@ def test_scan_tensors_off_16_byte_boundaries(vb, N, K, Cd, L, dt, at):
         got = vb.selective_scan_bwd(ts[0], ts[1], dev(A), ts[2], ts[3], dev(D), dev(bias), put(dout, at[0], torch.float32), True, ck)
         for name, x, r in zip(NAMES, got, ref):
             assert O.max_rel_err(host(x), r) <= TOL[dt], name
+
+
+@pytest.mark.parametrize("dt", ["f32", "bf16"])
+@pytest.mark.parametrize("scans", [0, 1, 2, 3])
+@pytest.mark.parametrize("shape,offset", [((1, 1, 1, 1), 0), ((2, 3, 1, 9), 1), ((2, 3, 9, 1), 0), ((3, 50, 7, 7), 3), ((2, 37, 5, 6), 2), ((5, 61, 16, 32), 0),
+                                          ((1, 3, 64, 32), 4), ((1, 3, 56, 58), 1), ((1, 2, 96, 96), 0), ((1, 2, 109, 113), 1), ((1, 2, 192, 192), 0),
+                                          ((1, 2, 33, 161), 1), ((1, 2, 200, 190), 0), ((1, 1, 2, 9001), 0), ((1, 1, 20000, 3), 1), ((2, 2, 247, 231), 5)])
+def test_cross_of_any_plane_and_alignment(vb, shape, offset, scans, dt):
+    """CrossScan and CrossMerge at the edges of their kernels: single pixels and lines, planes that share a CTA, lines in one bank, pairs, the
+    largest planes taken whole and the smallest in tiles, tensors that start anywhere.  The merge is rounded after every addition."""
+    Bt, Cc, H, W = shape
+    rng, td = np.random.default_rng(H * W + scans), TD[dt]
+
+    def at_offset(a):
+        room = torch.full((a.size + offset,), float("nan"), device="cuda", dtype=td)
+        room[offset:] = dev(a.reshape(-1), td)
+        return room[offset:].view(a.shape)
+    rnd = (lambda a: a) if dt == "f32" else O.round_bf16
+    x, ys = rnd(rng.standard_normal(shape, dtype=np.float32)), rnd(rng.standard_normal((Bt, 4, Cc, H, W), dtype=np.float32))
+    assert np.array_equal(host(vb.cross_scan_fn(at_offset(x), scans=scans)), O.cross_scan(x, scans).reshape(Bt, 4, Cc, H * W))
+    place = O.cross_scan(np.arange(H * W, dtype=np.float32).reshape(1, 1, H, W), scans).reshape(4, H * W).astype(np.int64)
+    y = [torch.empty(Bt, Cc, H * W, dtype=td) for _ in range(4)]
+    for k in range(4):
+        y[k][..., torch.from_numpy(place[k])] = torch.from_numpy(ys[:, k].reshape(Bt, Cc, H * W)).to(td)
+    if scans == 1:
+        want = (((y[0].float() + y[1].float()) + y[2].float()) + y[3].float()).to(td)
+    else:
+        want = ((y[0] + y[1]) + y[2]) + y[3] if scans == 3 else (y[0] + y[2]) + (y[1] + y[3])
+    assert torch.equal(vb.cross_merge_fn(at_offset(ys), scans=scans).cpu().view(Bt, Cc, H * W), want)
