@@ -213,6 +213,7 @@ struct SegAddr {
 // planes' scans share their barriers.
 template <typename T, int VEC, int NPL, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) core_plane_kernel(const CoreArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) float smem[];
     __shared__ ScanScratch scr;
     constexpr bool kPrecise = sizeof(T) == 4;
@@ -455,12 +456,12 @@ static int launch_core_n(const CoreArgs& a, const PlaneConfig& c, unsigned grid,
         auto kern = core_plane_kernel<T, VEC, NPL, 448, 2>;
         e = ensure_dynamic_smem((const void*)kern, c.smem);
         if (e != cudaSuccess) return SS2D_ECUDA;
-        kern<<<grid, c.threads, c.smem, st>>>(a);
+        launch(kern, grid, c.threads, c.smem, st, a);
     } else {
         auto kern = core_plane_kernel<T, VEC, NPL, 1024, 1>;
         e = ensure_dynamic_smem((const void*)kern, c.smem);
         if (e != cudaSuccess) return SS2D_ECUDA;
-        kern<<<grid, c.threads, c.smem, st>>>(a);
+        launch(kern, grid, c.threads, c.smem, st, a);
     }
     count_launch();
     return check_launch();
@@ -543,7 +544,7 @@ template <typename T, int S, int SV, int MINB, int kRoll>
 static int launch_routes_k(const RouteArgs& a, const RoutePlan& r, unsigned grid, cudaStream_t st) {
     auto kern = core_route_kernel<T, S, SV, MINB, kRoll>;
     if (ensure_dynamic_smem((const void*)kern, r.smem) != cudaSuccess) return SS2D_ECUDA;
-    kern<<<grid, 128, r.smem, st>>>(a);
+    launch(kern, grid, 128, r.smem, st, a);
     count_launch();
     return check_launch();
 }
@@ -558,7 +559,7 @@ template <typename T, int MINB>
 static int launch_pad(const RouteArgs& a, const RoutePlan& r, unsigned grid, cudaStream_t st) {
     auto kern = core_route_pad_kernel<T, 8, MINB>;
     if (ensure_dynamic_smem((const void*)kern, r.smem) != cudaSuccess) return SS2D_ECUDA;
-    kern<<<grid, 128, r.smem, st>>>(a);
+    launch(kern, grid, 128, r.smem, st, a);
     count_launch();
     return check_launch();
 }

@@ -221,6 +221,7 @@ __device__ __forceinline__ void walk_route(const RouteArgs& a, const int b, cons
 // in the column-major copy (W a multiple of SV; the merge needs W to be a multiple of 4).
 template <typename T, int S, int SV, int MINB, int kRoll>
 __global__ void __launch_bounds__(128, MINB) core_route_kernel(const RouteArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int L = a.L, H = a.H, W = a.W, D = a.D;
     float* accR = reinterpret_cast<float*>(smem_raw);          // routes 0, 2: row-major
@@ -295,6 +296,7 @@ __global__ void __launch_bounds__(128, MINB) core_route_kernel(const RouteArgs a
 // Shared memory: (8 + 2 sizeof(T)) bytes per element of a row.
 template <typename T, int S, int MINB>
 __global__ void __launch_bounds__(128, MINB) core_route_pad_kernel(const RouteArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int Lp = a.L, L = a.plane, H = a.H, W = a.W, D = a.D;
     float* accR = reinterpret_cast<float*>(smem_raw);

@@ -77,6 +77,7 @@ template <typename T> __device__ __forceinline__ void run_pad(const RunArgs& a, 
 // V: pixels of a thread at a time, 1, or 2 of 16-bit maps with even sides whose planes start on words.
 template <typename T, int SCANS, int V, bool kPad>
 __global__ void __launch_bounds__(512) cross_scan_runs_kernel(const RunArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) unsigned char smraw[];
     constexpr bool kCols = SCANS == 0 || SCANS == 3;
     const int b = blockIdx.x / a.blocks, c0 = (blockIdx.x - b * a.blocks) * a.PP, np = min(a.PP, a.C - c0);
@@ -124,6 +125,7 @@ __global__ void __launch_bounds__(512) cross_scan_runs_kernel(const RunArgs a) {
 // `back`).  The CrossScan of rows that each belong to one route.
 template <typename T>
 __global__ void __launch_bounds__(512) cross_rows_kernel(const RunArgs a, const int scans, const int back) {
+    follow_previous();
     extern __shared__ __align__(16) unsigned char smraw[];
     const int bk = blockIdx.x / a.blocks, k = bk & 3, c0 = (blockIdx.x - bk * a.blocks) * a.PP, np = min(a.PP, a.C - c0);
     const int L = a.L, S = a.S, H = a.H, W = a.W, n = np * L;
@@ -147,6 +149,7 @@ __global__ void __launch_bounds__(512) cross_rows_kernel(const RunArgs a, const 
 // V: as above, of routes that start on words.
 template <typename T, int SCANS, int V>
 __global__ void __launch_bounds__(512) cross_merge_runs_kernel(const RunArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) unsigned char smraw[];
     T* sm = reinterpret_cast<T*>(smraw);
     constexpr bool kCols = SCANS == 0 || SCANS == 3;

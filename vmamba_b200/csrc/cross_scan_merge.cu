@@ -49,6 +49,7 @@ struct CrossArgs {
 // pair at the mirrored address with its halves swapped.
 constexpr int kPairTile = 64;
 __global__ void __launch_bounds__(256) cross_scan_pair_kernel(const CrossArgs a) {
+    follow_previous();
     __shared__ __align__(4) uint16_t tile[kPairTile][kPairTile + 2];       // pitch 33 words
     const unsigned t = blockIdx.x, tiles_w = (unsigned)a.tiles_w, tiles_h = (unsigned)a.tiles_h, C = (unsigned)a.C;
     const unsigned tw = t % tiles_w, rest = t / tiles_w, th = rest % tiles_h, plane = rest / tiles_h;
@@ -119,17 +120,17 @@ static bool plan_tiles(const ss2d_cross_params* p, int slots, TileArgs& a, size_
 static unsigned tile_grid(const TileArgs& a, int64_t images) { return (unsigned)(images * a.C * a.tiles_h * a.tiles_w); }
 template <typename T>
 static int launch_scan_tiles(const TileArgs& a, int64_t B, size_t smem, cudaStream_t st) {
-    cross_scan_tiles_kernel<T><<<tile_grid(a, B), kTileThreads, smem, st>>>(a);
+    launch(cross_scan_tiles_kernel<T>, tile_grid(a, B), kTileThreads, smem, st, a);
     count_launch();
     return check_launch();
 }
 template <typename T, int V>
 static int merge_tiles_v(const TileArgs& a, int64_t B, int scans, size_t smem, cudaStream_t st) {
     const unsigned g = tile_grid(a, B);
-    if (scans == 0) cross_merge_tiles_kernel<T, 0, V><<<g, kTileThreads, smem, st>>>(a);
-    else if (scans == 1) cross_merge_tiles_kernel<T, 1, V><<<g, kTileThreads, smem, st>>>(a);
-    else if (scans == 2) cross_merge_tiles_kernel<T, 2, V><<<g, kTileThreads, smem, st>>>(a);
-    else cross_merge_tiles_kernel<T, 3, V><<<g, kTileThreads, smem, st>>>(a);
+    if (scans == 0) launch(cross_merge_tiles_kernel<T, 0, V>, g, kTileThreads, smem, st, a);
+    else if (scans == 1) launch(cross_merge_tiles_kernel<T, 1, V>, g, kTileThreads, smem, st, a);
+    else if (scans == 2) launch(cross_merge_tiles_kernel<T, 2, V>, g, kTileThreads, smem, st, a);
+    else launch(cross_merge_tiles_kernel<T, 3, V>, g, kTileThreads, smem, st, a);
     count_launch();
     return check_launch();
 }
@@ -167,14 +168,14 @@ template <typename K> static int run_attr(K k, size_t smem) {
 template <typename T, int SCANS, int V, bool kPad> static int launch_scan_runs(const RunArgs& a, int64_t B, int threads, size_t smem, cudaStream_t st) {
     auto k = cross_scan_runs_kernel<T, SCANS, V, kPad>;
     if (const int rc = run_attr(k, smem)) return rc;
-    k<<<(unsigned)(B * a.blocks), threads, smem, st>>>(a);
+    launch(k, (unsigned)(B * a.blocks), threads, smem, st, a);
     count_launch();
     return check_launch();
 }
 template <typename T, int SCANS, int V> static int launch_merge_runs(const RunArgs& a, int64_t B, int threads, size_t smem, cudaStream_t st) {
     auto k = cross_merge_runs_kernel<T, SCANS, V>;
     if (const int rc = run_attr(k, smem)) return rc;
-    k<<<(unsigned)(B * a.blocks), threads, smem, st>>>(a);
+    launch(k, (unsigned)(B * a.blocks), threads, smem, st, a);
     count_launch();
     return check_launch();
 }
@@ -234,8 +235,8 @@ static int launch_rows(const ss2d_cross_params* p, bool back, cudaStream_t st) {
     const unsigned grid = (unsigned)(p->B * 4 * a.blocks);
     const int rc = p->dtype == SS2D_F32 ? run_attr(cross_rows_kernel<float>, smem) : run_attr(cross_rows_kernel<uint16_t>, smem);
     if (rc) return rc;
-    if (p->dtype == SS2D_F32) cross_rows_kernel<float><<<grid, threads, smem, st>>>(a, p->scans, back);
-    else cross_rows_kernel<uint16_t><<<grid, threads, smem, st>>>(a, p->scans, back);
+    if (p->dtype == SS2D_F32) launch(cross_rows_kernel<float>, grid, threads, smem, st, a, p->scans, back);
+    else launch(cross_rows_kernel<uint16_t>, grid, threads, smem, st, a, p->scans, back);
     count_launch();
     return check_launch();
 }
@@ -287,7 +288,7 @@ int cross_scan(const ss2d_cross_params* p, cudaStream_t st) {
         CrossArgs q = a;
         q.tiles_h = (p->H + kPairTile - 1) / kPairTile;
         q.tiles_w = (p->W + kPairTile - 1) / kPairTile;
-        cross_scan_pair_kernel<<<(unsigned)(q.tiles_h * q.tiles_w * p->B * p->C), dim3(32, 8), 0, st>>>(q);
+        launch(cross_scan_pair_kernel, (unsigned)(q.tiles_h * q.tiles_w * p->B * p->C), dim3(32, 8), 0, st, q);
         count_launch();
         return check_launch();
     }
@@ -353,6 +354,7 @@ __device__ __forceinline__ void ex_decompose(const CrossExArgs& a, long long i, 
 
 template <typename T>
 __global__ void __launch_bounds__(256) cross_scan_ex_kernel(const CrossExArgs a) {
+    follow_previous();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.total; i += (long long)gridDim.x * blockDim.x) {
         long long b, c, p;
         ex_decompose(a, i, b, c, p);
@@ -368,6 +370,7 @@ __global__ void __launch_bounds__(256) cross_scan_ex_kernel(const CrossExArgs a)
 
 template <typename T>
 __global__ void __launch_bounds__(256) cross_merge_ex_kernel(const CrossExArgs a) {
+    follow_previous();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.total; i += (long long)gridDim.x * blockDim.x) {
         long long b, c, p;
         ex_decompose(a, i, b, c, p);
@@ -418,8 +421,8 @@ template <typename T, bool kScan>
 static int launch_ex(const CrossExArgs& a, cudaStream_t st) {
     long long ctas = (a.total + 255) / 256;
     if (ctas > 148LL * 32) ctas = 148LL * 32;
-    if constexpr (kScan) cross_scan_ex_kernel<T><<<(unsigned)ctas, 256, 0, st>>>(a);
-    else cross_merge_ex_kernel<T><<<(unsigned)ctas, 256, 0, st>>>(a);
+    if constexpr (kScan) launch(cross_scan_ex_kernel<T>, (unsigned)ctas, 256, 0, st, a);
+    else launch(cross_merge_ex_kernel<T>, (unsigned)ctas, 256, 0, st, a);
     count_launch();
     return check_launch();
 }

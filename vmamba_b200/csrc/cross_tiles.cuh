@@ -77,6 +77,7 @@ template <bool kByRow, int V, typename F, typename U> __device__ __forceinline__
 // a row keeps the phase it has in global memory; pieces that reach beyond the map are taken by single elements.
 template <typename T>
 __global__ void __launch_bounds__(kTileThreads) cross_scan_tiles_kernel(const TileArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) unsigned char smraw[];
     T* sm = reinterpret_cast<T*>(smraw);
     constexpr int E = 16 / (int)sizeof(T);
@@ -134,6 +135,7 @@ __global__ void __launch_bounds__(kTileThreads) cross_scan_tiles_kernel(const Ti
 // even sides whose planes start on words.
 template <typename T, int SCANS, int V>
 __global__ void __launch_bounds__(kTileThreads, 6) cross_merge_tiles_kernel(const TileArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) unsigned char smraw[];
     T* sm = reinterpret_cast<T*>(smraw);             // [slot][th][pitch]
     constexpr bool kCols = SCANS == 0 || SCANS == 3;

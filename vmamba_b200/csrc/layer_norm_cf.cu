@@ -33,6 +33,7 @@ struct NormArgs {
 // Without the per-channel tests of the general form the kernel issues about half the instructions.
 template <typename Tio, int NTY, int CACHE, int PV, int TX, int MODE>
 __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * PV <= 24) ? 2 : 1) layer_norm_cf_kernel(const NormArgs a) {
+    follow_previous();
     static_assert(TX == 16 && NTY % 4 == 0, "a warp is two channel slices of 16 items");
     constexpr int NP = NTY / 2;                      // partial sums per item after the in-warp step
     __shared__ float red[2][NP][TX][PV];
@@ -251,11 +252,11 @@ static void launch_one(const NormArgs& a, cudaStream_t st) {
             if (!a.add && !a.add_bias && !a.sum_out) mode = 1;
             else if (a.add && a.sum_out) mode = a.add_bias ? 3 : 2;
         }
-        if (mode == 1) { layer_norm_cf_kernel<Tio, NTY, CACHE, PV, kItemsPerCta, 1><<<grid, block, 0, st>>>(a); return; }
-        if (mode == 2) { layer_norm_cf_kernel<Tio, NTY, CACHE, PV, kItemsPerCta, 2><<<grid, block, 0, st>>>(a); return; }
-        if (mode == 3) { layer_norm_cf_kernel<Tio, NTY, CACHE, PV, kItemsPerCta, 3><<<grid, block, 0, st>>>(a); return; }
+        if (mode == 1) { launch(layer_norm_cf_kernel<Tio, NTY, CACHE, PV, kItemsPerCta, 1>, grid, block, 0, st, a); return; }
+        if (mode == 2) { launch(layer_norm_cf_kernel<Tio, NTY, CACHE, PV, kItemsPerCta, 2>, grid, block, 0, st, a); return; }
+        if (mode == 3) { launch(layer_norm_cf_kernel<Tio, NTY, CACHE, PV, kItemsPerCta, 3>, grid, block, 0, st, a); return; }
     }
-    layer_norm_cf_kernel<Tio, NTY, CACHE, PV, kItemsPerCta, 0><<<grid, block, 0, st>>>(a);
+    launch(layer_norm_cf_kernel<Tio, NTY, CACHE, PV, kItemsPerCta, 0>, grid, block, 0, st, a);
 }
 
 template <typename Tio>

@@ -26,6 +26,7 @@ struct NormBwdArgs {
 // PV: pixels per lane (neighbours, one access).  IT > 0: a warp's IT groups of channels stay in registers (D <= 32 * IT).
 template <typename Tg, int PV, int IT>
 __global__ void __launch_bounds__(kLnbWarps * 32, 3) layer_norm_cf_bwd_kernel(const NormBwdArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) float lnb_sm[];                // [2][D] sums of dw, db
     __shared__ float red[3][kLnbWarps][32 * PV];
     using VY = Vec<float, PV>;
@@ -172,15 +173,16 @@ static void launch_lnb(const NormBwdArgs& a, int pv, unsigned ctas, cudaStream_t
     const size_t smem = (size_t)2 * a.D * sizeof(float);
     const int threads = kLnbWarps * 32;
     if (pv == 2) {
-        if (a.D <= 96) layer_norm_cf_bwd_kernel<Tg, 2, 3><<<ctas, threads, smem, st>>>(a);
-        else layer_norm_cf_bwd_kernel<Tg, 2, 0><<<ctas, threads, smem, st>>>(a);
+        if (a.D <= 96) launch(layer_norm_cf_bwd_kernel<Tg, 2, 3>, ctas, threads, smem, st, a);
+        else launch(layer_norm_cf_bwd_kernel<Tg, 2, 0>, ctas, threads, smem, st, a);
     } else {
-        if (a.D <= 96) layer_norm_cf_bwd_kernel<Tg, 1, 3><<<ctas, threads, smem, st>>>(a);
-        else layer_norm_cf_bwd_kernel<Tg, 1, 0><<<ctas, threads, smem, st>>>(a);
+        if (a.D <= 96) launch(layer_norm_cf_bwd_kernel<Tg, 1, 3>, ctas, threads, smem, st, a);
+        else launch(layer_norm_cf_bwd_kernel<Tg, 1, 0>, ctas, threads, smem, st, a);
     }
 }
 
 __global__ void __launch_bounds__(256) layer_norm_cf_bwd_fold_kernel(const float* part, int ctas, int D, float* dw, float* db) {
+    follow_previous();
     __shared__ float red[8][32];
     const int i = blockIdx.x * 32 + (threadIdx.x & 31), row = threadIdx.x >> 5;
     float s = 0.f;
@@ -234,7 +236,7 @@ int layer_norm_cf_bwd(const ss2d_norm_bwd_params* p, cudaStream_t st) {
     if (p->g_dtype == SS2D_F32) launch_lnb<float>(a, pv, ctas, st);
     else if (p->g_dtype == SS2D_BF16) launch_lnb<__nv_bfloat16>(a, pv, ctas, st);
     else launch_lnb<__half>(a, pv, ctas, st);
-    layer_norm_cf_bwd_fold_kernel<<<(unsigned)((2 * p->D + 31) / 32), 256, 0, st>>>(a.part, (int)ctas, a.D, (float*)p->dweight, (float*)p->dbias);
+    launch(layer_norm_cf_bwd_fold_kernel, (unsigned)((2 * p->D + 31) / 32), 256, 0, st, a.part, (int)ctas, a.D, (float*)p->dweight, (float*)p->dbias);
     count_launch(2);
     return check_launch();
 }

@@ -51,6 +51,7 @@ struct LinearArgs {
 template <typename T, bool kBias>
 __global__ void __launch_bounds__(kThreads, 1)
 linear_cf_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const LinearArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* ring = sm + a.w_bytes;                      // W first: [K / 32][Mpad rows][64 B], 64-byte swizzle
@@ -237,7 +238,7 @@ int launch_linear(const ss2d_linear_params* p, cudaStream_t st) {
     a.tiles = (int)((p->N + kTilePx - 1) / kTilePx);
     a.error_flag = dev_flag;
     const int grid = a.tiles < sms ? a.tiles : sms;
-    kern<<<grid, kThreads, kSmemBytes, st>>>(tmX, tmW, a);
+    launch(kern, grid, kThreads, kSmemBytes, st, tmX, tmW, a);
     count_launch();
     return check_launch();
 }

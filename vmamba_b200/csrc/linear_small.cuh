@@ -35,6 +35,7 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool ok) 
 
 template <typename T>
 __global__ void __launch_bounds__(kLsWarps * 32) linear_small_kernel(const LinearSmallArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) unsigned char ls_raw[];
     const int K = a.K, M = a.M, WP = K + 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     T* xs = reinterpret_cast<T*>(ls_raw);                  // [K][72]
@@ -135,7 +136,7 @@ template <typename T> static int launch_linear_small(const ss2d_linear_params* p
     const size_t smem = linear_small_smem(p->K);
     auto kern = linear_small_kernel<T>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
-    kern<<<dim3((unsigned)((p->N + kLsN - 1) / kLsN), (unsigned)((p->M + kLsM - 1) / kLsM)), kLsWarps * 32, smem, st>>>(a);
+    launch(kern, dim3((unsigned)((p->N + kLsN - 1) / kLsN), (unsigned)((p->M + kLsM - 1) / kLsM)), kLsWarps * 32, smem, st, a);
     count_launch();
     return check_launch();
 }

@@ -66,6 +66,7 @@ template <typename T, int C>
 __global__ void __launch_bounds__(kThreads, 1)
 mlp_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW1,
                  const __grid_constant__ CUtensorMap tmW2, const MlpArgs a) {
+    follow_previous();
     using S = MlpSmem<C>;
     constexpr int NCH = S::NCH;
     constexpr int kTmemCols = 512;
@@ -302,7 +303,7 @@ int launch_mlp(const ss2d_mlp_params* p, cudaStream_t st) {
     a.tiles = (int)((N + kTilePx - 1) / kTilePx);
     a.error_flag = dev_flag;
     const int grid = a.tiles < sms ? a.tiles : sms;
-    kern<<<grid, kThreads, smem, st>>>(tmX, tmW1, tmW2, a);
+    launch(kern, grid, kThreads, smem, st, tmX, tmW1, tmW2, a);
     count_launch();
     return check_launch();
 }

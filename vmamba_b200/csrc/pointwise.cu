@@ -25,6 +25,7 @@ struct BiasActArgs {
 // pair of values); the rational erfc form with rcp / ex2 took 25 and left the kernel bound by instruction issue.
 template <typename T, int PV, int ACT>
 __global__ void __launch_bounds__(256) bias_act_kernel(const BiasActArgs a) {
+    follow_previous();
     // x may be y: a store orders every later load behind it, so each pass loads kU vectors first
     constexpr int kU = 4;
     const long long row = blockIdx.x / a.chunks_per_row;
@@ -69,9 +70,9 @@ static void launch_bias_act(BiasActArgs a, int act, cudaStream_t st) {
     while ((long long)chunks * a.rows > (1LL << 30) && chunks > 1) chunks >>= 1;
     a.chunks_per_row = chunks;
     const unsigned g = (unsigned)(a.rows * chunks);
-    if (act == ACT_GELU) bias_act_kernel<T, PV, ACT_GELU><<<g, 256, 0, st>>>(a);
-    else if (act == ACT_SILU) bias_act_kernel<T, PV, ACT_SILU><<<g, 256, 0, st>>>(a);
-    else bias_act_kernel<T, PV, ACT_NONE><<<g, 256, 0, st>>>(a);
+    if (act == ACT_GELU) launch(bias_act_kernel<T, PV, ACT_GELU>, g, 256, 0, st, a);
+    else if (act == ACT_SILU) launch(bias_act_kernel<T, PV, ACT_SILU>, g, 256, 0, st, a);
+    else launch(bias_act_kernel<T, PV, ACT_NONE>, g, 256, 0, st, a);
 }
 
 template <typename T>
@@ -133,6 +134,7 @@ struct DwStripArgs {
 
 template <typename T, int PV, int KR, int ACT>
 __global__ void __launch_bounds__(256, PV == 8 ? 2 : 3) dwconv3x3_strip_kernel(const DwStripArgs a) {
+    follow_previous();
     const int H = a.H, W = a.W;
     const int lane = threadIdx.x & 31;
     const long long gi = (long long)blockIdx.x * 256 + threadIdx.x;
@@ -258,9 +260,9 @@ __global__ void __launch_bounds__(256, PV == 8 ? 2 : 3) dwconv3x3_strip_kernel(c
 
 template <typename T, int PV, int KR>
 static int launch_dw_strip_a(const DwStripArgs& a, int act, unsigned grid, cudaStream_t st) {
-    if (act == ACT_SILU) dwconv3x3_strip_kernel<T, PV, KR, ACT_SILU><<<grid, 256, 0, st>>>(a);
-    else if (act == ACT_GELU) dwconv3x3_strip_kernel<T, PV, KR, ACT_GELU><<<grid, 256, 0, st>>>(a);
-    else dwconv3x3_strip_kernel<T, PV, KR, ACT_NONE><<<grid, 256, 0, st>>>(a);
+    if (act == ACT_SILU) launch(dwconv3x3_strip_kernel<T, PV, KR, ACT_SILU>, grid, 256, 0, st, a);
+    else if (act == ACT_GELU) launch(dwconv3x3_strip_kernel<T, PV, KR, ACT_GELU>, grid, 256, 0, st, a);
+    else launch(dwconv3x3_strip_kernel<T, PV, KR, ACT_NONE>, grid, 256, 0, st, a);
     count_launch();
     return check_launch();
 }

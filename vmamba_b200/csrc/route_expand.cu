@@ -43,6 +43,7 @@ constexpr int kDChunk = 128;   // channels per CTA (grid.z walks the slices)
 
 template <typename T, int VEC, int NI>
 __global__ void __launch_bounds__(kExpThreads) route_expand_kernel(const ExpandArgs a) {
+    follow_previous();
     constexpr int NDG = kExpThreads / NI;   // channel groups working side by side
     constexpr int NP = (VEC + 1) / 2;
     extern __shared__ __align__(16) float sm[];
@@ -167,6 +168,7 @@ template <typename T> __device__ __forceinline__ uint32_t pack2(float x, float y
 
 template <typename T, int KP>
 __global__ void __launch_bounds__(256, 4) route_expand_mma_kernel(const ExpandArgs a) {
+    follow_previous();
     constexpr int PIX = kMmaPix;
     constexpr int KPAD = KP + 8, XPAD = PIX + 8;       // pitches (elements): conflict-free fragment loads and vector stores
     __shared__ __align__(16) T Ws[kDChunk * KPAD];     // [channel][k]
@@ -322,10 +324,10 @@ static int launch_expand_mma(ExpandArgs a, cudaStream_t st) {
     const long long tiles = (long long)a.B * ((tiles_per_run + a.mma_tiles - 1) / a.mma_tiles);
     if (tiles > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
     const dim3 grid((unsigned)tiles, 4, (unsigned)cuts);
-    if (kp == 16) route_expand_mma_kernel<T, 16><<<grid, threads, 0, st>>>(a);
-    else if (kp == 32) route_expand_mma_kernel<T, 32><<<grid, threads, 0, st>>>(a);
-    else if (kp == 48) route_expand_mma_kernel<T, 48><<<grid, threads, 0, st>>>(a);
-    else if (kp == 64) route_expand_mma_kernel<T, 64><<<grid, threads, 0, st>>>(a);
+    if (kp == 16) launch(route_expand_mma_kernel<T, 16>, grid, threads, 0, st, a);
+    else if (kp == 32) launch(route_expand_mma_kernel<T, 32>, grid, threads, 0, st, a);
+    else if (kp == 48) launch(route_expand_mma_kernel<T, 48>, grid, threads, 0, st, a);
+    else if (kp == 64) launch(route_expand_mma_kernel<T, 64>, grid, threads, 0, st, a);
     else return SS2D_ENOTSUP;
     count_launch();
     return check_launch();
@@ -338,7 +340,7 @@ static int launch_expand(const ExpandArgs& a, cudaStream_t st) {
     auto kern = route_expand_kernel<T, VEC, NI>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
     const dim3 grid((unsigned)((a.items_total + NI - 1) / NI), 4, (unsigned)((a.D + kDChunk - 1) / kDChunk));
-    kern<<<grid, kExpThreads, smem, st>>>(a);
+    launch(kern, grid, kExpThreads, smem, st, a);
     count_launch();
     return check_launch();
 }
@@ -373,6 +375,7 @@ struct TransArgs {
 
 template <typename T>
 __global__ void __launch_bounds__(256) plane_transpose_kernel(const TransArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) unsigned char traw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const int P = a.W + 1, psz = a.H * P;
@@ -436,6 +439,7 @@ long long route_expand_workspace_bytes(const ss2d_expand_params* p) {
 // that leaves SMs idle, a CTA (104 planes of 62 x 64: 28 us with warps).
 template <typename T, bool kCta>
 __global__ void __launch_bounds__(256) orient_rows_kernel(const TransArgs a, const int pad) {
+    follow_previous();
     extern __shared__ __align__(16) unsigned char traw[];
     const int step = kCta ? blockDim.x : 32, lane = kCta ? threadIdx.x : threadIdx.x & 31;
     const int warp = kCta ? 0 : threadIdx.x >> 5, nwarps = kCta ? 1 : blockDim.x >> 5;
@@ -479,7 +483,7 @@ static int launch_orient(const ss2d_expand_params* p, cudaStream_t st) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
     long long ctas = (t.planes + warps - 1) / warps;
     if (ctas > 148 * 16) ctas = 148 * 16;
-    kern<<<(unsigned)ctas, cta ? 256 : warps * 32, smem, st>>>(t, (int)p->image_row);
+    launch(kern, (unsigned)ctas, cta ? 256 : warps * 32, smem, st, t, (int)p->image_row);
     count_launch();
     return check_launch();
 }
@@ -502,7 +506,7 @@ static int launch_transpose(const ss2d_expand_params* p, cudaStream_t st) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
     long long ctas = (t.planes + warps - 1) / warps;
     if (ctas > 148 * 16) ctas = 148 * 16;
-    kern<<<(unsigned)ctas, warps * 32, smem, st>>>(t);
+    launch(kern, (unsigned)ctas, warps * 32, smem, st, t);
     count_launch();
     return check_launch();
 }

@@ -91,6 +91,7 @@ __device__ __forceinline__ void softplus_pair(float2 x, float2& sp, float2& dsp)
 // bf16, all gradients: 245 us with pieces; single elements cost 9 %, the choice inside one kernel 4 %.)
 template <typename Tin, typename Tg, int AL, int LPR, int BC>
 __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) float n1_sm[];
     constexpr int G = 32 / LPR, kChunk = LPR * 8, kStep = kN1Warps * G;     // kStep: rows of the CTA that are worked on at a time
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, R = a.R, L = a.L, ln = lane & (LPR - 1), wr = warp * G + lane / LPR;
@@ -281,6 +282,7 @@ __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArg
 // What a segment does to e: a warp per (row, segment), chunks of 256 elements from the segment's end.
 template <typename Tin, typename Tg, int AL, int BC>
 __global__ void __launch_bounds__(kN1Warps * 32) n1_bwd_segments_kernel(const N1BwdArgs a) {
+    follow_previous();
     const int lane = threadIdx.x & 31, L = a.L;
     const int64_t w = (int64_t)blockIdx.x * kN1Warps + (threadIdx.x >> 5);
     const int64_t row = w / (a.S - 1);

@@ -54,6 +54,7 @@ template <int NS> struct StBwdSmem {
 
 template <typename Tin, typename Tg, int NS, int VW>
 __global__ void __launch_bounds__(StLayout<NS>::kWarps * 32, 8 / StLayout<NS>::kWarps) st_bwd_kernel(const StBwdArgs a) {
+    follow_previous();
     using Y = StLayout<NS>;
     using M = StBwdSmem<NS>;
     constexpr int RPW = Y::RPW, SL = Y::SL, P = kStPitch, W = Y::kWarps, kRow = RPW * P;
@@ -376,6 +377,7 @@ __global__ void __launch_bounds__(StLayout<NS>::kWarps * 32, 8 / StLayout<NS>::k
 // What a segment does to the reverse state: its value from zero and the sum of its step sizes.  Segment 0 is read by nobody.
 template <typename Tin, typename Tg, int NS, int VW>
 __global__ void __launch_bounds__(StLayout<NS>::kWarps * 32) st_bwd_segments_kernel(const StBwdArgs a) {
+    follow_previous();
     using Y = StLayout<NS>;
     constexpr int RPW = Y::RPW, SL = Y::SL, P = kStPitch, W = Y::kWarps, kRow = RPW * P;
     extern __shared__ __align__(16) float st_sm[];

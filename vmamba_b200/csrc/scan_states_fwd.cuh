@@ -30,6 +30,7 @@ struct StFwdArgs {
 
 template <typename Tin, typename Tout, int NS, int R_, int VW, bool kOut>
 __global__ void __launch_bounds__(StLayout<NS, R_>::kWarps * 32) st_fwd_kernel(const StFwdArgs a) {
+    follow_previous();
     using Y = StLayout<NS, R_>;
     constexpr int RPW = Y::RPW, SL = Y::SL, R = Y::R, RL = Y::RL, P = kStPitch;
     constexpr int kRow = RPW * P, kBC = kStChunk * Y::BCP;
@@ -233,7 +234,7 @@ static int st_launch_fwd(const StFwdArgs& a, int64_t batch, cudaStream_t st) {
     static_assert(smem <= 48 * 1024, "default shared-memory limit");
     const int64_t ctas = batch * a.n_groups * a.parts * a.S;
     if (ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
-    st_fwd_kernel<Tin, Tout, NS, R, VW, kOut><<<(unsigned)ctas, Y::kWarps * 32, smem, st>>>(a);
+    launch(st_fwd_kernel<Tin, Tout, NS, R, VW, kOut>, (unsigned)ctas, Y::kWarps * 32, smem, st, a);
     count_launch();
     return check_launch();
 }

@@ -42,6 +42,7 @@ constexpr int kWarpsPerCta = 4;
 // fp32 rows of any alignment are held to 128 registers, four CTAs per SM (12 288 rows of 3 137 elements: 170 -> 132 us).
 template <typename Tin, typename Tout, int AL, int W, int LPR>
 __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32, W == 1 && AL == 0 && sizeof(Tin) == 4 ? 4 : 0) selscan_fwd_n1_kernel(const ScanArgs a) {
+    follow_previous();
     static_assert(W == 1 || LPR == 32, "rows of several warps take whole warps");
     constexpr int VEC = 8, WSTEP = LPR * VEC, STEP = W * WSTEP;
     __shared__ AB agg[2][W];
@@ -166,6 +167,7 @@ __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32, W == 1 &&
 // d_state > 1: the carry of each state lives in shared memory (one slot per warp and state).
 template <typename Tin, typename Tout, int VEC>
 __global__ void __launch_bounds__(kWarpsPerCta * 32) selscan_fwd_nx_kernel(const ScanArgs a) {
+    follow_previous();
     __shared__ float carry_s[kWarpsPerCta][SS2D_MAX_DSTATE];
     __shared__ float A2_s[kWarpsPerCta][SS2D_MAX_DSTATE];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -265,12 +267,12 @@ static int launch_n1(const ScanArgs& a, cudaStream_t st) {
     const int64_t per_cta = kWarpsPerCta * (32 / lpr), ctas = w == 1 ? (a.rows + per_cta - 1) / per_cta : a.rows;
     if (ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
     const unsigned g = (unsigned)ctas;
-    if (w == 8) selscan_fwd_n1_kernel<Tin, Tout, AL, 8, 32><<<g, 256, 0, st>>>(a);
-    else if (w == 4) selscan_fwd_n1_kernel<Tin, Tout, AL, 4, 32><<<g, 128, 0, st>>>(a);
-    else if (w == 2) selscan_fwd_n1_kernel<Tin, Tout, AL, 2, 32><<<g, 64, 0, st>>>(a);
-    else if (lpr == 8) selscan_fwd_n1_kernel<Tin, Tout, AL, 1, 8><<<g, kWarpsPerCta * 32, 0, st>>>(a);
-    else if (lpr == 16) selscan_fwd_n1_kernel<Tin, Tout, AL, 1, 16><<<g, kWarpsPerCta * 32, 0, st>>>(a);
-    else selscan_fwd_n1_kernel<Tin, Tout, AL, 1, 32><<<g, kWarpsPerCta * 32, 0, st>>>(a);
+    if (w == 8) launch(selscan_fwd_n1_kernel<Tin, Tout, AL, 8, 32>, g, 256, 0, st, a);
+    else if (w == 4) launch(selscan_fwd_n1_kernel<Tin, Tout, AL, 4, 32>, g, 128, 0, st, a);
+    else if (w == 2) launch(selscan_fwd_n1_kernel<Tin, Tout, AL, 2, 32>, g, 64, 0, st, a);
+    else if (lpr == 8) launch(selscan_fwd_n1_kernel<Tin, Tout, AL, 1, 8>, g, kWarpsPerCta * 32, 0, st, a);
+    else if (lpr == 16) launch(selscan_fwd_n1_kernel<Tin, Tout, AL, 1, 16>, g, kWarpsPerCta * 32, 0, st, a);
+    else launch(selscan_fwd_n1_kernel<Tin, Tout, AL, 1, 32>, g, kWarpsPerCta * 32, 0, st, a);
     count_launch();
     return check_launch();
 }
@@ -279,7 +281,7 @@ template <typename Tin, typename Tout, int VEC>
 static int launch_nx(const ScanArgs& a, cudaStream_t st) {
     const int64_t ctas = (a.rows + kWarpsPerCta - 1) / kWarpsPerCta;
     if (ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
-    selscan_fwd_nx_kernel<Tin, Tout, VEC><<<(unsigned)ctas, kWarpsPerCta * 32, 0, st>>>(a);
+    launch(selscan_fwd_nx_kernel<Tin, Tout, VEC>, (unsigned)ctas, kWarpsPerCta * 32, 0, st, a);
     count_launch();
     return check_launch();
 }

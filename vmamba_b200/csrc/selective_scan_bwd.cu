@@ -51,6 +51,7 @@ struct BwdArgs {
 
 template <typename Tin, typename Tg, int VEC>
 __global__ void __launch_bounds__(256) selscan_bwd_kernel(const BwdArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) float sm[];
     constexpr int STEP = 32 * VEC;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, RW = blockDim.x >> 5;
@@ -242,6 +243,7 @@ __global__ void __launch_bounds__(256) selscan_bwd_kernel(const BwdArgs a) {
 // row's u / delta / dout vectors are fetched before the current row's arithmetic.
 template <typename Tin, typename Tg, int VEC>
 __global__ void __launch_bounds__(256) selscan_bwd_n1_kernel(const BwdArgs a, const int R) {
+    follow_previous();
     extern __shared__ __align__(16) float sm[];
     constexpr int STEP = 32 * VEC;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, RW = blockDim.x >> 5;
@@ -457,6 +459,7 @@ constexpr int kBwdFloatsPerWarp = 4 * kBwdTile * kBwdPitch + 8 * 32 + 2 * kBwdTi
 
 template <typename Tin, typename Tg>
 __global__ void __launch_bounds__(kBwdRowsWarps * 32, 4) selscan_bwd_rows_kernel(const BwdArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) float sm[];
     constexpr int T = kBwdTile, P = kBwdPitch, PE = 4;         // PE: elements per piece (8 bytes of a 16-bit tensor)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -630,6 +633,7 @@ template <int NS> struct BwdRowsN {
 
 template <typename Tin, typename Tg, int NS>
 __global__ void __launch_bounds__(kBwdRowsWarps * 32, 2) selscan_bwd_rows_nx_kernel(const BwdArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) float sm[];
     constexpr int T = kBwdTile, P = kBwdPitch, PE = 4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -848,6 +852,7 @@ template <typename Tin>
 __global__ void selscan_bwd_fold_kernel(const float* rowred, const float* bcpart, float* dA, float* dD, float* dbias,
                                         Tin* dB, Tin* dC, int64_t batch, int64_t images, int64_t dim, int N, int64_t L, int64_t Lp,
                                         int n_groups, int parts, int64_t out_gs) {
+    follow_previous();
     const int64_t n_small = dim * (N + 2);
     const int64_t n_bc = batch * n_groups * N * L;       // per tensor
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_small + 2 * n_bc;
@@ -983,11 +988,11 @@ static int launch_bwd(const BwdArgs& a, const BwdPlan& c, int64_t ctas, cudaStre
     if (a.N == 1) {
         auto kern = selscan_bwd_n1_kernel<Tin, Tg, VEC>;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem) != cudaSuccess) return SS2D_ECUDA;
-        kern<<<(unsigned)ctas, c.rw * 32, c.smem, st>>>(a, c.R);
+        launch(kern, (unsigned)ctas, c.rw * 32, c.smem, st, a, c.R);
     } else {
         auto kern = selscan_bwd_kernel<Tin, Tg, VEC>;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem) != cudaSuccess) return SS2D_ECUDA;
-        kern<<<(unsigned)ctas, c.rw * 32, c.smem, st>>>(a);
+        launch(kern, (unsigned)ctas, c.rw * 32, c.smem, st, a);
     }
     count_launch();
     return check_launch();
@@ -1003,7 +1008,7 @@ static int launch_bwd_rows(const BwdArgs& a, const BwdPlan& c, cudaStream_t st) 
     const int64_t warps = a.rows / 32;
     const int64_t ctas = (warps + kBwdRowsWarps - 1) / kBwdRowsWarps;
     if (ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
-    kern<<<(unsigned)ctas, kBwdRowsWarps * 32, c.smem, st>>>(a);
+    launch(kern, (unsigned)ctas, kBwdRowsWarps * 32, c.smem, st, a);
     count_launch();
     return check_launch();
 }
@@ -1021,7 +1026,7 @@ static int launch_fold(const ss2d_scan_bwd_params* p, const BwdFold& f, cudaStre
     const int64_t total = p->dim * (p->dstate + 2) + 2 * p->batch * p->n_groups * p->dstate * p->seqlen;
     int64_t blocks = (total + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    selscan_bwd_fold_kernel<Tin><<<(unsigned)blocks, 256, 0, st>>>(f.rowred, f.bcpart, (float*)p->dA, (float*)p->dD, (float*)p->ddelta_bias,
+    launch(selscan_bwd_fold_kernel<Tin>, (unsigned)blocks, 256, 0, st, f.rowred, f.bcpart, (float*)p->dA, (float*)p->dD, (float*)p->ddelta_bias,
                                                                    (Tin*)p->dB, (Tin*)p->dC, p->batch, f.images, p->dim, (int)p->dstate,
                                                                    p->seqlen, f.Lp, (int)p->n_groups, f.parts,
                                                                    p->bc_out_group_stride ? p->bc_out_group_stride : p->dstate * p->seqlen);

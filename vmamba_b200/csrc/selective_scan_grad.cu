@@ -121,10 +121,10 @@ static int launch_n1_bwd(const N1BwdArgs& a, cudaStream_t st) {
     const int64_t ctas = a.batch * a.n_groups * a.parts * a.S, seg_ctas = (a.batch * a.dim * (a.S - 1) + kN1Warps - 1) / kN1Warps;
     if (ctas > 0x7fffffffLL || seg_ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
     if (a.S > 1) {
-        n1_bwd_segments_kernel<Tin, Tg, AL, BC><<<(unsigned)seg_ctas, kN1Warps * 32, 0, st>>>(a);
+        launch(n1_bwd_segments_kernel<Tin, Tg, AL, BC>, (unsigned)seg_ctas, kN1Warps * 32, 0, st, a);
         count_launch();
     }
-    kern<<<(unsigned)ctas, kN1Warps * 32, smem, st>>>(a);
+    launch(kern, (unsigned)ctas, kN1Warps * 32, smem, st, a);
     count_launch();
     return check_launch();
 }
@@ -140,10 +140,10 @@ static int launch_st_bwd(const StBwdArgs& a, cudaStream_t st) {
     if (ctas > 0x7fffffffLL || seg_ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
     if (a.S > 1) {
         const size_t s2 = sizeof(float) * (2 * kStRows * kStPitch + kStChunk * Y::BCP);
-        st_bwd_segments_kernel<Tin, Tg, NS, VW><<<(unsigned)seg_ctas, Y::kWarps * 32, s2, st>>>(a);
+        launch(st_bwd_segments_kernel<Tin, Tg, NS, VW>, (unsigned)seg_ctas, Y::kWarps * 32, s2, st, a);
         count_launch();
     }
-    kern<<<(unsigned)ctas, Y::kWarps * 32, smem, st>>>(a);
+    launch(kern, (unsigned)ctas, Y::kWarps * 32, smem, st, a);
     count_launch();
     return check_launch();
 }

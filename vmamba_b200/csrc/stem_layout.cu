@@ -29,6 +29,7 @@ struct StemArgs {
 
 template <typename T, int C0>
 __global__ void __launch_bounds__(128, 4) stem_conv_norm_act_kernel(const StemArgs a) {
+    follow_previous();
     // weights as [tap][channel] fp32 so that one 16-byte broadcast load brings a tap's weights of four channels
     __shared__ __align__(16) float sw[27 * C0];
     __shared__ float sb[3 * C0];
@@ -149,6 +150,7 @@ __global__ void __launch_bounds__(128, 4) stem_conv_norm_act_kernel(const StemAr
 // costs 1.5 per output and what remains is the GELU.
 template <typename T, int C0>
 __global__ void __launch_bounds__(512, 1) stem_mma_kernel(const StemArgs a, int rows_total, int vec_ok) {
+    follow_previous();
     extern __shared__ __align__(16) unsigned char stem_smem[];
     constexpr int NT = C0 / 8;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthreads = blockDim.x;
@@ -314,9 +316,9 @@ static int launch_stem_mma(const StemArgs& a, int C0, cudaStream_t st) {
     const long long rows = (long long)a.B * a.Ho;
     // persistent CTAs, four per SM's worth (224 x 224 images, batch 128: 2 or 4 per SM 164 us, 8: 169, 32: 184)
     const unsigned grid = (unsigned)(rows < 148 * 4 ? rows : 148 * 4);
-    if (C0 == 32) stem_mma_kernel<T, 32><<<grid, threads, smem, st>>>(a, (int)rows, vec_ok);
-    else if (C0 == 48) stem_mma_kernel<T, 48><<<grid, threads, smem, st>>>(a, (int)rows, vec_ok);
-    else stem_mma_kernel<T, 64><<<grid, threads, smem, st>>>(a, (int)rows, vec_ok);
+    if (C0 == 32) launch(stem_mma_kernel<T, 32>, grid, threads, smem, st, a, (int)rows, vec_ok);
+    else if (C0 == 48) launch(stem_mma_kernel<T, 48>, grid, threads, smem, st, a, (int)rows, vec_ok);
+    else launch(stem_mma_kernel<T, 64>, grid, threads, smem, st, a, (int)rows, vec_ok);
     count_launch();
     return check_launch();
 }
@@ -343,7 +345,7 @@ int stem_conv_norm_act(const ss2d_stem_params* p, cudaStream_t st) {
     }
     const long long total = 2LL * a.B * a.Ho * ((a.Wo + 1) / 2);      // two threads per pixel pair
     const unsigned grid = (unsigned)((total + 127) / 128);
-#define SS2D_STEM_CASE(TT, CC) stem_conv_norm_act_kernel<TT, CC><<<grid, 128, 0, st>>>(a)
+#define SS2D_STEM_CASE(TT, CC) launch(stem_conv_norm_act_kernel<TT, CC>, grid, 128, 0, st, a)
 #define SS2D_STEM_T(TT) \
     switch (p->C0) { case 32: SS2D_STEM_CASE(TT, 32); break; case 48: SS2D_STEM_CASE(TT, 48); break; \
                      case 64: SS2D_STEM_CASE(TT, 64); break; default: return SS2D_ENOTSUP; }
@@ -374,6 +376,7 @@ struct RowsArgs {
 
 template <typename Tin, typename Tout, int TP>
 __global__ void __launch_bounds__(256) pixels_norm_to_planes_kernel(const RowsArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) float tile[];                       // [TP][C + 1], then part[256 / TP][TP], scale[TP], shift[TP]
     const long long n0 = (long long)blockIdx.x * TP;
     const int C = a.C, P = C + 1;
@@ -468,7 +471,7 @@ int pixels_norm_to_planes(const ss2d_relayout_params* p, cudaStream_t st) {
     if (ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
 #define SS2D_ROWS_LAUNCH_TP(TI, TO, TPV) { auto kern = pixels_norm_to_planes_kernel<TI, TO, TPV>; \
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA; \
-        kern<<<(unsigned)ctas, 256, smem, st>>>(a); }
+        launch(kern, (unsigned)ctas, 256, smem, st, a); }
 #define SS2D_ROWS_LAUNCH(TI, TO) { if (tp == 32) SS2D_ROWS_LAUNCH_TP(TI, TO, 32) else SS2D_ROWS_LAUNCH_TP(TI, TO, 16) }
     const int ri = p->rows_dtype, po = p->planes_dtype;
     if (ri == SS2D_F32 && po == SS2D_F32) SS2D_ROWS_LAUNCH(float, float)
@@ -499,6 +502,7 @@ struct PlanesArgs {
 
 template <typename T, int TP>
 __global__ void __launch_bounds__(256) planes_to_pixels_kernel(const PlanesArgs a) {
+    follow_previous();
     extern __shared__ __align__(16) float tile[];                       // [TP][C + 1]
     const long long n0 = (long long)blockIdx.x * TP;
     const int C = a.C, P = C + 1;
@@ -607,7 +611,7 @@ int planes_to_pixels(const ss2d_relayout_params* p, cudaStream_t st) {
     if (ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
 #define SS2D_PLANES_LAUNCH_TP(TT, TPV) { auto kern = planes_to_pixels_kernel<TT, TPV>; \
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA; \
-        kern<<<(unsigned)ctas, 256, smem, st>>>(a); }
+        launch(kern, (unsigned)ctas, 256, smem, st, a); }
 #define SS2D_PLANES_LAUNCH(TT) { if (tp == 32) SS2D_PLANES_LAUNCH_TP(TT, 32) else SS2D_PLANES_LAUNCH_TP(TT, 16) }
     if (p->rows_dtype == SS2D_F32) SS2D_PLANES_LAUNCH(float)
     else if (p->rows_dtype == SS2D_BF16) SS2D_PLANES_LAUNCH(__nv_bfloat16)
