@@ -10,9 +10,10 @@
 // Segments: where the rows do not fill the chip they are cut into S segments; a first kernel leaves each segment's
 // effect on e (its value from zero, and the sum of its step sizes), and a segment starts from the fold of those behind it.
 //
-// Bound: latency at three CTAs of four warps per SM (153 to 168 registers).  32 x 384 rows of 3 136 elements, bf16, 150 us: an SM issues
-// in half of its cycles with 2.5 warps per scheduler, 0.7 of them eligible; the arithmetic alone (about 45 instructions per
-// element, four on the MUFU pipe) is 47 us, the bytes 74 us at the copy rate (38 % of the DRAM rate).
+// Bound: latency at three CTAs of four warps per SM (153 to 168 registers).  32 x 384 rows of 3 136 elements, bf16, 138 us (150 with the
+// addresses of every row formed from its number): an SM issues in half of its cycles with 2.5 warps per scheduler, and of a warp's five
+// cycles per instruction 1.4 wait for the one before it, 0.7 for shuffles and exponentials and 0.5 for memory; the bytes are 74 us at the copy
+// rate.  Not faster: four elements per lane and twice the warps (190), rows through shared memory three deep (135; fp32 174 -> 228).
 #pragma once
 #include "scan_row.cuh"
 
@@ -131,22 +132,34 @@ __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArg
     }
     __syncwarp();
 
+    // The rows of a set.  The next one's lie a fixed step behind, but for shared warps (their last set) and shared step sizes.  Stepping saves the
+    // products of row number and stride, but holds ten registers: fp32 vectors (160 -> 163 us at 1 x 1 024 x 16 384) and pieces of 16-bit rows
+    // (243 -> 247 at 32 x 384 x 3 137) are at their limit.
+    constexpr bool kStepped = (AL != 0) == (sizeof(Tin) == 2);
+    struct Rows { const Tin *u, *d; const Tg* g; const float* ck; int64_t out; };
+    auto rows_of = [&](int i) {
+        const int64_t r = (int64_t)k * gs + min(first + i * kStep, gs - 1);
+        return Rows{u + r * a.u_ds, dt + (a.dratio == 1 ? r : r / a.dratio) * a.d_ds, gp + r * a.g_ds, a.ckpt + (out0 + r) * nck, (out0 + r) * L};
+    };
+    auto advance = [&](Rows& w, int i) {
+        if (!kStepped || G > 1 || a.dratio != 1) w = rows_of(i);
+        else { w.u += kStep * a.u_ds; w.d += kStep * a.d_ds; w.g += kStep * a.g_ds; w.ck += kStep * nck; w.out += (int64_t)kStep * L; }
+    };
     Row8<Tin, AL> nu, nd;
     Row8<Tg, AL> ng;
     float nh = 0.f;
-    auto row_of = [&](int i) { return (int64_t)k * gs + min(first + i * kStep, gs - 1); };
-    auto delta_row = [&](int64_t r) { return dt + (a.dratio == 1 ? r : r / a.dratio) * a.d_ds; };
-    auto fetch = [&](int i, int pos) {
-        const int64_t r = row_of(i);
-        nu.load(u + r * a.u_ds, pos, 0, L); nd.load(delta_row(r), pos, 0, L); ng.load(gp + r * a.g_ds, pos, 0, L);
-        nh = pos < L ? __ldg(a.ckpt + (out0 + r) * nck + (pos >> 3)) : 0.f;
+    auto fetch = [&](const Rows& w, int pos) {
+        nu.load(w.u, pos, 0, L); nd.load(w.d, pos, 0, L); ng.load(w.g, pos, 0, L);
+        nh = pos < L ? __ldg(w.ck + (pos >> 3)) : 0.f;
     };
     int buf = 0;
     const int first_w = first - lane / LPR, mine = first_w < gs ? min(R, (gs - first_w + kStep - 1) / kStep) : 0;     // row sets of this warp
+    const Rows row0 = rows_of(0);
     for (int c = (hi - 1) / kChunk; c * kChunk >= lo; --c, buf ^= 1) {
         const int pos = c * kChunk + ln * 8;
         float2 bv[4], cv[4], accB[4], accC[4];
-        if (mine) fetch(0, pos);
+        Rows row = row0;
+        if (mine) fetch(row, pos);
         {
             Row8<Tin, BC> rb, rc;
             rb.load(Bm, pos, 0, L); rc.load(Cm, pos, 0, L);
@@ -156,11 +169,11 @@ __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArg
         for (int i = 0; i < 4; ++i) accB[i] = accC[i] = pk(0.f);
 #pragma unroll 1
         for (int i = 0; i < mine; ++i) {
-            const int64_t r = row_of(i);
             float2 uv[4], d[4], g[4];
-            row8_pairs(nu, u + r * a.u_ds, pos, L, uv); row8_pairs(nd, delta_row(r), pos, L, d); row8_pairs(ng, gp + r * a.g_ds, pos, L, g);
+            row8_pairs(nu, row.u, pos, L, uv); row8_pairs(nd, row.d, pos, L, d); row8_pairs(ng, row.g, pos, L, g);
             float h = nh;
-            if (i + 1 < mine) fetch(i + 1, pos);
+            const int64_t out = row.out;
+            if (i + 1 < mine) { advance(row, i + 1); fetch(row, pos); }
             const float4 pr = par[i * kStep + wr];
             const float An = pr.x;
             const bool real = G == 1 || first + i * kStep < gs;   // spare lanes repeat the last row and take part in nothing
@@ -231,8 +244,8 @@ __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArg
             }
             float* q = racc + (i * kN1Warps + warp) * 96 + lane;
             q[0] += dA.x + dA.y; q[32] += dD.x + dD.y; q[64] += db.x + db.y;
-            row8_store<Tin, AL, LPR>((Tin*)a.du + (out0 + r) * L, pos, real ? L : 0, duo, stage, lane);
-            row8_store<Tin, AL, LPR>((Tin*)a.ddelta + (out0 + r) * L, pos, real ? L : 0, ddo, stage, lane);
+            row8_store<Tin, AL, LPR>((Tin*)a.du + out, pos, real ? L : 0, duo, stage, lane);
+            row8_store<Tin, AL, LPR>((Tin*)a.ddelta + out, pos, real ? L : 0, ddo, stage, lane);
         }
         if constexpr (G > 1) {                                   // the rows that share the warp
 #pragma unroll
@@ -273,7 +286,7 @@ __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArg
             for (int off = LPR / 2; off > 0; off >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], off);
         }
         if (ln == 0 && first + i * kStep < gs) {
-            float* rr = a.rowred + (((int64_t)seg * a.batch + b) * a.dim + row_of(i)) * 3;
+            float* rr = a.rowred + (((int64_t)seg * a.batch + b) * a.dim + (int64_t)k * gs + first + i * kStep) * 3;
             rr[0] = v[0]; rr[1] = v[1]; rr[2] = v[2];
         }
     }
