@@ -200,12 +200,14 @@ template <typename T, int NS, int WARPS> struct StRawBC<T, NS, 0, WARPS> {
 
 // Number of segments a row is cut into (1: none) and their length, given the warps that whole rows fill.  Cutting costs a
 // second pass, so it starts below four warps per SM and then goes up to sixteen (16 states, bf16: 768 rows of 3 136
-// elements 116 -> 49 us, 384 rows of 65 536 4.4 -> 0.33 ms; 6 144 rows, which fill five warps, 0.25 uncut, 0.28 cut).
+// elements 116 -> 49 us, 384 rows of 65 536 4.4 -> 0.29 ms; 6 144 rows, which fill five warps, 0.25 uncut, 0.28 cut).
+// `resident`: sixteen is what the SM holds, and more would be a second round (rows of vectors: 3 072 rows of 3 136, 16 states, fp32, 206 us with
+// seven segments, 188 with six); where it holds more, the number is rounded up (4 608 rows of 8 594, 4 states, bf16, 308 against 318).
 struct StSegments { int count, len; };
-inline StSegments st_segments(int64_t warps, int64_t L) {
+inline StSegments st_segments(int64_t warps, int64_t L, bool resident) {
     const int64_t want = 148 * 16;
     if (warps * 4 > want || L < 192) return {1, (int)((L + 63) / 64 * 64)};
-    int64_t s = (want + warps - 1) / warps;
+    int64_t s = (resident ? want : want + warps - 1) / warps;
     const int64_t most = (L + 63) / 64;
     if (s > most) s = most;
     const int64_t len = (((L + s - 1) / s) + 63) / 64 * 64;

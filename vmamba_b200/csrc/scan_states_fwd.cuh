@@ -2,11 +2,14 @@
 //   kOut          the result, and the states in front of every `every`-th element where the backward pass wants them;
 //   !kOut         no result: the end states of every segment (the first of the two passes over rows cut into segments), or
 //                 the states in front of every `every`-th element alone (a backward call without the forward's).
-// Bound: the write-back of the shared-memory reads (scan_states.cuh, R) and the warps in flight.  16 x 768 rows of 3 136 elements, 16
-// states, bf16, 311 us: shared memory at 80 % of its rate, issue 42 % with 2.6 warps per scheduler (384 CTAs on 740 places);
-// the exponentials, one per (element, state), are 132 us, DRAM is at 11 %.  Per (element, state) a lane issues about 4.5
-// instructions: half of a packed multiply each for dl * A and du * B, half of a packed fma each for the state and the
-// result, the exponential, and its share of the three shared-memory reads and of the sum over the lanes of a row.
+// Bound: latency with 2.6 warps per scheduler (384 CTAs on 592 places), then the write-back of the shared-memory reads (scan_states.cuh, R).
+// 16 x 768 rows of 3 136 elements, 16 states, bf16, 294 us; of a warp's six cycles per instruction 1.5 wait for shared memory and
+// exponentials and 1.4 for the instruction in front.  B and C of a group of elements are therefore read while the group in front is
+// worked on, which the compiler undoes unless it may use the registers that so few warps leave (312 -> 294 us, fp32 385 -> 339; packing
+// 16-bit B and C, which halves their reads but unpacks them, 306).  The exponentials, one per (element, state), are 132 us, DRAM is at 11 %.
+// Per (element, state) a lane issues about 7 instructions: half of a packed multiply each for dl * A and du * B, half of a packed fma
+// each for the state and the result, the exponential, and its share of the shared-memory reads, of the sum over the lanes of a
+// row and of the staging.
 #pragma once
 #include "scan_states.cuh"
 
@@ -28,13 +31,16 @@ struct StFwdArgs {
     int every;               // a multiple of 32
 };
 
+// Registers for sixteen warps an SM; twelve with two rows per lane (49 152 rows, 16 states, fp32 1 142 against 1 062 us); pieces (VW 0) as the compiler
+// likes (4 608 rows of 8 594, 4 states, 438 us with sixteen, 308).
 template <typename Tin, typename Tout, int NS, int R_, int VW, bool kOut>
-__global__ void __launch_bounds__(StLayout<NS, R_>::kWarps * 32) st_fwd_kernel(const StFwdArgs a) {
+__global__ void __launch_bounds__(StLayout<NS, R_>::kWarps * 32, VW == 0 ? 0 : (R_ == 2 ? 12 : 16) / StLayout<NS, R_>::kWarps) st_fwd_kernel(const StFwdArgs a) {
     follow_previous();
     using Y = StLayout<NS, R_>;
     constexpr int RPW = Y::RPW, SL = Y::SL, R = Y::R, RL = Y::RL, P = kStPitch;
     constexpr int kRow = RPW * P, kBC = kStChunk * Y::BCP;
     using Raw = StRaw<Tin, RPW, VW>;
+    constexpr bool kAhead = R == 1;                  // B and C of a group, too, are read in front of it
     constexpr bool kPre = sizeof(Raw) <= (VW == 0 ? 128 : 64);         // the next chunk is fetched into registers while this one is worked on
     extern __shared__ __align__(16) float st_sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rl = lane / SL, sl = lane % SL, n0 = sl * 4;
@@ -132,8 +138,15 @@ __global__ void __launch_bounds__(StLayout<NS, R_>::kWarps * 32) st_fwd_kernel(c
         const float* sC = sB + kBC;
         // A group's decays are formed while the group in front of it is worked on: the exponentials (one per eight
         // cycles and scheduler) then run beside the other arithmetic of the same warp.
-        struct Group { float2 dec[R][4][2], x[R][2]; float y[R][4]; } grp[2];
+        struct Group { float2 dec[R][4][2], x[R][2]; float y[R][4]; float4 b[kAhead ? 4 : 1], c[kAhead ? 4 : 1]; } grp[2];
         auto prepare = [&](int t, Group& g) {
+            if constexpr (kAhead) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    g.b[e] = *reinterpret_cast<const float4*>(sB + (t + e) * Y::BCP);
+                    if constexpr (kOut) g.c[e] = *reinterpret_cast<const float4*>(sC + (t + e) * Y::BCP);
+                }
+            }
 #pragma unroll
             for (int j = 0; j < R; ++j) {
                 const float4 d4 = *reinterpret_cast<const float4*>(sd + (rl + j * RL) * P + t);
@@ -163,11 +176,11 @@ __global__ void __launch_bounds__(StLayout<NS, R_>::kWarps * 32) st_fwd_kernel(c
             if (t + 4 < kStChunk) prepare(t + 4, grp[((t >> 2) & 1) ^ 1]);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const float4 b4 = *reinterpret_cast<const float4*>(sB + (t + e) * Y::BCP);
+                const float4 b4 = kAhead ? g.b[kAhead ? e : 0] : *reinterpret_cast<const float4*>(sB + (t + e) * Y::BCP);
                 const float2 bb[2] = {make_float2(b4.x, b4.y), make_float2(b4.z, b4.w)};
                 float2 cc[2];
                 if constexpr (kOut) {
-                    const float4 c4 = *reinterpret_cast<const float4*>(sC + (t + e) * Y::BCP);
+                    const float4 c4 = kAhead ? g.c[kAhead ? e : 0] : *reinterpret_cast<const float4*>(sC + (t + e) * Y::BCP);
                     cc[0] = make_float2(c4.x, c4.y); cc[1] = make_float2(c4.z, c4.w);
                 }
 #pragma unroll
@@ -176,8 +189,8 @@ __global__ void __launch_bounds__(StLayout<NS, R_>::kWarps * 32) st_fwd_kernel(c
 #pragma unroll
                     for (int q = 0; q < 2; ++q) h[j][q] = __ffma2_rn(dec[j][e][q], h[j][q], __fmul2_rn(f2(xe), bb[q]));
                     if constexpr (kOut) {
-                        const float2 s = __ffma2_rn(cc[1], h[j][1], __fmul2_rn(cc[0], h[j][0]));
-                        y[j][e] += s.x + s.y;
+                        const float2 s = __ffma2_rn(cc[1], h[j][1], __ffma2_rn(cc[0], h[j][0], make_float2(y[j][e], 0.f)));
+                        y[j][e] = s.x + s.y;
                     }
                 }
             }

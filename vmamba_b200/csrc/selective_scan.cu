@@ -355,7 +355,7 @@ static int fwd_vec(const ss2d_scan_params* p) {
 // How the rows of a 2 .. 16 state problem are cut: segments, and the floats of their end states and sums.
 static StSegments fwd_segments(const ss2d_scan_params* p, int64_t& floats) {
     const int NS = st_pad_states(p->dstate), parts = st_parts(p->dim / p->n_groups);
-    const StSegments s = st_segments(p->batch * p->n_groups * parts * (NS / 4), p->seqlen);
+    const StSegments s = st_segments(p->batch * p->n_groups * parts * (NS / 4), p->seqlen, fwd_vec(p) >= 4);
     floats = s.count > 1 ? p->batch * p->dim * s.count * (NS + 1) : 0;
     return s;
 }
