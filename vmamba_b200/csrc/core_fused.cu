@@ -21,6 +21,7 @@
 // by all channels of an image and stay in L1/L2.  They are read in the activation type (the type
 // the projection produced them in): every thread re-reads them for every plane, and with 16-bit
 // elements a warp's load is one contiguous 512-byte run instead of two half-used 1 KB runs.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -41,11 +42,13 @@ struct CoreArgs {
     long long d_bs[4], d_cs[4], bc_bs[4];
     long long x_bs, x_cs;
     int B, D, H, W, L, G, PP, Wp, groups_per_image;
+    int back;                             // warps that a plane reaches back from the one that holds its last segment
+    int same_rows;                        // the four step sizes have one channel stride
     unsigned magic_G, magic_W, magic_H;   // ceil(2^32 / d): n / d == umulhi(n, magic) for n * d < 2^32
 };
 
 struct ScanScratch {
-    AB wtot[4][32];          // [2 * stream + direction][warp]
+    AB wtot[2][4][32];       // [orientation][2 * stream + direction][warp]
     float wpre[4][32];
 };
 
@@ -53,43 +56,59 @@ __device__ __forceinline__ int fast_div(int n, unsigned magic) { return magic ? 
 
 // CTA-wide scan of per-thread aggregates in thread order (forward) and in reverse thread order
 // (backward), for NS independent streams at once (a thread may hold segments of NS planes: the streams
-// share the two barriers).  The state before the first thread is zero, so only the state entering each
+// share the barrier).  The state before the first thread is zero, so only the state entering each
 // thread is needed: hin_f for the forward route, hin_b for the backward route.
+// A warp scans its lanes and leaves its totals; behind the barrier it folds those of the `back` warps in front of it (behind it), which
+// are all that a plane with a thread in this warp can reach.  Where those are more than four, one warp scans the totals, and a second
+// barrier passes its result on.
 template <int NS>
-__device__ __forceinline__ void cta_scan_pair(const AB (&f)[NS], const AB (&bk)[NS], int lane, int warp, int nwarps,
-                                              ScanScratch& s, float (&hin_f)[NS], float (&hin_b)[NS]) {
+__device__ __forceinline__ void cta_scan_pair(const AB (&f)[NS], const AB (&bk)[NS], int lane, int warp, int nwarps, int back,
+                                              AB (&tot)[4][32], float (&pre)[4][32], float (&hin_f)[NS], float (&hin_b)[NS]) {
     AB inc_f[NS], inc_b[NS];
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
-        inc_f[q] = warp_scan_inclusive(f[q], lane);
-        inc_b[q] = warp_scan_inclusive_rev(bk[q], lane);
-        if (lane == 31) s.wtot[2 * q][warp] = inc_f[q];
-        if (lane == 0) s.wtot[2 * q + 1][warp] = inc_b[q];
+        inc_f[q] = f[q]; inc_b[q] = bk[q];
+        scan_step_up<1>(inc_f[q].a, inc_f[q].b); scan_step_down<1>(inc_b[q].a, inc_b[q].b);
+        scan_step_up<2>(inc_f[q].a, inc_f[q].b); scan_step_down<2>(inc_b[q].a, inc_b[q].b);
+        scan_step_up<4>(inc_f[q].a, inc_f[q].b); scan_step_down<4>(inc_b[q].a, inc_b[q].b);
+        scan_step_up<8>(inc_f[q].a, inc_f[q].b); scan_step_down<8>(inc_b[q].a, inc_b[q].b);
+        scan_step_up<16>(inc_f[q].a, inc_f[q].b); scan_step_down<16>(inc_b[q].a, inc_b[q].b);
+        if (lane == 31) tot[2 * q][warp] = inc_f[q];
+        if (lane == 0) tot[2 * q + 1][warp] = inc_b[q];
     }
     __syncthreads();
-    for (int job = warp; job < 2 * NS; job += nwarps) {         // one warp per (stream, direction)
-        const AB t = (lane < nwarps) ? s.wtot[job][lane] : AB{1.f, 0.f};
-        if ((job & 1) == 0) {
-            const AB sc = warp_scan_inclusive(t, lane);
-            float e = __shfl_up_sync(0xffffffffu, sc.b, 1);
-            if (lane == 0) e = 0.f;
-            s.wpre[job][lane] = e;
-        } else {
-            const AB sc = warp_scan_inclusive_rev(t, lane);
-            float e = __shfl_down_sync(0xffffffffu, sc.b, 1);
-            if (lane == 31) e = 0.f;
-            s.wpre[job][lane] = e;
+    float hf[NS], hb[NS];
+#pragma unroll
+    for (int q = 0; q < NS; ++q) hf[q] = hb[q] = 0.f;
+    if (back > 4) {
+        for (int job = warp; job < 2 * NS; job += nwarps) {      // one warp per (stream, direction)
+            AB t = lane < nwarps ? tot[job][lane] : AB{1.f, 0.f};
+            if ((job & 1) == 0) {
+                t = warp_scan_inclusive(t, lane);
+                pre[job][lane] = entering_state<false>(t.b, 0.f);
+            } else {
+                t = warp_scan_inclusive_rev(t, lane);
+                pre[job][lane] = entering_state<true>(t.b, 0.f);
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < NS; ++q) { hf[q] = pre[2 * q][warp]; hb[q] = pre[2 * q + 1][warp]; }
+        back = 0;
+    }
+#pragma unroll 1
+    for (int j = back; j > 0; --j) {                 // the farthest first
+#pragma unroll
+        for (int q = 0; q < NS; ++q) {
+            const AB x = tot[2 * q][max(warp - j, 0)], y = tot[2 * q + 1][min(warp + j, nwarps - 1)];
+            if (warp >= j) hf[q] = fmaf(x.a, hf[q], x.b);
+            if (warp + j < nwarps) hb[q] = fmaf(y.a, hb[q], y.b);
         }
     }
-    __syncthreads();
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
-        float ea = __shfl_up_sync(0xffffffffu, inc_f[q].a, 1), eb = __shfl_up_sync(0xffffffffu, inc_f[q].b, 1);
-        if (lane == 0) { ea = 1.f; eb = 0.f; }
-        hin_f[q] = fmaf(ea, s.wpre[2 * q][warp], eb);
-        float ra = __shfl_down_sync(0xffffffffu, inc_b[q].a, 1), rb = __shfl_down_sync(0xffffffffu, inc_b[q].b, 1);
-        if (lane == 31) { ra = 1.f; rb = 0.f; }
-        hin_b[q] = fmaf(ra, s.wpre[2 * q + 1][warp], rb);
+        hin_f[q] = entering_state<false>(fmaf(inc_f[q].a, hf[q], inc_f[q].b), hf[q]);
+        hin_b[q] = entering_state<true>(fmaf(inc_b[q].a, hb[q], inc_b[q].b), hb[q]);
     }
 }
 
@@ -251,10 +270,13 @@ __global__ void __launch_bounds__(MAXT, MINB) core_plane_kernel(const CoreArgs a
 #pragma unroll
     for (int s = 0; s < NPL; ++s) {
         rx[s] = VT::load_raw((const T*)a.x + b * a.x_bs + d[s] * a.x_cs + e0);
-        rd0[s] = VT::load_raw((const T*)a.delta[0] + b * a.d_bs[0] + d[s] * a.d_cs[0] + e0);
-        rd2[s] = VT::load_raw((const T*)a.delta[2] + b * a.d_bs[2] + d[s] * a.d_cs[2] + e0);
-        rd1[s] = VT::load_raw((const T*)a.delta[1] + b * a.d_bs[1] + d[s] * a.d_cs[1] + e0);
-        rd3[s] = VT::load_raw((const T*)a.delta[3] + b * a.d_bs[3] + d[s] * a.d_cs[3] + e0);
+        const long long o0 = d[s] * a.d_cs[0] + e0;
+        long long o1 = o0, o2 = o0, o3 = o0;
+        if (!a.same_rows) { o1 = d[s] * a.d_cs[1] + e0; o2 = d[s] * a.d_cs[2] + e0; o3 = d[s] * a.d_cs[3] + e0; }
+        rd0[s] = VT::load_raw((const T*)a.delta[0] + b * a.d_bs[0] + o0);
+        rd2[s] = VT::load_raw((const T*)a.delta[2] + b * a.d_bs[2] + o2);
+        rd1[s] = VT::load_raw((const T*)a.delta[1] + b * a.d_bs[1] + o1);
+        rd3[s] = VT::load_raw((const T*)a.delta[3] + b * a.d_bs[3] + o3);
     }
     float2 ul[NPL][NP], yrow[NPL][NP];
 
@@ -304,7 +326,7 @@ __global__ void __launch_bounds__(MAXT, MINB) core_plane_kernel(const CoreArgs a
             if (!active[s]) { af[s] = AB{1.f, 0.f}; ab[s] = AB{1.f, 0.f}; }
         }
         float hf[NPL], hb[NPL];
-        cta_scan_pair<NPL>(af, ab, lane, warp, nwarps, scr, hf, hb);   // its barriers also order the x stores before the reads below
+        cta_scan_pair<NPL>(af, ab, lane, warp, nwarps, a.back, scr.wtot[0], scr.wpre, hf, hb);   // its barrier also orders the x stores before the reads below
 #pragma unroll
         for (int s = 0; s < NPL; ++s) {
             if (first) hf[s] = 0.f;
@@ -351,7 +373,7 @@ __global__ void __launch_bounds__(MAXT, MINB) core_plane_kernel(const CoreArgs a
             if (!active[s]) { af[s] = AB{1.f, 0.f}; ab[s] = AB{1.f, 0.f}; }
         }
         float hf[NPL], hb[NPL];
-        cta_scan_pair<NPL>(af, ab, lane, warp, nwarps, scr, hf, hb);   // every x value has been read before these barriers
+        cta_scan_pair<NPL>(af, ab, lane, warp, nwarps, a.back, scr.wtot[1], scr.wpre, hf, hb);   // every x value has been read before this barrier
 #pragma unroll
         for (int s = 0; s < NPL; ++s) {
             if (first) hf[s] = 0.f;
@@ -677,6 +699,9 @@ static int run_planes(const ss2d_core_params* p, const PlaneConfig& c, float* me
     auto magic = [](long long d) { return (unsigned)(((1ULL << 32) + (unsigned long long)d - 1) / (unsigned long long)d); };
     a.magic_G = c.G > 1 ? magic(c.G) : 0; a.magic_W = p->W > 1 ? magic(p->W) : 0; a.magic_H = p->H > 1 ? magic(p->H) : 0;
     a.groups_per_image = (int)((p->D + c.PP - 1) / c.PP);
+    a.back = std::min((c.G + 30) / 32, c.threads / 32 - 1);
+    a.same_rows = p->delta_channel_stride[0] == p->delta_channel_stride[1] && p->delta_channel_stride[0] == p->delta_channel_stride[2] &&
+                  p->delta_channel_stride[0] == p->delta_channel_stride[3];
     const long long grid = (long long)p->B * a.groups_per_image;
     if (grid > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
     if (p->act_dtype == SS2D_F32) return launch_core_v<float>(a, c, (unsigned)grid, st);
