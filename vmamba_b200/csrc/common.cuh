@@ -153,6 +153,18 @@ __device__ __forceinline__ float softplus_fast(float x) {
     return (x > 20.0f) ? x : sp;
 }
 
+// the same of a pair, bit for bit: half the multiplications and additions issued
+__device__ __forceinline__ float2 splat2(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 softplus_fast2(float2 x) {
+    const float2 t = __fmul2_rn(x, splat2(kLog2e));
+    const float2 e = make_float2(ex2_approx(t.x), ex2_approx(t.y));
+    const float2 series = __fmul2_rn(e, __ffma2_rn(e, __ffma2_rn(e, splat2(0.33333334f), splat2(-0.5f)), splat2(1.0f)));
+    const float2 w = __fadd2_rn(e, splat2(1.0f));
+    const float2 full = __fmul2_rn(make_float2(lg2_approx(w.x), lg2_approx(w.y)), splat2(kLn2));
+    const float2 s = make_float2(e.x < 0.015625f ? series.x : full.x, e.y < 0.015625f ? series.y : full.y);
+    return make_float2(x.x > 20.0f ? x.x : s.x, x.y > 20.0f ? x.y : s.y);
+}
+
 // softplus(x) and its derivative sigmoid(x) = e^x / (1 + e^x) from one exponential (threshold 20 as torch:
 // above it softplus is x and the derivative 1)
 __device__ __forceinline__ void softplus_and_grad(float x, float& sp, float& dsp) {

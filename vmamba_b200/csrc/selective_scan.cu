@@ -31,8 +31,9 @@ constexpr int kWarpsPerCta = 4;
 // per lane, and scans its lanes' (a, b) pairs by shuffle; with several warps per row their totals meet in shared memory
 // (one barrier per step) and every warp folds the ones in front of it.  How many: n1_warps.  The next step's vectors are
 // fetched in front of this one's arithmetic.
-// Bound, 1 024 rows of 16 385 elements (four warps each, 51 us, 20 % of the DRAM rate): instruction issue, 72 % of the slots of an SM
-// that has work, and 1 024 CTAs on the 740 places that 91 registers leave, so that the second wave is a third full.
+// Bound, 1 024 rows of 16 385 elements (four warps each, 46 us, 20 % of the DRAM rate): instruction issue, 72 % of the slots of an SM
+// that has work, and 1 024 CTAs on the 740 places that 91 registers leave, so that the second wave is a third full.  32 x 384 rows of
+// 3 136 with the states kept, 66 us: issue (79 %) and HBM (330 MB, 50 us at the copy rate).  Arithmetic in pairs, 50 and 70 us before.
 // AL is the vector width of every access (8 or 4 elements), or 0 for rows of any alignment: a row is then walked from
 // the 16-byte boundary in front of its result, so that the results leave as vectors, and the inputs are cut out of the
 // aligned pieces around them.  Elements of the tensors' first and last rows whose pieces would reach beyond a tensor (at most
@@ -44,6 +45,8 @@ template <typename Tin, typename Tout, int AL, int W, int LPR>
 __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32, W == 1 && AL == 0 && sizeof(Tin) == 4 ? 4 : 0) selscan_fwd_n1_kernel(const ScanArgs a) {
     follow_previous();
     static_assert(W == 1 || LPR == 32, "rows of several warps take whole warps");
+    // elementwise arithmetic in pairs; fp32 pieces are at their 128 registers and would spill (12 288 rows of 3 137 elements 124 -> 136 us).
+    constexpr bool kPacked = !(AL == 0 && sizeof(Tin) == 4);
     constexpr int VEC = 8, WSTEP = LPR * VEC, STEP = W * WSTEP;
     __shared__ AB agg[2][W];
     const int lane = threadIdx.x & (LPR - 1), wi = W == 1 ? 0 : threadIdx.x >> 5;
@@ -93,16 +96,35 @@ __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32, W == 1 &&
         ru.get(u, pos, l0, l1, uv); rd.get(dt, pos, l0, l1, dv); rb.get(Bm, pos, l0, l1, bv); rc.get(Cm, pos, l0, l1, cv);
         fetch(pos + STEP);
         float p = 1.f, h = 0.f;
+        if constexpr (!kPacked) {
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) {
-            float dl = dv[i] + bias;
-            if (sp) dl = softplus_fast(dl);
-            // outside the row: a step of zero leaves the state as it is (whole vectors are tested once below)
-            if constexpr (AL != 8) dl = pos + (AL ? i / (AL ? AL : 1) * AL : i) < l1 && (AL || pos + i >= l0) ? dl : 0.f;
-            const float aa = decay_fast(dl, A2);
-            h = fmaf(aa, h, dl * bv[i] * uv[i]);
-            p *= aa;
-            P[i] = p; hl[i] = h;
+            for (int i = 0; i < VEC; ++i) {
+                float dl = dv[i] + bias;
+                if (sp) dl = softplus_fast(dl);
+                dl = pos + i < l1 && pos + i >= l0 ? dl : 0.f;
+                const float aa = decay_fast(dl, A2);
+                h = fmaf(aa, h, dl * bv[i] * uv[i]);
+                p *= aa;
+                P[i] = p; hl[i] = h;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < VEC; i += 2) {
+                float2 dl = __fadd2_rn(make_float2(dv[i], dv[i + 1]), splat2(bias));
+                if (sp) dl = softplus_fast2(dl);
+                // outside the row: a step of zero leaves the state as it is (whole vectors are tested once below)
+                if constexpr (AL != 8) {
+                    dl.x = pos + (AL ? i / (AL ? AL : 1) * AL : i) < l1 && (AL || pos + i >= l0) ? dl.x : 0.f;
+                    dl.y = pos + (AL ? (i + 1) / (AL ? AL : 1) * AL : i + 1) < l1 && (AL || pos + i + 1 >= l0) ? dl.y : 0.f;
+                }
+                const float2 t = __fmul2_rn(dl, splat2(A2));
+                const float2 aa = make_float2(ex2_approx(t.x), ex2_approx(t.y));
+                const float2 x = __fmul2_rn(__fmul2_rn(dl, make_float2(bv[i], bv[i + 1])), make_float2(uv[i], uv[i + 1]));
+                h = fmaf(aa.x, h, x.x); p *= aa.x;
+                P[i] = p; hl[i] = h;
+                h = fmaf(aa.y, h, x.y); p *= aa.y;
+                P[i + 1] = p; hl[i + 1] = h;
+            }
         }
         float ia = p, ib = h;
         if constexpr (AL == 8) { const bool in = pos < L; ia = in ? p : 1.f; ib = in ? h : 0.f; }
@@ -141,8 +163,18 @@ __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32, W == 1 &&
         }
         if (!a.states_only && real) {
             float ov[VEC];
+            if constexpr (!kPacked) {
 #pragma unroll
-            for (int i = 0; i < VEC; ++i) ov[i] = fmaf(Dv, uv[i], cv[i] * fmaf(P[i], hin, hl[i]));
+                for (int i = 0; i < VEC; ++i) ov[i] = fmaf(Dv, uv[i], cv[i] * fmaf(P[i], hin, hl[i]));
+            } else {
+#pragma unroll
+                for (int i = 0; i < VEC; i += 2) {
+                    const float2 y = __ffma2_rn(splat2(Dv), make_float2(uv[i], uv[i + 1]),
+                                                __fmul2_rn(make_float2(cv[i], cv[i + 1]),
+                                                           __ffma2_rn(make_float2(P[i], P[i + 1]), splat2(hin), make_float2(hl[i], hl[i + 1]))));
+                    ov[i] = y.x; ov[i + 1] = y.y;
+                }
+            }
             constexpr int SV = AL && AL < OV ? AL : OV;          // elements per store
 #pragma unroll
             for (int j = 0; j < VEC; j += SV) {
