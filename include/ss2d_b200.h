@@ -371,6 +371,29 @@ typedef struct ss2d_linear_params {
 int ss2d_linear_supported(const ss2d_linear_params *p);
 int ss2d_linear_fwd(const ss2d_linear_params *p, void *cuda_stream);
 
+/* --------------------------------------------------------------------------------
+ * Sums of products of rows:  out (groups, M, N) fp32 = sum over o, l of a (outer, groups, M, L) . b (outer, groups, N, L), the weight
+ * gradients of the core's projections (autograd of F.conv1d / einsum, vmamba.py:1536-1538, 1542-1543).
+ *   a, b   dtype (SS2D_BF16 or SS2D_F16), 16-byte aligned, every stride (elements) and L a multiple of 8, N <= 64
+ *   turned 1: out is (groups, N, M)
+ * Returns SS2D_ENOTSUP for what it does not take; ss2d_row_products_workspace_bytes returns -1 for those.
+ * -------------------------------------------------------------------------------- */
+typedef struct ss2d_row_products_params {
+    const void *a;
+    const void *b;
+    void *out;
+    void *workspace;
+    int64_t workspace_bytes;
+    int64_t outer, groups, M, N, L;
+    int64_t a_outer_stride, a_group_stride, a_row_stride;
+    int64_t b_outer_stride, b_group_stride, b_row_stride;
+    int32_t dtype;
+    int32_t turned;
+} ss2d_row_products_params;
+
+int64_t ss2d_row_products_workspace_bytes(const ss2d_row_products_params *p);
+int ss2d_row_products(const ss2d_row_products_params *p, void *cuda_stream);
+
 /* Debug checks (off by default; on with the environment variable SS2D_DEBUG_CHECKS=1 at load time or by this call).
  * When on, every entry point that launches kernels first asks the driver about each pointer it was given
  * (cudaPointerGetAttributes) and returns SS2D_EINVAL_DEVICE, before any launch, for host memory or memory of a GPU

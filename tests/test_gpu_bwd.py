@@ -338,3 +338,32 @@ def test_scan_gradients_of_the_c_interface_by_default(vb, Bt, K, Cd, N, L, dt, c
     assert _lib.lib().ss2d_selective_scan_bwd(p, torch.cuda.current_stream().cuda_stream) == _lib.SS2D_OK
     for (name, x), r in zip(out.items(), O.selective_scan_bwd(u, delta, A, B, C, D, bias, dout, True, dt)):
         assert O.max_rel_err(host(x), r) <= TOL[dt], name
+
+
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("outer,groups,M,N,L,turned", [(1, 1, 1, 1, 8, 0), (2, 4, 96, 6, 3136, 0), (3, 4, 40, 13, 1000, 1), (1, 1, 17, 64, 72, 0), (5, 1, 192, 56, 784, 1),
+                                                       (1, 4, 130, 8, 40000, 0), (2, 3, 31, 33, 264, 1), (1, 2, 300, 24, 56, 0)])
+def test_row_products(vb, outer, groups, M, N, L, turned, dt):
+    """The weight gradients' sums of row products, on rows that are parts of larger ones: edges of the blocks of rows, of the vectors and of the parts.
+    A sum is one of at most L / 16 and some forty partial ones, each rounded to fp32 (2^-22 covers the tensor core's truncation)."""
+    from vmamba_b200 import _lib
+    td = {"bf16": torch.bfloat16, "f16": torch.float16}[dt]
+    g = torch.Generator(device="cuda").manual_seed(M * N + L)
+    a = torch.randn(outer, groups, M + 2, L + 16, device="cuda", generator=g).to(td)[:, :, 1:M + 1, 8:L + 8]
+    b = torch.randn(outer, groups, N + 1, L + 8, device="cuda", generator=g).to(td)[:, :, :N, :L]
+    out = torch.full((groups, N, M) if turned else (groups, M, N), float("nan"), device="cuda")
+    p = _lib.RowProductsParams(a=a.data_ptr(), b=b.data_ptr(), out=out.data_ptr(), outer=outer, groups=groups, M=M, N=N, L=L,
+                               a_outer_stride=a.stride(0), a_group_stride=a.stride(1), a_row_stride=a.stride(2),
+                               b_outer_stride=b.stride(0), b_group_stride=b.stride(1), b_row_stride=b.stride(2),
+                               dtype={"bf16": _lib.SS2D_BF16, "f16": _lib.SS2D_F16}[dt], turned=turned)
+    need = _lib.lib().ss2d_row_products_workspace_bytes(p)
+    assert need > 0
+    ws = torch.empty(need, device="cuda", dtype=torch.uint8)
+    p.workspace, p.workspace_bytes = ws.data_ptr(), need
+    assert _lib.lib().ss2d_row_products(p, torch.cuda.current_stream().cuda_stream) == _lib.SS2D_OK
+    x, y = a.double(), b.double()
+    want, size = (x @ y.transpose(2, 3)).sum(0), (x.abs() @ y.abs().transpose(2, 3)).sum(0)
+    got = out.transpose(1, 2) if turned else out
+    assert ((got.double() - want).abs() <= (L / 16 + 48) * 2.0 ** -22 * size).all()
+    p.N = 65
+    assert _lib.lib().ss2d_row_products_workspace_bytes(p) == -1

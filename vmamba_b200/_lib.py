@@ -116,6 +116,12 @@ class LinearParams(ctypes.Structure):
                [(n, _i64) for n in ("M", "K", "N", "x_row_stride", "out_row_stride")] + [("dtype", _i32), ("act", _i32)]
 
 
+class RowProductsParams(ctypes.Structure):
+    _fields_ = [(n, _vp) for n in ("a", "b", "out", "workspace")] + \
+               [(n, _i64) for n in ("workspace_bytes", "outer", "groups", "M", "N", "L", "a_outer_stride", "a_group_stride", "a_row_stride",
+                                    "b_outer_stride", "b_group_stride", "b_row_stride")] + [("dtype", _i32), ("turned", _i32)]
+
+
 EXPORTS = {
     # name: (restype, argtypes)
     "ss2d_selective_scan_fwd": (ctypes.c_int, [ctypes.POINTER(ScanParams), _vp]),
@@ -129,6 +135,8 @@ EXPORTS = {
     "ss2d_cross_padding_supported": (ctypes.c_int, [ctypes.POINTER(CrossParams)]),
     "ss2d_layer_norm_cf_bwd": (ctypes.c_int, [ctypes.POINTER(NormBwdParams), _vp]),
     "ss2d_layer_norm_cf_bwd_workspace_bytes": (_i64, [ctypes.POINTER(NormBwdParams)]),
+    "ss2d_row_products": (ctypes.c_int, [ctypes.POINTER(RowProductsParams), _vp]),
+    "ss2d_row_products_workspace_bytes": (_i64, [ctypes.POINTER(RowProductsParams)]),
     "ss2d_cross_scan_ex": (ctypes.c_int, [ctypes.POINTER(CrossExParams), _vp]),
     "ss2d_cross_merge_ex": (ctypes.c_int, [ctypes.POINTER(CrossExParams), _vp]),
     "ss2d_core_workspace_bytes": (_i64, [ctypes.POINTER(CoreParams)]),

@@ -19,6 +19,8 @@ int cross_rows(const ss2d_cross_params* p, int back, cudaStream_t st);
 int cross_padding_supported(const ss2d_cross_params* p);
 long long layer_norm_cf_bwd_workspace_bytes(const ss2d_norm_bwd_params* p);
 int layer_norm_cf_bwd(const ss2d_norm_bwd_params* p, cudaStream_t st);
+long long row_products_workspace_bytes(const ss2d_row_products_params* p);
+int row_products(const ss2d_row_products_params* p, cudaStream_t st);
 int cross_scan_ex(const ss2d_cross_ex_params* p, cudaStream_t st);
 int cross_merge_ex(const ss2d_cross_ex_params* p, cudaStream_t st);
 int layer_norm_cf(const ss2d_norm_params* p, cudaStream_t st);
@@ -114,6 +116,12 @@ int ss2d_layer_norm_cf_bwd(const ss2d_norm_bwd_params* p, void* stream) {
     ss2d::Range nvtx_("ss2d_layer_norm_cf_bwd");
     if (p) SS2D_CHECK_PTRS(p->y, p->g, p->weight, p->dy, p->dweight, p->dbias, p->workspace);
     return ss2d::layer_norm_cf_bwd(p, (cudaStream_t)stream);
+}
+int64_t ss2d_row_products_workspace_bytes(const ss2d_row_products_params* p) { return ss2d::row_products_workspace_bytes(p); }
+int ss2d_row_products(const ss2d_row_products_params* p, void* stream) {
+    ss2d::Range nvtx_("ss2d_row_products");
+    if (p) SS2D_CHECK_PTRS(p->a, p->b, p->out, p->workspace);
+    return ss2d::row_products(p, (cudaStream_t)stream);
 }
 int ss2d_cross_scan_ex(const ss2d_cross_ex_params* p, void* stream) {
     ss2d::Range nvtx_("ss2d_cross_scan_ex");

@@ -36,8 +36,24 @@ static Tensor per_image(const Tensor& w, int64_t B) {
     return w.unsqueeze(0).expand({B, 4, w.size(1), w.size(2)}).reshape({B * 4, w.size(1), w.size(2)});
 }
 
-// sum over the images of a . b^T (rows of equal length): per-image products accumulated and summed in fp32
+// sum over the images of a . b^T (rows of equal length), in fp32; a, b: (images * groups, rows, elements)
 static Tensor row_products(const Tensor& a, const Tensor& b, int64_t groups) {
+    const bool turned = b.size(1) > a.size(1);                        // the shorter one is the kernel's b
+    const Tensor &x = turned ? b : a, &y = turned ? a : b;
+    if (a.scalar_type() != at::kFloat && x.stride(2) == 1 && y.stride(2) == 1) {
+        ss2d_row_products_params p = {};
+        p.a = x.data_ptr(); p.b = y.data_ptr(); p.dtype = dtype_code(a); p.turned = turned;
+        p.outer = a.size(0) / groups; p.groups = groups; p.M = x.size(1); p.N = y.size(1); p.L = a.size(2);
+        p.a_outer_stride = groups * x.stride(0); p.a_group_stride = x.stride(0); p.a_row_stride = x.stride(1);
+        p.b_outer_stride = groups * y.stride(0); p.b_group_stride = y.stride(0); p.b_row_stride = y.stride(1);
+        const int64_t need = ss2d_row_products_workspace_bytes(&p);
+        if (need > 0 && (uintptr_t)p.a % 16 == 0 && (uintptr_t)p.b % 16 == 0) {
+            Tensor out = at::empty({groups, a.size(1), b.size(1)}, a.options().dtype(at::kFloat)), ws = bytes(need, a);
+            p.out = out.data_ptr(); p.workspace = ws.data_ptr(); p.workspace_bytes = need;
+            check(ss2d_row_products(&p, stream_of(a)), "ss2d_row_products");
+            return out;
+        }
+    }
     const Tensor bt = b.transpose(1, 2);
     const Tensor p = a.scalar_type() == at::kFloat ? at::bmm(a, bt) : at::bmm(a, bt, at::kFloat);
     return p.view({-1, groups, p.size(1), p.size(2)}).sum(0);
