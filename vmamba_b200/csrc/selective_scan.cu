@@ -384,10 +384,19 @@ static int fwd_vec(const ss2d_scan_params* p) {
                         p->C_state_stride, ptr_el(p->u, si), ptr_el(p->delta, si), ptr_el(p->B, si), ptr_el(p->C, si), ptr_el(p->out, so)}, 8);
 }
 
+// Vector width of the 2 .. 16 state kernels: 8, 4, 1, or 0 for pieces (st_dispatch_fwd).
+static int states_vw(const ss2d_scan_params* p) {
+    const int v = fwd_vec(p);
+    if (v >= 4) return v >= 8 ? 8 : 4;
+    const ScanSpans s = scan_spans(*p, dtype_size(p->in_dtype));
+    const bool pieces = whole_pieces(s.u) && whole_pieces(s.delta) && whole_pieces(s.B) && whole_pieces(s.C);
+    return pieces && (dtype_size(p->in_dtype) == 2 || st_pad_states(p->dstate) == 4) ? 0 : 1;
+}
+
 // How the rows of a 2 .. 16 state problem are cut: segments, and the floats of their end states and sums.
 static StSegments fwd_segments(const ss2d_scan_params* p, int64_t& floats) {
     const int NS = st_pad_states(p->dstate), parts = st_parts(p->dim / p->n_groups);
-    const StSegments s = st_segments(p->batch * p->n_groups * parts * (NS / 4), p->seqlen, fwd_vec(p) >= 4);
+    const StSegments s = st_segments(p->batch * p->n_groups * parts * (NS / 4), p->seqlen, states_vw(p) != 0);
     floats = s.count > 1 ? p->batch * p->dim * s.count * (NS + 1) : 0;
     return s;
 }
@@ -438,10 +447,7 @@ static int selective_scan_states(const ss2d_scan_params* p, cudaStream_t st) {
     a.S = s.count; a.seg_len = s.len;
     a.ends = floats ? (float*)p->workspace : nullptr;
     a.sums = floats ? a.ends + p->batch * p->dim * s.count * st_pad_states(p->dstate) : nullptr;
-    // 0: no vectors, but pieces (16-byte boundaries at the tensors' ends)
-    const ScanSpans s4 = scan_spans(*p, dtype_size(p->in_dtype));
-    const bool pieces = whole_pieces(s4.u) && whole_pieces(s4.delta) && whole_pieces(s4.B) && whole_pieces(s4.C);
-    const int v = fwd_vec(p), vw = v >= 8 ? 8 : v >= 4 ? 4 : pieces ? 0 : 1;
+    const int vw = states_vw(p);
     const bool of32 = p->out_dtype == SS2D_F32;
     if (p->in_dtype == SS2D_F32) return states_fwd<float, float>(a, p, vw, st);
     if (p->in_dtype == SS2D_BF16) return of32 ? states_fwd<__nv_bfloat16, float>(a, p, vw, st) : states_fwd<__nv_bfloat16, __nv_bfloat16>(a, p, vw, st);
