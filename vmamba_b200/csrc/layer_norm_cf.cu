@@ -100,6 +100,20 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
         for (int i = 0; i < PV; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], 16);
     };
 
+    // Weight and bias are read behind the statistics.  A grid of few CTAs has nothing else to do meanwhile and brings them into L1 (one captured
+    // image, with the shorter vectors of few pixels, 786 -> 764 us; with many CTAs the requests are in the way: 128 images 5 737 -> 6 410).
+    if constexpr (CACHE > 0) {
+        if (gridDim.x <= 32) {
+#pragma unroll
+            for (int c0 = 0; c0 < CACHE; c0 += TX) {
+                const int d = ty + (c0 + tx) * NTY;
+                if (c0 + tx < CACHE && d < D) {
+                    if (MODE || a.w) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.w + d));
+                    if (MODE || a.b) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.b + d));
+                }
+            }
+        }
+    }
     float cache[CACHE > 0 ? CACHE : 1][PV];
     float s[PV];
 #pragma unroll
@@ -266,6 +280,7 @@ static void launch_norm(NormArgs a, int pv, long long B, cudaStream_t st) {
     // (more threads per CTA: keep about 64 registers per thread so that several CTAs share an SM)
     if (D > 32 * 32) pv = 1;
     else if (D > 16 * 12 && pv > 2) pv = 2;
+    while (pv > 1 && B * (a.L / pv) < 74 * kItemsPerCta) pv /= 2;      // few pixels: shorter vectors on more SMs
     a.nv = a.L / pv;
     a.items = (int)(B * a.nv);
     // widths that are 16 per channel slice (128, 256, 512: the VMamba-B dims) get exact shapes of their own,
