@@ -462,6 +462,49 @@ def test_fused_core_detection_map_sizes(vb, shape, dtype):
     assert O.max_rel_err(host(y), ref) <= (TOL_F32 if dtype == "f32" else TOL_BF16)
 
 
+def test_core_plane_kernel_adds_in_one_order(vb):
+    """Planes whose threads span up to four warps: the totals of the warps are added as a scan over them adds (in pairs, then pairs of pairs), whichever
+    of the two forms of the kernel passes them on.  Steps of one element (decay 1, C = 1) leave sums alone, which are followed here term by term."""
+    from vmamba_b200 import fused
+    H = W = 28
+    L, V = H * W, 8
+    rng = np.random.default_rng(28)
+    f = np.float32
+    x = rng.standard_normal((1, 1, H, W), dtype=f)
+    delta = rng.uniform(21, 40, (4, L)).astype(f)                # above 20 the softplus is the identity
+
+    def entering(h):                                             # what enters every thread, given what each of them adds; the walk goes up
+        lanes = np.zeros(-(-len(h) // 32) * 32, f)
+        lanes[:len(h)] = h
+        lanes = lanes.reshape(-1, 32)
+        for off in (1, 2, 4, 8, 16):
+            lanes[:, off:] = lanes[:, off:] + lanes[:, :-off]
+        tot = [f(0)] * 4 + list(lanes[:, 31])
+        pre = np.array([(tot[w + 3] + tot[w + 2]) + (tot[w + 1] + tot[w]) for w in range(len(lanes))], f)
+        return np.concatenate([pre[:, None], pre[:, None] + lanes[:, :-1]], 1).reshape(-1)[:len(h)]
+
+    def orientation(u, up, down):                                # both routes over one order of the pixels
+        ul = (u * f(0.6931471805599453)).astype(f)
+        add = [((d * f(1.4426950408889634)) * ul).reshape(-1, V) for d in (up, down)]
+        fwd, bwd = np.zeros_like(add[0]), np.zeros_like(add[1])
+        for i in range(V):
+            fwd[:, i] = add[0][:, i] + (fwd[:, i - 1] if i else f(0))
+            bwd[:, V - 1 - i] = add[1][:, V - 1 - i] + (bwd[:, V - i] if i else f(0))
+        # the lanes behind the last thread add nothing: the walk down may start at that thread's warp end
+        pad = -(-len(bwd) // 32) * 32
+        back = entering(np.concatenate([bwd[:, 0], np.zeros(pad - len(bwd), f)])[::-1])[::-1][:len(bwd)]
+        return (entering(fwd[:, -1])[:, None] + (back[:, None] + (bwd + fwd))).reshape(-1)
+
+    row = orientation(x.reshape(-1), delta[0], delta[2]).reshape(H, W)
+    col = orientation(x[0, 0].T.reshape(-1), delta[1], delta[3]).reshape(W, H).T
+    zero = dev(np.zeros((4, 1), f))
+    w = vb.CoreWeights(dev(np.zeros((12, 1), f)), dev(np.zeros((4, 1, 1), f)), zero, zero.view(-1), zero.view(-1), None, None, 1, 1, 1)
+    ones = dev(np.ones((1, 2, 2, L), f))
+    proj = fused.RouteStreams(ones, ones, dev(delta[[0, 2]][None, :, None]), dev(delta[[1, 3]][None, :, None]))
+    got = fused.scan_merge_norm(dev(x), proj, w, with_norm=False)
+    assert np.array_equal(host(got)[0, 0], row + col)
+
+
 @pytest.mark.parametrize("shape", [(1, 16, 56, 56), (1, 8, 14, 14)])
 def test_fused_core_extreme_step_sizes(vb, shape):
     """delta + bias from -40 to +60: softplus in its two tails.  The 16-bit fast path computes log2(1 + 2^x') with the

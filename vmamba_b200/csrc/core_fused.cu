@@ -11,7 +11,7 @@
 // planes of one image side by side (PP*G threads).  Per orientation the forward route and the
 // backward route are evaluated on the same registers: each thread runs the recurrence over its
 // VEC elements in both directions, the thread aggregates (a, b) are combined by one CTA-wide
-// scan per direction (warp shuffle scan, then a scan of the warp totals), plane boundaries being
+// scan per direction (warp shuffle scan, then a fold of the totals of the warps that a plane spans), plane boundaries being
 // expressed as a = 0 on the first (last) thread of a plane.  The column-major orientation needs
 // x transposed and gives its result transposed: both go through a padded fp32 plane in shared
 // memory, which is also where the four routes are summed.  No atomics; output is the merged fp32
@@ -60,7 +60,8 @@ __device__ __forceinline__ int fast_div(int n, unsigned magic) { return magic ? 
 // thread is needed: hin_f for the forward route, hin_b for the backward route.
 // A warp scans its lanes and leaves its totals; behind the barrier it folds those of the `back` warps in front of it (behind it), which
 // are all that a plane with a thread in this warp can reach.  Where those are more than four, one warp scans the totals, and a second
-// barrier passes its result on.
+// barrier passes its result on.  Up to four are folded in pairs, which is the order in which that scan adds them: the state that enters a
+// thread does not depend on the path.
 template <int NS>
 __device__ __forceinline__ void cta_scan_pair(const AB (&f)[NS], const AB (&bk)[NS], int lane, int warp, int nwarps, int back,
                                               AB (&tot)[4][32], float (&pre)[4][32], float (&hin_f)[NS], float (&hin_b)[NS]) {
@@ -78,8 +79,6 @@ __device__ __forceinline__ void cta_scan_pair(const AB (&f)[NS], const AB (&bk)[
     }
     __syncthreads();
     float hf[NS], hb[NS];
-#pragma unroll
-    for (int q = 0; q < NS; ++q) hf[q] = hb[q] = 0.f;
     if (back > 4) {
         for (int job = warp; job < 2 * NS; job += nwarps) {      // one warp per (stream, direction)
             AB t = lane < nwarps ? tot[job][lane] : AB{1.f, 0.f};
@@ -94,15 +93,20 @@ __device__ __forceinline__ void cta_scan_pair(const AB (&f)[NS], const AB (&bk)[
         __syncthreads();
 #pragma unroll
         for (int q = 0; q < NS; ++q) { hf[q] = pre[2 * q][warp]; hb[q] = pre[2 * q + 1][warp]; }
-        back = 0;
-    }
-#pragma unroll 1
-    for (int j = back; j > 0; --j) {                 // the farthest first
+    } else {
 #pragma unroll
         for (int q = 0; q < NS; ++q) {
-            const AB x = tot[2 * q][max(warp - j, 0)], y = tot[2 * q + 1][min(warp + j, nwarps - 1)];
-            if (warp >= j) hf[q] = fmaf(x.a, hf[q], x.b);
-            if (warp + j < nwarps) hb[q] = fmaf(y.a, hb[q], y.b);
+            // of the j-th warp in front of this one (behind it); none is the identity
+            const auto f_of = [&](int j) { return warp >= j ? tot[2 * q][warp - j] : AB{1.f, 0.f}; };
+            const auto b_of = [&](int j) { return warp + j < nwarps ? tot[2 * q + 1][warp + j] : AB{1.f, 0.f}; };
+            AB x = f_of(1), y = b_of(1);
+            if (back > 1) { x = combine(f_of(2), x); y = combine(b_of(2), y); }
+            hf[q] = x.b; hb[q] = y.b;
+            if (back > 2) {
+                AB u = f_of(3), v = b_of(3);
+                if (back > 3) { u = combine(f_of(4), u); v = combine(b_of(4), v); }
+                hf[q] = fmaf(x.a, u.b, x.b); hb[q] = fmaf(y.a, v.b, y.b);
+            }
         }
     }
 #pragma unroll
