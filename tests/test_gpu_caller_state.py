@@ -196,3 +196,29 @@ def test_a_captured_graph_keeps_its_weights(vb):
         assert not torch.equal(m(x), first)              # the model's own object is made anew, and the old one let go
         junk = [torch.full_like(t, float("nan")) for stage in m.blocks for b in stage for t in (b.w_in, b.w_dw, b.w_out, b.w1, b.w2)]
         assert torch.equal(runner(x), first) and len(junk) == 20
+
+
+def test_threads_with_planes_of_other_sizes(vb):
+    """The limit of a kernel's shared memory belongs to all threads: calls on planes of 51 KB and of 71 KB of routes, which take the same kernel, in two
+    threads at once."""
+    import threading
+
+    from vmamba_b200 import _lib
+    done = {}
+
+    def calls(H, W):
+        stream = torch.cuda.Stream()
+        ys = torch.randn(1, 4, 8, H, W, device="cuda")
+        out = torch.empty(1, 8, H, W, device="cuda")
+        torch.cuda.synchronize()
+        p = _lib.CrossParams(in_=ys.data_ptr(), out=out.data_ptr(), dtype=_lib.SS2D_F32, scans=1, B=1, C=8, H=H, W=W)
+        done[H, W] = {_lib.lib().ss2d_cross_merge(p, stream.cuda_stream) for _ in range(4000)}
+        stream.synchronize()
+        done[H, W].add(torch.equal(out, ((ys[:, 0] + ys[:, 1]) + ys[:, 2]) + ys[:, 3]))
+
+    threads = [threading.Thread(target=calls, args=(56, 57 + 14 * i)) for i in (0, 1, 0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert done == {(56, 57): {_lib.SS2D_OK, True}, (56, 71): {_lib.SS2D_OK, True}}

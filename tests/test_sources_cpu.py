@@ -14,3 +14,9 @@ def test_dynamic_shared_memory_declares_its_alignment():
             assert re.search(r"__align__\((16|32|64|128|1024)\)", line), (os.path.basename(path), line)
             found += 1
     assert found > 10
+
+
+def test_limits_of_shared_memory_only_grow():
+    """They belong to a kernel and all threads that launch it: one function sets them, under a lock."""
+    sets = {os.path.basename(p): open(p).read().count("cudaFuncSetAttribute(") for p in glob.glob(os.path.join(CSRC, "*")) if os.path.isfile(p)}
+    assert {p: n for p, n in sets.items() if n} == {"api.cu": 1}

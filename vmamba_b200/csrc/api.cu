@@ -2,6 +2,9 @@
 #include <atomic>
 #include <cstdlib>
 #include <initializer_list>
+#include <map>
+#include <mutex>
+#include <utility>
 
 #include <nvtx3/nvToolsExt.h>
 
@@ -73,6 +76,24 @@ struct Range {
 
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 int check_launch() { return cudaPeekAtLastError() == cudaSuccess ? SS2D_OK : SS2D_ECUDA; }
+
+// A launch that needs less than another thread's never takes that thread's limit away between its two calls.
+int allow_dynamic_smem(const void* kern, size_t bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, size_t> allowed;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return SS2D_ECUDA;
+    std::lock_guard<std::mutex> lock(mu);
+    try {
+        size_t& now = allowed[{kern, dev}];
+        if (now >= bytes) return SS2D_OK;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return SS2D_ECUDA;
+        now = bytes;
+    } catch (...) {                                  // no memory for the entry
+        return SS2D_ECUDA;
+    }
+    return SS2D_OK;
+}
 }  // namespace ss2d
 
 extern "C" {

@@ -297,4 +297,9 @@ inline bool aligned_to(const void* p, size_t a) { return (reinterpret_cast<uintp
 void count_launch(int n = 1);
 int check_launch();   // cudaPeekAtLastError -> SS2D_OK / SS2D_ECUDA
 
+// Lets launches of a kernel on the current device have `bytes` of dynamic shared memory: SS2D_OK or SS2D_ECUDA.  The limit belongs to
+// the kernel and all threads that launch it, so it only ever grows (api.cu).
+int allow_dynamic_smem(const void* kern, size_t bytes);
+template <typename... P> inline int allow_dynamic_smem(void (*kern)(P...), size_t bytes) { return allow_dynamic_smem((const void*)kern, bytes); }
+
 }  // namespace ss2d

@@ -404,28 +404,6 @@ __global__ void __launch_bounds__(MAXT, MINB) core_plane_kernel(const CoreArgs a
     }
 }
 
-
-// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per (kernel, device): the attribute only ever has to grow.
-static cudaError_t ensure_dynamic_smem(const void* kern, size_t bytes) {
-    struct Entry { const void* kern; int dev; size_t bytes; };
-    static std::mutex mu;
-    static std::vector<Entry> seen;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lock(mu);
-    for (Entry& en : seen)
-        if (en.kern == kern && en.dev == dev) {
-            if (en.bytes >= bytes) return cudaSuccess;
-            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-            if (e == cudaSuccess) en.bytes = bytes;
-            return e;
-        }
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) seen.push_back(Entry{kern, dev, bytes});
-    return e;
-}
-
 struct PlaneConfig { int vec, G, PP, threads, Wp, npl; size_t smem; };
 
 static bool plan_planes(const ss2d_core_params* p, PlaneConfig& c) {
@@ -477,16 +455,13 @@ static bool plan_planes(const ss2d_core_params* p, PlaneConfig& c) {
 
 template <typename T, int VEC, int NPL>
 static int launch_core_n(const CoreArgs& a, const PlaneConfig& c, unsigned grid, cudaStream_t st) {
-    cudaError_t e;
     if (c.threads <= 448) {           // 72 registers per thread at two CTAs per SM
         auto kern = core_plane_kernel<T, VEC, NPL, 448, 2>;
-        e = ensure_dynamic_smem((const void*)kern, c.smem);
-        if (e != cudaSuccess) return SS2D_ECUDA;
+        if (const int rc = allow_dynamic_smem(kern, c.smem)) return rc;
         launch(kern, grid, c.threads, c.smem, st, a);
     } else {
         auto kern = core_plane_kernel<T, VEC, NPL, 1024, 1>;
-        e = ensure_dynamic_smem((const void*)kern, c.smem);
-        if (e != cudaSuccess) return SS2D_ECUDA;
+        if (const int rc = allow_dynamic_smem(kern, c.smem)) return rc;
         launch(kern, grid, c.threads, c.smem, st, a);
     }
     count_launch();
@@ -569,7 +544,7 @@ static bool plan_padded(const ss2d_core_params* p, RoutePlan& r) {
 template <typename T, int S, int SV, int MINB, int kRoll>
 static int launch_routes_k(const RouteArgs& a, const RoutePlan& r, unsigned grid, cudaStream_t st) {
     auto kern = core_route_kernel<T, S, SV, MINB, kRoll>;
-    if (ensure_dynamic_smem((const void*)kern, r.smem) != cudaSuccess) return SS2D_ECUDA;
+    if (const int rc = allow_dynamic_smem(kern, r.smem)) return rc;
     launch(kern, grid, 128, r.smem, st, a);
     count_launch();
     return check_launch();
@@ -584,7 +559,7 @@ static int launch_routes_t(const RouteArgs& a, const RoutePlan& r, unsigned grid
 template <typename T, int MINB>
 static int launch_pad(const RouteArgs& a, const RoutePlan& r, unsigned grid, cudaStream_t st) {
     auto kern = core_route_pad_kernel<T, 8, MINB>;
-    if (ensure_dynamic_smem((const void*)kern, r.smem) != cudaSuccess) return SS2D_ECUDA;
+    if (const int rc = allow_dynamic_smem(kern, r.smem)) return rc;
     launch(kern, grid, 128, r.smem, st, a);
     count_launch();
     return check_launch();

@@ -162,19 +162,16 @@ static bool plan_runs(const ss2d_cross_params* p, long long images, int copies, 
     threads = PP * L > 4096 ? 512 : PP * L > 1024 ? 256 : 128;
     return true;
 }
-template <typename K> static int run_attr(K k, size_t smem) {
-    return smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ? SS2D_ECUDA : SS2D_OK;
-}
 template <typename T, int SCANS, int V, bool kPad> static int launch_scan_runs(const RunArgs& a, int64_t B, int threads, size_t smem, cudaStream_t st) {
     auto k = cross_scan_runs_kernel<T, SCANS, V, kPad>;
-    if (const int rc = run_attr(k, smem)) return rc;
+    if (const int rc = allow_dynamic_smem(k, smem)) return rc;
     launch(k, (unsigned)(B * a.blocks), threads, smem, st, a);
     count_launch();
     return check_launch();
 }
 template <typename T, int SCANS, int V> static int launch_merge_runs(const RunArgs& a, int64_t B, int threads, size_t smem, cudaStream_t st) {
     auto k = cross_merge_runs_kernel<T, SCANS, V>;
-    if (const int rc = run_attr(k, smem)) return rc;
+    if (const int rc = allow_dynamic_smem(k, smem)) return rc;
     launch(k, (unsigned)(B * a.blocks), threads, smem, st, a);
     count_launch();
     return check_launch();
@@ -233,7 +230,7 @@ static int launch_rows(const ss2d_cross_params* p, bool back, cudaStream_t st) {
     if (!padding_fits(p, dtype_size(p->dtype), 1) || !plan_runs(p, p->B * 4, 1, kRunMost, a, threads, smem)) return SS2D_ENOTSUP;
     if (!aligned_to(p->in, 8) || !aligned_to(p->out, 8) || (a.S != a.L && a.S % 8 != 0)) return SS2D_EINVAL_ALIGN;
     const unsigned grid = (unsigned)(p->B * 4 * a.blocks);
-    const int rc = p->dtype == SS2D_F32 ? run_attr(cross_rows_kernel<float>, smem) : run_attr(cross_rows_kernel<uint16_t>, smem);
+    const int rc = p->dtype == SS2D_F32 ? allow_dynamic_smem(cross_rows_kernel<float>, smem) : allow_dynamic_smem(cross_rows_kernel<uint16_t>, smem);
     if (rc) return rc;
     if (p->dtype == SS2D_F32) launch(cross_rows_kernel<float>, grid, threads, smem, st, a, p->scans, back);
     else launch(cross_rows_kernel<uint16_t>, grid, threads, smem, st, a, p->scans, back);

@@ -221,15 +221,10 @@ int launch_linear(const ss2d_linear_params* p, cudaStream_t st) {
     if (*host_flag) return SS2D_ECUDA;                     // an earlier launch on this device gave up on a wait
     int* dev_flag = nullptr;
     if (cudaHostGetDevicePointer((void**)&dev_flag, host_flag, 0) != cudaSuccess) return SS2D_ECUDA;
-    static bool attr_ok[64][2] = {};
+    auto kern = p->bias ? linear_cf_kernel<T, true> : linear_cf_kernel<T, false>;
+    if (const int rc = allow_dynamic_smem(kern, kSmemBytes)) return rc;
     int dev = 0;
     cudaGetDevice(&dev);
-    const int hb = p->bias ? 1 : 0;
-    auto kern = hb ? linear_cf_kernel<T, true> : linear_cf_kernel<T, false>;
-    if (!attr_ok[dev & 63][hb]) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess) return SS2D_ECUDA;
-        attr_ok[dev & 63][hb] = true;
-    }
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return SS2D_ECUDA;
     a.bias = (const float*)p->bias; a.out = p->out; a.N = p->N;

@@ -135,7 +135,7 @@ template <typename T> static int launch_linear_small(const ss2d_linear_params* p
                          p->out_row_stride ? p->out_row_stride : p->N};
     const size_t smem = linear_small_smem(p->K);
     auto kern = linear_small_kernel<T>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
+    if (const int rc = allow_dynamic_smem(kern, smem)) return rc;
     launch(kern, dim3((unsigned)((p->N + kLsN - 1) / kLsN), (unsigned)((p->M + kLsM - 1) / kLsM)), kLsWarps * 32, smem, st, a);
     count_launch();
     return check_launch();

@@ -289,13 +289,9 @@ int launch_mlp(const ss2d_mlp_params* p, cudaStream_t st) {
     if (cudaHostGetDevicePointer((void**)&dev_flag, host_flag, 0) != cudaSuccess) return SS2D_ECUDA;
     auto kern = mlp_fused_kernel<T, C>;
     constexpr int smem = S::kTotal + 1024;
-    static bool attr_ok[64] = {};
+    if (const int rc = allow_dynamic_smem(kern, smem)) return rc;
     int dev = 0;
     cudaGetDevice(&dev);
-    if (!attr_ok[dev & 63]) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return SS2D_ECUDA;
-        attr_ok[dev & 63] = true;
-    }
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return SS2D_ECUDA;
     MlpArgs a;

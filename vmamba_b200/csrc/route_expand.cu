@@ -338,7 +338,7 @@ static int launch_expand(const ExpandArgs& a, cudaStream_t st) {
     const size_t smem = ((size_t)a.C * NI * VEC + (size_t)a.R * kDChunk) * sizeof(float);
     if (smem > 200 * 1024) return SS2D_ENOTSUP;
     auto kern = route_expand_kernel<T, VEC, NI>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
+    if (const int rc = allow_dynamic_smem(kern, smem)) return rc;
     const dim3 grid((unsigned)((a.items_total + NI - 1) / NI), 4, (unsigned)((a.D + kDChunk - 1) / kDChunk));
     launch(kern, grid, kExpThreads, smem, st, a);
     count_launch();
@@ -480,7 +480,7 @@ static int launch_orient(const ss2d_expand_params* p, cudaStream_t st) {
     warps = warps < 1 ? 1 : warps > 8 ? 8 : warps;
     auto kern = cta ? orient_rows_kernel<T, true> : orient_rows_kernel<T, false>;
     const size_t smem = plane_bytes * warps;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
+    if (const int rc = allow_dynamic_smem(kern, smem)) return rc;
     long long ctas = (t.planes + warps - 1) / warps;
     if (ctas > 148 * 16) ctas = 148 * 16;
     launch(kern, (unsigned)ctas, cta ? 256 : warps * 32, smem, st, t, (int)p->image_row);
@@ -503,7 +503,7 @@ static int launch_transpose(const ss2d_expand_params* p, cudaStream_t st) {
     if (warps > 8) warps = 8;
     const size_t smem = plane_bytes * warps;
     auto kern = plane_transpose_kernel<T>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
+    if (const int rc = allow_dynamic_smem(kern, smem)) return rc;
     long long ctas = (t.planes + warps - 1) / warps;
     if (ctas > 148 * 16) ctas = 148 * 16;
     launch(kern, (unsigned)ctas, warps * 32, smem, st, t);

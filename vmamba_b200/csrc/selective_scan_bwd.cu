@@ -987,11 +987,11 @@ template <typename Tin, typename Tg, int VEC>
 static int launch_bwd(const BwdArgs& a, const BwdPlan& c, int64_t ctas, cudaStream_t st) {
     if (a.N == 1) {
         auto kern = selscan_bwd_n1_kernel<Tin, Tg, VEC>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem) != cudaSuccess) return SS2D_ECUDA;
+        if (const int rc = allow_dynamic_smem(kern, c.smem)) return rc;
         launch(kern, (unsigned)ctas, c.rw * 32, c.smem, st, a, c.R);
     } else {
         auto kern = selscan_bwd_kernel<Tin, Tg, VEC>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem) != cudaSuccess) return SS2D_ECUDA;
+        if (const int rc = allow_dynamic_smem(kern, c.smem)) return rc;
         launch(kern, (unsigned)ctas, c.rw * 32, c.smem, st, a);
     }
     count_launch();
@@ -1004,7 +1004,7 @@ static int launch_bwd_rows(const BwdArgs& a, const BwdPlan& c, cudaStream_t st) 
     if (a.N == 16) kern = selscan_bwd_rows_nx_kernel<Tin, Tg, 16>;
     else if (a.N == 8) kern = selscan_bwd_rows_nx_kernel<Tin, Tg, 8>;
     else if (a.N == 4) kern = selscan_bwd_rows_nx_kernel<Tin, Tg, 4>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem) != cudaSuccess) return SS2D_ECUDA;
+    if (const int rc = allow_dynamic_smem(kern, c.smem)) return rc;
     const int64_t warps = a.rows / 32;
     const int64_t ctas = (warps + kBwdRowsWarps - 1) / kBwdRowsWarps;
     if (ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;

@@ -117,7 +117,7 @@ static int launch_n1_bwd(const N1BwdArgs& a, cudaStream_t st) {
     const size_t smem = sizeof(float) * (2 * kN1Warps * 2 * kN1Chunk + (size_t)kN1Warps * a.R * (4 * (32 / n1_lanes(a.L)) + 96) + (AL ? 0 : kN1Warps * 264));
     const int lpr = n1_lanes(a.L);
     auto kern = lpr == 8 ? n1_bwd_kernel<Tin, Tg, AL, 8, BC> : lpr == 16 ? n1_bwd_kernel<Tin, Tg, AL, 16, BC> : n1_bwd_kernel<Tin, Tg, AL, 32, BC>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
+    if (const int rc = allow_dynamic_smem(kern, smem)) return rc;
     const int64_t ctas = a.batch * a.n_groups * a.parts * a.S, seg_ctas = (a.batch * a.dim * (a.S - 1) + kN1Warps - 1) / kN1Warps;
     if (ctas > 0x7fffffffLL || seg_ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
     if (a.S > 1) {
@@ -134,7 +134,7 @@ static int launch_st_bwd(const StBwdArgs& a, cudaStream_t st) {
     using Y = StLayout<NS>;
     const size_t smem = StBwdSmem<NS>::bytes(a.sets);
     auto kern = st_bwd_kernel<Tin, Tg, NS, VW>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA;
+    if (const int rc = allow_dynamic_smem(kern, smem)) return rc;
     const int64_t ctas = a.batch * a.n_groups * a.parts * a.S;
     const int64_t seg_ctas = a.batch * a.n_groups * ((a.group_size + kStRows - 1) / kStRows) * (a.S - 1);
     if (ctas > 0x7fffffffLL || seg_ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;

@@ -470,7 +470,7 @@ int pixels_norm_to_planes(const ss2d_relayout_params* p, cudaStream_t st) {
     const long long ctas = (p->N + tp - 1) / tp;
     if (ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
 #define SS2D_ROWS_LAUNCH_TP(TI, TO, TPV) { auto kern = pixels_norm_to_planes_kernel<TI, TO, TPV>; \
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA; \
+        if (const int rc = allow_dynamic_smem(kern, smem)) return rc; \
         launch(kern, (unsigned)ctas, 256, smem, st, a); }
 #define SS2D_ROWS_LAUNCH(TI, TO) { if (tp == 32) SS2D_ROWS_LAUNCH_TP(TI, TO, 32) else SS2D_ROWS_LAUNCH_TP(TI, TO, 16) }
     const int ri = p->rows_dtype, po = p->planes_dtype;
@@ -610,7 +610,7 @@ int planes_to_pixels(const ss2d_relayout_params* p, cudaStream_t st) {
     const long long ctas = (p->N + tp - 1) / tp;
     if (ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
 #define SS2D_PLANES_LAUNCH_TP(TT, TPV) { auto kern = planes_to_pixels_kernel<TT, TPV>; \
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SS2D_ECUDA; \
+        if (const int rc = allow_dynamic_smem(kern, smem)) return rc; \
         launch(kern, (unsigned)ctas, 256, smem, st, a); }
 #define SS2D_PLANES_LAUNCH(TT) { if (tp == 32) SS2D_PLANES_LAUNCH_TP(TT, 32) else SS2D_PLANES_LAUNCH_TP(TT, 16) }
     if (p->rows_dtype == SS2D_F32) SS2D_PLANES_LAUNCH(float)
