@@ -80,7 +80,8 @@ typedef struct ss2d_scan_params {
 } ss2d_scan_params;
 
 int ss2d_selective_scan_fwd(const ss2d_scan_params *p, void *cuda_stream);
-int64_t ss2d_selective_scan_fwd_workspace_bytes(const ss2d_scan_params *p);       /* < 0: invalid arguments; 0: none is used */
+/* < 0: invalid arguments; 0: none is used.  A size of the shape alone, wherever the tensors lie. */
+int64_t ss2d_selective_scan_fwd_workspace_bytes(const ss2d_scan_params *p);
 int64_t ss2d_selective_scan_checkpoint_every(int64_t dstate, int64_t delta_ratio);   /* the spacing that the backward call reads */
 
 /* ------------------------------------------------------------------------------------

@@ -320,3 +320,32 @@ def test_gradient_planner_deals_rows_while_two_ctas_per_sm_are_left():
     assert parts(8, 96, 3136) == 12                                # 384 of 2; 4 would leave 192
     assert parts(16, 192, 784) == 6                                # 384 of 8
     assert parts(4, 96, 3136) == 24                                # 384 of 1
+
+
+def test_scan_workspace_serves_tensors_of_any_alignment():
+    """The size that a scan asks for is one of its shape: rows are cut into more segments where their tensors start on 16-byte boundaries, but a
+    workspace that was sized from others has room for them."""
+    L = _lib.lib()
+    for states, length in ((4, 15686), (8, 7686), (16, 8594), (16, 4096)):
+        for dtype in (_lib.SS2D_F32, _lib.SS2D_F16, _lib.SS2D_BF16):
+            sizes = set()
+            for offset in (0, 1, 2, 4):
+                f, g = _lib.ScanParams(), _lib.ScanBwdParams()
+                size = 4 if dtype == _lib.SS2D_F32 else 2
+                for p in (f, g):
+                    for at, name in enumerate(("u", "delta", "B", "C")):       # nothing is read
+                        setattr(p, name, (at + 1) << 40 | offset * size)
+                    p.A = 1 << 45
+                    p.batch, p.dim, p.dstate, p.seqlen, p.n_groups = 1, 4 * 384, states, length, 4
+                    p.u_dim_stride = p.delta_dim_stride = p.B_state_stride = p.C_state_stride = length
+                    p.u_batch_stride = p.delta_batch_stride = 4 * 384 * length
+                    p.B_batch_stride = p.C_batch_stride = 4 * states * length
+                    p.B_group_stride = p.C_group_stride = states * length
+                    p.in_dtype = dtype
+                f.out, f.out_dtype, f.out_batch_stride, f.out_dim_stride = 1 << 46, dtype, 4 * 384 * length, length
+                g.dout, g.dout_dtype, g.dout_batch_stride, g.dout_dim_stride = 1 << 46, dtype, 4 * 384 * length, length
+                for at, name in enumerate(("du", "ddelta", "dA", "dB", "dC")):
+                    setattr(g, name, (at + 1) << 47)
+                g.checkpoint_every = L.ss2d_selective_scan_checkpoint_every(states, 1)
+                sizes.add((L.ss2d_selective_scan_fwd_workspace_bytes(f), L.ss2d_selective_scan_bwd_workspace_bytes(g)))
+            assert len(sizes) == 1 and min(min(s) for s in sizes) > 0, (states, length, dtype, sizes)

@@ -367,3 +367,56 @@ def test_row_products(vb, outer, groups, M, N, L, turned, dt):
     assert ((got.double() - want).abs() <= (L / 16 + 48) * 2.0 ** -22 * size).all()
     p.N = 65
     assert _lib.lib().ss2d_row_products_workspace_bytes(p) == -1
+
+
+def test_scan_in_a_workspace_of_tensors_that_lie_elsewhere(vb):
+    """Sized from tensors that start off 16-byte boundaries, used with ones that start on them, whose rows are cut into more segments: they are cut
+    (two launches), and the gradients without the forward call's states fit."""
+    from vmamba_b200 import _lib
+    K, Cd, N, L = 4, 384, 8, 7686
+    u, delta, A, B, C, D, bias, dout = _random_case(1, K, Cd, N, L, seed=8)
+    td = torch.bfloat16
+    ts = dict(u=dev(u, td), delta=dev(delta, td), A=dev(A), B=dev(B, td), C=dev(C, td), D=dev(D), delta_bias=dev(bias))
+    out = torch.full((1, K * Cd, L), float("nan"), device="cuda", dtype=td)
+    grads = dict(du=torch.empty_like(ts["u"]), ddelta=torch.empty_like(ts["u"]), dA=torch.empty_like(ts["A"]), dB=torch.empty_like(ts["B"]),
+                 dC=torch.empty_like(ts["C"]), dD=torch.empty_like(ts["D"]), ddelta_bias=torch.empty_like(ts["D"]))
+    g = dev(dout)
+    lib, st = _lib.lib(), torch.cuda.current_stream().cuda_stream
+
+    def params(kind, offset, **more):
+        p = kind(in_dtype=_lib.SS2D_BF16, delta_softplus=1, batch=1, dim=K * Cd, dstate=N, seqlen=L, n_groups=K,
+                 checkpoint_every=lib.ss2d_selective_scan_checkpoint_every(N, 1), **{k: t.data_ptr() for k, t in {**ts, **more}.items()})
+        for name in ("u", "delta", "dout" if kind is _lib.ScanBwdParams else "out"):
+            setattr(p, name + "_batch_stride", K * Cd * L)
+            setattr(p, name + "_dim_stride", L)
+        for name in ("B", "C"):
+            setattr(p, name + "_batch_stride", K * N * L)
+            setattr(p, name + "_group_stride", N * L)
+            setattr(p, name + "_state_stride", L)
+        p.u += offset                                        # of the queries, which read nothing
+        return p
+
+    def room(size):
+        t = torch.empty(size, device="cuda", dtype=torch.uint8)
+        return dict(workspace=t.data_ptr(), workspace_bytes=size), t
+
+    forward = params(_lib.ScanParams, 0, out=out)
+    forward.out_dtype = _lib.SS2D_BF16
+    query = params(_lib.ScanParams, 2, out=out)
+    query.out_dtype = _lib.SS2D_BF16
+    fields, hold = room(lib.ss2d_selective_scan_fwd_workspace_bytes(query))
+    for k, v in fields.items():
+        setattr(forward, k, v)
+    before = _lib.launch_count()
+    assert lib.ss2d_selective_scan_fwd(forward, st) == _lib.SS2D_OK
+    assert _lib.launch_count() - before == 2
+    assert torch.equal(out, vb.selective_scan_fn(*ts.values(), True, False))
+    backward = params(_lib.ScanBwdParams, 0, dout=g, **grads)
+    query = params(_lib.ScanBwdParams, 2, dout=g, **grads)
+    fields, hold = room(lib.ss2d_selective_scan_bwd_workspace_bytes(query))
+    for k, v in fields.items():
+        setattr(backward, k, v)
+    assert lib.ss2d_selective_scan_bwd(backward, st) == _lib.SS2D_OK
+    want = vb.selective_scan_bwd(*ts.values(), g, True)
+    for x, y in zip(grads.values(), want):
+        assert torch.equal(x, y)

@@ -393,12 +393,14 @@ static int states_vw(const ss2d_scan_params* p) {
     return pieces && (dtype_size(p->in_dtype) == 2 || st_pad_states(p->dstate) == 4) ? 0 : 1;
 }
 
-// How the rows of a 2 .. 16 state problem are cut: segments, and the floats of their end states and sums.
-static StSegments fwd_segments(const ss2d_scan_params* p, int64_t& floats) {
-    const int NS = st_pad_states(p->dstate), parts = st_parts(p->dim / p->n_groups);
-    const StSegments s = st_segments(p->batch * p->n_groups * parts * (NS / 4), p->seqlen, states_vw(p) != 0);
-    floats = s.count > 1 ? p->batch * p->dim * s.count * (NS + 1) : 0;
-    return s;
+// How the rows of a 2 .. 16 state problem are cut, and the floats that the segments' end states and sums take.  The number of segments depends on
+// where the tensors lie (`resident`, st_segments); the workspace that callers are asked for is of the larger number, so that one
+// of this shape serves tensors of any alignment.
+static StSegments fwd_segments(const ss2d_scan_params* p, bool resident) {
+    return st_segments(p->batch * p->n_groups * st_parts(p->dim / p->n_groups) * (st_pad_states(p->dstate) / 4), p->seqlen, resident);
+}
+static int64_t segment_floats(const ss2d_scan_params* p, StSegments s) {
+    return s.count > 1 ? p->batch * p->dim * s.count * (st_pad_states(p->dstate) + 1) : 0;
 }
 
 long long selective_scan_checkpoint_every(int64_t dstate, int64_t delta_ratio) {
@@ -408,9 +410,7 @@ long long selective_scan_checkpoint_every(int64_t dstate, int64_t delta_ratio) {
 long long selective_scan_fwd_workspace_bytes(const ss2d_scan_params* p) {
     if (validate_fwd(p) != SS2D_OK) return -1;
     if (!st_states(p)) return 0;
-    int64_t floats;
-    fwd_segments(p, floats);
-    return (long long)floats * 4;
+    return (long long)segment_floats(p, fwd_segments(p, false)) * 4;
 }
 
 template <typename Tin, typename Tout>
@@ -440,14 +440,14 @@ static int selective_scan_states(const ss2d_scan_params* p, cudaStream_t st) {
     a.parts = st_parts(a.group_size);
     a.every = p->checkpoint_every ? (int)p->checkpoint_every : 128;
     a.ckpt = (float*)p->checkpoints; a.nck = (p->seqlen + a.every - 1) / a.every;
-    int64_t floats;
-    StSegments s = fwd_segments(p, floats);
+    const int vw = states_vw(p);
+    StSegments s = fwd_segments(p, vw != 0);
+    int64_t floats = segment_floats(p, s);
     if (floats && (!p->workspace || p->workspace_bytes < floats * 4)) { s = {1, (a.L + 63) / 64 * 64}; floats = 0; }   // uncut: slower, same result
     if (floats && !aligned_to(p->workspace, 16)) return SS2D_EINVAL_ALIGN;
     a.S = s.count; a.seg_len = s.len;
     a.ends = floats ? (float*)p->workspace : nullptr;
     a.sums = floats ? a.ends + p->batch * p->dim * s.count * st_pad_states(p->dstate) : nullptr;
-    const int vw = states_vw(p);
     const bool of32 = p->out_dtype == SS2D_F32;
     if (p->in_dtype == SS2D_F32) return states_fwd<float, float>(a, p, vw, st);
     if (p->in_dtype == SS2D_BF16) return of32 ? states_fwd<__nv_bfloat16, float>(a, p, vw, st) : states_fwd<__nv_bfloat16, __nv_bfloat16>(a, p, vw, st);
