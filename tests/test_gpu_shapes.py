@@ -231,3 +231,16 @@ def test_cross_of_any_plane_and_alignment(vb, shape, offset, scans, dt):
     else:
         want = ((y[0] + y[1]) + y[2]) + y[3] if scans == 3 else (y[0] + y[2]) + (y[1] + y[3])
     assert torch.equal(vb.cross_merge_fn(at_offset(ys), scans=scans).cpu().view(Bt, Cc, H * W), want)
+
+
+def test_cross_of_single_pixels_of_very_many_images(vb):
+    """The number of a route, four times the image's, is beyond 32 bits."""
+    n = (1 << 29) + 3
+    x = torch.arange(n, device="cuda", dtype=torch.int32).to(torch.int16).view(torch.bfloat16).view(n, 1, 1, 1)
+    ys = vb.cross_scan_fn(x)
+    assert ys.shape == (n, 4, 1, 1) and all(torch.equal(ys[:, k, 0, 0].view(torch.int16), x.view(-1).view(torch.int16)) for k in range(4))
+    ys = torch.ones(n, 4, 1, 1, 1, device="cuda", dtype=torch.bfloat16)
+    del x
+    ys[-2:] = 2
+    y = vb.cross_merge_fn(ys)
+    assert bool((y[:-2] == 4).all()) and bool((y[-2:] == 8).all())

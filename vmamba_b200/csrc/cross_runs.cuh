@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(512) cross_scan_runs_kernel(const RunArgs a) {
     T* out[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        out[k] = (T*)a.out + ((long long)(b * 4 + k) * a.C + c0) * S;
+        out[k] = (T*)a.out + (((long long)b * 4 + k) * a.C + c0) * S;
         run_pad(a, np, out[k]);
     }
     piece_wait();
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(512) cross_merge_runs_kernel(const RunArgs a) 
     const T* in[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-        in[k] = run_fetch((const T*)a.in + ((long long)(b * 4 + k) * a.C + c0) * S, (np - 1) * S + L, sm + k * a.slot, H, kCols && k % 2 ? pad : 0);
+        in[k] = run_fetch((const T*)a.in + (((long long)b * 4 + k) * a.C + c0) * S, (np - 1) * S + L, sm + k * a.slot, H, kCols && k % 2 ? pad : 0);
     T* __restrict__ out = (T*)a.out + ((long long)b * a.C + c0) * L;
     piece_wait();
     const int n = np * L, last = W * Hp - pad - 1;
