@@ -86,9 +86,6 @@ __global__ void __launch_bounds__(256) cross_scan_pair_kernel(const CrossArgs a)
     }
 }
 
-// Rounds to the storage type after every addition, as elementwise tensor additions do.
-template <typename T> __device__ __forceinline__ T add_t(T x, T y) { return from_f<T>(to_f<T>(x) + to_f<T>(y)); }
-
 // How the tile kernels cut a plane.  Scan: sides of at most 64 pixels, shared rows of an odd number of pieces.  Merge: whole rows, or equal
 // parts of at most 128 pixels, of 32 lines or 4 096 pixels; `slots` tiles in shared memory.
 static bool plan_tiles(const ss2d_cross_params* p, int slots, TileArgs& a, size_t& smem) {
@@ -383,11 +380,7 @@ __global__ void __launch_bounds__(256) cross_merge_ex_kernel(const CrossExArgs a
 #pragma unroll
             for (int k = 0; k < 4; ++k) ((T*)a.out)[x_index(a, b, k, c, p)] = v[k];
         } else {
-            T r;
-            if (a.scans == 0 || a.scans == 2) r = add_t(add_t(v[0], v[2]), add_t(v[1], v[3]));
-            else if (a.scans == 3) r = add_t(add_t(add_t(v[0], v[1]), v[2]), v[3]);
-            else r = from_f<T>(((to_f<T>(v[0]) + to_f<T>(v[1])) + to_f<T>(v[2])) + to_f<T>(v[3]));
-            ((T*)a.out)[x_index(a, b, 0, c, p)] = r;
+            ((T*)a.out)[x_index(a, b, 0, c, p)] = flat_sum<T>(a.scans, v[0], v[1], v[2], v[3]);
         }
     }
 }

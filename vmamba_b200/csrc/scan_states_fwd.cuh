@@ -252,6 +252,9 @@ static int st_launch_fwd(const StFwdArgs& a, int64_t batch, cudaStream_t st) {
     return check_launch();
 }
 
+// Rows without vectors are read by pieces: 16-bit ones, and fp32 ones where a warp holds more than 16 of them (4 608 rows of 8 593, 16 states: 1.36 ms,
+// 0.82 by single elements; 4 states: 445 against 508 us).
+constexpr bool st_takes_pieces(size_t esize, int NS) { return esize == 2 || NS == 4; }
 inline int st_pad_states(int64_t N) { return N <= 4 ? 4 : N <= 8 ? 8 : 16; }
 inline int st_parts(int64_t group_size) { return (int)((group_size + kStRows - 1) / kStRows); }
 
@@ -265,9 +268,13 @@ static int st_rows_per_lane(const StFwdArgs& a, int64_t batch, cudaStream_t st) 
     return st_launch_fwd<Tin, Tout, NS, 1, VW, kOut>(a, batch, st);
 }
 
-// vw: vector width of the global accesses, 8, 4, 1, or 0 for rows without vectors in tensors that start and end on 16-byte
-// boundaries (no piece reaches beyond them then): pieces of 16-bit rows (above), but single elements of fp32 rows where a warp holds no more than 16 of them (4 608 rows of 8 593, 16 states: 0.82 against 1.36 ms with pieces; 4 states:
-// 508 against 445 us).
+template <typename Tin, typename Tout, int NS, bool kOut> static int st_pieces(const StFwdArgs& a, int64_t batch, cudaStream_t st) {
+    if constexpr (st_takes_pieces(sizeof(Tin), NS)) return st_rows_per_lane<Tin, Tout, NS, 0, kOut>(a, batch, st);
+    return SS2D_ENOTSUP;                             // never chosen
+}
+
+// vw: vector width of the global accesses, 8, 4, 1, or 0 for pieces (st_takes_pieces), in tensors that start and end on 16-byte boundaries
+// (no piece reaches beyond them then).
 template <typename Tin, typename Tout, bool kOut>
 static int st_dispatch_fwd(const StFwdArgs& a, int64_t batch, int vw, cudaStream_t st) {
     const int NS = st_pad_states(a.N);
@@ -275,7 +282,7 @@ static int st_dispatch_fwd(const StFwdArgs& a, int64_t batch, int vw, cudaStream
     if (NS == NS_)                                                                              \
         return vw == 8   ? st_rows_per_lane<Tin, Tout, NS_, 8, kOut>(a, batch, st)              \
                : vw == 4 ? st_rows_per_lane<Tin, Tout, NS_, 4, kOut>(a, batch, st)              \
-               : vw == 0 ? st_rows_per_lane<Tin, Tout, NS_, (sizeof(Tin) == 2 || NS_ == 4 ? 0 : 1), kOut>(a, batch, st) \
+               : vw == 0 ? st_pieces<Tin, Tout, NS_, kOut>(a, batch, st)                        \
                          : st_rows_per_lane<Tin, Tout, NS_, 1, kOut>(a, batch, st);
     SS2D_ST(4)
     SS2D_ST(8)

@@ -390,7 +390,7 @@ static int states_vw(const ss2d_scan_params* p) {
     if (v >= 4) return v >= 8 ? 8 : 4;
     const ScanSpans s = scan_spans(*p, dtype_size(p->in_dtype));
     const bool pieces = whole_pieces(s.u) && whole_pieces(s.delta) && whole_pieces(s.B) && whole_pieces(s.C);
-    return pieces && (dtype_size(p->in_dtype) == 2 || st_pad_states(p->dstate) == 4) ? 0 : 1;
+    return pieces && st_takes_pieces(dtype_size(p->in_dtype), st_pad_states(p->dstate)) ? 0 : 1;
 }
 
 // How the rows of a 2 .. 16 state problem are cut, and the floats that the segments' end states and sums take.  The number of segments depends on
