@@ -222,3 +222,31 @@ def test_threads_with_planes_of_other_sizes(vb):
     for t in threads:
         t.join()
     assert done == {(56, 57): {_lib.SS2D_OK, True}, (56, 71): {_lib.SS2D_OK, True}}
+
+
+def test_results_of_kernels_in_front(vb):
+    """Library kernels write what the next call reads, and it what they read, call behind call on one stream: as with a wait for the GPU between them."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(4, 96, 28, 28, device="cuda", generator=g).bfloat16()
+    w = torch.randn(96, 96, device="cuda", generator=g).mul(96 ** -0.5).bfloat16()
+    A, D = -torch.rand(384, 1, device="cuda", generator=g), torch.ones(384, device="cuda")
+
+    def chain(between):
+        h, out = x, []
+        for i in range(24):
+            h = torch.matmul(w, h.flatten(2)).view_as(x)
+            between()
+            xs = vb.cross_scan_fn(h)
+            between()
+            s = torch.matmul(w[:4], h.flatten(2)).repeat(1, 4, 1).view(4, 4, 4, 784)
+            y = vb.selective_scan_fn(xs.view(4, 384, 784), xs.view(4, 384, 784), A, s[:, :, :1], s[:, :, 1:2], D, None, True, True)
+            between()
+            h = vb.cross_merge_fn(y.view(4, 4, 96, 28, 28)).view_as(x)
+            between()
+            h = (h / h.std()).bfloat16()
+            out.append(h)
+        return torch.stack(out)
+
+    want = chain(torch.cuda.synchronize)
+    for _ in range(8):
+        assert torch.equal(chain(lambda: None), want)

@@ -32,3 +32,18 @@ def test_forward_scans_keep_their_values_in_registers():
     spills = re.findall(r"entry function '(\w*st_fwd_kernel\w*)'.*?(\d+) bytes spill stores, (\d+) bytes spill loads", open(log).read(), re.S)
     assert len(spills) > 100
     assert not [s for s in spills if int(s[1]) > 24 or int(s[2]) > 24]
+
+
+def test_kernels_that_follow_one_another_read_with_ordinary_loads():
+    """`launch` lets a kernel start while the one in front of it, of this library or any other, still writes.  What it waits for is
+    promised to its ordinary loads alone: not to the read-only path, whose loads may also be moved in front of the wait."""
+    kernels = 0
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu*"))):
+        src = re.sub(r"//[^\n]*", "", open(path).read())
+        src = re.sub(r"#else\n#define piece_load __ldg[^\n]*", "", src)          # of host builds
+        assert "<<<" not in src and not re.search(r"__ldg|\bld\.global\.nc|ldu", src), os.path.basename(path)
+        for k in re.finditer(r"__global__\s+void[^{;]*\{\s*([^;]*;)", src):
+            assert k.group(1) == "follow_previous();", (os.path.basename(path), k.group(0)[:200])
+            assert "__restrict__" not in k.group(0)                              # a kernel argument that is: read-only by the compiler's own choice
+            kernels += 1
+    assert kernels > 35

@@ -52,27 +52,26 @@ template <typename T, int VEC> struct Vec {
     static constexpr int kWords = (kBytes + 3) / 4;
     struct Raw { uint32_t w[kWords]; };
 
-    template <bool kReadOnly = true>
     static __device__ __forceinline__ Raw load_raw(const T* p) {
         Raw r;
         if constexpr (kBytes % 16 == 0) {
 #pragma unroll
             for (int i = 0; i < kBytes / 16; ++i) {
                 const uint4* q = reinterpret_cast<const uint4*>(p) + i;
-                const uint4 t = kReadOnly ? __ldg(q) : *q;
+                const uint4 t = *q;
                 r.w[4 * i] = t.x; r.w[4 * i + 1] = t.y; r.w[4 * i + 2] = t.z; r.w[4 * i + 3] = t.w;
             }
         } else if constexpr (kBytes == 8) {
             const uint2* q = reinterpret_cast<const uint2*>(p);
-            const uint2 t = kReadOnly ? __ldg(q) : *q;
+            const uint2 t = *q;
             r.w[0] = t.x; r.w[1] = t.y;
         } else if constexpr (kBytes == 4) {
             const uint32_t* q = reinterpret_cast<const uint32_t*>(p);
-            r.w[0] = kReadOnly ? __ldg(q) : *q;
+            r.w[0] = *q;
         } else {
             static_assert(kBytes == 2, "unsupported vector width");
             const uint16_t* q = reinterpret_cast<const uint16_t*>(p);
-            r.w[0] = kReadOnly ? __ldg(q) : *q;
+            r.w[0] = *q;
         }
         return r;
     }
@@ -104,8 +103,6 @@ template <typename T, int VEC> struct Vec {
         }
     }
     static __device__ __forceinline__ void load(const T* p, float (&v)[VEC]) { unpack(load_raw(p), v); }
-    // for shared memory (or global data written earlier in the same kernel): no read-only path
-    static __device__ __forceinline__ void load_plain(const T* p, float (&v)[VEC]) { unpack(load_raw<false>(p), v); }
     static __device__ __forceinline__ void store(T* p, const float (&v)[VEC]) {
         Raw r;
         if constexpr (sizeof(T) == 4) {
@@ -267,10 +264,12 @@ template <> struct MmaK16<__half> {
 };
 
 // ---- launches that follow one another -----------------------------------------------------------------
-// A kernel of this library is launched while the one in front of it drains: its CTAs are placed as soon as that kernel's have
-// ended, and the first thing each of them does is wait for its results.  No kernel lets its successor go ahead of its own end
-// (griddepcontrol.launch_dependents): nothing that a successor reads through the read-only path can have been cached in front of
-// the write.  us a pass: features of 427 x 640 photographs, 290 launches on a stream, 2 564 -> 2 170; the core on 64 x 192 planes of 28 x 28
+// A kernel of this library is launched while the one in front of it on its stream drains: its CTAs are placed as soon as that kernel's have
+// ended, or as it allows it, and the first thing each of them does is wait for its results.  What is in front may be any library's kernel that
+// lets its successors in early, so a CTA may be on the chip while its inputs are still written.  The wait makes them visible to ordinary loads:
+// no kernel reads global memory through the read-only path (__ldg), which asks for data that nothing writes as long as the kernel lives, and
+// whose loads a compiler may move in front of the wait.  None lets its own successor in early.
+// us a pass: features of 427 x 640 photographs, 290 launches on a stream, 2 564 -> 2 170; the core on 64 x 192 planes of 28 x 28
 // 121 -> 112, its training step 565 -> 537.
 __device__ __forceinline__ void follow_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Not in a stream that is being captured: a graph's own gaps are as short (three captured backbones of one image in turn 855 us, and 871

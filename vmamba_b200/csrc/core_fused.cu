@@ -186,11 +186,10 @@ __device__ __forceinline__ AB route_local(const float2 (&ul)[(VEC + 1) / 2], con
 // constants, the two CTA-wide scans) is then shared by seven elements instead of one.
 template <typename T, int VEC> struct VecScalar {
     struct Raw { T e[VEC]; };
-    template <bool kReadOnly = true>
     static __device__ __forceinline__ Raw load_raw(const T* p) {
         Raw r;
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) r.e[i] = kReadOnly ? __ldg(p + i) : p[i];
+        for (int i = 0; i < VEC; ++i) r.e[i] = p[i];
         return r;
     }
     static __device__ __forceinline__ void unpack(const Raw& r, float (&v)[VEC]) {
@@ -304,7 +303,7 @@ __global__ void __launch_bounds__(MAXT, MINB) core_plane_kernel(const CoreArgs a
         AB af[NPL], ab[NPL];
 #pragma unroll
         for (int s = 0; s < NPL; ++s) {
-            const float2 Dsum = splat(__ldg(a.Dskip + d[s]) + __ldg(a.Dskip + 2 * D + d[s]));
+            const float2 Dsum = splat(a.Dskip[d[s]] + a.Dskip[2 * D + d[s]]);
 #pragma unroll
             for (int j = 0; j < NP; ++j) { yrow[s][j] = mul2(Dsum, ul[s][j]); ul[s][j] = mul2(ul[s][j], splat(kLn2)); }
         }
@@ -313,7 +312,7 @@ __global__ void __launch_bounds__(MAXT, MINB) core_plane_kernel(const CoreArgs a
 #pragma unroll
         for (int s = 0; s < NPL; ++s) {
             RouteConst rc;
-            rc.A = __ldg(a.A + d[s]); rc.bias = __ldg(a.bias + d[s]); rc.bias2 = rc.bias * kLog2e;
+            rc.A = a.A[d[s]]; rc.bias = a.bias[d[s]]; rc.bias2 = rc.bias * kLog2e;
             unpack_pairs<T, VEC>(rd0[s], dv);
             af[s] = route_local<VEC, true, kPrecise>(ul[s], dv, bv, cv, rc, cPf[s], yrow[s]);
         }
@@ -322,7 +321,7 @@ __global__ void __launch_bounds__(MAXT, MINB) core_plane_kernel(const CoreArgs a
 #pragma unroll
         for (int s = 0; s < NPL; ++s) {
             RouteConst rc;
-            rc.A = __ldg(a.A + 2 * D + d[s]); rc.bias = __ldg(a.bias + 2 * D + d[s]); rc.bias2 = rc.bias * kLog2e;
+            rc.A = a.A[2 * D + d[s]]; rc.bias = a.bias[2 * D + d[s]]; rc.bias2 = rc.bias * kLog2e;
             unpack_pairs<T, VEC>(rd2[s], dv);
             ab[s] = route_local<VEC, false, kPrecise>(ul[s], dv, bv, cv, rc, cPb[s], yrow[s]);
             if (first) af[s].a = 0.f;
@@ -351,7 +350,7 @@ __global__ void __launch_bounds__(MAXT, MINB) core_plane_kernel(const CoreArgs a
                 ul[s][j].x = plane[s][cs.at(2 * j, Wp)];
                 ul[s][j].y = (2 * j + 1 < VEC) ? plane[s][cs.at(2 * j + 1, Wp)] : 0.f;
             }
-            const float2 Dsum = splat(__ldg(a.Dskip + D + d[s]) + __ldg(a.Dskip + 3 * D + d[s]));
+            const float2 Dsum = splat(a.Dskip[D + d[s]] + a.Dskip[3 * D + d[s]]);
 #pragma unroll
             for (int j = 0; j < NP; ++j) { ycol[s][j] = mul2(Dsum, ul[s][j]); ul[s][j] = mul2(ul[s][j], splat(kLn2)); }
         }
@@ -360,7 +359,7 @@ __global__ void __launch_bounds__(MAXT, MINB) core_plane_kernel(const CoreArgs a
 #pragma unroll
         for (int s = 0; s < NPL; ++s) {
             RouteConst rc;
-            rc.A = __ldg(a.A + D + d[s]); rc.bias = __ldg(a.bias + D + d[s]); rc.bias2 = rc.bias * kLog2e;
+            rc.A = a.A[D + d[s]]; rc.bias = a.bias[D + d[s]]; rc.bias2 = rc.bias * kLog2e;
             unpack_pairs<T, VEC>(rd1[s], dv);
             af[s] = route_local<VEC, true, kPrecise>(ul[s], dv, bv, cv, rc, cPf[s], ycol[s]);
         }
@@ -369,7 +368,7 @@ __global__ void __launch_bounds__(MAXT, MINB) core_plane_kernel(const CoreArgs a
 #pragma unroll
         for (int s = 0; s < NPL; ++s) {
             RouteConst rc;
-            rc.A = __ldg(a.A + 3 * D + d[s]); rc.bias = __ldg(a.bias + 3 * D + d[s]); rc.bias2 = rc.bias * kLog2e;
+            rc.A = a.A[3 * D + d[s]]; rc.bias = a.bias[3 * D + d[s]]; rc.bias2 = rc.bias * kLog2e;
             unpack_pairs<T, VEC>(rd3[s], dv);
             ab[s] = route_local<VEC, false, kPrecise>(ul[s], dv, bv, cv, rc, cPb[s], ycol[s]);
             if (first) af[s].a = 0.f;

@@ -68,10 +68,10 @@ __device__ __forceinline__ void walk_route(const RouteArgs& a, const int b, cons
     const T* __restrict__ dp = (const T*)a.delta[k] + b * a.d_bs[k] + d * a.d_cs[k];
     const T* __restrict__ Bp = (const T*)a.Bm[k] + b * a.bc_bs[k];
     const T* __restrict__ Cp = (const T*)a.Cm[k] + b * a.bc_bs[k];
-    const float Ak = __ldg(a.A + k * a.D + d) * (kPrecise ? kLog2e : 1.f);
-    const float bias = __ldg(a.bias + k * a.D + d) * (kPrecise ? 1.f : kLog2e);
+    const float Ak = a.A[k * a.D + d] * (kPrecise ? kLog2e : 1.f);
+    const float bias = a.bias[k * a.D + d] * (kPrecise ? 1.f : kLog2e);
     // 16-bit maps accumulate in units of 1 / ln 2 (the step size stays a base-2 logarithm); the merge rescales
-    const float Dk = __ldg(a.Dskip + k * a.D + d) * (kPrecise ? 1.f : 1.f / kLn2);
+    const float Dk = a.Dskip[k * a.D + d] * (kPrecise ? 1.f : 1.f / kLn2);
     const bool first_lane = lane == (kBack ? 31 : 0);
     const bool swap_units = (lane & 4) != 0;
     const int last_seg = L - S;                        // L is a multiple of S
@@ -89,7 +89,7 @@ __device__ __forceinline__ void walk_route(const RouteArgs& a, const int b, cons
         const int o = offset_of(e);
         rd = VT::load_raw(dp + o);
         rb = VT::load_raw(Bp + o);
-        rx = VT::template load_raw<false>(xsrc + o);
+        rx = VT::load_raw(xsrc + o);
         rc = VT::load_raw(Cp + o);
     }
 #pragma unroll 1
@@ -100,7 +100,7 @@ __device__ __forceinline__ void walk_route(const RouteArgs& a, const int b, cons
         if constexpr (kRoll == 0) {
             rd = VT::load_raw(dp + o_next);
             rb = VT::load_raw(Bp + o_next);
-            rx = VT::template load_raw<false>(xsrc + o_next);
+            rx = VT::load_raw(xsrc + o_next);
             rc = VT::load_raw(Cp + o_next);
         }
         float2 aa[NP], bb[NP], du[NP];
@@ -113,7 +113,7 @@ __device__ __forceinline__ void walk_route(const RouteArgs& a, const int b, cons
             if constexpr (kRoll == 1) {
                 // the raw registers of these three streams are free: the next chunk's loads fly during the rest of this one
                 rb = VT::load_raw(Bp + o_next);
-                rx = VT::template load_raw<false>(xsrc + o_next);
+                rx = VT::load_raw(xsrc + o_next);
             }
 #pragma unroll
             for (int j = 0; j < NP; ++j) {
@@ -165,7 +165,7 @@ __device__ __forceinline__ void walk_route(const RouteArgs& a, const int b, cons
         if constexpr (kRoll == 2) rd = VT::load_raw(dp + o_next);
         if constexpr (kRoll == 2 || kRoll == 3) {
             rb = VT::load_raw(Bp + o_next);
-            rx = VT::template load_raw<false>(xsrc + o_next);
+            rx = VT::load_raw(xsrc + o_next);
         }
         float2 y[NP];
         {
@@ -188,8 +188,8 @@ __device__ __forceinline__ void walk_route(const RouteArgs& a, const int b, cons
             float2 v0 = swap_units ? y[0] : y[2], v1 = swap_units ? y[1] : y[3];     // unit accessed second
             if (s >= nA) {                                       // same for the whole warp
                 float o[4], w[4];
-                Vec<float, 4>::load_plain(q + first, o);
-                Vec<float, 4>::load_plain(q + second, w);
+                Vec<float, 4>::load(q + first, o);
+                Vec<float, 4>::load(q + second, w);
                 u0 = __fadd2_rn(u0, make_float2(o[0], o[1])); u1 = __fadd2_rn(u1, make_float2(o[2], o[3]));
                 v0 = __fadd2_rn(v0, make_float2(w[0], w[1])); v1 = __fadd2_rn(v1, make_float2(w[2], w[3]));
             }
@@ -201,7 +201,7 @@ __device__ __forceinline__ void walk_route(const RouteArgs& a, const int b, cons
         } else {
             if (s >= nA) {
                 float old[S];
-                Vec<float, S>::load_plain(q, old);
+                Vec<float, S>::load(q, old);
 #pragma unroll
                 for (int j = 0; j < NP; ++j) y[j] = __fadd2_rn(y[j], make_float2(old[2 * j], old[2 * j + 1]));
             }
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(128, MINB) core_route_kernel(const RouteArgs a
 #pragma unroll 2
                 for (int w0 = wsub; w0 < W; w0 += 8) {
                     float r[4], o[4];
-                    Vec<float, 4>::load_plain(accR + h * W + w0, r);
+                    Vec<float, 4>::load(accR + h * W + w0, r);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) o[i] = scale * (r[i] + accC[(w0 + i) * H + h]);
                     Vec<float, 4>::store(out + h * W + w0, o);

@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
             return;
         }
         const long long off = (long long)d * a.cs;
-        if (has_in) Vec<float, PV>::load_plain(src + off, v);      // `in` may alias `sum_out`: no read-only path
+        if (has_in) Vec<float, PV>::load(src + off, v);
         else {
 #pragma unroll
             for (int i = 0; i < PV; ++i) v[i] = 0.f;
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
             for (int i = 0; i < PV; ++i) v[i] += t[i];
         }
         if (has_ab) {
-            const float bb = __ldg(a.add_bias + d);
+            const float bb = a.add_bias[d];
 #pragma unroll
             for (int i = 0; i < PV; ++i) v[i] += bb;
         }
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
 #pragma unroll
         for (int j = 0; j < NP / 2; ++j) {
             float t[PV];
-            Vec<float, PV>::load_plain(&red[which][h * (NP / 2) + j][tx][0], t);
+            Vec<float, PV>::load(&red[which][h * (NP / 2) + j][tx][0], t);
 #pragma unroll
             for (int i = 0; i < PV; ++i) v[i] += t[i];
         }
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
 #pragma unroll
         for (int c = 0; c < CACHE; ++c) {
             const int d = ty + c * NTY;
-            if (live && in_range(d) && has_in) Vec<float, PV>::load_plain(src + (long long)d * a.cs, cache[c]);
+            if (live && in_range(d) && has_in) Vec<float, PV>::load(src + (long long)d * a.cs, cache[c]);
             else {
 #pragma unroll
                 for (int i = 0; i < PV; ++i) cache[c][i] = 0.f;
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
                     for (int i = 0; i < PV; ++i) cache[c][i] += tv[i];
                 }
                 if (has_ab) {
-                    const float bb = __ldg(a.add_bias + d);
+                    const float bb = a.add_bias[d];
 #pragma unroll
                     for (int i = 0; i < PV; ++i) cache[c][i] += bb;
                 }
@@ -187,8 +187,8 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
             return;
         }
         const long long off = (long long)d * a.cs;
-        if (again) { Vec<float, PV>::load_plain(again + off, v); return; }
-        if (has_in) Vec<float, PV>::load_plain(src + off, v);
+        if (again) { Vec<float, PV>::load(again + off, v); return; }
+        if (has_in) Vec<float, PV>::load(src + off, v);
         else {
 #pragma unroll
             for (int i = 0; i < PV; ++i) v[i] = 0.f;
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
             for (int i = 0; i < PV; ++i) v[i] += t[i];
         }
         if (has_ab) {
-            const float bb = __ldg(a.add_bias + d);
+            const float bb = a.add_bias[d];
 #pragma unroll
             for (int i = 0; i < PV; ++i) v[i] += bb;
         }
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
     Tio* __restrict__ dst = (Tio*)a.out + (long long)bimg * a.obs + pix;
     const bool has_w = MODE ? true : (norm && a.w), has_b = MODE ? true : (norm && a.b);
     auto emit = [&](int d, const float (&v)[PV]) {
-        const float g = has_w ? __ldg(a.w + d) : 1.f, be = has_b ? __ldg(a.b + d) : 0.f;
+        const float g = has_w ? a.w[d] : 1.f, be = has_b ? a.b[d] : 0.f;
         float o[PV];
 #pragma unroll
         for (int i = 0; i < PV; ++i) o[i] = fmaf((v[i] - mean[i]) * rstd[i], g, be);

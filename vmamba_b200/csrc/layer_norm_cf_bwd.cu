@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(kLnbWarps * 32, 3) layer_norm_cf_bwd_kernel(co
             for (int i = 0; i < 4; ++i) {
                 float v[PV], gv[PV];
                 VY::unpack(qy[i], v); VG::unpack(qg[i], gv);
-                const float w = d0 + i < D ? (a.w ? __ldg(a.w + d0 + i) : 1.f) : 0.f;
+                const float w = d0 + i < D ? (a.w ? a.w[d0 + i] : 1.f) : 0.f;
 #pragma unroll
                 for (int p = 0; p < PV; ++p) {
                     const float c = d0 + i < D ? v[p] - mean[p] : 0.f, gw = gv[p] * w;
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kLnbWarps * 32, 3) layer_norm_cf_bwd_kernel(co
                 float c[PV], gv[PV], o[PV];
                 VY::unpack(qy[i], c); VG::unpack(qg[i], gv);
                 const bool real = d0 + i < D && in;
-                const float w = d0 + i < D ? (a.w ? __ldg(a.w + d0 + i) : 1.f) : 0.f;
+                const float w = d0 + i < D ? (a.w ? a.w[d0 + i] : 1.f) : 0.f;
                 v[2 * i] = v[2 * i + 1] = 0.f;
 #pragma unroll
                 for (int p = 0; p < PV; ++p) {

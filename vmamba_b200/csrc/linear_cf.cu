@@ -165,8 +165,8 @@ linear_cf_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
                 uint32_t w[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const float lo = __uint_as_float(r[2 * q]) + (kBias ? __ldg(bias + c0 + 2 * q) : 0.f);
-                    const float hi = __uint_as_float(r[2 * q + 1]) + (kBias ? __ldg(bias + c0 + 2 * q + 1) : 0.f);
+                    const float lo = __uint_as_float(r[2 * q]) + (kBias ? bias[c0 + 2 * q] : 0.f);
+                    const float hi = __uint_as_float(r[2 * q + 1]) + (kBias ? bias[c0 + 2 * q + 1] : 0.f);
                     const uint32_t own = Half2Of<T>::pack(lo, hi);
                     const uint32_t other = __shfl_xor_sync(0xffffffffu, own, 1);
                     w[q] = __byte_perm(own, other, sel);

@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kLsWarps * 32) linear_small_kernel(const Linea
         const int m = i >> 3, c = (i & 7) * 8;
         if (m0 + m >= M || n0 + c >= a.N) continue;
         float v[8];
-        const float b = a.bias ? __ldg(a.bias + m0 + m) : 0.f;
+        const float b = a.bias ? a.bias[m0 + m] : 0.f;
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = b;
 #pragma unroll

@@ -90,7 +90,7 @@ mlp_fused_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int i = threadIdx.x; i < S::HID; i += kThreads) reinterpret_cast<float*>(sm + S::kBias)[i] = __ldg(a.b1 + i);
+    for (int i = threadIdx.x; i < S::HID; i += kThreads) reinterpret_cast<float*>(sm + S::kBias)[i] = a.b1[i];
     if (warp == 1) { tmem_alloc(tmem_slot, kTmemCols); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();

@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(256) bias_act_kernel(const BiasActArgs a) {
     const long long row = blockIdx.x / a.chunks_per_row;
     const int chunk = blockIdx.x - (int)row * a.chunks_per_row;
     const int d = (int)((row / a.rows_per_channel) % a.D);
-    const float b = a.bias ? __ldg(a.bias + d) : 0.f;
+    const float b = a.bias ? a.bias[d] : 0.f;
     const T* __restrict__ xr = (const T*)a.x + row * (long long)a.nv * PV;
     T* __restrict__ yr = (T*)a.y + row * (long long)a.nv * PV;
     for (int it0 = chunk * 256 + threadIdx.x; it0 < a.nv; it0 += kU * 256 * a.chunks_per_row) {
@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(256) bias_act_kernel(const BiasActArgs a) {
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
             const int it = it0 + u * 256 * a.chunks_per_row;
-            if (it < a.nv) raw[u] = Vec<T, PV>::template load_raw<false>(xr + (long long)it * PV);
+            if (it < a.nv) raw[u] = Vec<T, PV>::load_raw(xr + (long long)it * PV);
         }
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(256, PV == 8 ? 2 : 3) dwconv3x3_strip_kernel(c
 #pragma unroll
         for (int j = 0; j < 9; ++j) k[j] = to_f<T>(wk[j]);
     }
-    const float b = a.bias ? __ldg(a.bias + d) : 0.f;
+    const float b = a.bias ? a.bias[d] : 0.f;
     const long long origin = chan * a.cstride + (long long)(plane - chan * a.ppc) * H * W + seg * PV;
     const T* __restrict__ px = (const T*)a.x + origin;
     T* __restrict__ py = (T*)a.y + origin;
@@ -170,8 +170,8 @@ __global__ void __launch_bounds__(256, PV == 8 ? 2 : 3) dwconv3x3_strip_kernel(c
 #pragma unroll
             for (int q = 0; q < VT::kWords; ++q) raw[j].w[q] = 0u;
         }
-        edge_l[j] = (in && lane == 0 && !at_left) ? to_f<T>(__ldg(row - 1)) : 0.f;
-        edge_r[j] = (in && lane == 31 && !at_right) ? to_f<T>(__ldg(row + PV)) : 0.f;
+        edge_l[j] = (in && lane == 0 && !at_left) ? to_f<T>(*(row - 1)) : 0.f;
+        edge_r[j] = (in && lane == 31 && !at_right) ? to_f<T>(row[PV]) : 0.f;
     }
     // window row: [left neighbour, PV own columns, right neighbour]
     auto open_row = [&](int j, float (&wv)[PV + 2]) {

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kExpThreads) route_expand_kernel(const ExpandA
     if (live && blockIdx.z == 0) {
         for (int n = dg; n < a.N2; n += NDG) {
             float v[VEC];
-            Vec<float, VEC>::load_plain(s_rows + (size_t)(a.R + n) * (NI * VEC) + it * VEC, v);
+            Vec<float, VEC>::load(s_rows + (size_t)(a.R + n) * (NI * VEC) + it * VEC, v);
             Vec<T, VEC>::store((T*)a.bc[k] + b * a.bc_bs[k] + (long long)n * a.bc_rs[k] + q0, v);
         }
     }
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(kExpThreads) route_expand_kernel(const ExpandA
 #pragma unroll 2
         for (int r = 0; r < a.R; ++r) {
             float sv[VEC];
-            Vec<float, VEC>::load_plain(s_rows + (size_t)r * (NI * VEC) + it * VEC, sv);
+            Vec<float, VEC>::load(s_rows + (size_t)r * (NI * VEC) + it * VEC, sv);
             const float4 w4 = *reinterpret_cast<const float4*>(s_w + r * kDChunk + dl0);
             const float wv[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
@@ -188,9 +188,9 @@ __global__ void __launch_bounds__(256, 4) route_expand_mma_kernel(const ExpandAr
     // one projected row of eight pixels, gathered column-major for the odd routes
     auto fetch8 = [&](int row, int q) {
         const T* rp = xd + (long long)row * a.xd_rs;
-        if (!col) return __ldg(reinterpret_cast<const uint4*>(rp + q));
+        if (!col) return *reinterpret_cast<const uint4*>(rp + q);
         if (a.xt)
-            return __ldg(reinterpret_cast<const uint4*>((const T*)a.xt + ((long long)(k >> 1) * a.C + row) * a.xt_rs + (long long)b * a.Limg + q));
+            return *reinterpret_cast<const uint4*>((const T*)a.xt + ((long long)(k >> 1) * a.C + row) * a.xt_rs + (long long)b * a.Limg + q);
         __align__(16) T v[8];
         const int img0 = (q / a.Limg) * a.Limg, qi = q - img0;
         int w = qi / a.H, h = qi - w * a.H, base = img0;
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(256, 4) route_expand_mma_kernel(const ExpandAr
         for (int i = tid; i < slice * (KP / 8); i += threads) {
             const int dl = i / (KP / 8), r = (i - dl * (KP / 8)) * 8;
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (dl < dn && r < a.R) v = __ldg(reinterpret_cast<const uint4*>(wk + (long long)(dc + dl) * a.R + r));
+            if (dl < dn && r < a.R) v = *reinterpret_cast<const uint4*>(wk + (long long)(dc + dl) * a.R + r);
             *reinterpret_cast<uint4*>(&Ws[dl * KPAD + r]) = v;
         }
     } else {
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(256) plane_transpose_kernel(const TransArgs a)
         if (vec) {
             for (int e = lane * PV; e < a.L; e += 32 * PV) {
                 T v[PV];
-                *reinterpret_cast<uint4*>(v) = __ldg(reinterpret_cast<const uint4*>(src + e));
+                *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(src + e);
                 int h = e / a.W, w = e - h * a.W;
 #pragma unroll
                 for (int i = 0; i < PV; ++i) {

@@ -39,10 +39,10 @@ __global__ void __launch_bounds__(kRpWarps * 32) row_products_kernel(const RowPr
 #pragma unroll 2
     for (int l = l_lo + t * 8; l - t * 8 < l_hi; l += 32) {
         const bool in = l < l_hi;
-        const uint4 x = in && in0 ? __ldg(reinterpret_cast<const uint4*>(a0 + l)) : zero, y = in && in1 ? __ldg(reinterpret_cast<const uint4*>(a1 + l)) : zero;
+        const uint4 x = in && in0 ? *reinterpret_cast<const uint4*>(a0 + l) : zero, y = in && in1 ? *reinterpret_cast<const uint4*>(a1 + l) : zero;
         uint4 v[NT];
 #pragma unroll
-        for (int n = 0; n < NT; ++n) v[n] = in && n * 8 + g < p.N ? __ldg(reinterpret_cast<const uint4*>(b + (n * 8 + g) * p.b_rs + l)) : zero;
+        for (int n = 0; n < NT; ++n) v[n] = in && n * 8 + g < p.N ? *reinterpret_cast<const uint4*>(b + (n * 8 + g) * p.b_rs + l) : zero;
         const uint32_t f0[4] = {x.x, y.x, x.y, y.y}, f1[4] = {x.z, y.z, x.w, y.w};
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(256) row_products_fold_kernel(const float* par
     const int lane = threadIdx.x & 31, run = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
     float s = 0.f;
     if (i < total)
-        for (int q = run; q < parts; q += 8) s += __ldg(part + (int64_t)q * total + i);
+        for (int q = run; q < parts; q += 8) s += part[(int64_t)q * total + i];
     sums[run][lane] = s;
     __syncthreads();
     if (run == 0 && i < total) {

@@ -123,11 +123,11 @@ __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArg
         for (int j = 0; j < 3; ++j) racc[((i * kN1Warps + warp) * 3 + j) * 32 + lane] = 0.f;
         if (ln == 0) {                                           // spare lanes of a shared warp: the group's last row
             const int64_t r = (int64_t)k * gs + min(ig, gs - 1);
-            const float An = __ldg(a.A + r);
+            const float An = a.A[r];
             float e = 0.f;
             for (int j = a.S - 1; j > seg; --j)                  // what the segments behind leave
-                e = fmaf(ex2_approx(__ldg(a.esum + (out0 + r) * a.S + j) * An * kLog2e), e, __ldg(a.eagg + (out0 + r) * a.S + j));
-            par[i * kStep + wr] = make_float4(An, a.bias ? __ldg(a.bias + (a.dratio == 1 ? r : r / a.dratio)) : 0.f, a.D ? __ldg(a.D + r) : 0.f, e);
+                e = fmaf(ex2_approx(a.esum[(out0 + r) * a.S + j] * An * kLog2e), e, a.eagg[(out0 + r) * a.S + j]);
+            par[i * kStep + wr] = make_float4(An, a.bias ? a.bias[a.dratio == 1 ? r : r / a.dratio] : 0.f, a.D ? a.D[r] : 0.f, e);
         }
     }
     __syncwarp();
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kN1Warps * 32, 3) n1_bwd_kernel(const N1BwdArg
     float nh = 0.f;
     auto fetch = [&](const Rows& w, int pos) {
         nu.load(w.u, pos, 0, L); nd.load(w.d, pos, 0, L); ng.load(w.g, pos, 0, L);
-        nh = pos < L ? __ldg(w.ck + (pos >> 3)) : 0.f;
+        nh = pos < L ? w.ck[pos >> 3] : 0.f;
     };
     int buf = 0;
     const int first_w = first - lane / LPR, mine = first_w < gs ? min(R, (gs - first_w + kStep - 1) / kStep) : 0;     // row sets of this warp
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kN1Warps * 32) n1_bwd_segments_kernel(const N1
     const Tin* __restrict__ dt = (const Tin*)a.delta + b * a.d_bs + rd * a.d_ds;
     const Tg* __restrict__ gp = (const Tg*)a.dout + b * a.g_bs + r * a.g_ds;
     const Tin* __restrict__ Cm = (const Tin*)a.C + b * a.C_bs + k * a.C_gs;
-    const float A2 = __ldg(a.A + r) * kLog2e, bias = a.bias ? __ldg(a.bias + rd) : 0.f;
+    const float A2 = a.A[r] * kLog2e, bias = a.bias ? a.bias[rd] : 0.f;
     const int lo = seg * a.seg_len, hi = min(L, lo + a.seg_len);
     float e = 0.f, sum = 0.f;                                    // over the chunks taken so far
     for (int c = (hi - 1) / kN1Chunk; c * kN1Chunk >= lo; --c) {

@@ -4,6 +4,12 @@
 
 namespace ss2d {
 
+#ifdef __CUDACC__
+template <typename T> __device__ __forceinline__ T piece_load(const T* p) { return *p; }
+#else
+#define piece_load __ldg                             // compiled for the host: what stands for common.cuh looks where it reads
+#endif
+
 // The bytes of a tensor of rows, and whether they start and end on 16-byte boundaries: then no aligned piece that holds an element
 // of a row reaches beyond them.
 struct Span { uintptr_t lo, hi; };
@@ -51,7 +57,7 @@ template <typename T> struct Row8<T, 0> {
         for (int i = 0; i <= kPieces; ++i) {
             uint4 t = make_uint4(0, 0, 0, 0);
             const int e = e0 + i * kPiece;
-            if (e < L && e + kPiece > from && (i < kPieces || off != 0)) t = __ldg(q + i);
+            if (e < L && e + kPiece > from && (i < kPieces || off != 0)) t = piece_load(q + i);
             w[4 * i] = t.x; w[4 * i + 1] = t.y; w[4 * i + 2] = t.z; w[4 * i + 3] = t.w;
         }
     }

@@ -226,8 +226,8 @@ __device__ __forceinline__ void st_fold_segments(float2 (&h)[2], const float2 (&
     h[0] = h[1] = make_float2(0.f, 0.f);
     const int from = kBack ? S - 1 : 0, step = kBack ? -1 : 1;
     for (int j = from; j != seg; j += step) {
-        const float d = __ldg(sums + row * S + j);
-        const float4 e = __ldg(reinterpret_cast<const float4*>(ends + (row * S + j) * NSpad + n0));
+        const float d = sums[row * S + j];
+        const float4 e = *reinterpret_cast<const float4*>(ends + (row * S + j) * NSpad + n0);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const float2 x = __fmul2_rn(f2(d), A2[q]);

@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(StLayout<NS>::kWarps * 32, 8 / StLayout<NS>::k
             const float* p = a.A + (g0 + row_in_group(s)) * a.N + n0;
             float t[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) t[i] = n0 + i < a.N ? __ldg(p + i) : 0.f;
+            for (int i = 0; i < 4; ++i) t[i] = n0 + i < a.N ? p[i] : 0.f;
             A_s[s * 32 + lane] = make_float4(t[0], t[1], t[2], t[3]);
             load_A(s, A);
         }
@@ -133,16 +133,16 @@ __global__ void __launch_bounds__(StLayout<NS>::kWarps * 32, 8 / StLayout<NS>::k
             xd.load(dt + o * a.d_ds, a.d_ds, count, t0, L, lane);
             xu.load(u + o * a.u_ds, a.u_ds, count, t0, L, lane);
             xg.load(gp + o * a.g_ds, a.g_ds, count, t0, L, lane);
-            const float bias_rl = a.bias ? __ldg(a.bias + g0 + row_in_group(s)) : 0.f;
+            const float bias_rl = a.bias ? a.bias[g0 + row_in_group(s)] : 0.f;
             {                                        // the state in front of the chunk
                 const float* ck = a.ckpt + ((b * a.dim + g0 + row_in_group(s)) * nck + t0 / kStChunk) * a.N + n0;
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (a.N == NS) v = __ldg(reinterpret_cast<const float4*>(ck));
+                if (a.N == NS) v = *reinterpret_cast<const float4*>(ck);
                 else {
-                    if (n0 < a.N) v.x = __ldg(ck);
-                    if (n0 + 1 < a.N) v.y = __ldg(ck + 1);
-                    if (n0 + 2 < a.N) v.z = __ldg(ck + 2);
-                    if (n0 + 3 < a.N) v.w = __ldg(ck + 3);
+                    if (n0 < a.N) v.x = *ck;
+                    if (n0 + 1 < a.N) v.y = ck[1];
+                    if (n0 + 2 < a.N) v.z = ck[2];
+                    if (n0 + 3 < a.N) v.w = ck[3];
                 }
                 hs[s * kStTiles * 32 + lane] = v;
             }
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(StLayout<NS>::kWarps * 32, 8 / StLayout<NS>::k
                             S[w][t] = (up ? S[w][t + n] : S[w][t]) + __shfl_xor_sync(0xffffffffu, up ? S[w][t] : S[w][t + n], off);
                 }
                 __syncwarp();                        // every lane of the row has read d, u, g of the tile
-                const float Dv = a.D ? __ldg(a.D + g0 + row_in_group(s)) : 0.f;
+                const float Dv = a.D ? a.D[g0 + row_in_group(s)] : 0.f;
                 float2 db = dDb[s * 32 + lane];
 #pragma unroll
                 for (int i = 0; i < E; ++i) {
@@ -400,10 +400,10 @@ __global__ void __launch_bounds__(StLayout<NS>::kWarps * 32) st_bwd_segments_ker
     {
         float t[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) t[i] = n0 + i < a.N ? __ldg(a.A + (g0 + ig) * a.N + n0 + i) * kLog2e : 0.f;
+        for (int i = 0; i < 4; ++i) t[i] = n0 + i < a.N ? a.A[(g0 + ig) * a.N + n0 + i] * kLog2e : 0.f;
         A2[0] = make_float2(t[0], t[1]); A2[1] = make_float2(t[2], t[3]);
     }
-    const float bias_rl = a.bias ? __ldg(a.bias + g0 + ig) : 0.f;
+    const float bias_rl = a.bias ? a.bias[g0 + ig] : 0.f;
     const bool sp = a.softplus != 0;
     const int lo = seg * a.seg_len, hi = min(L, lo + a.seg_len);
     float sum = 0.f;

@@ -73,10 +73,10 @@ __global__ void __launch_bounds__(StLayout<NS, R_>::kWarps * 32, !st_sixteen_war
         row[j] = b * a.dim + r;
         float t[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) t[i] = n0 + i < a.N ? __ldg(a.A + r * a.N + n0 + i) * kLog2e : 0.f;
+        for (int i = 0; i < 4; ++i) t[i] = n0 + i < a.N ? a.A[r * a.N + n0 + i] * kLog2e : 0.f;
         A2[j][0] = make_float2(t[0], t[1]); A2[j][1] = make_float2(t[2], t[3]);
-        bias[j] = a.bias ? __ldg(a.bias + r) : 0.f;
-        Dv[j] = kOut && a.D && sl == 0 ? __ldg(a.D + r) : 0.f;          // one lane of a row adds D u
+        bias[j] = a.bias ? a.bias[r] : 0.f;
+        Dv[j] = kOut && a.D && sl == 0 ? a.D[r] : 0.f;          // one lane of a row adds D u
         sum_d[j] = 0.f;
         if (a.fold) st_fold_segments<false>(h[j], A2[j], a.ends, a.sums, row[j], a.S, seg, n0, NS);
         else h[j][0] = h[j][1] = f2(0.f);

@@ -61,9 +61,9 @@ __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32, W == 1 &&
     const Tin* __restrict__ Bm = (const Tin*)a.B + b * a.B_bs + k * a.B_gs;
     const Tin* __restrict__ Cm = (const Tin*)a.C + b * a.C_bs + k * a.C_gs;
     Tout* __restrict__ out = (Tout*)a.out + b * a.o_bs + r * a.o_ds;
-    const float A2 = __ldg(a.A + r) * kLog2e;
-    const float Dv = a.D ? __ldg(a.D + r) : 0.f;
-    const float bias = a.bias ? __ldg(a.bias + rd_) : 0.f;
+    const float A2 = a.A[r] * kLog2e;
+    const float Dv = a.D ? a.D[r] : 0.f;
+    const float bias = a.bias ? a.bias[rd_] : 0.f;
     const bool sp = a.softplus != 0;
     const int L = (int)a.seqlen;
     constexpr int OV = 16 / (int)sizeof(Tout);       // elements per 16-byte store
@@ -214,12 +214,12 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) selscan_fwd_nx_kernel(const
     const int N = (int)a.dstate;
     for (int n = lane; n < N; n += 32) {
         carry_s[warp][n] = 0.f;
-        A2_s[warp][n] = __ldg(a.A + r * N + n) * kLog2e;
+        A2_s[warp][n] = a.A[r * N + n] * kLog2e;
     }
     __syncwarp();
     const bool has_D = a.D != nullptr;
-    const float Dv = has_D ? __ldg(a.D + r) : 0.f;
-    const float bias = a.bias ? __ldg(a.bias + r / a.dratio) : 0.f;
+    const float Dv = has_D ? a.D[r] : 0.f;
+    const float bias = a.bias ? a.bias[r / a.dratio] : 0.f;
     const bool sp = a.softplus != 0;
     const int L = (int)a.seqlen;
     constexpr int STEP = 32 * VEC;

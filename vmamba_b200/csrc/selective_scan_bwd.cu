@@ -78,15 +78,15 @@ __global__ void __launch_bounds__(256) selscan_bwd_kernel(const BwdArgs a) {
     Tin* __restrict__ du = (Tin*)a.du + (b * a.dim + r) * L;
     Tin* __restrict__ dd = (Tin*)a.ddelta + (b * a.dim + r) * L;
     const bool has_D = a.D != nullptr;
-    const float Dv = has_D ? __ldg(a.D + r) : 0.f;
-    const float bias = a.bias ? __ldg(a.bias + r / a.dratio) : 0.f;
+    const float Dv = has_D ? a.D[r] : 0.f;
+    const float bias = a.bias ? a.bias[r / a.dratio] : 0.f;
     const bool sp = a.softplus != 0;
     using VI = Vec<Tin, VEC>;
     using VG = Vec<Tg, VEC>;
 
     for (int n = lane; n < N; n += 32) {
         carry[n] = 0.f; dA_s[n] = 0.f;
-        A_s[n] = __ldg(a.A + r * N + n);
+        A_s[n] = a.A[r * N + n];
     }
     __syncwarp();
 
@@ -282,8 +282,8 @@ __global__ void __launch_bounds__(256) selscan_bwd_n1_kernel(const BwdArgs a, co
         }
         const Tin* __restrict__ u = (const Tin*)a.u + b * a.u_bs + r * a.u_ds;
         const Tin* __restrict__ dt = (const Tin*)a.delta + b * a.d_bs + (r / a.dratio) * a.d_ds;
-        const float A2 = __ldg(a.A + r) * kLog2e;
-        const float bias = a.bias ? __ldg(a.bias + r / a.dratio) : 0.f;
+        const float A2 = a.A[r] * kLog2e;
+        const float bias = a.bias ? a.bias[r / a.dratio] : 0.f;
         float hc = 0.f;
         typename VI::Raw ru = {}, rd = {}, rb = {};
         int pos = lane * VEC;
@@ -346,9 +346,9 @@ __global__ void __launch_bounds__(256) selscan_bwd_n1_kernel(const BwdArgs a, co
             const int64_t ig = row0 + lr;
             if (ig < a.group_size) {                    // uniform over the warp
                 const int64_t r = (int64_t)k * a.group_size + ig;
-                const float An = __ldg(a.A + r), A2 = An * kLog2e;
-                const float bias = a.bias ? __ldg(a.bias + r / a.dratio) : 0.f;
-                const float Dv = has_D ? __ldg(a.D + r) : 0.f;
+                const float An = a.A[r], A2 = An * kLog2e;
+                const float bias = a.bias ? a.bias[r / a.dratio] : 0.f;
+                const float Dv = has_D ? a.D[r] : 0.f;
                 float uv[VEC], dl[VEC], gv[VEC], dsp[VEC], av[VEC], P[VEC], hl[VEC], Q[VEC], El[VEC];
                 VI::unpack(ru, uv); VI::unpack(rd, dl); VG::unpack(rg, gv);
                 float p = 1.f, h = 0.f, dD_loc = 0.f;
@@ -484,10 +484,10 @@ __global__ void __launch_bounds__(kBwdRowsWarps * 32, 4) selscan_bwd_rows_kernel
     Tin* __restrict__ dd = (Tin*)a.ddelta + (b * a.dim + r0) * L;
     float* __restrict__ bc_out = a.bcpart + (((size_t)b * a.n_groups + k) * a.parts + part) * 2 * (size_t)L;
     const float* __restrict__ ck = a.ckpt + (b * a.dim + r) * a.nck;
-    const float An = __ldg(a.A + r), A2 = An * kLog2e;
+    const float An = a.A[r], A2 = An * kLog2e;
     const bool has_D = a.D != nullptr;
-    const float Dv = has_D ? __ldg(a.D + r) : 0.f;
-    const float bias = a.bias ? __ldg(a.bias + r) : 0.f;
+    const float Dv = has_D ? a.D[r] : 0.f;
+    const float bias = a.bias ? a.bias[r] : 0.f;
     const bool sp = a.softplus != 0;
     using VI = Vec<Tin, PE>;
     using VG = Vec<Tg, PE>;
@@ -661,10 +661,10 @@ __global__ void __launch_bounds__(kBwdRowsWarps * 32, 2) selscan_bwd_rows_nx_ker
     const float* __restrict__ ck = a.ckpt + (b * a.dim + r) * a.nck * NS;
     float A2[NS], e_carry[NS], dA_acc[NS];
 #pragma unroll
-    for (int n = 0; n < NS; ++n) { A2[n] = __ldg(a.A + r * NS + n) * kLog2e; e_carry[n] = 0.f; dA_acc[n] = 0.f; }
+    for (int n = 0; n < NS; ++n) { A2[n] = a.A[r * NS + n] * kLog2e; e_carry[n] = 0.f; dA_acc[n] = 0.f; }
     const bool has_D = a.D != nullptr;
-    const float Dv = has_D ? __ldg(a.D + r) : 0.f;
-    const float bias = a.bias ? __ldg(a.bias + r) : 0.f;
+    const float Dv = has_D ? a.D[r] : 0.f;
+    const float bias = a.bias ? a.bias[r] : 0.f;
     const bool sp = a.softplus != 0;
     using VI = Vec<Tin, PE>;
 

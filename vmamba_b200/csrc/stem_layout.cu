@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(512, 1) stem_mma_kernel(const StemArgs a, int 
             if (i < 9 * W8) {
                 const int r = i / W8, c8 = i - r * W8;
                 const int ci = r / 3, ky = r - ci * 3, iy = 2 * oy - 1 + ky;
-                if (iy >= 0 && iy < a.H) pre[sl] = __ldg(reinterpret_cast<const uint4*>(xb + ((long long)ci * a.H + iy) * a.W + 8 * c8));
+                if (iy >= 0 && iy < a.H) pre[sl] = *reinterpret_cast<const uint4*>(xb + ((long long)ci * a.H + iy) * a.W + 8 * c8);
             }
         }
     };
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(256) pixels_norm_to_planes_kernel(const RowsAr
         const bool full = p4 + 4 <= live && ((a.out_cs | n0) & 3) == 0;
 #pragma unroll 2
         for (int c = cw; c < C; c += 256 / Q4) {
-            const float w = a.lnw ? __ldg(a.lnw + c) : 1.f, bb = a.lnb ? __ldg(a.lnb + c) : 0.f;
+            const float w = a.lnw ? a.lnw[c] : 1.f, bb = a.lnb ? a.lnb[c] : 0.f;
             float o[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) o[i] = fmaf(fmaf(tile[(p4 + i) * P + c], sc[i], sh[i]), w, bb);
@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(256) planes_to_pixels_kernel(const PlanesArgs 
                     const int c = c0 + CW4 * j;
                     if (c < C) {
                         const long long off = (long long)c * a.cs + n0 + p4;
-                        Vec<float, 4>::load_plain(a.planes + off, v[j]);
+                        Vec<float, 4>::load(a.planes + off, v[j]);
                         if (a.add) {
                             float t[4];
                             Vec<T, 4>::load((const T*)a.add + off, t);
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(256) planes_to_pixels_kernel(const PlanesArgs 
                     const int c = c0 + CW4 * j;
                     if (c < C) {
                         if (a.bias) {
-                            const float bb = __ldg(a.bias + c);
+                            const float bb = a.bias[c];
 #pragma unroll
                             for (int i = 0; i < 4; ++i) v[j][i] += bb;
                         }
@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(256) planes_to_pixels_kernel(const PlanesArgs 
             for (int j = 0; j < 4; ++j) {
                 const int c = c0 + CW * j;
                 if (c < C) {
-                    if (a.bias) v[j] += __ldg(a.bias + c);
+                    if (a.bias) v[j] += a.bias[c];
                     if (a.write_back) a.planes[(long long)c * a.cs + n] = v[j];
                     tile[pl * P + c] = v[j];
                 }
