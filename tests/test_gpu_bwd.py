@@ -420,3 +420,26 @@ def test_scan_in_a_workspace_of_tensors_that_lie_elsewhere(vb):
     want = vb.selective_scan_bwd(*ts.values(), g, True)
     for x, y in zip(grads.values(), want):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("outer,groups,M,N,L,turned", [(1, 1, 1, 1, 8, 0), (2, 4, 96, 6, 3136, 0), (3, 4, 40, 13, 1000, 1), (1, 1, 17, 64, 72, 0), (1, 4, 130, 8, 40000, 0),
+                                                       (2, 3, 31, 33, 264, 1), (1, 1, 16, 8, 150000, 0)])
+def test_row_products_of_whole_numbers(vb, outer, groups, M, N, L, turned, dt):
+    """Products of whole numbers up to 3, whose sums (at most 9 x 150 000) are exact in any order: one element that is lost or taken twice, at the
+    end of a part or of a vector, shows however long the rows are."""
+    from vmamba_b200 import _lib
+    td = {"bf16": torch.bfloat16, "f16": torch.float16}[dt]
+    g = torch.Generator(device="cuda").manual_seed(M * N + L)
+    a = torch.randint(1, 4, (outer, groups, M, L), device="cuda", generator=g).to(td)
+    b = torch.randint(1, 4, (outer, groups, N, L), device="cuda", generator=g).to(td)
+    out = torch.full((groups, N, M) if turned else (groups, M, N), float("nan"), device="cuda")
+    p = _lib.RowProductsParams(a=a.data_ptr(), b=b.data_ptr(), out=out.data_ptr(), outer=outer, groups=groups, M=M, N=N, L=L,
+                               a_outer_stride=a.stride(0), a_group_stride=a.stride(1), a_row_stride=a.stride(2),
+                               b_outer_stride=b.stride(0), b_group_stride=b.stride(1), b_row_stride=b.stride(2),
+                               dtype={"bf16": _lib.SS2D_BF16, "f16": _lib.SS2D_F16}[dt], turned=turned)
+    ws = torch.empty(_lib.lib().ss2d_row_products_workspace_bytes(p), device="cuda", dtype=torch.uint8)
+    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
+    assert _lib.lib().ss2d_row_products(p, torch.cuda.current_stream().cuda_stream) == _lib.SS2D_OK
+    want = (a.double() @ b.double().transpose(2, 3)).sum(0)
+    assert torch.equal((out.transpose(1, 2) if turned else out).double(), want)
