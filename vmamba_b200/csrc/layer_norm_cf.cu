@@ -205,6 +205,21 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
             for (int i = 0; i < PV; ++i) v[i] += bb;
         }
     };
+    // Weight and bias of kBatch channels at a time, ahead of the stores of the channels in front (an ordinary load does not pass a store), the first
+    // ones ahead of the second statistic.
+    const bool has_w = MODE ? true : (norm && a.w), has_b = MODE ? true : (norm && a.b);
+    constexpr int kBatch = CACHE == 0 ? 4 : CACHE % 12 == 0 ? 6 : 8;
+    static_assert(CACHE % kBatch == 0, "");
+    float g[2][kBatch], be[2][kBatch];
+    auto fetch_wb = [&](int n, float (&gn)[kBatch], float (&bn)[kBatch]) {
+#pragma unroll
+        for (int j = 0; j < kBatch; ++j) {
+            const int d = ty + (n * kBatch + j) * NTY;
+            gn[j] = has_w && in_range(d) ? a.w[d] : 1.f;
+            bn[j] = has_b && in_range(d) ? a.b[d] : 0.f;
+        }
+    };
+    if constexpr (CACHE > 0) fetch_wb(0, g[0], be[0]);
     if (norm) {
         if constexpr (CACHE > 0) {
 #pragma unroll
@@ -229,9 +244,7 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
 #pragma unroll
     for (int i = 0; i < PV; ++i) rstd[i] = norm ? rsqrtf(fmaf(q[i], inv_d, a.eps)) : 1.f;
     Tio* __restrict__ dst = (Tio*)a.out + (long long)bimg * a.obs + pix;
-    const bool has_w = MODE ? true : (norm && a.w), has_b = MODE ? true : (norm && a.b);
-    auto emit = [&](int d, const float (&v)[PV]) {
-        const float g = has_w ? a.w[d] : 1.f, be = has_b ? a.b[d] : 0.f;
+    auto emit = [&](int d, const float (&v)[PV], float g, float be) {
         float o[PV];
 #pragma unroll
         for (int i = 0; i < PV; ++i) o[i] = fmaf((v[i] - mean[i]) * rstd[i], g, be);
@@ -239,15 +252,28 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
     };
     if constexpr (CACHE > 0) {
 #pragma unroll
-        for (int c = 0; c < CACHE; ++c) {
-            const int d = ty + c * NTY;
-            if (in_range(d)) emit(d, cache[c]);
+        for (int n = 0; n < CACHE / kBatch; ++n) {
+            if (n + 1 < CACHE / kBatch) fetch_wb(n + 1, g[(n + 1) & 1], be[(n + 1) & 1]);
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) {
+                const int c = n * kBatch + j, d = ty + c * NTY;
+                if (in_range(d)) emit(d, cache[c], g[n & 1][j], be[n & 1][j]);
+            }
         }
     } else {
-        for (int d = ty; d < D; d += NTY) {
-            float v[PV];
-            refetch(d, v);
-            emit(d, v);
+        for (int n = 0; n * kBatch * NTY + ty < D; ++n) {
+            float v[kBatch][PV];
+            fetch_wb(n, g[0], be[0]);
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) {
+                const int d = ty + (n * kBatch + j) * NTY;
+                if (d < D) refetch(d, v[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) {
+                const int d = ty + (n * kBatch + j) * NTY;
+                if (d < D) emit(d, v[j], g[0][j], be[0][j]);
+            }
         }
     }
 }

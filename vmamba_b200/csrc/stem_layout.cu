@@ -430,17 +430,36 @@ __global__ void __launch_bounds__(256) pixels_norm_to_planes_kernel(const RowsAr
 #pragma unroll
         for (int i = 0; i < 4; ++i) { sc[i] = stat[p4 + i]; sh[i] = stat[TP + p4 + i]; }
         const bool full = p4 + 4 <= live && ((a.out_cs | n0) & 3) == 0;
-#pragma unroll 2
-        for (int c = cw; c < C; c += 256 / Q4) {
-            const float w = a.lnw ? a.lnw[c] : 1.f, bb = a.lnb ? a.lnb[c] : 0.f;
-            float o[4];
+        // two channels at a time, weight and bias of the next two ahead of their stores (an ordinary load does not pass a store)
+        constexpr int kStep = 256 / Q4;
+        float w[2], bb[2];
+        const auto fetch = [&](int c0) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) o[i] = fmaf(fmaf(tile[(p4 + i) * P + c], sc[i], sh[i]), w, bb);
-            Tout* dst = (Tout*)a.out + (long long)c * a.out_cs + n0 + p4;
-            if (full) Vec<Tout, 4>::store(dst, o);
-            else {
+            for (int j = 0; j < 2; ++j) {
+                const int c = c0 + j * kStep;
+                w[j] = a.lnw && c < C ? a.lnw[c] : 1.f; bb[j] = a.lnb && c < C ? a.lnb[c] : 0.f;
+            }
+        };
+        fetch(cw);
+        for (int c0 = cw; c0 < C; c0 += 2 * kStep) {
+            float o[2][4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) if (p4 + i < live) dst[i] = from_f<Tout>(o[i]);
+            for (int j = 0; j < 2; ++j) {
+                const int c = min(c0 + j * kStep, C - 1);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) o[j][i] = fmaf(fmaf(tile[(p4 + i) * P + c], sc[i], sh[i]), w[j], bb[j]);
+            }
+            fetch(c0 + 2 * kStep);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int c = c0 + j * kStep;
+                if (c >= C) break;
+                Tout* dst = (Tout*)a.out + (long long)c * a.out_cs + n0 + p4;
+                if (full) Vec<Tout, 4>::store(dst, o[j]);
+                else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) if (p4 + i < live) dst[i] = from_f<Tout>(o[j][i]);
+                }
             }
         }
     }
