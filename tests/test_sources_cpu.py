@@ -3,8 +3,6 @@ import glob
 import os
 import re
 
-import pytest
-
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "vmamba_b200", "csrc")
 
 
@@ -22,16 +20,6 @@ def test_limits_of_shared_memory_only_grow():
     """They belong to a kernel and all threads that launch it: one function sets them, under a lock."""
     sets = {os.path.basename(p): open(p).read().count("cudaFuncSetAttribute(") for p in glob.glob(os.path.join(CSRC, "*")) if os.path.isfile(p)}
     assert {p: n for p, n in sets.items() if n} == {"api.cu": 1}
-
-
-def test_forward_scans_keep_their_values_in_registers():
-    """A bound on a kernel's registers that it does not fit makes it spill; the report of the build says how much."""
-    log = os.path.join(CSRC, "..", "build", "ptxas.log")
-    if not os.path.exists(log):
-        pytest.skip("not built here")
-    spills = re.findall(r"entry function '(\w*st_fwd_kernel\w*)'.*?(\d+) bytes spill stores, (\d+) bytes spill loads", open(log).read(), re.S)
-    assert len(spills) > 100
-    assert not [s for s in spills if int(s[1]) > 24 or int(s[2]) > 24]
 
 
 def test_kernels_that_follow_one_another_read_with_ordinary_loads():

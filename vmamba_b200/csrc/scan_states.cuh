@@ -198,10 +198,6 @@ template <typename T, int NS, int WARPS> struct StRawBC<T, NS, 0, WARPS> {
     }
 };
 
-// Whether the forward kernel is held to the registers of sixteen warps an SM (st_fwd_kernel).  Not pieces (VW 0: 4 608 rows of 8 594, 4 states, 438 us,
-// 308 without), nor 16-bit rows of up to four states by single elements, which spilled 64 to 120 bytes.
-constexpr bool st_sixteen_warps(size_t esize, int NS, int VW) { return VW > 1 || (VW == 1 && !(esize == 2 && NS == 4)); }
-
 // Number of segments a row is cut into (1: none) and their length, given the warps that whole rows fill.  Cutting costs a
 // second pass, so it starts below four warps per SM and then goes up to sixteen (16 states, bf16: 768 rows of 3 136
 // elements 116 -> 49 us, 384 rows of 65 536 4.4 -> 0.29 ms; 6 144 rows, which fill five warps, 0.25 uncut, 0.28 cut).

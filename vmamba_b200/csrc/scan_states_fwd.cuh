@@ -31,10 +31,10 @@ struct StFwdArgs {
     int every;               // a multiple of 32
 };
 
-// Registers for sixteen warps an SM; twelve with two rows per lane (49 152 rows, 16 states, fp32 1 142 against 1 062 us); as the compiler likes
-// where it would spill (st_sixteen_warps).
+// Registers for sixteen warps an SM; twelve with two rows per lane (49 152 rows, 16 states, fp32 1 142 against 1 062 us); pieces (VW 0) as the compiler
+// likes (4 608 rows of 8 594, 4 states, 438 us with sixteen, 308).
 template <typename Tin, typename Tout, int NS, int R_, int VW, bool kOut>
-__global__ void __launch_bounds__(StLayout<NS, R_>::kWarps * 32, !st_sixteen_warps(sizeof(Tin), NS, VW) ? 0 : (R_ == 2 ? 12 : 16) / StLayout<NS, R_>::kWarps) st_fwd_kernel(const StFwdArgs a) {
+__global__ void __launch_bounds__(StLayout<NS, R_>::kWarps * 32, VW == 0 ? 0 : (R_ == 2 ? 12 : 16) / StLayout<NS, R_>::kWarps) st_fwd_kernel(const StFwdArgs a) {
     follow_previous();
     using Y = StLayout<NS, R_>;
     constexpr int RPW = Y::RPW, SL = Y::SL, R = Y::R, RL = Y::RL, P = kStPitch;

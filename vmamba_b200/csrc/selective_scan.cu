@@ -441,7 +441,7 @@ static int selective_scan_states(const ss2d_scan_params* p, cudaStream_t st) {
     a.every = p->checkpoint_every ? (int)p->checkpoint_every : 128;
     a.ckpt = (float*)p->checkpoints; a.nck = (p->seqlen + a.every - 1) / a.every;
     const int vw = states_vw(p);
-    StSegments s = fwd_segments(p, st_sixteen_warps(dtype_size(p->in_dtype), st_pad_states(p->dstate), vw));
+    StSegments s = fwd_segments(p, vw != 0);
     int64_t floats = segment_floats(p, s);
     if (floats && (!p->workspace || p->workspace_bytes < floats * 4)) { s = {1, (a.L + 63) / 64 * 64}; floats = 0; }   // uncut: slower, same result
     if (floats && !aligned_to(p->workspace, 16)) return SS2D_EINVAL_ALIGN;
