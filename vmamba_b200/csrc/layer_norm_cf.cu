@@ -206,7 +206,8 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
         }
     };
     // Weight and bias of kBatch channels at a time, ahead of the stores of the channels in front (an ordinary load does not pass a store), the first
-    // ones ahead of the second statistic.
+    // ones ahead of the second statistic.  More than 32 values of a thread leave no registers for them
+    // (two maps of 1 536 channels in fp16, ahead 62 us, one by one 54).
     const bool has_w = MODE ? true : (norm && a.w), has_b = MODE ? true : (norm && a.b);
     constexpr int kBatch = CACHE == 0 ? 4 : CACHE % 12 == 0 ? 6 : 8;
     static_assert(CACHE % kBatch == 0, "");
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
             bn[j] = has_b && in_range(d) ? a.b[d] : 0.f;
         }
     };
-    if constexpr (CACHE > 0) fetch_wb(0, g[0], be[0]);
+    if constexpr (CACHE > 0 && CACHE <= 32) fetch_wb(0, g[0], be[0]);
     if (norm) {
         if constexpr (CACHE > 0) {
 #pragma unroll
@@ -250,7 +251,13 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
         for (int i = 0; i < PV; ++i) o[i] = fmaf((v[i] - mean[i]) * rstd[i], g, be);
         Vec<Tio, PV>::store(dst + (long long)d * a.ocs, o);
     };
-    if constexpr (CACHE > 0) {
+    if constexpr (CACHE > 32) {
+#pragma unroll
+        for (int c = 0; c < CACHE; ++c) {
+            const int d = ty + c * NTY;
+            if (in_range(d)) emit(d, cache[c], has_w ? a.w[d] : 1.f, has_b ? a.b[d] : 0.f);
+        }
+    } else if constexpr (CACHE > 0) {
 #pragma unroll
         for (int n = 0; n < CACHE / kBatch; ++n) {
             if (n + 1 < CACHE / kBatch) fetch_wb(n + 1, g[(n + 1) & 1], be[(n + 1) & 1]);
