@@ -31,10 +31,9 @@ struct StFwdArgs {
     int every;               // a multiple of 32
 };
 
-// Registers for sixteen warps an SM; twelve with two rows per lane (49 152 rows, 16 states, fp32 1 142 against 1 062 us); pieces (VW 0) as the compiler
-// likes (4 608 rows of 8 594, 4 states, 438 us with sixteen, 308).
-template <typename Tin, typename Tout, int NS, int R_, int VW, bool kOut>
-__global__ void __launch_bounds__(StLayout<NS, R_>::kWarps * 32, VW == 0 ? 0 : (R_ == 2 ? 12 : 16) / StLayout<NS, R_>::kWarps) st_fwd_kernel(const StFwdArgs a) {
+// Registers for sixteen warps an SM; twelve with two rows per lane (49 152 rows, 16 states, fp32 1 142 against 1 062 us), unless !kHeld (st_launch_fwd).
+template <typename Tin, typename Tout, int NS, int R_, int VW, bool kOut, bool kHeld>
+__global__ void __launch_bounds__(StLayout<NS, R_>::kWarps * 32, !kHeld ? 0 : (R_ == 2 ? 12 : 16) / StLayout<NS, R_>::kWarps) st_fwd_kernel(const StFwdArgs a) {
     follow_previous();
     using Y = StLayout<NS, R_>;
     constexpr int RPW = Y::RPW, SL = Y::SL, R = Y::R, RL = Y::RL, P = kStPitch;
@@ -247,7 +246,12 @@ static int st_launch_fwd(const StFwdArgs& a, int64_t batch, cudaStream_t st) {
     static_assert(smem <= 48 * 1024, "default shared-memory limit");
     const int64_t ctas = batch * a.n_groups * a.parts * a.S;
     if (ctas > 0x7fffffffLL) return SS2D_EINVAL_SHAPE;
-    launch(st_fwd_kernel<Tin, Tout, NS, R, VW, kOut>, (unsigned)ctas, Y::kWarps * 32, smem, st, a);
+    // Registers as the compiler likes for pieces (4 608 rows of 8 594, 4 states, 438 us with sixteen warps an SM, 308), and for 16-bit rows of up to
+    // four states by single elements where they are not cut: those spill at sixteen warps (64 to 120 bytes; 24 576 rows of 785 elements, f16 / bf16,
+    // 168 / 293 us, 143 / 268), which cut rows fill all the same (4 608 rows of 8 594 306 / 453, and 373 / 708).
+    constexpr bool spills = VW == 1 && NS == 4 && sizeof(Tin) == 2;
+    if (VW == 0 || (spills && a.S == 1)) launch(st_fwd_kernel<Tin, Tout, NS, R, VW, kOut, (VW != 0 && !spills)>, (unsigned)ctas, Y::kWarps * 32, smem, st, a);
+    else launch(st_fwd_kernel<Tin, Tout, NS, R, VW, kOut, VW != 0>, (unsigned)ctas, Y::kWarps * 32, smem, st, a);
     count_launch();
     return check_launch();
 }
