@@ -4,10 +4,23 @@
 
 namespace ss2d {
 
+// The piece at p, or zeros.  16-bit rows: as one predicated load, which the compiler leaves where it is (1 024 rows of 16 385 elements 44.4 us; as a plain one
+// under a condition 46.0).  fp32 rows, whose registers are full: as a plain one, which it may place (57 us, predicated 72).  Both come
+// behind the wait for the kernel in front (follow_previous), which is volatile too.
 #ifdef __CUDACC__
-template <typename T> __device__ __forceinline__ T piece_load(const T* p) { return *p; }
-#else
-#define piece_load __ldg                             // compiled for the host: what stands for common.cuh looks where it reads
+template <bool kPredicated> __device__ __forceinline__ uint4 piece_load(const uint4* p, bool in) {
+    uint4 t = make_uint4(0, 0, 0, 0);
+    if constexpr (!kPredicated) {
+        if (in) t = *p;
+    } else {
+        asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %5, 0;\n mov.b32 %0, 0;\n mov.b32 %1, 0;\n mov.b32 %2, 0;\n mov.b32 %3, 0;\n"
+                     " @p ld.global.v4.b32 {%0, %1, %2, %3}, [%4];\n}"
+                     : "=&r"(t.x), "=&r"(t.y), "=&r"(t.z), "=&r"(t.w) : "l"(p), "r"((int)in));
+    }
+    return t;
+}
+#else                                                // for the host: what stands for common.cuh looks where it reads
+template <bool kPredicated> uint4 piece_load(const uint4* p, bool in) { return in ? __ldg(p) : make_uint4(0, 0, 0, 0); }
 #endif
 
 // The bytes of a tensor of rows, and whether they start and end on 16-byte boundaries: then no aligned piece that holds an element
@@ -55,9 +68,8 @@ template <typename T> struct Row8<T, 0> {
         const int off = (int)(at & 15) / (int)sizeof(T), e0 = pos - off;       // e0: element at the start of the first piece
 #pragma unroll
         for (int i = 0; i <= kPieces; ++i) {
-            uint4 t = make_uint4(0, 0, 0, 0);
             const int e = e0 + i * kPiece;
-            if (e < L && e + kPiece > from && (i < kPieces || off != 0)) t = piece_load(q + i);
+            const uint4 t = piece_load<sizeof(T) == 2>(q + i, e < L && e + kPiece > from && (i < kPieces || off != 0));
             w[4 * i] = t.x; w[4 * i + 1] = t.y; w[4 * i + 2] = t.z; w[4 * i + 3] = t.w;
         }
     }
