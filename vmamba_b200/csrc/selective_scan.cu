@@ -4,6 +4,8 @@
 // one where channels share a row of step sizes: selscan_fwd_nx_kernel, a warp per row, the carry of every state in shared memory.
 // In all of them u and delta are read once and the result is written once; the B / C rows, shared by the channels of a
 // group, come from the caches.
+#include <type_traits>
+
 #include "scan_row.cuh"
 #include "scan_states_fwd.cuh"
 
@@ -45,8 +47,13 @@ template <typename Tin, typename Tout, int AL, int W, int LPR>
 __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32, W == 1 && AL == 0 && sizeof(Tin) == 4 ? 4 : 0) selscan_fwd_n1_kernel(const ScanArgs a) {
     follow_previous();
     static_assert(W == 1 || LPR == 32, "rows of several warps take whole warps");
-    // elementwise arithmetic in pairs; fp32 pieces are at their 128 registers and would spill (12 288 rows of 3 137 elements 124 -> 136 us).
-    constexpr bool kPacked = !(AL == 0 && sizeof(Tin) == 4);
+    // Elementwise arithmetic in pairs, but where it measured slower.  fp32 pieces are at their 128 registers and would spill (12 288 rows of 3 137
+    // elements 124 -> 136 us).  Whole vectors, in pairs / one by one: two warps of 16-bit rows, 2 048 rows of 65 536 elements bf16 215 / 194 us, f16 211 / 189,
+    // of 16 384 56 / 51 and 55 / 50; four warps of bf16 rows, 1 024 of 65 536 110 / 98 (f16 110 / 117); one warp of fp32 rows, 3 584 of
+    // 65 536 572 / 551.  Else 16-bit rows gain: 3 584 of 65 536 bf16 325 / 354, 256 of 65 536 35.0 / 37.3.
+    constexpr bool kOneByOne = (AL == 0 && sizeof(Tin) == 4) ||
+                               (AL == 8 && (sizeof(Tin) == 4 ? W == 1 : W == 2 || (W == 4 && std::is_same<Tin, __nv_bfloat16>::value)));
+    constexpr bool kPacked = !kOneByOne;
     constexpr int VEC = 8, WSTEP = LPR * VEC, STEP = W * WSTEP;
     __shared__ AB agg[2][W];
     const int lane = threadIdx.x & (LPR - 1), wi = W == 1 ? 0 : threadIdx.x >> 5;
@@ -101,7 +108,7 @@ __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32, W == 1 &&
             for (int i = 0; i < VEC; ++i) {
                 float dl = dv[i] + bias;
                 if (sp) dl = softplus_fast(dl);
-                dl = pos + i < l1 && pos + i >= l0 ? dl : 0.f;
+                if constexpr (AL == 0) dl = pos + i < l1 && pos + i >= l0 ? dl : 0.f;       // outside the row: a step of zero (below)
                 const float aa = decay_fast(dl, A2);
                 h = fmaf(aa, h, dl * bv[i] * uv[i]);
                 p *= aa;
