@@ -273,7 +273,9 @@ template <> struct MmaK16<__half> {
 // 121 -> 112, its training step 565 -> 537.
 __device__ __forceinline__ void follow_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Not in a stream that is being captured: a graph's own gaps are as short (three captured backbones of one image in turn 855 us, and 871
-// with it; of 128 images 5 792 and 5 816).  Not for grids of more CTAs, of which the gap is a small part.
+// with it; of 128 images 5 792 and 5 816).  Not for grids of more CTAs, of which the gap is a small part.  The core with no such launches / grids of up to 2 048 /
+// 8 192 / any: 64 x 192 planes of 28 x 28 115.7 / 111.0 / 108.7 / 108.8 us, 128 x 768 of 7 x 7 108.5 / 102.1 / 100.6 / 100.5, 64 x 192 of
+// 14 x 32 82.0 / 76.9 / 76.9 / 74.7.
 constexpr long long kFollowMost = 8192;
 template <typename... P, typename... A>
 inline void launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {

@@ -431,9 +431,9 @@ static bool plan_planes(const ss2d_core_params* p, PlaneConfig& c) {
     // ~14 warps per CTA, two CTAs per SM; seven-thread planes (7 x 7) in CTAs of seven warps, four per SM: 61.6 -> 51.4 us
     // per launch at 128 x 768 planes (the 14 x 14 launch takes 84 us with 448, 224 or 160 threads and 98 us with 320)
     // Seven warps and four CTAs too where at least two planes of 28 x 28 and less go into them, 57 to 112 segments: barriers of fewer
-    // warps.  Whole core, us, fourteen against seven warps: 64 x 192 planes of 28 x 28 (98 segments) 130 / 126 (ten warps 138),
-    // 24 x 24 (72) 100 / 94, 16 x 36 (72) 99 / 93; 64 x 384 of 18 x 14 (63) 116 / 112, 20 x 14 (70) 118 / 115; 16 x 384 of 28 x 28
-    // 82 / 79; 64 x 192 of 14 x 32 (112) 89 / 89 and 21 x 21 (63, seven-element segments) 106 / 107.
+    // warps.  Whole core, us, fourteen / ten / seven warps: 64 x 192 planes of 28 x 28 (98 segments) 115 / 121 / 109,
+    // 24 x 24 (72) and 16 x 36 (72) 86 / 82 / 80; 64 x 384 of 18 x 14 (63) 94 / 97 / 89, 20 x 14 (70) 99 / 95 / 94; 16 x 384 of 28 x 28
+    // 68 / 69 / 64; 64 x 192 of 14 x 32 (112) and 21 x 21 (63, seven-element segments) the same; 128 x 768 of 7 x 7 111 / 114 / 101.
     int PP = (int)((G <= 8 || (G > 56 && G <= 112) ? 224 : 448) / G);
     if (PP < 1) PP = 1;
     if (PP > p->D) PP = (int)p->D;

@@ -101,7 +101,8 @@ __global__ void __launch_bounds__(TX * NTY, (NTY == 32 && CACHE > 0 && CACHE * P
     };
 
     // Weight and bias are read behind the statistics.  A grid of few CTAs has nothing else to do meanwhile and brings them into L1 (one captured
-    // image, with the shorter vectors of few pixels, 786 -> 764 us; with many CTAs the requests are in the way: 128 images 5 737 -> 6 410).
+    // image, with the shorter vectors of few pixels, 786 -> 764 us; with many CTAs the requests are in the way: 128 images 5 737 -> 6 410; up to 32 / 74 /
+    // 148 CTAs, what they ask for in L2 already: 384 channels of 4 x 196 pixels 3.5 / 4.3 / 4.3 us, of 8 x 196 3.5 / 3.5 / 5.9, 768 of 2 x 280 4.5 / 4.9 / 4.9).
     if constexpr (CACHE > 0) {
         if (gridDim.x <= 32) {
 #pragma unroll
@@ -313,7 +314,9 @@ static void launch_norm(NormArgs a, int pv, long long B, cudaStream_t st) {
     // (more threads per CTA: keep about 64 registers per thread so that several CTAs share an SM)
     if (D > 32 * 32) pv = 1;
     else if (D > 16 * 12 && pv > 2) pv = 2;
-    while (pv > 1 && B * (a.L / pv) < 74 * kItemsPerCta) pv /= 2;      // few pixels: shorter vectors on more SMs
+    // few pixels: shorter vectors on more SMs, up to 74 CTAs (us never / 37 / 74 / 148: 768 channels of 2 x 280 pixels 5.8 / 4.5 / 4.5 / 4.5, 384 of 8 x 196
+    // 4.0 / 4.0 / 3.5 / 3.5, 192 of 2 x 784 3.0 / 2.7 / 2.7 / 2.9)
+    while (pv > 1 && B * (a.L / pv) < 74 * kItemsPerCta) pv /= 2;
     a.nv = a.L / pv;
     a.items = (int)(B * a.nv);
     // widths that are 16 per channel slice (128, 256, 512: the VMamba-B dims) get exact shapes of their own,

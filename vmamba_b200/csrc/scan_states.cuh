@@ -200,9 +200,10 @@ template <typename T, int NS, int WARPS> struct StRawBC<T, NS, 0, WARPS> {
 
 // Number of segments a row is cut into (1: none) and their length, given the warps that whole rows fill.  Cutting costs a
 // second pass, so it starts below four warps per SM and then goes up to sixteen (16 states, bf16: 768 rows of 3 136
-// elements 116 -> 49 us, 384 rows of 65 536 4.4 -> 0.29 ms; 6 144 rows, which fill five warps, 0.25 uncut, 0.28 cut).
-// `resident`: sixteen is what the SM holds, and more would be a second round (rows of vectors: 3 072 rows of 3 136, 16 states, fp32, 206 us with
-// seven segments, 188 with six); where it holds more, the number is rounded up (4 608 rows of 8 594, 4 states, bf16, 308 against 318).
+// elements 144 -> 36 us, 384 rows of 65 536 3.7 -> 0.29 ms; 6 144 rows, which fill five warps, 225 uncut, 255, 224 and 271 cut in two, three and
+// four; fp32, 6 144 rows of 1 001 83 uncut, 95 and 91 cut in two and three).
+// `resident`: sixteen is what the SM holds, and more would be a second round (rows of vectors: 3 072 rows of 3 136, 16 states, fp32, 161 us with
+// seven segments, 132 with six); where it holds more, the number is rounded up (4 608 rows of 8 594, 4 states, bf16, 308 against 318).
 struct StSegments { int count, len; };
 inline StSegments st_segments(int64_t warps, int64_t L, bool resident) {
     const int64_t want = 148 * 16;

@@ -33,7 +33,7 @@ constexpr int kWarpsPerCta = 4;
 // per lane, and scans its lanes' (a, b) pairs by shuffle; with several warps per row their totals meet in shared memory
 // (one barrier per step) and every warp folds the ones in front of it.  How many: n1_warps.  The next step's vectors are
 // fetched in front of this one's arithmetic.
-// Bound, 1 024 rows of 16 385 elements (four warps each, 46 us, 20 % of the DRAM rate): instruction issue, 72 % of the slots of an SM
+// Bound, 1 024 rows of 16 385 elements (four warps each, 45 us, 20 % of the DRAM rate): instruction issue, 72 % of the slots of an SM
 // that has work, and 1 024 CTAs on the 740 places that 91 registers leave, so that the second wave is a third full.  32 x 384 rows of
 // 3 136 with the states kept, 66 us: issue (79 %) and HBM (330 MB, 50 us at the copy rate).  Arithmetic in pairs, 50 and 70 us before.
 // AL is the vector width of every access (8 or 4 elements), or 0 for rows of any alignment: a row is then walked from
@@ -51,6 +51,7 @@ __global__ void __launch_bounds__(W == 1 ? kWarpsPerCta * 32 : W * 32, W == 1 &&
     // elements 124 -> 136 us).  Whole vectors, in pairs / one by one: two warps of 16-bit rows, 2 048 rows of 65 536 elements bf16 215 / 194 us, f16 211 / 189,
     // of 16 384 56 / 51 and 55 / 50; four warps of bf16 rows, 1 024 of 65 536 110 / 98 (f16 110 / 117); one warp of fp32 rows, 3 584 of
     // 65 536 572 / 551.  Else 16-bit rows gain: 3 584 of 65 536 bf16 325 / 354, 256 of 65 536 35.0 / 37.3.
+    // (Vectors of four, single warps, in pairs: bf16, 3 584 rows of 65 540 413, 385 before the pairs; of 3 140 20.1 and 22.6.)
     constexpr bool kOneByOne = (AL == 0 && sizeof(Tin) == 4) ||
                                (AL == 8 && (sizeof(Tin) == 4 ? W == 1 : W == 2 || (W == 4 && std::is_same<Tin, __nv_bfloat16>::value)));
     constexpr bool kPacked = !kOneByOne;
@@ -287,13 +288,15 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) selscan_fwd_nx_kernel(const
 // and 16 CTAs per SM of eight, four and two warps; unaligned ones 2, 5 and 10), because long rows gain from more warps in a
 // second wave too.  us with 1 / 2 / 4 / 8 warps, bf16, the rule's in brackets:
 //   rows    L = 3 136 (aligned)        L = 3 137                  L = 16 385
-//   256     16.4  12.3  11.0 [10.2]    19.2  14.4  12.4 [12.3]    61.4  37.9  25.6 [22.5]
-//   740     16.4  14.4  12.3 [14.3]    20.5  18.4  17.3 [20.5]    69.6  47.1  38.9 [48.1]
-//   1 024   17.5  14.4 [14.4] 16.4     21.4  20.5 [22.6] 24.6     70.8  55.3 [53.3] 62.5
-//   2 048   20.5 [18.5] 20.5  23.5     26.7 [28.7] 32.8  43.0
-//   3 584  [26.6] 27.5  30.7  34.8    [43.0] 43.0  51.2  69.7
-// It is within 3 % of the best but where CTAs of eight warps do not fit at once (444 to 740 rows, up to 24 %) and at its steps
-// (1 536 and 3 072 rows, up to 13 %).
+//   256      7.2   6.5   6.2  [7.3]    11.7   8.0   6.7  [6.2]    47.3  27.3  18.1 [16.1]
+//   740      8.6   7.3   6.3  [6.9]    13.7  11.3  10.8 [13.7]    55.2  38.4  31.2 [38.6]
+//   1 024    8.6   8.5  [8.1]  8.9     13.6  13.3 [14.2] 17.8     59.2  47.2 [44.6] 54.1
+//   1 536    9.9  11.2 [11.6] 13.0     16.7  19.2 [20.4] 26.7     70.4  74.1 [66.5] 81.9
+//   2 048   11.8 [12.8] 14.4  16.5     20.4 [21.3] 24.9  33.6     85.2 [81.0] 80.9 103.7
+//   3 072   16.1 [18.6] 20.4  24.1     30.2 [31.0] 36.1  49.5      134 [121]  119   153
+//   3 584  [18.2] 21.4  23.8  28.1    [33.6] 35.3  42.0  57.6     [146]  136   139   179
+// It is within 7 % of the best for rows of 16 385 and for 2 048 rows and more of 3 137, but where CTAs of eight warps do not fit at once (444 to 740
+// rows, up to 27 %); it gives a warp too many to 256 rows of 3 136 (18 %) and from 1 536 rows of about 3 100 on (up to 22 %).
 static int n1_warps(int64_t rows, int64_t L) {
     int w = 1;
     while (w < 8 && rows * w < 148 * 24 && (int64_t)w * 256 < L) w *= 2;
